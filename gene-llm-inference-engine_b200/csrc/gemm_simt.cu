@@ -1,11 +1,14 @@
 // Matrix product on the CUDA cores with 32-bit fused multiply-adds: C[M,N] (+)= A[M,K] * W[N,K]^T.
 //
 // This is the matrix product of the true 32-bit path (no tensor cores, no reduced-precision mode)
-// and accepts bfloat16 operands too (widened exactly), for any M, N, K. Every output element is one
-// chain of fmaf over k = 0..K-1 in increasing order, whatever M is and wherever the row sits in
+// and accepts bfloat16 operands too (widened exactly), for any M, N, K. All-32-bit products whose rows
+// are whole 16-byte pieces go to the tiled kernel of gemm_f32.cu; the kernel below takes the rest (bfloat16, or a K that is
+// no multiple of 4), one chain of fmaf over k = 0..K-1 in increasing order for every output element. In either, an element's
+// sum is the same whatever M is and wherever the row sits in
 // the batch: results do not depend on how tokens are cut into steps (the property the reference
 // states for its own kernels, src/gpu/device_kernels.inc:97-100).
 #include "common.cuh"
+#include "gemm_f32.cuh"
 
 namespace gi {
 
@@ -97,6 +100,9 @@ static int gi_gemm_simt_impl(const void* A, int a_dtype, const void* W, int w_dt
     GI_REQUIRE((M + kBM - 1) / kBM <= 65535, "gemm: M=%d exceeds the grid limit", M);
     GI_REQUIRE(c_dtype == kF32 || c_dtype == kBF16, "gemm: unsupported output dtype code %d", c_dtype);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (a_dtype == kF32 && w_dtype == kF32 && c_dtype == kF32 &&
+        gemm_f32_takes(static_cast<const float*>(A), static_cast<const float*>(W), M, N, K, lda, ldw))
+        return gemm_f32(static_cast<const float*>(A), static_cast<const float*>(W), static_cast<float*>(C), M, N, K, lda, ldw, ldc, accumulate, st);
     if (a_dtype == kF32 && w_dtype == kF32) return launch_simt<float, float>(A, W, C, c_dtype, accumulate, M, N, K, lda, ldw, ldc, st);
     if (a_dtype == kF32 && w_dtype == kBF16) return launch_simt<float, __nv_bfloat16>(A, W, C, c_dtype, accumulate, M, N, K, lda, ldw, ldc, st);
     if (a_dtype == kBF16 && w_dtype == kBF16) return launch_simt<__nv_bfloat16, __nv_bfloat16>(A, W, C, c_dtype, accumulate, M, N, K, lda, ldw, ldc, st);

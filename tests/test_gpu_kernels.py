@@ -90,6 +90,29 @@ def test_gemm_simt(a_dtype, w_dtype, c_dtype, M, N, K_):
             assert torch.equal(one[0], out[M - 1]), "a row alone differs from the row in the batch"
 
 
+@pytest.mark.parametrize("M,N,K_", [(1, 1, 4), (8, 127, 36), (9, 128, 512), (16, 129, 1024), (17, 300, 2052), (32, 2048, 2048), (33, 136, 4096),
+                                    (65, 130, 260), (70, 19000, 64)])
+def test_gemm_simt_tiled(M, N, K_):
+    """32-bit products in whole 16-byte pieces: every block height, edges of blocks and chunks, one to eight chunks of K.
+    Bound: each sum is at most K / 2 long, and a chain of n roundings of products that sum to s is off by about sqrt(n) 2^-24 |s|."""
+    g = torch.Generator().manual_seed(5)
+    a, w, base = (torch.randn(*shape, generator=g) for shape in ((M, K_), (N, K_), (M, N)))
+    want = a.double() @ w.double().T
+    bound = 4 * (K_ / 2) ** 0.5 * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T) + 1e-30
+    a, w = a.to(DEV), w.to(DEV)
+    out = torch.full((M, N), float("nan"), device=DEV)
+    K().gemm_simt(a, w, out)
+    assert ((out.cpu().double() - want).abs() <= bound).all()
+    acc = base.to(DEV)
+    K().gemm_simt(a, w, acc, accumulate=True)
+    assert torch.equal(acc, base.to(DEV) + out)
+    for rows in (1, 8, 9, 16, 17, 32, 33, 64):      # the same rows at every block height
+        if rows <= M:
+            part = torch.empty((rows, N), device=DEV)
+            K().gemm_simt(a[M - rows:].contiguous(), w, part)
+            assert torch.equal(part, out[M - rows:]), rows
+
+
 def _paged(dtype, n_pages, Hkv, ps, hd):
     kc = torch.full((n_pages, Hkv, ps, hd), float("nan"), dtype=dt(dtype), device=DEV)
     return kc, kc.clone()
