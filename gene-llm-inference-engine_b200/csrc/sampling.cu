@@ -11,26 +11,21 @@
 // kept on the host so that a request's stream does not depend on the batch it is in).
 //
 // The sorted order is never materialised. A position in it (the k-th token, the place where the
-// cumulative mass crosses a threshold) is found by a radix descent over the 32 bits of the
-// probabilities: histograms of counts and of double-precision masses per 8-bit digit, four
-// passes, then index order inside the last group of equal probabilities. One block per row.
+// cumulative mass crosses a threshold) is found by a radix descent over the bits of the
+// probabilities: histograms of counts and of exact masses per 10-bit digit, three
+// passes, then index order inside the last group of equal probabilities. One cluster of CTAs per row.
+#include <climits>
+#include <type_traits>
+
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace gi {
 
-constexpr int kSampleThreads = 1024;
+namespace cg = cooperative_groups;
 
-__device__ __forceinline__ double block_sum_double(double v, double* scratch) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if (lane == 0) scratch[warp] = v;
-    __syncthreads();
-    double total = 0.0;
-    for (int w = 0; w < (blockDim.x >> 5); ++w) total += scratch[w];
-    return total;
-}
+constexpr int kSampleThreads = 1024;
 
 // Greedy argmax in two steps: kArgmaxParts blocks per row each find the best of a slice of the
 // vocabulary (lowest index among equals), then one block per row picks among the slice winners.
@@ -91,147 +86,223 @@ argmax_final_kernel(const float* __restrict__ part_val, const int* __restrict__ 
     if (threadIdx.x == 0) out[blockIdx.x] = best_i == 0x7fffffff ? 0 : best_i;
 }
 
-// The bits fixed so far of the value searched for: elements with (bits & mask) == prefix remain.
-struct Descent {
-    unsigned prefix;
-    unsigned mask;
+// ---- temperature sampling: one cluster of kSampleParts CTAs per row ----
+//
+// A row is bound by latency, not by its bytes (0.5 MB at a vocabulary of 128,256, read once from memory and a few times from
+// L1): one block of 1024 threads per row took 1,560 us for six rows, most of it in double-precision atomics on
+// histograms in shared memory (loops of compare-and-swap, all on the few digits that the exponents have) and in loops of one
+// thread over 1024 ranges. Here eight CTAs share a row, every warp owns a contiguous piece of it, and a histogram's masses
+// are integers: the values of one bin have one exponent, so their sum is a sum of 24-bit mantissas, added exactly in two
+// 32-bit words by the hardware's integer atomics: 90 us for the same rows.
+constexpr int kSampleParts = 8, kBins = 1024, kDigit = 10;
+constexpr int kMassBits = 12;                  // a mantissa goes into two words of 12 bits: slices of up to 2^20 values cannot overflow them
+constexpr int kNarrowVocab = kSampleParts << 20;      // above: whole mantissas in 64-bit words (whose atomics are slower)
+
+template <bool kWide> struct SampleShared {
+    using Low = typename std::conditional<kWide, unsigned long long, unsigned>::type;
+    unsigned count[2][kBins];
+    Low low[2][kBins];
+    unsigned high[2][kBins];                   // histograms of this CTA's piece; the two sets take turns
+    double cta_max, cta_sum, cta_mass;         // each written once and read by the cluster behind its own barrier
+    int cta_equal;
+    double warp_mass[32];
+    double red[32];
+    int counts[32];
+    double scan_mass[32];
+    int scan_count[32];
+    int first, last;                           // positions of the bin chosen
+    double chosen_mass;
+    int chosen_count;
 };
 
-// Walks the values from the largest downwards, 8 bits per pass: in each pass the bucket is chosen in
-// which the running total of weights (1 per element if kByCount, else the probability), started
-// at `before`, first reaches (inclusive) or exceeds the target. On return d.prefix holds all 32
-// bits of the value found and `before` the total weight of the strictly larger values.
-template <bool kByCount>
-__device__ void radix_descend(const float* __restrict__ probs, int V, double target, bool inclusive,
-                              Descent& d, double& before, double* s_hist_w, unsigned* s_hist_c,
-                              int* s_choice) {
-    // kByCount: weight of an element is 1 (find the k-th element); else its probability.
-    for (int shift = 24; shift >= 0; shift -= 8) {
-        for (int b = threadIdx.x; b < 256; b += blockDim.x) { s_hist_w[b] = 0.0; s_hist_c[b] = 0u; }
+// What a descent has found: the value's bits, what is strictly above it, and how many values equal it.
+struct Found {
+    unsigned bits;
+    double mass_above;
+    int count_above, equal;
+};
+
+__device__ __forceinline__ unsigned long long sample_mantissa(unsigned bits) {
+    return (bits & 0x7fffffu) | ((bits >> 23) ? 0x800000u : 0u);
+}
+__device__ __forceinline__ double sample_scale(unsigned bits) {                    // the weight of the mantissa's last bit
+    const int e = static_cast<int>((bits >> 23) & 255u);
+    return ldexp(1.0, (e > 0 ? e : 1) - 150);
+}
+
+__device__ __forceinline__ double warp_sum_double(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+// Sum over the block in the order of the warps; each thread has it.
+__device__ __forceinline__ double block_sum_double(double v, double* scratch) {
+    v = warp_sum_double(v);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double total = 0.0;
+    for (int w = 0; w < kSampleThreads / 32; ++w) total += scratch[w];
+    return total;
+}
+
+// Walks the row's values from the largest downwards, ten bits of them per pass (values are at most 1: 30 bits): in each pass
+// the bin is chosen in which the running total (of ones if by_count, else of probabilities) first reaches (inclusive) or
+// exceeds the target. Where rounding never lets it, the lowest bin that weighs anything is chosen. The piece
+// [begin, end) is the calling warp's. `turn` counts the passes of the row.
+template <bool kWide>
+__device__ Found sample_descend(const float* __restrict__ probs, int begin, int end, bool by_count, double target, bool inclusive,
+                                SampleShared<kWide>& s, int& turn, cg::cluster_group& cluster) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    Found f{0u, 0.0, 0, 0};
+    unsigned mask = 0u;
+    for (int shift = 20; shift >= 0; shift -= kDigit) {
+        const int set = turn++ & 1;
+        s.count[set][threadIdx.x] = 0u;
+        s.low[set][threadIdx.x] = 0u;
+        s.high[set][threadIdx.x] = 0u;
+        if (threadIdx.x == 0) { s.first = kBins; s.last = -1; }
         __syncthreads();
-        for (int i = threadIdx.x; i < V; i += blockDim.x) {
+        for (int i = begin + lane; i < end; i += 32) {
             const unsigned bits = __float_as_uint(probs[i]);
-            if ((bits & d.mask) == d.prefix) {
-                const unsigned digit = (bits >> shift) & 255u;
-                if (kByCount) atomicAdd(&s_hist_c[digit], 1u);
-                else atomicAdd(&s_hist_w[digit], static_cast<double>(probs[i]));
+            if ((bits & mask) == f.bits) {
+                const unsigned digit = (bits >> shift) & (kBins - 1);
+                const unsigned m = static_cast<unsigned>(sample_mantissa(bits));
+                atomicAdd(&s.count[set][digit], 1u);
+                if constexpr (kWide) {
+                    atomicAdd(&s.low[set][digit], static_cast<unsigned long long>(m));
+                } else {
+                    atomicAdd(&s.low[set][digit], m & ((1u << kMassBits) - 1));
+                    atomicAdd(&s.high[set][digit], m >> kMassBits);
+                }
             }
         }
+        cluster.sync();
+        // thread t has the t-th bin from the top: its totals over the cluster, then a scan over the block
+        const int bin = kBins - 1 - threadIdx.x;
+        unsigned long long low = 0, high = 0;
+        int count = 0;
+#pragma unroll
+        for (int p = 0; p < kSampleParts; ++p) {
+            count += static_cast<int>(*cluster.map_shared_rank(&s.count[set][bin], p));
+            low += *cluster.map_shared_rank(&s.low[set][bin], p);
+            high += *cluster.map_shared_rank(&s.high[set][bin], p);
+        }
+        const double mass = static_cast<double>(low + (high << kMassBits)) * sample_scale(f.bits | (static_cast<unsigned>(bin) << shift));
+        double run = mass;
+        int runs = count;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double m = __shfl_up_sync(0xffffffffu, run, o);
+            const int c = __shfl_up_sync(0xffffffffu, runs, o);
+            if (lane >= o) { run += m; runs += c; }
+        }
+        if (lane == 31) { s.scan_mass[warp] = run; s.scan_count[warp] = runs; }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            double run = before, run_before = before;
-            int choice = 0;
-            for (int b = 255; b >= 0; --b) {
-                const double w = kByCount ? static_cast<double>(s_hist_c[b]) : s_hist_w[b];
-                if (w == 0.0) continue;
-                run_before = run;
-                choice = b;
-                const double next = run + w;
-                if (inclusive ? (next >= target) : (next > target)) break;
-                run = next;
-            }
-            // If rounding never reaches the target, the lowest non-empty bucket stays chosen and
-            // the total before it is reported: the caller's walk over equal values then ends on
-            // the last element.
-            s_choice[0] = choice;
-            s_hist_w[256] = run_before;
+        double ahead = f.mass_above;
+        int aheads = f.count_above;
+        for (int w = 0; w < warp; ++w) { ahead += s.scan_mass[w]; aheads += s.scan_count[w]; }
+        run += ahead;
+        runs += aheads;
+        const bool weighs = by_count ? count > 0 : mass > 0.0;
+        const double total = by_count ? static_cast<double>(runs) : run;
+        if (weighs && (inclusive ? total >= target : total > target)) atomicMin(&s.first, static_cast<int>(threadIdx.x));
+        if (weighs) atomicMax(&s.last, static_cast<int>(threadIdx.x));
+        __syncthreads();
+        const int chosen = s.first < kBins ? s.first : max(s.last, 0);
+        if (static_cast<int>(threadIdx.x) == chosen) {
+            s.chosen_mass = run - mass;
+            s.chosen_count = runs - count;
+            s.counts[0] = count;
         }
         __syncthreads();
-        before = s_hist_w[256];
-        d.prefix |= static_cast<unsigned>(s_choice[0]) << shift;
-        d.mask |= 255u << shift;
-        __syncthreads();
+        f.mass_above = s.chosen_mass;
+        f.count_above = s.chosen_count;
+        f.equal = s.counts[0];
+        f.bits |= static_cast<unsigned>(kBins - 1 - chosen) << shift;
+        mask |= static_cast<unsigned>(kBins - 1) << shift;
     }
+    return f;
 }
 
-// Among elements whose probability bits equal `bits`, in index order: the 0-based rank of the
-// first one at which before + (rank+1)*w reaches (inclusive) or exceeds the target; the element's
-// index is returned; `n_equal` receives the group size.
-__device__ int nth_equal_index(const float* __restrict__ probs, int V, unsigned bits, int rank, int* s_tmp) {
-    // rank-th (0-based) index with probs == bits, by a block-wide ordered count.
-    __shared__ int s_counts[kSampleThreads];
-    const int per = (V + blockDim.x - 1) / blockDim.x;
-    const int begin = threadIdx.x * per, end = min(V, begin + per);
-    int c = 0;
-    for (int i = begin; i < end; ++i) c += (__float_as_uint(probs[i]) == bits);
-    s_counts[threadIdx.x] = c;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int run = 0, owner = blockDim.x - 1, inner = 0;
-        for (int t = 0; t < static_cast<int>(blockDim.x); ++t) {
-            if (run + s_counts[t] > rank) { owner = t; inner = rank - run; break; }
-            run += s_counts[t];
-        }
-        s_tmp[0] = owner;
-        s_tmp[1] = inner;
-    }
-    __syncthreads();
-    const int owner = s_tmp[0], inner = s_tmp[1];
-    __syncthreads();
-    if (threadIdx.x == owner) {
-        int seen = 0, found = -1;
-        for (int i = begin; i < end; ++i) {
-            if (__float_as_uint(probs[i]) == bits) {
-                if (seen == inner) { found = i; break; }
-                ++seen;
-            }
-        }
-        s_tmp[2] = found;
-    }
-    __syncthreads();
-    return s_tmp[2];
+// The smallest c of 1 .. n with above + c * w >= target (inclusive) or > target; n where there is none.
+__device__ __forceinline__ int sample_count_to(double above, double w, int n, double target, bool inclusive) {
+    if (!(w > 0.0)) return n;
+    const double guess = (target - above) / w;
+    int c = guess >= n ? n : guess <= 1.0 ? 1 : static_cast<int>(guess);
+    auto reached = [&](int k) { const double cum = above + k * w; return inclusive ? cum >= target : cum > target; };
+    while (c > 1 && reached(c - 1)) --c;
+    while (c < n && !reached(c)) ++c;
+    return c;
 }
 
-__device__ int count_equal(const float* __restrict__ probs, int V, unsigned bits, double* scratch) {
-    double c = 0.0;
-    for (int i = threadIdx.x; i < V; i += blockDim.x) c += (__float_as_uint(probs[i]) == bits) ? 1.0 : 0.0;
-    return static_cast<int>(block_sum_double(c, scratch));
-}
-
-// One block per row. probs: scratch [rows, V] floats.
-__global__ void __launch_bounds__(kSampleThreads)
+// probs: scratch [rows, V] floats.
+template <bool kWide>
+__global__ void __cluster_dims__(kSampleParts, 1, 1) __launch_bounds__(kSampleThreads)
 sample_kernel(const float* __restrict__ logits, float* __restrict__ probs_all, int V,
               const float* __restrict__ temperature, const int* __restrict__ top_k,
               const float* __restrict__ top_p, const float* __restrict__ uniform, int* __restrict__ out) {
     pdl_prologue();
-    __shared__ double s_red[32];
-    __shared__ double s_hist_w[257];
-    __shared__ unsigned s_hist_c[256];
-    __shared__ int s_choice[4];
-    __shared__ float s_maxes[32];
-
-    const int r = blockIdx.x;
+    __shared__ SampleShared<kWide> s;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int r = blockIdx.x / kSampleParts, part = blockIdx.x % kSampleParts;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const float* row = logits + static_cast<size_t>(r) * V;
     float* probs = probs_all + static_cast<size_t>(r) * V;
     const float temp = temperature[r];
-    if (!(temp > 0.f)) return;          // a greedy row: out[r] keeps what the caller put there (its argmax)
+    if (!(temp > 0.f)) return;          // a greedy row (for the whole cluster): out[r] keeps what the caller put there (its argmax)
+
+    // this CTA's piece of the row, and this warp's piece of that
+    const int slice = (V + kSampleParts - 1) / kSampleParts, piece = (slice + 31) / 32;
+    const int slice_begin = min(V, part * slice), slice_end = min(V, slice_begin + slice);
+    const int begin = min(slice_end, slice_begin + warp * piece), end = min(slice_end, begin + piece);
 
     // max
     float mx = -INFINITY;
-    for (int i = threadIdx.x; i < V; i += blockDim.x) mx = fmaxf(mx, row[i]);
+    for (int i = begin + lane; i < end; i += 32) mx = fmaxf(mx, row[i]);
     mx = warp_max(mx);
-    if ((threadIdx.x & 31) == 0) s_maxes[threadIdx.x >> 5] = mx;
+    if (lane == 0) s.red[warp] = static_cast<double>(mx);
     __syncthreads();
+    if (threadIdx.x == 0) {
+        double m = s.red[0];
+        for (int w = 1; w < 32; ++w) m = fmax(m, s.red[w]);
+        s.cta_max = m;
+    }
+    cluster.sync();
     mx = -INFINITY;
-    for (int w = 0; w < (blockDim.x >> 5); ++w) mx = fmaxf(mx, s_maxes[w]);
+    for (int p = 0; p < kSampleParts; ++p) mx = fmaxf(mx, static_cast<float>(*cluster.map_shared_rank(&s.cta_max, p)));
 
     // p_i = exp((l_i - max)/T), sum in double, then scaled by (float)(1/sum)
-    double part = 0.0;
-    for (int i = threadIdx.x; i < V; i += blockDim.x) {
+    double mine = 0.0;
+    for (int i = begin + lane; i < end; i += 32) {
         const float e = expf((row[i] - mx) / temp);
         probs[i] = e;
-        part += static_cast<double>(e);
+        mine += static_cast<double>(e);
     }
-    const double sum = block_sum_double(part, s_red);
+    mine = block_sum_double(mine, s.red);
+    if (threadIdx.x == 0) s.cta_sum = mine;
+    cluster.sync();
+    double sum = 0.0;
+    for (int p = 0; p < kSampleParts; ++p) sum += *cluster.map_shared_rank(&s.cta_sum, p);
     const float inv_sum = static_cast<float>(1.0 / sum);
-    part = 0.0;
-    for (int i = threadIdx.x; i < V; i += blockDim.x) {
+    mine = 0.0;
+    for (int i = begin + lane; i < end; i += 32) {
         const float p = probs[i] * inv_sum;
         probs[i] = p;
-        part += static_cast<double>(p);
+        mine += static_cast<double>(p);
     }
+    mine = warp_sum_double(mine);
+    if (lane == 0) s.warp_mass[warp] = mine;
     __syncthreads();
-    const double all_mass = block_sum_double(part, s_red);
+    mine = 0.0;
+    for (int w = 0; w < 32; ++w) mine += s.warp_mass[w];
+    if (threadIdx.x == 0) s.cta_mass = mine;
+    cluster.sync();
+    double before = 0.0, all_mass = 0.0;              // `before`: the mass of the pieces ahead of this CTA's
+    for (int p = 0; p < kSampleParts; ++p) {
+        if (p == part) before = all_mass;
+        all_mass += *cluster.map_shared_rank(&s.cta_mass, p);
+    }
 
     const int k = top_k[r];
     const float tp = top_p[r];
@@ -239,118 +310,119 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ probs_all, i
     const bool use_p = tp < 1.0f;
     const double u = static_cast<double>(uniform[r]);
 
-    if (!use_k && !use_p) {
-        // index order: thread t owns a contiguous range; block scan of range masses in double
-        __shared__ double s_range[kSampleThreads];
-        const int per = (V + blockDim.x - 1) / blockDim.x;
-        const int begin = threadIdx.x * per, end = min(V, begin + per);
-        double mine = 0.0;
-        for (int i = begin; i < end; ++i) mine += static_cast<double>(probs[i]);
-        s_range[threadIdx.x] = mine;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            const double target = u * all_mass;
-            double run = 0.0;
+    if (!(sum == sum)) {                              // a row without probabilities (NaN, or infinities of one sign only)
+        if (part == 0 && threadIdx.x == 0) out[r] = use_p ? 0 : use_k ? k - 1 : V - 1;
+    } else if (!use_k && !use_p) {
+        // index order: the CTA, the warp, then the value at which the running mass exceeds the target
+        const double target = u * all_mass;
+        if (target >= all_mass) {
+            if (part == 0 && threadIdx.x == 0) out[r] = V - 1;          // rounding guard: u was (almost) 1
+        } else if (target >= before && target < before + mine) {
+            double run = before, next = before;       // run: the mass ahead of the owner, a warp that has some
             int owner = -1;
-            for (int t = 0; t < static_cast<int>(blockDim.x); ++t) {
-                if (target < run + s_range[t]) { owner = t; break; }
-                run += s_range[t];
+            for (int w = 0; w < 32 && !(target < next); ++w) {
+                if (s.warp_mass[w] > 0.0) { owner = w; run = next; }
+                next += s.warp_mass[w];
             }
-            s_choice[0] = owner;
-            s_hist_w[256] = run;
-        }
-        __syncthreads();
-        const int owner = s_choice[0];
-        if (owner < 0) {
-            if (threadIdx.x == 0) out[r] = V - 1;          // rounding guard: u was (almost) 1
-        } else if (threadIdx.x == owner) {
-            const double target = u * all_mass;
-            double cum = s_hist_w[256];
-            int pick = end - 1;
-            for (int i = begin; i < end; ++i) {
-                cum += static_cast<double>(probs[i]);
-                if (target < cum) { pick = i; break; }
+            if (owner == warp) {
+                int pick = -1, fallback = max(begin, end - 1);
+                for (int base = begin; base < end && pick < 0; base += 32) {
+                    const int i = base + lane;
+                    double cum = i < end ? static_cast<double>(probs[i]) : 0.0;
+                    const unsigned some = __ballot_sync(0xffffffffu, cum > 0.0);
+                    if (some) fallback = base + 31 - __clz(some);
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const double m = __shfl_up_sync(0xffffffffu, cum, o);
+                        if (lane >= o) cum += m;
+                    }
+                    cum += run;
+                    const unsigned over = __ballot_sync(0xffffffffu, i < end && target < cum);
+                    if (over) pick = base + __ffs(over) - 1;
+                    run = __shfl_sync(0xffffffffu, cum, 31);
+                }
+                if (lane == 0) out[r] = pick >= 0 ? pick : fallback;
             }
-            out[r] = pick;
         }
-        return;
-    }
+    } else {
+        // ---- the kept set is a prefix of the order (probability descending, index ascending) ----
+        // Its end is described by (boundary bits, number of boundary-valued elements kept).
+        // Start: everything kept.
+        double kept_mass = all_mass;
+        unsigned bound_bits = 0u;        // smallest kept probability's bits
+        int bound_take = 0;              // how many elements equal to it are kept (index order)
+        bool bounded = false;
+        int turn = 0;
 
-    // ---- the kept set is a prefix of the order (probability descending, index ascending) ----
-    // Its end is described by (boundary bits, number of boundary-valued elements kept).
-    // Start: everything kept.
-    double kept_mass = all_mass;
-    unsigned bound_bits = 0u;        // smallest kept probability's bits
-    int bound_take = 0;              // how many elements equal to it are kept (index order)
-    bool bounded = false;
-
-    if (use_k) {
-        Descent d{0u, 0u};
-        double before = 0.0;
-        radix_descend<true>(probs, V, static_cast<double>(k), true, d, before, s_hist_w, s_hist_c, s_choice);
-        bound_bits = d.prefix;
-        bound_take = k - static_cast<int>(before);           // before = count of strictly larger elements
-        bounded = true;
-        // mass of the kept set
-        double m = 0.0;
-        for (int i = threadIdx.x; i < V; i += blockDim.x)
-            if (__float_as_uint(probs[i]) > bound_bits) m += static_cast<double>(probs[i]);
-        __syncthreads();
-        kept_mass = block_sum_double(m, s_red) + static_cast<double>(bound_take) * static_cast<double>(__uint_as_float(bound_bits));
-    }
-
-    if (use_p) {
-        // shortest prefix with cum >= top_p * kept_mass, inside the current kept set.
-        const double threshold = static_cast<double>(tp) * kept_mass;
-        // The descent runs over all elements; as the kept set is a prefix of the same order, the
-        // crossing lies inside it unless rounding pushes it out, which is checked below.
-        Descent d{0u, 0u};
-        double before = 0.0;
-        radix_descend<false>(probs, V, threshold, true, d, before, s_hist_w, s_hist_c, s_choice);
-        unsigned nb = d.prefix;
-        const double w = static_cast<double>(__uint_as_float(nb));
-        int n_equal = count_equal(probs, V, nb, s_red);
-        // first rank (1-based count) with before + c*w >= threshold
-        int take = 1;
-        if (w > 0.0) {
-            double cum = before;
-            take = n_equal;
-            for (int c = 1; c <= n_equal; ++c) { cum += w; if (cum >= threshold) { take = c; break; } }
-        }
-        bool p_inside = true;
-        if (bounded) {
-            // the top-p end must not lie beyond the top-k end
-            if (nb < bound_bits || (nb == bound_bits && take > bound_take)) p_inside = false;
-        }
-        if (p_inside) {
-            bound_bits = nb;
-            bound_take = take;
+        if (use_k) {
+            const Found f = sample_descend(probs, begin, end, true, static_cast<double>(k), true, s, turn, cluster);
+            bound_bits = f.bits;
+            bound_take = k - f.count_above;
             bounded = true;
-            kept_mass = before + static_cast<double>(take) * w;
+            kept_mass = f.mass_above + static_cast<double>(bound_take) * static_cast<double>(__uint_as_float(bound_bits));
+        }
+        if (use_p) {
+            // shortest prefix with cum >= top_p * kept_mass, inside the current kept set. The descent runs over all elements;
+            // as the kept set is a prefix of the same order, the crossing lies inside it unless rounding pushes it out.
+            const double threshold = static_cast<double>(tp) * kept_mass;
+            const Found f = sample_descend(probs, begin, end, false, threshold, true, s, turn, cluster);
+            const double w = static_cast<double>(__uint_as_float(f.bits));
+            const int take = w > 0.0 ? sample_count_to(f.mass_above, w, f.equal, threshold, true) : 1;
+            if (!bounded || f.bits > bound_bits || (f.bits == bound_bits && take <= bound_take)) {
+                bound_bits = f.bits;
+                bound_take = take;
+                bounded = true;
+                kept_mass = f.mass_above + static_cast<double>(take) * w;
+            }
+        }
+
+        // ---- draw: first token in the order with u * kept_mass < cum ----
+        const double target = u * kept_mass;
+        const Found f = sample_descend(probs, begin, end, false, target, false, s, turn, cluster);
+        unsigned pick_bits = f.bits;
+        int rank = sample_count_to(f.mass_above, static_cast<double>(__uint_as_float(pick_bits)), f.equal, target, false) - 1;
+        // clamp to the kept set (rounding guard: the last kept token)
+        if (bounded && (pick_bits < bound_bits || (pick_bits == bound_bits && rank >= bound_take))) {
+            pick_bits = bound_bits;
+            rank = bound_take - 1;
+        }
+        // the rank-th (0-based) index with those bits: the CTA, the warp, then the place
+        int c = 0;
+        for (int i = begin + lane; i < end; i += 32) c += __float_as_uint(probs[i]) == pick_bits;
+        c = __reduce_add_sync(0xffffffffu, c);
+        __syncthreads();
+        if (lane == 0) s.counts[warp] = c;
+        __syncthreads();
+        int own = 0, ahead = 0;
+        for (int w = 0; w < 32; ++w) {
+            if (w == warp) ahead = own;
+            own += s.counts[w];
+        }
+        if (threadIdx.x == 0) s.cta_equal = own;
+        cluster.sync();
+        for (int p = 0; p < part; ++p) ahead += *cluster.map_shared_rank(&s.cta_equal, p);
+        if (rank >= ahead && rank < ahead + c) {
+            for (int base = begin; base < end; base += 32) {
+                const int i = base + lane;
+                const unsigned same = __ballot_sync(0xffffffffu, i < end && __float_as_uint(probs[i]) == pick_bits);
+                if (rank < ahead + __popc(same)) {
+                    if ((same >> lane & 1u) && ahead + __popc(same & ((1u << lane) - 1)) == rank) out[r] = i;
+                    break;
+                }
+                ahead += __popc(same);
+            }
         }
     }
+    cluster.sync();                                   // no CTA leaves while another may read its shared memory
+}
 
-    // ---- draw: first token in the order with u * kept_mass < cum ----
-    const double target = u * kept_mass;
-    Descent d{0u, 0u};
-    double before = 0.0;
-    radix_descend<false>(probs, V, target, false, d, before, s_hist_w, s_hist_c, s_choice);
-    unsigned pick_bits = d.prefix;
-    int rank = 0;
-    {
-        const double w = static_cast<double>(__uint_as_float(pick_bits));
-        const int n_equal = count_equal(probs, V, pick_bits, s_red);
-        rank = n_equal - 1;
-        double cum = before;
-        for (int c = 0; c < n_equal; ++c) { cum += w; if (target < cum) { rank = c; break; } }
-    }
-    // clamp to the kept set (rounding guard: the last kept token)
-    if (bounded && (pick_bits < bound_bits || (pick_bits == bound_bits && rank >= bound_take))) {
-        pick_bits = bound_bits;
-        rank = bound_take - 1;
-    }
-    const int idx = nth_equal_index(probs, V, pick_bits, rank, s_choice);
-    if (threadIdx.x == 0) out[r] = idx;
+int launch_sample(const float* logits, float* probs, int rows, int V, const float* temperature, const int* top_k, const float* top_p,
+                  const float* uniform, int* out, cudaStream_t st) {
+    GI_REQUIRE(rows <= INT_MAX / kSampleParts, "sample: %d rows exceed the grid limit", rows);
+    const dim3 grid(rows * kSampleParts), block(kSampleThreads);
+    if (V <= kNarrowVocab) launch_kernel((sample_kernel<false>), grid, block, 0, st, logits, probs, V, temperature, top_k, top_p, uniform, out);
+    else launch_kernel((sample_kernel<true>), grid, block, 0, st, logits, probs, V, temperature, top_k, top_p, uniform, out);
+    return check_launch("sample");
 }
 
 }  // namespace gi
@@ -376,9 +448,7 @@ static int gi_sample_impl(const float* logits, float* probs_scratch, int rows, i
                          const int* top_k, const float* top_p, const float* uniform, int* out, void* stream) {
     if (rows == 0) return 0;
     GI_REQUIRE(rows > 0 && V > 0, "sample: sizes must be positive (rows=%d, V=%d)", rows, V);
-    launch_kernel((sample_kernel), dim3(rows), dim3(kSampleThreads), 0, static_cast<cudaStream_t>(stream), 
-        logits, probs_scratch, V, temperature, top_k, top_p, uniform, out);
-    return check_launch("sample");
+    return launch_sample(logits, probs_scratch, rows, V, temperature, top_k, top_p, uniform, out, static_cast<cudaStream_t>(stream));
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -438,9 +508,7 @@ extern "C" int gi_sample_no_alloc(const float* logits, int rows, int vocab, cons
     float* work = nullptr;
     const int rc = work_area_for_current_device(&work);
     if (rc != 0) return rc;
-    launch_kernel((sample_kernel), dim3(rows), dim3(kSampleThreads), 0, static_cast<cudaStream_t>(stream), 
-        logits, work, vocab, temperature, top_k, top_p, uniform, out);
-    return check_launch("sample_no_alloc");
+    return launch_sample(logits, work, rows, vocab, temperature, top_k, top_p, uniform, out, static_cast<cudaStream_t>(stream));
 }
 
 // The exported names: each runs its implementation above and, while a launch program is recorded, leaves a copy of

@@ -343,6 +343,30 @@ def test_sample_matches_plain_sampler(V, temperature, top_k, top_p):
     assert not bad, f"rows (row, got, want): {bad}"
 
 
+@pytest.mark.parametrize("V,top_k,top_p", [(V, k, p) for V in (1, 7, 131, 8195, 128256) for k, p in ((0, 1.0), (3, 1.0), (0, 0.9), (40, 0.95))] +
+                         [((8 << 20) + 5, 40, 0.95)])
+def test_sample_rows_of_few_likely_tokens(V, top_k, top_p):
+    """Vocabularies around the pieces of a row (and above what its short words take), masked logits, rows without probabilities."""
+    g = torch.Generator().manual_seed(12)
+    logits = torch.full((4, V), float("-inf"))
+    at = torch.randperm(V, generator=g)[:min(V, 6)]
+    logits[0, at] = torch.arange(len(at)).float() * 0.5                         # six tokens, the rest masked
+    logits[1] = -200.0                                                          # one token, the rest underflow to 0
+    logits[1, V - 1] = 3.0
+    logits[2] = torch.randn(V, generator=g) * 2.5
+    if V > 10:
+        logits[2, 5] = logits[2, V // 2] = logits[2, V - 2] = 30.0              # equals across pieces
+    us = torch.tensor([0.62, 0.999, 0.5, 0.3])
+    out = torch.full((4,), -1, dtype=torch.int32, device=DEV)
+    K().sample(logits.to(DEV), torch.empty(4 * V, device=DEV), torch.ones(4, device=DEV),
+               torch.full((4,), top_k, dtype=torch.int32, device=DEV), torch.full((4,), top_p, device=DEV), us.to(DEV), out)
+    got = out.cpu().tolist()
+    for r in range(3):
+        near = {pm.PlainSampler(1.0, top_k, top_p).sample(logits[r].numpy(), u) for u in (float(us[r]) - 1e-6, float(us[r]), float(us[r]) + 1e-6)}
+        assert got[r] in near, (r, got[r], near)
+    assert got[3] == (0 if top_p < 1.0 else top_k - 1 if 0 < top_k < V else V - 1)      # no probabilities: an index, always the same
+
+
 @pytest.mark.parametrize("M,N,K_,plan", [
     (128, 256, 64, (False, 256, 1)), (128, 256, 512, (False, 256, 1)), (300, 520, 200, (False, 256, 1)),
     (129, 100, 96, (False, 128, 1)), (256, 64, 128, (False, 64, 1)),
