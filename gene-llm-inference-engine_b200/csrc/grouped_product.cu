@@ -169,13 +169,18 @@ grouped_product_kernel(const GroupedArgs p) {
     }
 }
 
-// The same products for few rows (decoding): the weights are what takes the time, so a warp streams whole rows of a
-// group's matrix with 16-byte loads, four rows after one another, and multiplies each with every row of the tile (at most
-// 16, read through the cache); a block of eight warps covers 32 output rows, so a matrix of a few thousand rows is spread
-// over more than a hundred blocks per tile. An output element is the sum of its lanes' partial sums (lane l takes the
+// The same products for few rows (decoding): the weights are what takes the time. A warp streams four output rows of a
+// group's matrix (gated: and their up rows) through a ring in shared memory, 512 bytes of each a step, by asynchronous copies
+// of 16 bytes; every lane copies exactly the pieces that it multiplies itself, so the ring needs no barrier, and 48 KB or more
+// are in flight per block whatever the warps are doing. (With the loads in registers, eight a lane and none while it
+// multiplied, eight experts of 2 x 4096 x 2048 values and sixteen pairs took 124 us, 1.9 TB/s.) Each step's
+// pieces are multiplied with up to eight rows of the tile, read through the cache; more rows stream the weights again, from
+// L2. An output element is the sum of its lanes' partial sums (lane l takes the
 // pieces l, l + 32, ...), added by a fixed xor tree: it depends on its own row only.
-constexpr int kGrRows = 32;           // output rows per block
-constexpr int kGrFew = 4;             // rows of a tile that are multiplied with a piece of the weights while it is in registers
+constexpr int kGrWarps = 4, kGrWarpRows = 4;
+constexpr int kGrRows = kGrWarps * kGrWarpRows;      // output rows per block
+constexpr int kGrFew = 8;             // rows of a tile that are multiplied with a piece of the weights while it is in registers
+constexpr int kGrSmem = 64 * 1024;    // the block's ring: three blocks an SM
 
 template <typename T> struct Vec16;
 template <> struct Vec16<float> {
@@ -195,118 +200,6 @@ template <> struct Vec16<__nv_bfloat16> {
     }
 };
 
-// PIECE: values per step of a lane = the weights' 16 bytes (8 bfloat16 or 4 floats); the inputs are read in as many.
-template <typename TA, typename TW, bool GATED>
-__global__ void __launch_bounds__(256)
-grouped_rows_kernel(const GroupedArgs p) {
-    pdl_prologue();
-    constexpr int PIECE = Vec16<TW>::N;
-    __shared__ int s_row[kGpTM];
-    __shared__ int s_count;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    int g;
-    if (p.tile_group) {
-        if (static_cast<int>(blockIdx.x) >= *p.n_tiles) return;
-        g = p.tile_group[blockIdx.x];
-    } else {
-        g = blockIdx.x % p.groups;
-    }
-    if (tid == 0) {             // the tile's rows, the empty places left out
-        int n = 0;
-        for (int i = 0; i < kGpTM; ++i) {
-            int r;
-            if (p.tile_group) r = p.sorted_rows[blockIdx.x * kGpTM + i];
-            else { r = (blockIdx.x / p.groups) * kGpTM + i; if (r >= p.rows) r = -1; }
-            if (r >= 0) s_row[n++] = r;
-        }
-        s_count = n;
-    }
-    __syncthreads();
-    const int m_count = s_count;
-    const TA* A = static_cast<const TA*>(p.a) + p.a_off + static_cast<size_t>(g) * p.a_gs;
-    const TW* W = static_cast<const TW*>(p.w) + static_cast<size_t>(g) * p.w_gs;
-    const int pieces = p.K / PIECE;
-    // The warp's four weight rows are streamed together, eight 16-byte loads of a lane in flight, and every input piece is
-    // read once for the four. The tile's rows are taken four at a time (a tile of a decode step seldom has more); a
-    // second group of four streams the same weight rows again, from the L2 cache.
-    const int n_first = blockIdx.y * kGrRows + warp * 4;
-    if (n_first >= p.N) return;
-    const TW* wrow[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) wrow[r] = W + static_cast<size_t>(min(n_first + r, p.N - 1)) * p.ldw;
-    for (int m0 = 0; m0 < m_count; m0 += kGrFew) {
-        const int m_here = min(kGrFew, m_count - m0);
-        float acc[4][kGrFew], acc_up[GATED ? 4 : 1][kGrFew];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-#pragma unroll
-            for (int i = 0; i < kGrFew; ++i) { acc[r][i] = 0.f; if (GATED) acc_up[GATED ? r : 0][i] = 0.f; }
-        }
-        // the output gate's values of the warp's 4 x kGrFew outputs, a lane each, asked for before the weights stream
-        float gate_z = 0.f;
-        if (p.gate != nullptr && lane < 4 * kGrFew) {
-            const int gr = lane / kGrFew, gi_ = lane % kGrFew;
-            if (gi_ < m_here && n_first + gr < p.N)
-                gate_z = gp_gate_value(p, s_row[m0 + gi_], g, n_first + gr);
-        }
-        for (int c = lane; c < pieces; c += 32) {
-            float wv[4][8], uv[GATED ? 4 : 1][8];
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                Vec16<TW>::load(wrow[r] + c * PIECE, wv[r]);
-                if (GATED) Vec16<TW>::load(wrow[r] + p.up_off + c * PIECE, uv[GATED ? r : 0]);
-            }
-#pragma unroll
-            for (int i = 0; i < kGrFew; ++i) {
-                if (i < m_here) {
-                    const TA* arow = A + static_cast<size_t>(s_row[m0 + i] / p.a_div) * p.lda + c * PIECE;
-                    float av[8];
-                    if (sizeof(TA) == 4 && PIECE == 8) {          // 32-bit inputs against bfloat16 weights: two loads
-                        float lo4[8], hi4[8];
-                        Vec16<float>::load(reinterpret_cast<const float*>(arow), lo4);
-                        Vec16<float>::load(reinterpret_cast<const float*>(arow) + 4, hi4);
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) { av[j] = lo4[j]; av[4 + j] = hi4[j]; }
-                    } else {
-                        Vec16<TA>::load(arow, av);
-                    }
-#pragma unroll
-                    for (int r = 0; r < 4; ++r) {
-#pragma unroll
-                        for (int j = 0; j < PIECE; ++j) {
-                            acc[r][i] = fmaf(av[j], wv[r][j], acc[r][i]);
-                            if (GATED) acc_up[GATED ? r : 0][i] = fmaf(av[j], uv[GATED ? r : 0][j], acc_up[GATED ? r : 0][i]);
-                        }
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-#pragma unroll
-            for (int i = 0; i < kGrFew; ++i) {
-                if (i < m_here && n_first + r < p.N) {
-                    const float sc = p.scales ? p.scales[s_row[m0 + i]] : 1.f;
-                    float v = sc * warp_sum(acc[r][i]);
-                    if (GATED) v = gated_value(v, sc * warp_sum(acc_up[GATED ? r : 0][i]), p.act, p.act_limit);
-                    else v = plain_value(v, p.out_act);
-                    if (p.gate != nullptr) v *= 1.0f / (1.0f + expf(-__shfl_sync(0xffffffffu, gate_z, r * kGrFew + i)));
-                    if (lane == 0) {
-                        const size_t o = static_cast<size_t>(s_row[m0 + i]) * p.ldo + p.o_off + static_cast<size_t>(g) * p.o_gs + n_first + r;
-                        if (p.out_is_f32) static_cast<float*>(p.out)[o] = v;
-                        else static_cast<__nv_bfloat16*>(p.out)[o] = __float2bfloat16_rn(v);
-                    }
-                }
-            }
-        }
-    }
-}
-
-// The heads form for many rows (prompt portions): tiles of 64 rows x 64 outputs, a thread 4 x 4 of them, so that two
-// 16-byte reads of shared memory feed sixteen multiply-adds. Inputs 32-bit or bfloat16, weights likewise; rows of four
-// values must be aligned (the caller checks). An output element is one chain of multiply-adds in the order of k.
-constexpr int kG64 = 64, kG64K = 16;
-
 template <typename T> __device__ __forceinline__ float4 load4(const T* p);
 template <> __device__ __forceinline__ float4 load4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
 template <> __device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bfloat16* p) {
@@ -315,6 +208,150 @@ template <> __device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bf
     const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
     return make_float4(a.x, a.y, b.x, b.y);
 }
+
+// What a warp of the few-row form works on.
+template <typename TA, typename TW>
+struct RowsWork {
+    const TA* A;                 // the group's inputs
+    const TW* wrow[kGrWarpRows]; // the warp's rows of weights
+    uint4* ring;                 // this lane's place in the warp's first stage
+    const int* rows;             // the tile's rows
+    int g, n_first, lane;
+};
+
+// MR rows of the tile (m_here of them are real, the last is repeated) against the warp's output rows.
+template <int MR, typename TA, typename TW, bool GATED>
+__device__ __forceinline__ void grouped_rows_few(const GroupedArgs& p, const RowsWork<TA, TW>& q, int m0, int m_here) {
+    constexpr int PIECE = Vec16<TW>::N;              // values per step of a lane: the weights' 16 bytes
+    constexpr int kW = GATED ? 2 * kGrWarpRows : kGrWarpRows;
+    constexpr int kStages = kGrSmem / (kGrWarps * kW * 512);
+    const int pieces = p.K / PIECE, steps = (pieces + 31) / 32;
+    auto load = [&](int step) {
+        const int c = step * 32 + q.lane;
+        if (c < pieces) {
+            const unsigned at = static_cast<unsigned>(__cvta_generic_to_shared(q.ring + (step % kStages) * (kW * 32)));
+#pragma unroll
+            for (int r = 0; r < kW; ++r) {
+                const TW* src = q.wrow[r % kGrWarpRows] + (r >= kGrWarpRows ? p.up_off : 0) + c * PIECE;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(at + r * 512), "l"(src) : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int i = 0; i < kStages - 1; ++i) load(i);
+    const TA* arow[MR];
+#pragma unroll
+    for (int i = 0; i < MR; ++i) arow[i] = q.A + static_cast<size_t>(q.rows[m0 + min(i, m_here - 1)] / p.a_div) * p.lda;
+    // the output gate's values of the warp's 4 x 8 outputs, a lane each, asked for before the weights arrive
+    float gate_z = 0.f;
+    if (p.gate != nullptr) {
+        const int gr = q.lane / kGrFew, gi_ = q.lane % kGrFew;
+        if (gi_ < m_here && q.n_first + gr < p.N) gate_z = gp_gate_value(p, q.rows[m0 + gi_], q.g, q.n_first + gr);
+    }
+    float acc[kW][MR];
+#pragma unroll
+    for (int r = 0; r < kW; ++r)
+#pragma unroll
+        for (int i = 0; i < MR; ++i) acc[r][i] = 0.f;
+    for (int step = 0; step < steps; ++step) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+        const int c = step * 32 + q.lane;
+        if (c < pieces) {
+            const uint4* stage = q.ring + (step % kStages) * (kW * 32);
+#pragma unroll
+            for (int h = 0; h < PIECE; h += 4) {
+                float av[MR][4];
+#pragma unroll
+                for (int i = 0; i < MR; ++i) {
+                    const float4 v = load4<TA>(arow[i] + c * PIECE + h);
+                    av[i][0] = v.x; av[i][1] = v.y; av[i][2] = v.z; av[i][3] = v.w;
+                }
+#pragma unroll
+                for (int r = 0; r < kW; ++r) {
+                    float wv[8];
+                    Vec16<TW>::load(reinterpret_cast<const TW*>(stage + r * 32), wv);
+#pragma unroll
+                    for (int i = 0; i < MR; ++i)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) acc[r][i] = fmaf(av[i][j], wv[h + j], acc[r][i]);
+                }
+            }
+        }
+        load(step + kStages - 1);                     // into the stage read a step ago, by this lane alone
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+    for (int r = 0; r < kGrWarpRows; ++r) {
+#pragma unroll
+        for (int i = 0; i < MR; ++i) {
+            if (i < m_here && q.n_first + r < p.N) {
+                const int row = q.rows[m0 + i];
+                const float sc = p.scales ? p.scales[row] : 1.f;
+                float v = sc * warp_sum(acc[r][i]);
+                if (GATED) v = gated_value(v, sc * warp_sum(acc[GATED ? r + kGrWarpRows : 0][i]), p.act, p.act_limit);
+                else v = plain_value(v, p.out_act);
+                if (p.gate != nullptr) v *= 1.0f / (1.0f + expf(-__shfl_sync(0xffffffffu, gate_z, r * kGrFew + i)));
+                if (q.lane == 0) {
+                    const size_t o = static_cast<size_t>(row) * p.ldo + p.o_off + static_cast<size_t>(q.g) * p.o_gs + q.n_first + r;
+                    if (p.out_is_f32) static_cast<float*>(p.out)[o] = v;
+                    else static_cast<__nv_bfloat16*>(p.out)[o] = __float2bfloat16_rn(v);
+                }
+            }
+        }
+    }
+}
+
+template <typename TA, typename TW, bool GATED>
+__global__ void __launch_bounds__(kGrWarps * 32, 3)
+grouped_rows_kernel(const GroupedArgs p) {
+    extern __shared__ uint4 s_ring[];
+    __shared__ int s_row[kGpTM];
+    __shared__ int s_count;
+    pdl_prologue();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int g;
+    if (p.tile_group) {
+        if (static_cast<int>(blockIdx.x) >= *p.n_tiles) return;
+        g = p.tile_group[blockIdx.x];
+    } else {
+        g = blockIdx.x % p.groups;
+    }
+    if (warp == 0) {             // the tile's rows, the empty places left out
+        int r = -1;
+        if (lane < kGpTM) {
+            if (p.tile_group) r = p.sorted_rows[blockIdx.x * kGpTM + lane];
+            else { r = (blockIdx.x / p.groups) * kGpTM + lane; if (r >= p.rows) r = -1; }
+        }
+        const unsigned some = __ballot_sync(0xffffffffu, r >= 0);
+        if (r >= 0) s_row[__popc(some & ((1u << lane) - 1))] = r;
+        if (lane == 0) s_count = __popc(some);
+    }
+    __syncthreads();
+    const int m_count = s_count;
+    constexpr int kW = GATED ? 2 * kGrWarpRows : kGrWarpRows;
+    constexpr int kStages = kGrSmem / (kGrWarps * kW * 512);
+    RowsWork<TA, TW> q;
+    q.n_first = blockIdx.y * kGrRows + warp * kGrWarpRows;
+    if (q.n_first >= p.N) return;
+    q.g = g; q.lane = lane; q.rows = s_row;
+    q.A = static_cast<const TA*>(p.a) + p.a_off + static_cast<size_t>(g) * p.a_gs;
+    q.ring = s_ring + warp * (kStages * kW * 32) + lane;
+    const TW* W = static_cast<const TW*>(p.w) + static_cast<size_t>(g) * p.w_gs;
+#pragma unroll
+    for (int r = 0; r < kGrWarpRows; ++r) q.wrow[r] = W + static_cast<size_t>(min(q.n_first + r, p.N - 1)) * p.ldw;
+    for (int m0 = 0; m0 < m_count; m0 += kGrFew) {
+        const int m_here = min(kGrFew, m_count - m0);
+        if (m_here == 1) grouped_rows_few<1, TA, TW, GATED>(p, q, m0, m_here);
+        else if (m_here == 2) grouped_rows_few<2, TA, TW, GATED>(p, q, m0, m_here);
+        else if (m_here <= 4) grouped_rows_few<4, TA, TW, GATED>(p, q, m0, m_here);
+        else grouped_rows_few<8, TA, TW, GATED>(p, q, m0, m_here);
+    }
+}
+
+// The heads form for many rows (prompt portions): tiles of 64 rows x 64 outputs, a thread 4 x 4 of them, so that two
+// 16-byte reads of shared memory feed sixteen multiply-adds. Inputs 32-bit or bfloat16, weights likewise; rows of four
+// values must be aligned (the caller checks). An output element is one chain of multiply-adds in the order of k.
+constexpr int kG64 = 64, kG64K = 16;
 
 template <typename TA, typename TW>
 __global__ void __launch_bounds__(256)
@@ -575,13 +612,18 @@ static bool rows_form_fits(const GroupedArgs& p, int a_dtype, int w_dtype) {
     return p.lda % a_piece == 0 && p.a_off % a_piece == 0 && p.a_gs % a_piece == 0;
 }
 
+template <typename TA, typename TW, bool GATED>
+static int launch_grouped_rows_as(const GroupedArgs& p, unsigned tiles, cudaStream_t st) {
+    static const cudaError_t ready = cudaFuncSetAttribute(grouped_rows_kernel<TA, TW, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGrSmem);
+    if (ready != cudaSuccess) { set_error("grouped_product (rows): %s", cudaGetErrorString(ready)); return 1; }
+    launch_kernel((grouped_rows_kernel<TA, TW, GATED>), dim3(tiles, (p.N + kGrRows - 1) / kGrRows), dim3(kGrWarps * 32), kGrSmem, st, p);
+    return check_launch("grouped_product (rows)");
+}
 template <bool GATED>
 static int launch_grouped_rows(const GroupedArgs& p, int a_dtype, int w_dtype, unsigned tiles, cudaStream_t st) {
-    dim3 grid(tiles, (p.N + kGrRows - 1) / kGrRows);
-    if (a_dtype == kF32 && w_dtype == kF32) launch_kernel((grouped_rows_kernel<float, float, GATED>), grid, dim3(256), 0, st, p);
-    else if (a_dtype == kF32 && w_dtype == kBF16) launch_kernel((grouped_rows_kernel<float, __nv_bfloat16, GATED>), grid, dim3(256), 0, st, p);
-    else launch_kernel((grouped_rows_kernel<__nv_bfloat16, __nv_bfloat16, GATED>), grid, dim3(256), 0, st, p);
-    return check_launch("grouped_product (rows)");
+    if (a_dtype == kF32 && w_dtype == kF32) return launch_grouped_rows_as<float, float, GATED>(p, tiles, st);
+    if (a_dtype == kF32 && w_dtype == kBF16) return launch_grouped_rows_as<float, __nv_bfloat16, GATED>(p, tiles, st);
+    return launch_grouped_rows_as<__nv_bfloat16, __nv_bfloat16, GATED>(p, tiles, st);
 }
 
 template <bool GATED>

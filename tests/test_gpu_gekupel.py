@@ -259,6 +259,32 @@ def test_routing_and_expert_products(dtype, T, E, top, D, I):
     _close(y.cpu(), want, torch.float32, "routed experts", f32=1e-5)
 
 
+@pytest.mark.parametrize("gated", ["silu", None])
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("N, K", [(18, 8), (33, 264), (16, 2056)])
+def test_expert_products_of_few_rows(dtype, N, K, gated):
+    """Every count of rows in a tile, rows of one to nine steps with a ragged last one, blocks of outputs with a ragged last one.
+    Bound: K products of values of about 1 and 0.1 in 32-bit, each lane's chain K / 32 long."""
+    from geneinfer_b200.ops import kernels
+    g = torch.Generator().manual_seed(21)
+    counts = [1, 2, 3, 4, 5, 7, 8, 9, 13, 16]
+    E, tm, T = len(counts), kernels.grouped_tile_rows(), sum(counts)
+    a, w = _bf(torch.randn(T, K, generator=g)), _bf(torch.randn(E, (2 if gated else 1) * N, K, generator=g) * 0.1)
+    rows = torch.randperm(T, generator=g).to(torch.int32).split(counts)
+    srt = torch.full((E, tm), -1, dtype=torch.int32)
+    for e, r in enumerate(rows):
+        srt[e, torch.randperm(tm, generator=g)[:len(r)]] = r          # empty places anywhere in a tile
+    grp = torch.arange(E, dtype=torch.int32).flip(0)
+    out = torch.full((T, N), float("nan"), device=DEV)
+    kernels.expert_product(a.to(DEV).to(dtype), 1, w.to(DEV).to(dtype), out, srt.flip(0).reshape(-1).to(DEV), grp.to(DEV),
+                           torch.tensor([E], dtype=torch.int32, device=DEV), gated=gated)
+    want = torch.empty(T, N, dtype=torch.float64)
+    for e, r in enumerate(rows):
+        z = a[r.long()].double() @ w[e].double().T
+        want[r.long()] = torch.nn.functional.silu(z[:, :N]) * z[:, N:] if gated else z
+    _close(out.cpu(), want, torch.float32, "few rows", f32=1e-5)
+
+
 # ------------------------------------------------------------------------------------------ mixers alone
 ATT = {"heads": 6, "kv_heads": 2, "dim": 16, "vdim": 24, "mask": {"size": 11}, "scale": 0.45}
 LAT = {"heads": 3, "dim": 24, "rot_dim": 8, "vdim": 40, "q_rank": 32, "kv_rank": 48, "mask": {"size": 13}, "scale": 0.3,
