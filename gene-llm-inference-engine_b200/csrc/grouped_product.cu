@@ -173,12 +173,12 @@ grouped_product_kernel(const GroupedArgs p) {
 // group's matrix (gated: and their up rows) through a ring in shared memory, 512 bytes of each a step, by asynchronous copies
 // of 16 bytes; every lane copies exactly the pieces that it multiplies itself, so the ring needs no barrier, and 48 KB or more
 // are in flight per block whatever the warps are doing. (With the loads in registers, eight a lane and none while it
-// multiplied, eight experts of 2 x 4096 x 2048 values and sixteen pairs took 124 us, 1.9 TB/s.) Each step's
+// multiplied, eight experts of 2 x 4096 x 2048 values and sixteen pairs took 124 us, 1.9 TB/s; with the ring and a block per
+// sixteen output rows 74 us, a third of it the blocks' beginnings and ends.) Each step's
 // pieces are multiplied with up to eight rows of the tile, read through the cache; more rows stream the weights again, from
 // L2. An output element is the sum of its lanes' partial sums (lane l takes the
 // pieces l, l + 32, ...), added by a fixed xor tree: it depends on its own row only.
 constexpr int kGrWarps = 4, kGrWarpRows = 4;
-constexpr int kGrRows = kGrWarps * kGrWarpRows;      // output rows per block
 constexpr int kGrFew = 8;             // rows of a tile that are multiplied with a piece of the weights while it is in registers
 constexpr int kGrSmem = 64 * 1024;    // the block's ring: three blocks an SM
 
@@ -209,61 +209,104 @@ template <> __device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bf
     return make_float4(a.x, a.y, b.x, b.y);
 }
 
-// What a warp of the few-row form works on.
-template <typename TA, typename TW>
-struct RowsWork {
-    const TA* A;                 // the group's inputs
-    const TW* wrow[kGrWarpRows]; // the warp's rows of weights
-    uint4* ring;                 // this lane's place in the warp's first stage
-    const int* rows;             // the tile's rows
-    int g, n_first, lane;
-};
+// The few-row form's units of work, taken by the grid's warps in turn: (tile, four output rows), and for a tile of more than
+// kGrFew rows a second pass over the same weights. A warp's ring runs on from unit to unit.
+template <typename TA, typename TW, bool GATED>
+struct RowsStream {
+    static constexpr int kPiece = Vec16<TW>::N;          // values per step of a lane: the weights' 16 bytes
+    static constexpr int kW = GATED ? 2 * kGrWarpRows : kGrWarpRows;
+    static constexpr int kStages = kGrSmem / (kGrWarps * kW * 512);
 
-// MR rows of the tile (m_here of them are real, the last is repeated) against the warp's output rows.
-template <int MR, typename TA, typename TW, bool GATED>
-__device__ __forceinline__ void grouped_rows_few(const GroupedArgs& p, const RowsWork<TA, TW>& q, int m0, int m_here) {
-    constexpr int PIECE = Vec16<TW>::N;              // values per step of a lane: the weights' 16 bytes
-    constexpr int kW = GATED ? 2 * kGrWarpRows : kGrWarpRows;
-    constexpr int kStages = kGrSmem / (kGrWarps * kW * 512);
-    const int pieces = p.K / PIECE, steps = (pieces + 31) / 32;
-    auto load = [&](int step) {
-        const int c = step * 32 + q.lane;
-        if (c < pieces) {
-            const unsigned at = static_cast<unsigned>(__cvta_generic_to_shared(q.ring + (step % kStages) * (kW * 32)));
+    const GroupedArgs& p;
+    uint4* ring;                 // this lane's place in the warp's first stage
+    int lane, units, per_tile, stride, pieces, steps;
+    // the step that is requested next
+    int unit, pass, passes, step, issued = 0;
+    const TW* wrow[kGrWarpRows];
+
+    // Group and rows of tile x; lane i gets the i-th of its rows.
+    __device__ __forceinline__ int tile(int x, int& g, int& row) const {
+        int r = -1;
+        if (p.tile_group) {
+            g = p.tile_group[x];
+            if (lane < kGpTM) r = p.sorted_rows[x * kGpTM + lane];
+        } else {
+            g = x % p.groups;
+            if (lane < kGpTM) r = x / p.groups * kGpTM + lane;
+            if (r >= p.rows) r = -1;
+        }
+        const unsigned some = __ballot_sync(0xffffffffu, r >= 0);       // the empty places left out
+        row = r;
+        if (some & (some + 1)) row = __shfl_sync(0xffffffffu, r, __fns(some, 0, lane + 1) & 31);
+        return __popc(some);
+    }
+    __device__ __forceinline__ void seek() {
+        for (; unit < units; unit += stride) {
+            int g, row;
+            passes = (tile(unit / per_tile, g, row) + kGrFew - 1) / kGrFew;
+            if (passes == 0) continue;
+            const TW* W = static_cast<const TW*>(p.w) + static_cast<size_t>(g) * p.w_gs;
+            const int n_first = unit % per_tile * kGrWarpRows;
 #pragma unroll
-            for (int r = 0; r < kW; ++r) {
-                const TW* src = q.wrow[r % kGrWarpRows] + (r >= kGrWarpRows ? p.up_off : 0) + c * PIECE;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(at + r * 512), "l"(src) : "memory");
+            for (int r = 0; r < kGrWarpRows; ++r) wrow[r] = W + static_cast<size_t>(min(n_first + r, p.N - 1)) * p.ldw;
+            pass = step = 0;
+            return;
+        }
+    }
+    __device__ __forceinline__ void request() {
+        if (unit < units) {
+            const int c = step * 32 + lane;
+            if (c < pieces) {
+                const unsigned at = static_cast<unsigned>(__cvta_generic_to_shared(ring + (issued % kStages) * (kW * 32)));
+#pragma unroll
+                for (int r = 0; r < kW; ++r) {
+                    const TW* src = wrow[r % kGrWarpRows] + (r >= kGrWarpRows ? p.up_off : 0) + c * kPiece;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(at + r * 512), "l"(src) : "memory");
+                }
+            }
+            if (++step == steps) {
+                step = 0;
+                if (++pass == passes) { unit += stride; seek(); }
             }
         }
+        ++issued;
         asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    for (int i = 0; i < kStages - 1; ++i) load(i);
+    }
+};
+
+// MR rows of a tile (m_here of them are real, the last is repeated) against the four output rows from n_first on. ``row``:
+// lane i has the tile's i-th row; ``done``: steps of the warp's ring taken so far.
+template <int MR, typename TA, typename TW, bool GATED>
+__device__ __forceinline__ void grouped_rows_unit(RowsStream<TA, TW, GATED>& q, int g, int row, int n_first, int m0, int m_here, int& done) {
+    const GroupedArgs& p = q.p;
+    constexpr int kW = RowsStream<TA, TW, GATED>::kW, kStages = RowsStream<TA, TW, GATED>::kStages, kPiece = Vec16<TW>::N;
+    const TA* A = static_cast<const TA*>(p.a) + p.a_off + static_cast<size_t>(g) * p.a_gs;
     const TA* arow[MR];
 #pragma unroll
-    for (int i = 0; i < MR; ++i) arow[i] = q.A + static_cast<size_t>(q.rows[m0 + min(i, m_here - 1)] / p.a_div) * p.lda;
-    // the output gate's values of the warp's 4 x 8 outputs, a lane each, asked for before the weights arrive
+    for (int i = 0; i < MR; ++i) arow[i] = A + static_cast<size_t>(__shfl_sync(0xffffffffu, row, m0 + min(i, m_here - 1)) / p.a_div) * p.lda;
+    // the output gate's values of the unit's 4 x 8 outputs, a lane each, asked for before the weights arrive
     float gate_z = 0.f;
     if (p.gate != nullptr) {
         const int gr = q.lane / kGrFew, gi_ = q.lane % kGrFew;
-        if (gi_ < m_here && q.n_first + gr < p.N) gate_z = gp_gate_value(p, q.rows[m0 + gi_], q.g, q.n_first + gr);
+        const int gate_row = __shfl_sync(0xffffffffu, row, m0 + min(gi_, m_here - 1));
+        if (gi_ < m_here && n_first + gr < p.N) gate_z = gp_gate_value(p, gate_row, g, n_first + gr);
     }
     float acc[kW][MR];
 #pragma unroll
     for (int r = 0; r < kW; ++r)
 #pragma unroll
         for (int i = 0; i < MR; ++i) acc[r][i] = 0.f;
-    for (int step = 0; step < steps; ++step) {
+    for (int step = 0; step < q.steps; ++step, ++done) {
         asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
         const int c = step * 32 + q.lane;
-        if (c < pieces) {
-            const uint4* stage = q.ring + (step % kStages) * (kW * 32);
+        if (c < q.pieces) {
+            const uint4* stage = q.ring + (done % kStages) * (kW * 32);
 #pragma unroll
-            for (int h = 0; h < PIECE; h += 4) {
+            for (int h = 0; h < kPiece; h += 4) {
                 float av[MR][4];
 #pragma unroll
                 for (int i = 0; i < MR; ++i) {
-                    const float4 v = load4<TA>(arow[i] + c * PIECE + h);
+                    const float4 v = load4<TA>(arow[i] + c * kPiece + h);
                     av[i][0] = v.x; av[i][1] = v.y; av[i][2] = v.z; av[i][3] = v.w;
                 }
 #pragma unroll
@@ -277,75 +320,63 @@ __device__ __forceinline__ void grouped_rows_few(const GroupedArgs& p, const Row
                 }
             }
         }
-        load(step + kStages - 1);                     // into the stage read a step ago, by this lane alone
+        q.request();                                  // into the stage read a step ago, by this lane alone
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
-    for (int r = 0; r < kGrWarpRows; ++r) {
+    for (int i = 0; i < MR; ++i) {
+        if (i >= m_here) break;
+        const int out_row = __shfl_sync(0xffffffffu, row, m0 + i);
+        const float sc = p.scales ? p.scales[out_row] : 1.f;
+        float mine = 0.f;                             // lane r ends up with output row r
 #pragma unroll
-        for (int i = 0; i < MR; ++i) {
-            if (i < m_here && q.n_first + r < p.N) {
-                const int row = q.rows[m0 + i];
-                const float sc = p.scales ? p.scales[row] : 1.f;
-                float v = sc * warp_sum(acc[r][i]);
-                if (GATED) v = gated_value(v, sc * warp_sum(acc[GATED ? r + kGrWarpRows : 0][i]), p.act, p.act_limit);
-                else v = plain_value(v, p.out_act);
-                if (p.gate != nullptr) v *= 1.0f / (1.0f + expf(-__shfl_sync(0xffffffffu, gate_z, r * kGrFew + i)));
-                if (q.lane == 0) {
-                    const size_t o = static_cast<size_t>(row) * p.ldo + p.o_off + static_cast<size_t>(q.g) * p.o_gs + q.n_first + r;
-                    if (p.out_is_f32) static_cast<float*>(p.out)[o] = v;
-                    else static_cast<__nv_bfloat16*>(p.out)[o] = __float2bfloat16_rn(v);
-                }
-            }
+        for (int r = 0; r < kGrWarpRows; ++r) {
+            float v = sc * warp_sum(acc[r][i]);
+            if (GATED) v = gated_value(v, sc * warp_sum(acc[GATED ? r + kGrWarpRows : 0][i]), p.act, p.act_limit);
+            else v = plain_value(v, p.out_act);
+            if (p.gate != nullptr) v *= 1.0f / (1.0f + expf(-__shfl_sync(0xffffffffu, gate_z, r * kGrFew + i)));
+            if (q.lane == r) mine = v;
+        }
+        if (q.lane < kGrWarpRows && n_first + q.lane < p.N) {
+            const size_t o = static_cast<size_t>(out_row) * p.ldo + p.o_off + static_cast<size_t>(g) * p.o_gs + n_first + q.lane;
+            if (p.out_is_f32) static_cast<float*>(p.out)[o] = mine;
+            else static_cast<__nv_bfloat16*>(p.out)[o] = __float2bfloat16_rn(mine);
         }
     }
 }
 
+// tiles: how many there are (experts form: at most; the number is read on the device)
 template <typename TA, typename TW, bool GATED>
 __global__ void __launch_bounds__(kGrWarps * 32, 3)
-grouped_rows_kernel(const GroupedArgs p) {
+grouped_rows_kernel(const GroupedArgs p, int tiles) {
     extern __shared__ uint4 s_ring[];
-    __shared__ int s_row[kGpTM];
-    __shared__ int s_count;
     pdl_prologue();
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    int g;
-    if (p.tile_group) {
-        if (static_cast<int>(blockIdx.x) >= *p.n_tiles) return;
-        g = p.tile_group[blockIdx.x];
-    } else {
-        g = blockIdx.x % p.groups;
-    }
-    if (warp == 0) {             // the tile's rows, the empty places left out
-        int r = -1;
-        if (lane < kGpTM) {
-            if (p.tile_group) r = p.sorted_rows[blockIdx.x * kGpTM + lane];
-            else { r = (blockIdx.x / p.groups) * kGpTM + lane; if (r >= p.rows) r = -1; }
+    using Stream = RowsStream<TA, TW, GATED>;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    Stream q{p};
+    q.ring = s_ring + warp * (Stream::kStages * Stream::kW * 32) + lane;
+    q.lane = lane;
+    q.per_tile = (p.N + kGrWarpRows - 1) / kGrWarpRows;
+    q.units = (p.tile_group ? *p.n_tiles : tiles) * q.per_tile;
+    q.stride = gridDim.x * kGrWarps;
+    q.pieces = p.K / Stream::kPiece;
+    q.steps = (q.pieces + 31) / 32;
+    const int first = blockIdx.x * kGrWarps + warp;
+    q.unit = first;
+    q.seek();
+    for (int i = 0; i < Stream::kStages - 1; ++i) q.request();
+    int done = 0, x = -1, g = 0, row = -1, m_count = 0;
+    for (int unit = first; unit < q.units; unit += q.stride) {
+        if (unit / q.per_tile != x) { x = unit / q.per_tile; m_count = q.tile(x, g, row); }
+        const int n_first = unit % q.per_tile * kGrWarpRows;
+        for (int m0 = 0; m0 < m_count; m0 += kGrFew) {
+            const int m_here = min(kGrFew, m_count - m0);
+            if (m_here == 1) grouped_rows_unit<1>(q, g, row, n_first, m0, m_here, done);
+            else if (m_here == 2) grouped_rows_unit<2>(q, g, row, n_first, m0, m_here, done);
+            else if (m_here <= 4) grouped_rows_unit<4>(q, g, row, n_first, m0, m_here, done);
+            else grouped_rows_unit<8>(q, g, row, n_first, m0, m_here, done);
         }
-        const unsigned some = __ballot_sync(0xffffffffu, r >= 0);
-        if (r >= 0) s_row[__popc(some & ((1u << lane) - 1))] = r;
-        if (lane == 0) s_count = __popc(some);
     }
-    __syncthreads();
-    const int m_count = s_count;
-    constexpr int kW = GATED ? 2 * kGrWarpRows : kGrWarpRows;
-    constexpr int kStages = kGrSmem / (kGrWarps * kW * 512);
-    RowsWork<TA, TW> q;
-    q.n_first = blockIdx.y * kGrRows + warp * kGrWarpRows;
-    if (q.n_first >= p.N) return;
-    q.g = g; q.lane = lane; q.rows = s_row;
-    q.A = static_cast<const TA*>(p.a) + p.a_off + static_cast<size_t>(g) * p.a_gs;
-    q.ring = s_ring + warp * (kStages * kW * 32) + lane;
-    const TW* W = static_cast<const TW*>(p.w) + static_cast<size_t>(g) * p.w_gs;
-#pragma unroll
-    for (int r = 0; r < kGrWarpRows; ++r) q.wrow[r] = W + static_cast<size_t>(min(q.n_first + r, p.N - 1)) * p.ldw;
-    for (int m0 = 0; m0 < m_count; m0 += kGrFew) {
-        const int m_here = min(kGrFew, m_count - m0);
-        if (m_here == 1) grouped_rows_few<1, TA, TW, GATED>(p, q, m0, m_here);
-        else if (m_here == 2) grouped_rows_few<2, TA, TW, GATED>(p, q, m0, m_here);
-        else if (m_here <= 4) grouped_rows_few<4, TA, TW, GATED>(p, q, m0, m_here);
-        else grouped_rows_few<8, TA, TW, GATED>(p, q, m0, m_here);
-    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 // The heads form for many rows (prompt portions): tiles of 64 rows x 64 outputs, a thread 4 x 4 of them, so that two
@@ -616,7 +647,13 @@ template <typename TA, typename TW, bool GATED>
 static int launch_grouped_rows_as(const GroupedArgs& p, unsigned tiles, cudaStream_t st) {
     static const cudaError_t ready = cudaFuncSetAttribute(grouped_rows_kernel<TA, TW, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGrSmem);
     if (ready != cudaSuccess) { set_error("grouped_product (rows): %s", cudaGetErrorString(ready)); return 1; }
-    launch_kernel((grouped_rows_kernel<TA, TW, GATED>), dim3(tiles, (p.N + kGrRows - 1) / kGrRows), dim3(kGrWarps * 32), kGrSmem, st, p);
+    int sms = 0, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const long long blocks = (static_cast<long long>(tiles) * ((p.N + kGrWarpRows - 1) / kGrWarpRows) + kGrWarps - 1) / kGrWarps;
+    GI_REQUIRE(blocks * kGrWarps <= 2147483647LL - 3 * 1024 * kGrWarps, "grouped_product: too many tiles");
+    launch_kernel((grouped_rows_kernel<TA, TW, GATED>), dim3(static_cast<unsigned>(blocks < 3LL * sms ? blocks : 3LL * sms)), dim3(kGrWarps * 32), kGrSmem, st, p,
+                  static_cast<int>(tiles));
     return check_launch("grouped_product (rows)");
 }
 template <bool GATED>
