@@ -322,81 +322,88 @@ scan_link_kernel(const ScanArgs p) {
     slot[e] = S;
 }
 
-// o_t += A_t S_p^T q_t for the tokens of one part, one head and 32 columns: the start state's columns and 16 tokens'
-// queries (transposed) in shared memory, a warp per four tokens, a lane per column.
-template <int kDk>
+// o_t += A_t S_p^T q_t for 64 tokens of a part, one head and kDv columns (64 or 128): a small matrix product whose tiles lie in
+// registers. The queries (by channel) in shared memory, the start state's rows staged 16 at a time; a thread has 8 tokens x
+// kDv / 16 columns, a warp 16 tokens. (16 tokens x 32 columns a block, four sums a thread, read shared memory twice for
+// every four multiply-adds: 72 us at twelve parts of 16 heads of 128 x 128, of which the multiply-adds need 11.)
+constexpr int kApplyRows = 64, kApplyStep = 16;
+
+template <int kDk, int kDv>
 __global__ void __launch_bounds__(128)
-scan_apply_kernel(const ScanArgs p) {
+scan_apply_kernel(const ScanArgs p, int blocks_per_part) {            // grid (column blocks x token blocks of a part, H, requests x parts)
     pdl_prologue();
-    constexpr int kChunk = kDk > 128 ? kScanChunk / 2 : kScanChunk;
-    __shared__ float s_S[kDk][kScanCols];
-    __shared__ __align__(16) float s_qT[kDk][kChunk + 4];      // rows 80 bytes apart: fewer bank conflicts when a chunk is laid down
-    const int tile = blockIdx.x, h = blockIdx.y;
-    const int r = blockIdx.z / p.max_parts, part_idx = blockIdx.z % p.max_parts;
-    const int g = h / p.group;
+    constexpr int kT = kApplyRows + 4, kX = kDv + 4, kTN = kDv / 16, kPer = kApplyStep * kDv / 128;
+    extern __shared__ __align__(16) float apply_smem[];
+    float* s_q = apply_smem;                           // [kDk][kT]
+    float* s_x = s_q + kDk * kT;                       // [kApplyStep][kX]
+    const int h = blockIdx.y, g = h / p.group;
+    const int r = blockIdx.z / p.max_parts, part_idx = blockIdx.z % p.max_parts, t0 = blockIdx.x % blocks_per_part * kApplyRows;
     int n = p.seg_len[r], s0 = p.seg_start[r];
     if (part_idx * p.part_len >= n) return;
     s0 += part_idx * p.part_len;
     n = min(p.part_len, n - part_idx * p.part_len);
+    if (t0 >= n) return;
+    s0 += t0;
+    const int tid = threadIdx.x, rows = min(kApplyRows, n - t0), c0 = blockIdx.x / blocks_per_part * kDv;
+    const int tm = tid / 16 * 8, tn = tid % 16 * 4;    // this thread's tokens tm .. tm + 7; columns tn .. tn + 3 (and 64 further on)
+    const bool works = tid / 32 * 16 < rows;
     const float* S = p.ws_state + (static_cast<size_t>(parts_before(p, r) + part_idx) * p.H + h) * p.dk * p.dv;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int j = tile * kScanCols + lane;
-    for (int e = threadIdx.x; e < kDk * kScanCols; e += 128) {
-        const int i = e / kScanCols, jj = tile * kScanCols + e % kScanCols;
-        s_S[i][e % kScanCols] = (i < p.dk && jj < p.dv) ? S[static_cast<size_t>(i) * p.dv + jj] : 0.f;
-    }
-    // the queries of a chunk are requested while the chunk before it is worked on
-    constexpr int kPerThread = kChunk * kDk / 128;
-    float qv[kPerThread], cv[kPerThread];
-    auto request = [&](int c0) {
-        const int m = min(kChunk, n - c0);
+    float xv[kPer];
+    auto request = [&](int i0) {                       // asked for while the rows before them are worked on
 #pragma unroll
-        for (int u = 0; u < kPerThread; ++u) {
-            const int e = threadIdx.x + u * 128;
-            const int tt = e / kDk, i = e % kDk;
-            const bool in = tt < m && i < p.dk;
-            qv[u] = in ? p.q[static_cast<size_t>(s0 + c0 + tt) * p.ld_q + p.q_off + g * p.dk + i] : 0.f;
-            // per-row decays: the product since the part's start scales the query's own channel
-            cv[u] = (in && p.gate_raw) ? p.ws_decay[(static_cast<size_t>(s0 + c0 + tt) * p.H + h) * p.dk + i] : 1.f;
+        for (int u = 0; u < kPer; ++u) {
+            const int e = tid + u * 128, i = i0 + e / kDv, j = c0 + e % kDv;
+            xv[u] = (i < p.dk && j < p.dv) ? S[static_cast<size_t>(i) * p.dv + j] : 0.f;
         }
     };
     request(0);
-    for (int c0 = 0; c0 < n; c0 += kChunk) {
-        const int m = min(kChunk, n - c0);
-        __syncthreads();
-#pragma unroll
-        for (int u = 0; u < kPerThread; ++u) {
-            const int e = threadIdx.x + u * 128;
-            s_qT[e % kDk][e / kDk] = (p.act ? silu_f(qv[u]) : qv[u]) * p.q_scale * cv[u];
-        }
-        __syncthreads();
-        if (c0 + kChunk < n) request(c0 + kChunk);
-        // what the sums are added to, and the decays that scale them, are on their way meanwhile
-        float old[4], dec[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int tt = warp * 4 + u;
-            const bool in = tt < m && j < p.dv;
-            const size_t t = static_cast<size_t>(s0 + c0 + (in ? tt : 0));
-            old[u] = in ? p.out[t * p.H * p.dv + h * p.dv + j] : 0.f;
-            dec[u] = !in ? 0.f : p.gate_raw ? 1.f : p.ws_decay[t * p.H + h];
-        }
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};
-        if (warp * 4 < kChunk)
 #pragma unroll 8
-        for (int i = 0; i < kDk; ++i) {
-            const float sv = s_S[i][lane];
-            const float4 q4 = *reinterpret_cast<const float4*>(&s_qT[i][warp * 4]);
-            acc[0] = fmaf(q4.x, sv, acc[0]);
-            acc[1] = fmaf(q4.y, sv, acc[1]);
-            acc[2] = fmaf(q4.z, sv, acc[2]);
-            acc[3] = fmaf(q4.w, sv, acc[3]);
+    for (int e = tid; e < kApplyRows * kDk; e += 128) {
+        const int t = e / kDk, i = e % kDk;
+        float v = 0.f;
+        if (t < rows && i < p.dk) {
+            v = p.q[static_cast<size_t>(s0 + t) * p.ld_q + p.q_off + g * p.dk + i];
+            v = (p.act ? silu_f(v) : v) * p.q_scale;
+            // per-row decays: the product since the part's start scales the query's own channel
+            if (p.gate_raw) v *= p.ws_decay[(static_cast<size_t>(s0 + t) * p.H + h) * p.dk + i];
         }
+        s_q[i * kT + t] = v;
+    }
+    float acc[8][kTN];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int tt = warp * 4 + u;
-            if (tt < m && j < p.dv)
-                p.out[static_cast<size_t>(s0 + c0 + tt) * p.H * p.dv + h * p.dv + j] = fmaf(dec[u], acc[u], old[u]);
+    for (int m = 0; m < 8; ++m)
+#pragma unroll
+        for (int j = 0; j < kTN; ++j) acc[m][j] = 0.f;
+    for (int i0 = 0; i0 < p.dk; i0 += kApplyStep) {
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < kPer; ++u) { const int e = tid + u * 128; s_x[e / kDv * kX + e % kDv] = xv[u]; }
+        __syncthreads();
+        if (i0 + kApplyStep < p.dk) request(i0 + kApplyStep);
+        if (!works) continue;
+#pragma unroll
+        for (int i = 0; i < kApplyStep; ++i) {
+            float l[8], x[kTN];
+            *reinterpret_cast<float4*>(&l[0]) = *reinterpret_cast<const float4*>(s_q + (i0 + i) * kT + tm);
+            *reinterpret_cast<float4*>(&l[4]) = *reinterpret_cast<const float4*>(s_q + (i0 + i) * kT + tm + 4);
+#pragma unroll
+            for (int j = 0; j < kTN; j += 4) *reinterpret_cast<float4*>(&x[j]) = *reinterpret_cast<const float4*>(s_x + i * kX + tn + j * 16);
+#pragma unroll
+            for (int m = 0; m < 8; ++m)
+#pragma unroll
+                for (int j = 0; j < kTN; ++j) acc[m][j] = fmaf(l[m], x[j], acc[m][j]);
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+        if (tm + m >= rows) continue;
+        const size_t t = static_cast<size_t>(s0 + tm + m);
+        const float f = p.gate_raw ? 1.f : p.ws_decay[t * p.H + h];
+        float* o = p.out + t * p.H * p.dv + h * p.dv;
+#pragma unroll
+        for (int j = 0; j < kTN; ++j) {
+            const int col = c0 + tn + (j & 3) + (j & 4) * 16;
+            if (col < p.dv) o[col] = fmaf(f, acc[m][j], o[col]);
         }
     }
 }
@@ -556,6 +563,15 @@ static int gi_causal_conv_impl(const float* in, int ld, int in_off, const float*
     return check_launch("causal_conv");
 }
 
+template <int kDk, int kDv>
+static void launch_apply(const ScanArgs& a, int R, cudaStream_t st) {
+    constexpr int smem = (kDk * (kApplyRows + 4) + kApplyStep * (kDv + 4)) * 4;
+    static const cudaError_t ready = cudaFuncSetAttribute(scan_apply_kernel<kDk, kDv>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    (void)ready;                                      // a failure shows at the launch
+    const int blocks = (a.part_len + kApplyRows - 1) / kApplyRows;
+    launch_kernel((scan_apply_kernel<kDk, kDv>), dim3((a.dv + kDv - 1) / kDv * blocks, a.H, R * a.max_parts), dim3(128), smem, st, a, blocks);
+}
+
 template <int kDk, int kRT>
 static void launch_scan(const ScanArgs& a, int R, cudaStream_t st) {
     const unsigned tiles = (a.dv + kScanCols - 1) / kScanCols;
@@ -570,7 +586,8 @@ static void launch_scan(const ScanArgs& a, int R, cudaStream_t st) {
     else launch_kernel((linear_scan_kernel<kDk, kRT, true, false>), dim3(tiles, a.H, R * a.max_parts), dim3(kThreads), 0, st, a);
     const size_t elements = static_cast<size_t>(a.H) * a.dk * a.dv;
     launch_kernel((scan_link_kernel), dim3(static_cast<unsigned>((elements + 255) / 256), R), dim3(256), 0, st, a);
-    launch_kernel((scan_apply_kernel<kDk>), dim3(tiles, a.H, R * a.max_parts), dim3(128), 0, st, a);
+    if (a.dv <= 64) launch_apply<kDk, 64>(a, R, st);
+    else launch_apply<kDk, 128>(a, R, st);
 }
 
 // part_len 0: every segment is walked from the request's state by one block per head and column tile. Otherwise

@@ -186,6 +186,48 @@ def test_recurrence_with_a_decay_per_row(H, dk, dv):
         assert not state[:, :5].any() and not state[2].any()
 
 
+@pytest.mark.parametrize("stepped", [False, True])
+@pytest.mark.parametrize("H, group, dk, dv", [(4, 2, 16, 24), (2, 1, 48, 64), (3, 3, 128, 65), (2, 1, 100, 130)])
+def test_recurrence_cut_into_parts(H, group, dk, dv, stepped):
+    """Constant decays (one of them 0) and decays from step sizes: parts whose last one has a token, tokens around the 64 of an
+    output block, a segment of one token, against the walk in 64 bits and against the walk without parts."""
+    from geneinfer_b200.ops import kernels
+    g = torch.Generator().manual_seed(H * 100 + dk + stepped)
+    lens, G = [257, 1, 65, 17, 192], H // group
+    T = sum(lens)
+    ld = 2 * G * dk + H * dv + H + 1
+    x = torch.randn(T, ld, generator=g) * 0.5
+    decay = torch.tensor([0.9, 0.0, 0.999, 0.5][:H])
+    bias, a_log, skip = torch.randn(H, generator=g), torch.randn(H, generator=g) * 0.3, torch.randn(H, generator=g)
+    starts = np.cumsum([0] + lens)
+    s0 = torch.randn(len(lens), H, dk, dv, generator=g) * 0.1
+    q, k, v, dt = x[:, 1:].split([G * dk, G * dk, H * dv, H], 1)
+    act = (lambda z: z * torch.sigmoid(z)) if stepped else (lambda z: z)
+    q, k = (act(t.double()).view(T, G, dk).repeat_interleave(group, 1) for t in (q, k))
+    v = act(v.double()).view(T, H, dv)
+    step = pf.softplus(dt.double() + bias.double())
+    a = torch.exp(-torch.exp(a_log.double()) * step) if stepped else decay.double().expand(T, H)
+    want, ends = torch.empty(T, H, dv, dtype=F), []
+    for r in range(len(lens)):
+        S = s0[r].double()
+        for t in range(starts[r], starts[r + 1]):
+            S = a[t][:, None, None] * S + (step[t][:, None] * k[t] if stepped else k[t])[:, :, None] * v[t][:, None, :]
+            want[t] = torch.einsum("hkv,hk->hv", S, q[t] * 0.7) + skip.double()[:, None] * v[t]
+        ends.append(S)
+    ints = lambda z: torch.tensor(z, dtype=torch.int32, device=DEV)  # noqa: E731
+    xd, results = x.to(DEV), []
+    form = dict(dt=xd, dt_offset=1 + 2 * G * dk + H * dv, dt_bias=bias.to(DEV), a_log=a_log.to(DEV)) if stepped else dict(decay=decay.to(DEV))
+    for part in (128, 70, 0):
+        state = s0.reshape(len(lens), -1).to(DEV).clone()
+        out = torch.full((T, H * dv), float("nan"), device=DEV)
+        extra = {} if not part else {"part_len": part, "ws_state": torch.full((kernels.scan_parts(T, len(lens), part), H * dk * dv), float("nan"), device=DEV),
+                                     "ws_decay": torch.full((T, H), float("nan"), device=DEV)}
+        kernels.linear_scan(xd, 1, xd, 1 + G * dk, xd, 1 + 2 * G * dk, H, group, dk, dv, stepped, state, 0, ints(starts[:-1].tolist()), ints(lens),
+                            ints(list(range(len(lens)))), out, skip=skip.to(DEV), q_scale=0.7, **form, **extra)
+        _close(out.cpu(), want.reshape(T, -1), torch.float32, f"outputs, parts of {part}", f32=1e-5)
+        _close(state.cpu(), torch.stack(ends).reshape(len(lens), -1), torch.float32, f"states, parts of {part}", f32=1e-5)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("W, groups", [(96, 3), (70, 5), (256, 1)])
 def test_group_norm_with_a_silu_gate_after_it(dtype, W, groups):
