@@ -344,9 +344,14 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
 
 // ------------------------------------------------------------------------------------------ decode, fed by TMA
 // The same arithmetic as attention_decode_kernel per 256-key chunk, organised for bandwidth: one
-// persistent CTA per SM, whose four warps are independent. A warp takes whole chunks (work item =
-// request x key/value head x chunk, dealt round-robin), walks a chunk's tiles in order with the
+// persistent CTA per SM, whose warps are independent. A warp takes whole chunks (work item =
+// request x key/value head x chunk), walks a chunk's tiles in order with the
 // online softmax, and writes the chunk's partial result itself, so no warp ever waits for another.
+// With 16 requests or more every CTA takes an equal run of the items that some query sees, dealt to its warps in turn: an SM's share
+// of the bytes decides when it is done (its warps share one path to memory), and with requests of different lengths, or
+// windows, many (request, chunk) pairs of the rectangle n_rows x n_chunks are empty: 64 requests of 380 to 1,900 positions
+// 42.9 -> 36.2 us a layer of the 1B sizes, 23 requests beside a portion at the 3B sizes 37.8 -> 29.2. Finding the items costs what
+// a few requests seldom give back: a step of eight requests of one length is 0.4 % faster with the rectangle dealt out as it is.
 // Each warp owns a ring of three stages (K tile + V tile) filled by TMA: one lane issues one box
 // per page and head (pages [pages, Hkv, page_size, hd] are rows of a 2D tensor map), running up to
 // three tiles ahead, across chunk borders. Pages wholly outside a query's range are not fetched.
@@ -366,7 +371,7 @@ struct DecodeTma {
     static constexpr int kQBytes = 16 * HD * 2;
     static constexpr int kMetaRows = 512;          // requests whose (row, position, request) are staged in shared memory
     static constexpr int kBarBytes = 256;
-    static constexpr int kSmemBytes = kWarps * kStages * kStageBytes + kWarps * kQBytes + kBarBytes + 3 * kMetaRows * 4 + 1024;
+    static constexpr int kSmemBytes = kWarps * kStages * kStageBytes + kWarps * kQBytes + kBarBytes + 4 * kMetaRows * 4 + 1024;
 };
 
 __device__ __forceinline__ void att_mbar_init(uint32_t bar) { asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar)); }
@@ -406,7 +411,8 @@ struct DecodeItem {
 
 // WIDE: a group has more than 8 query heads (both row halves of the 16-row tile are worked on); a kernel of its own,
 // so that the usual one carries half as much code (short kernels pay for the instructions they fetch).
-template <int HD, bool WIDE>
+// COMPACT: see above; the other deals the whole rectangle, empty items among them.
+template <int HD, bool WIDE, bool COMPACT>
 __global__ void __launch_bounds__(DecodeTma<HD>::kThreads, 1)
 attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                             const __nv_bfloat16* __restrict__ q, const int* __restrict__ rows, int n_rows,
@@ -451,23 +457,63 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
         meta[2 * Cfg::kMetaRows + i] = row_req[t];
     }
     __syncthreads();
-
-    const int total = n_rows * Hkv * n_chunks;
-    const int stride = gridDim.x * Cfg::kWarps;
+    // ends[i]: the items that requests 0 .. i have; every warp adds them up for itself (the same values to the same places), which
+    // costs less than another barrier
+    int* ends = meta + 3 * Cfg::kMetaRows;
+    int first_item = 0, total = n_rows * Hkv * n_chunks, stride = gridDim.x * Cfg::kWarps;       // (total: the end of this CTA's items)
+    if constexpr (COMPACT) {
+        int all = 0;
+        for (int base = 0; base < n_rows; base += 32) {
+            int n = 0;
+            if (base + lane < n_rows) {
+                const int pos = meta[Cfg::kMetaRows + base + lane];
+                const int lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
+                n = (pos / kChunkKeys - lo / kChunkKeys + 1) * Hkv;
+            }
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, n, d);
+                if (lane >= d) n += up;
+            }
+            if (base + lane < n_rows) ends[base + lane] = all + n;
+            all += __shfl_sync(0xffffffffu, n, 31);
+        }
+        __syncwarp();
+        const int share = all / static_cast<int>(gridDim.x), odd = all % static_cast<int>(gridDim.x), cta = static_cast<int>(blockIdx.x);
+        first_item = cta * share + min(cta, odd) + warp;
+        total = cta * share + min(cta, odd) + share + (cta < odd ? 1 : 0);
+        stride = Cfg::kWarps;
+    } else {
+        // neighbouring items to a CTA's warps, and to each CTA only its share when there are fewer than warps
+        const int per_cta = total < stride ? (total + gridDim.x - 1) / gridDim.x : Cfg::kWarps;
+        first_item = warp < per_cta ? static_cast<int>(blockIdx.x) * per_cta + warp : total;
+    }
     const int box_rows = page_size < kTile ? page_size : kTile;
     const int boxes = kTile / box_rows;
 
     auto item_at = [&](int w, DecodeItem& it) {
-        it.chunk = w % n_chunks;
-        const int rest = w / n_chunks;
-        it.g = rest % Hkv;
-        it.idx = rest / Hkv;
+        if constexpr (COMPACT) {
+            it.idx = 0;
+            for (int base = 0; base < n_rows; base += 32) {
+                const unsigned past = __ballot_sync(0xffffffffu, base + lane >= n_rows || ends[base + lane] > w);
+                if (past) { it.idx = base + __ffs(past) - 1; break; }
+            }
+        } else {
+            it.chunk = w % n_chunks;
+            it.g = w / n_chunks % Hkv;
+            it.idx = w / n_chunks / Hkv;
+        }
         if (it.idx < Cfg::kMetaRows) {
             it.t = meta[it.idx]; it.pos = meta[Cfg::kMetaRows + it.idx]; it.req = meta[2 * Cfg::kMetaRows + it.idx];
         } else {
             it.t = rows[it.idx]; it.pos = positions[it.t]; it.req = row_req[it.t];
         }
         it.lo = (window > 0 && it.pos - window + 1 > 0) ? it.pos - window + 1 : 0;
+        if constexpr (COMPACT) {
+            const int rel = w - (it.idx > 0 ? ends[it.idx - 1] : 0), seen = it.pos / kChunkKeys - it.lo / kChunkKeys + 1;
+            it.g = rel / seen;
+            it.chunk = it.lo / kChunkKeys + rel % seen;
+        }
         it.c0 = it.chunk * kChunkKeys;
         it.visible = it.c0 <= it.pos && it.c0 + kChunkKeys > it.lo;
         it.tile0 = it.lo > it.c0 ? (it.lo - it.c0) / kTile : 0;
@@ -477,10 +523,6 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
 
     // ---- producer cursor: the next tile to request
     DecodeItem pi;
-    // A CTA's warps take neighbouring items (neighbouring chunks of one request lie next to each other
-    // in memory); when there are fewer items than warps, each CTA takes only its share so that all SMs work.
-    const int per_cta = total < static_cast<int>(gridDim.x) * Cfg::kWarps ? (total + gridDim.x - 1) / gridDim.x : Cfg::kWarps;
-    const int first_item = warp < per_cta ? static_cast<int>(blockIdx.x) * per_cta + warp : total;
     int pw = first_item, ptile = 0, n_issued = 0;
     int p_pages = 0;                           // lane i: the page of the chunk's i-th page-sized run of keys
     const int pages_per_chunk = kChunkKeys / page_size > 0 ? kChunkKeys / page_size : 1;
@@ -661,75 +703,139 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     if (lane == 0) timeline_record(kTlAttentionDecode, 6);
 }
 
-// grid (H, decode requests), four warps. Warp w sums the chunks first + w, first + w + 4, ... in
-// increasing order, each lane its own head dims, with every load requested before the first is
-// used; the four sums are then added in warp order. The order depends on the row's own chunks only.
+// Merges the chunks' partial results of one (token, query head): the chunks first + w, first + w + 4, ... make sum w, in
+// increasing order; the four sums are then added in the order of w. The order depends on the row's own chunks only.
+// kSpread (long contexts): a block of four warps per row, warp w takes sum w, with every load requested before the first is used.
+// Otherwise (up to eight chunks) a warp takes a whole row and a block four rows: a block per row, 2,048 of them at 64 requests of 32
+// heads, needed more than one round over the SMs of loads that wait for one another, 10.5 us.
 constexpr int kCombineWarps = 4;
-constexpr int kCombineMaxDims = 4;                 // head dims per lane: the head sizes of these kernels end at 128
+constexpr int kCombineFew = 8;                     // chunks up to which a warp takes a row alone
 
+// kVals: head dims per lane, neighbours (1 also for head sizes below 32).
+template <int kVals, bool kSpread>
 __global__ void __launch_bounds__(kCombineWarps * 32)
 attention_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                          const int* __restrict__ rows, const int* __restrict__ positions,
                          __nv_bfloat16* __restrict__ out, int H, int HD, int max_chunks, int window, int skip_single,
                          const AttEpilogue ep) {
-    __shared__ float s_acc[kCombineWarps][kCombineMaxDims * 32];
+    __shared__ float s_acc[kSpread ? kCombineWarps : 1][kVals * 32];
     __shared__ float s_l[kCombineWarps];
-    const int h = blockIdx.x, idx = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int h = kSpread ? blockIdx.x : blockIdx.x * kCombineWarps + warp, idx = blockIdx.y;
     const int t = rows[idx];
     const int pos = positions[t];
     const int lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
     const int first = lo / kChunkKeys, last = pos / kChunkKeys;
     pdl_prologue();
+    if (h >= H) return;
     if (skip_single && first == last) return;        // the attention kernel wrote this token's result itself
     const float* ml = part_ml + (static_cast<size_t>(idx) * H + h) * max_chunks * 2;
-    const float* po = part_o + (static_cast<size_t>(idx) * H + h) * max_chunks * HD;
-    float M = -INFINITY;
-    for (int c = first + lane; c <= last; c += 32) M = fmaxf(M, ml[c * 2]);
-    M = warp_max(M);
-    float acc[kCombineMaxDims];
+    const float* po = part_o + (static_cast<size_t>(idx) * H + h) * max_chunks * HD + lane * kVals;
+    const bool mine = lane * kVals < HD;
+    auto load = [&](int c, float (&v)[kVals]) {
 #pragma unroll
-    for (int i = 0; i < kCombineMaxDims; ++i) acc[i] = 0.f;
-    float L = 0.f;
+        for (int i = 0; i < kVals; ++i) v[i] = 0.f;
+        if (c > last || !mine) return;
+        const float* src = po + static_cast<size_t>(c) * HD;
+        if constexpr (kVals == 1) {
+            v[0] = *src;
+        } else {
+#pragma unroll
+            for (int i = 0; i < kVals; i += 2) *reinterpret_cast<float2*>(&v[i]) = *reinterpret_cast<const float2*>(src + i);
+        }
+    };
     constexpr int kBatch = 8;                       // chunks whose loads are in flight together
-    for (int c0 = first + warp; c0 <= last; c0 += kCombineWarps * kBatch) {
-        float v[kBatch][kCombineMaxDims], mc[kBatch], lc[kBatch];
+    float o[kVals], M = -INFINITY, total = 0.f;
 #pragma unroll
-        for (int j = 0; j < kBatch; ++j) {
-            const int c = c0 + j * kCombineWarps;
-            const bool in = c <= last;
-            mc[j] = in ? ml[c * 2] : -INFINITY;
-            lc[j] = in ? ml[c * 2 + 1] : 0.f;
+    for (int i = 0; i < kVals; ++i) o[i] = 0.f;
+    if constexpr (kSpread) {
+        for (int c = first + lane; c <= last; c += 32) M = fmaxf(M, ml[c * 2]);
+        M = warp_max(M);
+        float acc[kVals], L = 0.f;
 #pragma unroll
-            for (int i = 0; i < kCombineMaxDims; ++i) {
-                const int d = lane + 32 * i;
-                v[j][i] = (in && d < HD) ? po[static_cast<size_t>(c) * HD + d] : 0.f;
+        for (int i = 0; i < kVals; ++i) acc[i] = 0.f;
+        for (int c0 = first + warp; c0 <= last; c0 += kCombineWarps * kBatch) {
+            float v[kBatch][kVals], mc[kBatch], lc[kBatch];
+#pragma unroll
+            for (int j = 0; j < kBatch; ++j) {
+                const int c = c0 + j * kCombineWarps;
+                mc[j] = c <= last ? ml[c * 2] : -INFINITY;
+                lc[j] = c <= last ? ml[c * 2 + 1] : 0.f;
+                load(c, v[j]);
+            }
+#pragma unroll
+            for (int j = 0; j < kBatch; ++j) {
+                const float f = (mc[j] == -INFINITY) ? 0.f : exp2f(mc[j] - M);
+                L += lc[j] * f;
+#pragma unroll
+                for (int i = 0; i < kVals; ++i) acc[i] += v[j][i] * f;
             }
         }
 #pragma unroll
-        for (int j = 0; j < kBatch; ++j) {
-            const float f = (mc[j] == -INFINITY) ? 0.f : exp2f(mc[j] - M);
-            L += lc[j] * f;
+        for (int i = 0; i < kVals; ++i) s_acc[warp][lane * kVals + i] = acc[i];
+        if (lane == 0) s_l[warp] = L;
+        __syncthreads();
+        if (warp != 0) return;
 #pragma unroll
-            for (int i = 0; i < kCombineMaxDims; ++i) acc[i] += v[j][i] * f;
+        for (int w = 0; w < kCombineWarps; ++w) {
+            total += s_l[w];
+#pragma unroll
+            for (int i = 0; i < kVals; ++i) o[i] += s_acc[w][lane * kVals + i];
+        }
+    } else {
+        float v[kCombineFew][kVals], mc[kCombineFew], lc[kCombineFew];
+#pragma unroll
+        for (int j = 0; j < kCombineFew; ++j) {
+            const int c = first + j;
+            mc[j] = c <= last ? ml[c * 2] : -INFINITY;
+            lc[j] = c <= last ? ml[c * 2 + 1] : 0.f;
+            load(c, v[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < kCombineFew; ++j) M = fmaxf(M, mc[j]);
+#pragma unroll
+        for (int w = 0; w < kCombineWarps; ++w) {
+            float acc[kVals], L = 0.f;
+#pragma unroll
+            for (int i = 0; i < kVals; ++i) acc[i] = 0.f;
+#pragma unroll
+            for (int j = w; j < kCombineFew; j += kCombineWarps) {
+                const float f = (mc[j] == -INFINITY) ? 0.f : exp2f(mc[j] - M);
+                L += lc[j] * f;
+#pragma unroll
+                for (int i = 0; i < kVals; ++i) acc[i] += v[j][i] * f;
+            }
+            total += L;
+#pragma unroll
+            for (int i = 0; i < kVals; ++i) o[i] += acc[i];
         }
     }
-#pragma unroll
-    for (int i = 0; i < kCombineMaxDims; ++i) s_acc[warp][lane + 32 * i] = acc[i];
-    if (lane == 0) s_l[warp] = L;
-    __syncthreads();
-    float total = 0.f;
-#pragma unroll
-    for (int w = 0; w < kCombineWarps; ++w) total += s_l[w];
+    if (!mine) return;
     const float f = ep.plain() ? 0.f : att_finish(ep, total, M, t, h);
     const float* gz = att_gate_row(ep, t, h);
-    for (int d = threadIdx.x; d < HD; d += kCombineWarps * 32) {
-        float o = 0.f;
+    __nv_bfloat16* dst = out + (static_cast<size_t>(t) * H + h) * HD + lane * kVals;
 #pragma unroll
-        for (int w = 0; w < kCombineWarps; ++w) o += s_acc[w][d];
-        if (gz) o *= sigmoid_f(gz[d]);
-        out[(static_cast<size_t>(t) * H + h) * HD + d] = __float2bfloat16_rn(ep.plain() ? o / total : o * f);
+    for (int i = 0; i < kVals; ++i) {
+        if (gz) o[i] *= sigmoid_f(gz[lane * kVals + i]);
+        o[i] = ep.plain() ? o[i] / total : o[i] * f;
     }
+    if constexpr (kVals == 1) {
+        *dst = __float2bfloat16_rn(o[0]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < kVals; i += 2) *reinterpret_cast<__nv_bfloat162*>(dst + i) = __floats2bfloat162_rn(o[i], o[i + 1]);
+    }
+}
+
+template <int kVals>
+static void launch_combine_as(const float* part_o, const float* part_ml, const int* rows, const int* positions, __nv_bfloat16* out, int H,
+                              int HD, int max_chunks, int n_chunks, int n_rows, int window, int skip_single, const AttEpilogue& ep, cudaStream_t st) {
+    if (n_chunks <= kCombineFew)
+        launch_kernel((attention_combine_kernel<kVals, false>), dim3((H + kCombineWarps - 1) / kCombineWarps, n_rows), dim3(kCombineWarps * 32), 0, st,
+                      part_o, part_ml, rows, positions, out, H, HD, max_chunks, window, skip_single, ep);
+    else
+        launch_kernel((attention_combine_kernel<kVals, true>), dim3(H, n_rows), dim3(kCombineWarps * 32), 0, st,
+                      part_o, part_ml, rows, positions, out, H, HD, max_chunks, window, skip_single, ep);
 }
 
 // ------------------------------------------------------------------------------------------ prefill
@@ -1045,9 +1151,7 @@ static int launch_decode(const void* q, const void* kc, const void* vc, void* ou
         static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(kc), static_cast<const __nv_bfloat16*>(vc),
         rows, row_req, positions, tables, table_stride, H, Hkv, page_size, scale * kLog2e, window, part_o, part_ml, max_chunks);
     if (check_launch("attention_decode")) return 1;
-    dim3 grid2(H, n_rows);
-    launch_kernel((attention_combine_kernel), dim3(grid2), dim3(kCombineWarps * 32), 0, st, part_o, part_ml, rows, positions,
-                                                                   static_cast<__nv_bfloat16*>(out), H, HD, max_chunks, window, 0, ep);
+    launch_combine_as<(HD + 31) / 32>(part_o, part_ml, rows, positions, static_cast<__nv_bfloat16*>(out), H, HD, max_chunks, n_chunks, n_rows, window, 0, ep, st);
     return check_launch("attention_combine");
 }
 
@@ -1061,8 +1165,10 @@ static int launch_decode_tma(const void* q, const void* kc, const void* vc, void
     using Cfg = DecodeTma<HD>;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attention_decode_tma_kernel<HD, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_decode_tma_kernel<HD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+        cudaError_t e = cudaFuncSetAttribute(attention_decode_tma_kernel<HD, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_decode_tma_kernel<HD, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_decode_tma_kernel<HD, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_decode_tma_kernel<HD, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
         if (e != cudaSuccess) { set_error("attention_decode: %s", cudaGetErrorString(e)); return 1; }
         configured = true;
     }
@@ -1078,21 +1184,18 @@ static int launch_decode_tma(const void* q, const void* kc, const void* vc, void
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int items = n_rows * Hkv * n_chunks;
     int grid = items < sms ? items : sms;           // few items: fewer per CTA rather than fewer CTAs
-    if (H / Hkv > 8)
-        launch_kernel((attention_decode_tma_kernel<HD, true>), dim3(grid), dim3(Cfg::kThreads), Cfg::kSmemBytes, st, mk, mv,
+    const bool compact = n_rows >= 16 && n_rows <= Cfg::kMetaRows && items > grid;
+    auto launch = [&](auto kernel) {
+        launch_kernel(kernel, dim3(grid), dim3(Cfg::kThreads), Cfg::kSmemBytes, st, mk, mv,
                   static_cast<const __nv_bfloat16*>(q), rows, n_rows, row_req, positions, tables, table_stride, H, Hkv,
                   page_size, scale * kLog2e, window, part_o, part_ml, max_chunks, n_chunks, static_cast<__nv_bfloat16*>(out), status,
                   (g_stream_kv && n_rows <= 32) ? 1 : 0, ep);     // (evict-first) measured: 2 % faster at 8 requests, no gain at 64
-    else
-        launch_kernel((attention_decode_tma_kernel<HD, false>), dim3(grid), dim3(Cfg::kThreads), Cfg::kSmemBytes, st, mk, mv,
-                  static_cast<const __nv_bfloat16*>(q), rows, n_rows, row_req, positions, tables, table_stride, H, Hkv,
-                  page_size, scale * kLog2e, window, part_o, part_ml, max_chunks, n_chunks, static_cast<__nv_bfloat16*>(out), status,
-                  (g_stream_kv && n_rows <= 32) ? 1 : 0, ep);     // (evict-first) measured: 2 % faster at 8 requests, no gain at 64
+    };
+    if (H / Hkv > 8) { if (compact) launch(attention_decode_tma_kernel<HD, true, true>); else launch(attention_decode_tma_kernel<HD, true, false>); }
+    else { if (compact) launch(attention_decode_tma_kernel<HD, false, true>); else launch(attention_decode_tma_kernel<HD, false, false>); }
     if (check_launch("attention_decode_tma")) return 1;
     if (n_chunks == 1) return 0;                     // every token's keys lie in one chunk: nothing to merge
-    dim3 grid2(H, n_rows);
-    launch_kernel((attention_combine_kernel), dim3(grid2), dim3(kCombineWarps * 32), 0, st, part_o, part_ml, rows, positions,
-                  static_cast<__nv_bfloat16*>(out), H, HD, max_chunks, window, 1, ep);
+    launch_combine_as<(HD + 31) / 32>(part_o, part_ml, rows, positions, static_cast<__nv_bfloat16*>(out), H, HD, max_chunks, n_chunks, n_rows, window, 1, ep, st);
     return check_launch("attention_combine");
 }
 
