@@ -470,6 +470,16 @@ def test_attention_decode_contexts_of_one_chunk(H, Hkv, hd, ps, decode_chunks):
     close(got, want, "bfloat16", "attention of a short window", bf16_tol=1e-2)
 
 
+@pytest.mark.parametrize("window", [None, 300])
+@pytest.mark.parametrize("hd,requests", [(64, 33), (128, 70), (32, 513)])
+def test_attention_decode_of_many_lengths(hd, requests, window):
+    """Requests of one chunk to six beside each other, more than one round of a warp over them, and more than the
+    descriptors in shared memory hold."""
+    lens = [1 + (i * 397) % 1400 if requests < 100 or i % 50 == 0 else 1 + (i * 37) % 80 for i in range(requests)]
+    got, want = _attention_case("bfloat16", 4, 2, hd, 16, ctx_lens=lens, q_lens=[1] * requests, window=window, seed=31, fast=True)
+    close(got, want, "bfloat16", "attention of many lengths", bf16_tol=1e-2)
+
+
 @pytest.mark.parametrize("far", [0, 15, 16, 63, 64, 255, 256, 511, 597])
 @pytest.mark.parametrize("q_len", [1, 3])
 def test_attention_tensor_cores_far_key(far, q_len):
