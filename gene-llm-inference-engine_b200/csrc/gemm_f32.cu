@@ -55,7 +55,7 @@ struct F32Tile {
 };
 using Tile8 = F32Tile<8, 64, 8, 2, 32, 5, 4>;
 using Tile16 = F32Tile<16, 64, 8, 4, 32, 4, 4>;
-using Tile32 = F32Tile<32, 128, 8, 8, 32, 3, 3>;
+using Tile32 = F32Tile<32, 128, 8, 4, 32, 3, 3>;
 using Tile64 = F32Tile<64, 128, 8, 8, 32, 4, 2>;
 
 // grid (chunks, blocks of rows, blocks of columns), clusters of `chunks` along x. kc: length of a chunk.
