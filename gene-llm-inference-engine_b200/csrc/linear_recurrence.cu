@@ -66,6 +66,100 @@ conv_state_update_kernel(const float* __restrict__ in, int ld, int in_off, float
     for (int j = 0; j < keep; ++j) st[static_cast<size_t>(j) * C + c] = vals[j];
 }
 
+// The same for channels in whole fours whose rows are 16-byte aligned and 2 to 4 taps; the arithmetic of an output is the one
+// above. A thread has four channels.
+__device__ __forceinline__ void conv_tap(float4& acc, const float (&w)[16], int taps, int j, const float4& u) {
+    acc.x = fmaf(w[j], u.x, acc.x); acc.y = fmaf(w[taps + j], u.y, acc.y);
+    acc.z = fmaf(w[2 * taps + j], u.z, acc.z); acc.w = fmaf(w[3 * taps + j], u.w, acc.w);
+}
+template <int TAPS>
+__device__ __forceinline__ void conv_weights(float (&w)[16], float4& first, const float* weight, const float* bias, int c) {
+#pragma unroll
+    for (int j = 0; j < TAPS; ++j)          // 4 TAPS values in a row
+        *reinterpret_cast<float4*>(&w[4 * j]) = __ldg(reinterpret_cast<const float4*>(weight + static_cast<size_t>(c) * TAPS) + j);
+    first = bias ? __ldg(reinterpret_cast<const float4*>(bias + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+__device__ __forceinline__ void conv_store(float* out, float4 v, int act) {
+    if (act) { v.x = silu_f(v.x); v.y = silu_f(v.y); v.z = silu_f(v.z); v.w = silu_f(v.w); }
+    *reinterpret_cast<float4*>(out) = v;
+}
+
+// Long segments: RUN consecutive rows a thread, every row asked for once and all at once (a value at a time and once per tap,
+// 2,048 rows of 3,072 channels took 37 us; the bytes need 8).
+template <int TAPS, int RUN>
+__global__ void __launch_bounds__(128)
+causal_conv_run_kernel(const float* __restrict__ in, int ld, int in_off, const float* __restrict__ weight,
+                       const float* __restrict__ bias, const float* __restrict__ state, long long slot_stride,
+                       const int* __restrict__ row_req, const int* __restrict__ seg_start,
+                       const int* __restrict__ state_slots, float* __restrict__ out, int C, int T, int act) {
+    pdl_launch_dependents();
+    const int c = (blockIdx.x * 128 + threadIdx.x) * 4, t0 = blockIdx.y * RUN;
+    if (c >= C) return;
+    float w[16];
+    float4 first;
+    conv_weights<TAPS>(w, first, weight, bias, c);      // the weights belong to no earlier kernel
+    pdl_wait();
+    float4 u[RUN + TAPS - 1];                           // rows t0 - (TAPS - 1) .. t0 + RUN - 1
+#pragma unroll
+    for (int k = 0; k < RUN + TAPS - 1; ++k) {
+        const int t = t0 - (TAPS - 1) + k;
+        u[k] = (t >= 0 && t < T) ? *reinterpret_cast<const float4*>(in + static_cast<size_t>(t) * ld + in_off + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int k = 0; k < RUN; ++k) {
+        const int t = t0 + k;
+        if (t >= T) break;
+        const int r = row_req[t], rel = t - seg_start[r];
+        float4 acc = first;
+        if (rel >= TAPS - 1) {
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j) conv_tap(acc, w, TAPS, j, u[k + j]);
+        } else {
+            const float* st = state + static_cast<long long>(state_slots[r]) * slot_stride + c;
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j) {
+                const int back = TAPS - 1 - j;
+                conv_tap(acc, w, TAPS, j, back <= rel ? u[k + j] : *reinterpret_cast<const float4*>(st + static_cast<size_t>(TAPS - 1 + rel - back) * C));
+            }
+        }
+        conv_store(out + static_cast<size_t>(t) * C + c, acc, act);
+    }
+}
+
+// Segments of a token each (decoding): a thread walks through a whole segment and leaves the state behind it (one launch
+// less, and the state is read once).
+template <int TAPS>
+__global__ void __launch_bounds__(128)
+causal_conv_walk_kernel(const float* __restrict__ in, int ld, int in_off, const float* __restrict__ weight,
+                        const float* __restrict__ bias, float* __restrict__ state, long long slot_stride,
+                        const int* __restrict__ seg_start, const int* __restrict__ seg_len,
+                        const int* __restrict__ state_slots, float* __restrict__ out, int C, int act) {
+    pdl_launch_dependents();
+    const int c = (blockIdx.x * 128 + threadIdx.x) * 4, r = blockIdx.y;
+    if (c >= C) return;
+    float w[16];
+    float4 first;
+    conv_weights<TAPS>(w, first, weight, bias, c);
+    pdl_wait();
+    const int n = seg_len[r], s0 = seg_start[r];
+    if (n <= 0) return;
+    float* st = state + static_cast<long long>(state_slots[r]) * slot_stride + c;
+    float4 u[TAPS];
+#pragma unroll
+    for (int j = 0; j < TAPS - 1; ++j) u[j] = *reinterpret_cast<const float4*>(st + static_cast<size_t>(j) * C);
+    for (int t = s0; t < s0 + n; ++t) {
+        u[TAPS - 1] = *reinterpret_cast<const float4*>(in + static_cast<size_t>(t) * ld + in_off + c);
+        float4 acc = first;
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) conv_tap(acc, w, TAPS, j, u[j]);
+        conv_store(out + static_cast<size_t>(t) * C + c, acc, act);
+#pragma unroll
+        for (int j = 0; j < TAPS - 1; ++j) u[j] = u[j + 1];
+    }
+#pragma unroll
+    for (int j = 0; j < TAPS - 1; ++j) *reinterpret_cast<float4*>(st + static_cast<size_t>(j) * C) = u[j];
+}
+
 // ---------------------------------------------------------------------------------- the recurrence
 // A block owns 32 columns of one head's state of one request, each thread a few rows x 4 columns of it in registers.
 // Tokens are staged a chunk at a time in shared memory (activated, with their a and b).
@@ -554,8 +648,31 @@ static int gi_causal_conv_impl(const float* in, int ld, int in_off, const float*
     GI_REQUIRE(T <= 65535 && R <= 65535, "causal_conv: %d rows in one step exceed the grid limit 65535", T);
     GI_REQUIRE(in_off >= 0 && in_off + C <= ld, "causal_conv: the channels lie outside the input row of %d", ld);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const unsigned cb = (C + 255) / 256;
-    launch_kernel((causal_conv_kernel), dim3(cb, T), dim3(256), 0, st, in, ld, in_off, weight, bias,
+    const unsigned cb = (C + 255) / 256, cb4 = (C / 4 + 127) / 128;
+    auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+    const bool fours = C % 4 == 0 && ld % 4 == 0 && in_off % 4 == 0 && slot_stride % 4 == 0 && state_off % 4 == 0 && taps >= 2 && taps <= 4 &&
+                       aligned(in) && aligned(weight) && aligned(bias) && aligned(state) && aligned(out);
+    if (fours && T == R) {
+        auto walk = [&](auto kernel) {
+            launch_kernel(kernel, dim3(cb4, R), dim3(128), 0, st, in, ld, in_off, weight, bias, state + state_off, slot_stride, seg_start, seg_len, state_slots,
+                          out, C, act);
+        };
+        if (taps == 2) walk(causal_conv_walk_kernel<2>);
+        else if (taps == 3) walk(causal_conv_walk_kernel<3>);
+        else walk(causal_conv_walk_kernel<4>);
+        return check_launch("causal_conv");
+    }
+    if (fours) {
+        // runs of eight rows once they fill the SMs (four blocks of 128 threads each), else of two
+        const bool longer = static_cast<long long>(cb4) * ((T + 7) / 8) >= 148 * 4;
+        auto run = [&](auto kernel, int rows) {
+            launch_kernel(kernel, dim3(cb4, (T + rows - 1) / rows), dim3(128), 0, st, in, ld, in_off, weight, bias, static_cast<const float*>(state + state_off),
+                          slot_stride, row_req, seg_start, state_slots, out, C, T, act);
+        };
+        if (taps == 2) { if (longer) run(causal_conv_run_kernel<2, 8>, 8); else run(causal_conv_run_kernel<2, 2>, 2); }
+        else if (taps == 3) { if (longer) run(causal_conv_run_kernel<3, 8>, 8); else run(causal_conv_run_kernel<3, 2>, 2); }
+        else { if (longer) run(causal_conv_run_kernel<4, 8>, 8); else run(causal_conv_run_kernel<4, 2>, 2); }
+    } else launch_kernel((causal_conv_kernel), dim3(cb, T), dim3(256), 0, st, in, ld, in_off, weight, bias,
                   static_cast<const float*>(state + state_off), slot_stride, row_req, seg_start, state_slots, out, C, taps, T, act);
     if (taps > 1)
         launch_kernel((conv_state_update_kernel), dim3(cb, R), dim3(256), 0, st, in, ld, in_off, state + state_off, slot_stride,

@@ -835,7 +835,7 @@ def causal_conv(proj: torch.Tensor, offset: int, weight: torch.Tensor, bias: Opt
                                int(state_offset), _dev(row_req, "row_req", torch.int32), _dev(seg_start, "seg_start", torch.int32),
                                _dev(seg_len, "seg_len", torch.int32), _dev(state_slots, "state_slots", torch.int32),
                                _dev(out, "out", torch.float32), C, taps, T, R, int(bool(activate)), _stream()), "causal_conv")
-    if taps > 1:
+    if taps > 1 and T > R:                   # (a token per segment: one kernel does both)
         count_launches(1)
 
 

@@ -128,6 +128,41 @@ def test_convolution_without_bias_or_activation_and_its_state(taps):
     assert not state[:, :3].any() and not state[1].any()
 
 
+@pytest.mark.parametrize("bias", [False, True])
+@pytest.mark.parametrize("taps", [2, 3, 4])
+def test_convolution_of_channels_in_fours(taps, bias):
+    """Runs of eight rows and of two across the borders of segments shorter than the filter, walks over single tokens, and the
+    state between steps of either kind. Equal to the bit to the general form (the same channels one column further on)."""
+    from geneinfer_b200.ops import kernels
+    g = torch.Generator().manual_seed(taps)
+    C, total = 2056, [1500, 13, 700]
+    w, b = torch.randn(C, taps, generator=g), torch.randn(C, generator=g)
+    seqs = [torch.randn(n, C + 4, generator=g) for n in total]
+    ints = lambda z: torch.tensor(z, dtype=torch.int32, device=DEV)  # noqa: E731
+    results = []
+    for off in (4, 3):                       # off 3: rows that no 16-byte piece starts
+        state = torch.zeros(3, 4 + (taps - 1) * C, device=DEV)
+        got, at = [[] for _ in seqs], [0, 0, 0]
+        for lengths in ([1, 1, 2], [2, 3, 0], [17, 1, 40], [1, 1, 1], [1, 0, 1], [1478, 7, 656]):
+            live = [r for r, n in enumerate(lengths) if n]
+            rows = torch.cat([seqs[r][at[r]:at[r] + lengths[r]] for r in live]).to(DEV)
+            if off == 3:
+                rows = rows.roll(-1, 1).contiguous()
+            starts = np.cumsum([0] + [lengths[r] for r in live])
+            row_req = torch.cat([torch.full((lengths[r],), i) for i, r in enumerate(live)]).int().to(DEV)
+            out = torch.full((rows.shape[0], C), float("nan"), device=DEV)
+            kernels.causal_conv(rows, off, w.to(DEV), b.to(DEV) if bias else None, state, 4, row_req, ints(starts[:-1].tolist()),
+                                ints([lengths[r] for r in live]), ints(live), out, activate=bias)
+            for i, r in enumerate(live):
+                got[r].append(out[starts[i]:starts[i + 1]].cpu())
+                at[r] += lengths[r]
+        results.append([torch.cat(o) for o in got] + [state.cpu()])
+    for one, two in zip(*results):
+        assert torch.equal(one, two)
+    want = pf.short_conv(seqs[0][:, 4:].double(), w.double()) + (b.double() if bias else 0.0)
+    _close(results[0][0], want * torch.sigmoid(want) if bias else want, torch.float32, "convolution", f32=2e-6)
+
+
 def _plain_row_decay_scan(q, k, v, z, tau, S0=None):
     T, H, dk = q.shape
     dv = v.shape[2]
