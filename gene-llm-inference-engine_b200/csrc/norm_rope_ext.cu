@@ -21,6 +21,8 @@
 //                   neighbours or of the two halves) behind it
 //
 // All arithmetic is 32-bit; only stores round. A row's result depends on that row only.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace gi {
@@ -67,6 +69,84 @@ residual_norm_kernel(const float* __restrict__ acc_in, const float* __restrict__
         if (acc_out) acc_out[row + d] = alpha * v;
         if (xn_out) xn_out[row + d] = from_float<TOut>(v);
     }
+}
+
+template <typename T> __device__ __forceinline__ void store_four(T* p, float a, float b, float c, float d);
+template <> __device__ __forceinline__ void store_four<float>(float* p, float a, float b, float c, float d) {
+    *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
+}
+template <> __device__ __forceinline__ void store_four<__nv_bfloat16>(__nv_bfloat16* p, float a, float b, float c, float d) {
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(a, b), hi = __floats2bfloat162_rn(c, d);
+    uint2 raw;
+    raw.x = *reinterpret_cast<const uint32_t*>(&lo);
+    raw.y = *reinterpret_cast<const uint32_t*>(&hi);
+    *reinterpret_cast<uint2*>(p) = raw;
+}
+
+// residual_norm (kAdd false: x = w * unit(a), acc_out = alpha * x) and add_normed (kAdd: x += w * unit(a), acc_out = a if it
+// is to be cleared) for rows that the block holds in registers: at most 1024 PIECES values in 16-byte pieces (the host checks).
+// Everything that is read is asked for at once (the weights even before the wait: they belong to no earlier kernel), where
+// the general kernels go to memory a second time once the sum is known, a value at a time: add_normed of 2,048 values took
+// 7.5 us for eight rows and 13.6 us for 1,273, of which the bytes need 7.
+template <typename TOut, int PIECES, bool kAdd>
+__global__ void __launch_bounds__(256)
+normed_rows_kernel(const float* a_in, const float* __restrict__ weight, float* __restrict__ x, float* acc_out,
+                   TOut* __restrict__ xn_out, int D, float eps, float alpha) {
+    __shared__ float warp_part[8];
+    pdl_launch_dependents();
+    const int n4 = D / 4;
+    const size_t row = static_cast<size_t>(blockIdx.x) * D;
+    float4 w[PIECES], a[PIECES], old[PIECES];
+#pragma unroll
+    for (int k = 0; k < PIECES; ++k) {
+        const int i = threadIdx.x + k * 256;
+        w[k] = i < n4 ? __ldg(reinterpret_cast<const float4*>(weight) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    pdl_wait();
+#pragma unroll
+    for (int k = 0; k < PIECES; ++k) {
+        const int i = threadIdx.x + k * 256;
+        a[k] = old[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i < n4) a[k] = reinterpret_cast<const float4*>(a_in + row)[i];
+        if (kAdd && i < n4) old[k] = reinterpret_cast<const float4*>(x + row)[i];
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < PIECES; ++k) {
+        ss = fmaf(a[k].x, a[k].x, ss); ss = fmaf(a[k].y, a[k].y, ss);
+        ss = fmaf(a[k].z, a[k].z, ss); ss = fmaf(a[k].w, a[k].w, ss);
+    }
+    ss = warp_sum(ss);
+    if ((threadIdx.x & 31) == 0) warp_part[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    float total = 0.f;
+#pragma unroll
+    for (int v = 0; v < 8; ++v) total += warp_part[v];
+    const float scale = 1.0f / sqrtf(total / static_cast<float>(D) + eps);
+#pragma unroll
+    for (int k = 0; k < PIECES; ++k) {
+        const int i = threadIdx.x + k * 256;
+        if (i >= n4) continue;
+        float v[4] = {w[k].x * (scale * a[k].x), w[k].y * (scale * a[k].y), w[k].z * (scale * a[k].z), w[k].w * (scale * a[k].w)};
+        if (kAdd) { v[0] += old[k].x; v[1] += old[k].y; v[2] += old[k].z; v[3] += old[k].w; }
+        store_four<float>(x + row + 4 * i, v[0], v[1], v[2], v[3]);
+        if (acc_out) {
+            if (kAdd) store_four<float>(acc_out + row + 4 * i, 0.f, 0.f, 0.f, 0.f);
+            else store_four<float>(acc_out + row + 4 * i, alpha * v[0], alpha * v[1], alpha * v[2], alpha * v[3]);
+        }
+        if (xn_out) store_four<TOut>(xn_out + row + 4 * i, v[0], v[1], v[2], v[3]);
+    }
+}
+
+// Launches it where the rows fit; false where they do not.
+template <typename TOut, bool kAdd>
+static bool launch_normed_rows(const float* a_in, const float* weight, float* x, float* acc_out, TOut* xn_out, int rows, int D, float eps,
+                               float alpha, cudaStream_t st) {
+    auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+    if (D % 4 != 0 || D > 4096 || !aligned(a_in) || !aligned(weight) || !aligned(x) || !aligned(acc_out) || !aligned(xn_out)) return false;
+    if (D <= 2048) launch_kernel((normed_rows_kernel<TOut, 2, kAdd>), dim3(rows), dim3(256), 0, st, a_in, weight, x, acc_out, xn_out, D, eps, alpha);
+    else launch_kernel((normed_rows_kernel<TOut, 4, kAdd>), dim3(rows), dim3(256), 0, st, a_in, weight, x, acc_out, xn_out, D, eps, alpha);
+    return true;
 }
 
 template <typename TOut>
@@ -116,13 +196,15 @@ gated_act4_kernel(const float* __restrict__ gu, const float* __restrict__ bias, 
 constexpr int kNrsWarps = 4;
 constexpr int kNrsMaxHead = 256;
 
-// A warp per head (query heads first, then key heads), a lane per pair of dimensions: both members of a rotation
+// A warp per head (query heads, key heads, then value heads), a lane per pair of dimensions: both members of a rotation
 // pair are the lane's own, the head's sum of squares is one warp reduction, nothing goes through shared memory but
-// the token's sines and cosines, which all heads of the block share. Many rows: a block per token; few rows (decoding):
-// a block per token and four heads. Head sizes up to 256 (four pairs a lane), even.
+// the token's sines and cosines, which all heads of the block share. Many rows: a block per token, a warp asking for
+// four heads' values at once (two of up to 128 dimensions, one beyond: as many registers); one head after the other, each
+// waiting for its own, 2,048 rows of 48 heads of 64 took 43 us, three times what their bytes need. Few rows (decoding):
+// a block per token and four heads. Head sizes up to 256 (kPairs: 1, 2 or 4 pairs a lane), even.
 constexpr int kNrsPairs = kNrsMaxHead / 64;
 
-template <typename T>
+template <typename T, int kPairs>
 __global__ void __launch_bounds__(kNrsWarps * 32)
 norm_rope_store_kernel(const float* __restrict__ in, int ld, int q_off, int k_off, int v_off, const float* __restrict__ bias,
                        const float* __restrict__ q_norm, const float* __restrict__ k_norm, float eps,
@@ -166,68 +248,88 @@ norm_rope_store_kernel(const float* __restrict__ in, int ld, int q_off, int k_of
         kv_base = (static_cast<size_t>(page) * Hkv * page_size + (pos % page_size)) * hd;
         v_base = (static_cast<size_t>(page) * Hkv * page_size + (pos % page_size)) * vd;
     }
-    const int n_heads = H + (write_kv ? Hkv : 0);
-    const int n_pairs = hd / 2;
-    for (int head = blockIdx.y * kNrsWarps + warp; head < n_heads; head += kNrsWarps * gridDim.y) {
-        const bool is_q = head < H;
-        const int col = is_q ? q_off + head * hd : k_off + (head - H) * hd;
-        const float* src = row + col;
-        const float* sbias = bias ? bias + col : nullptr;
-        const float* nw = is_q ? q_norm : k_norm;
-        if (nw && wide) nw += (is_q ? head : head - H) * hd;
-        float va[kNrsPairs], vb[kNrsPairs];
-        int ia[kNrsPairs], ib[kNrsPairs];
-        float ss = 0.f;
-#pragma unroll
-        for (int u = 0; u < kNrsPairs; ++u) {
-            const int pr = lane + 32 * u;
-            // pair pr: a rotation pair while pr < half, else two neighbouring dimensions behind the rotated ones
-            if (interleaved || pr >= half) {
-                const int base = interleaved ? 2 * pr : 2 * half + 2 * (pr - half);
-                ia[u] = base; ib[u] = base + 1;
+    // values that fit the lanes' pairs are items like the heads (nothing is done to them); others are copied with their key head
+    const bool plain_values = vd % 2 == 0 && vd <= 64 * kPairs;
+    const int n_heads = H + (write_kv ? Hkv : 0), n_items = n_heads + (write_kv && plain_values ? Hkv : 0);
+    constexpr int kBatch = kNrsPairs / kPairs;
+    const int step = kNrsWarps * gridDim.y;
+    for (int first = blockIdx.y * kNrsWarps + warp; first < n_items; first += step * kBatch) {
+        float va[kBatch][kPairs], vb[kBatch][kPairs];
+        // dimensions of pair pr: a rotation pair while pr < half, else two neighbouring dimensions behind the rotated ones
+        auto dims = [&](int pr, bool value, int& ia, int& ib) {
+            if (value || interleaved || pr >= half) {
+                ia = 2 * pr; ib = ia + 1;              // (2 * half + 2 * (pr - half))
             } else {
-                ia[u] = pr; ib[u] = pr + half;
+                ia = pr; ib = pr + half;
             }
-            const bool in_head = pr < n_pairs;
-            va[u] = in_head ? src[ia[u]] : 0.f;
-            vb[u] = in_head ? src[ib[u]] : 0.f;
-            if (sbias && in_head) { va[u] += sbias[ia[u]]; vb[u] += sbias[ib[u]]; }
-            ss = fmaf(va[u], va[u], ss);
-            ss = fmaf(vb[u], vb[u], ss);
-        }
-        T* dst = is_q ? q_out + (static_cast<size_t>(t) * H + head) * hd
-                      : k_cache + kv_base + static_cast<size_t>(head - H) * page_size * hd;
-        if (!is_q) {
-            // the values: copied from their columns as they are (the keys themselves where the design says so)
-            const int vcol = v_off + (head - H) * vd;
-            const float* vsrc = row + vcol;
-            const float* vbias = bias ? bias + vcol : nullptr;
-            T* vdst = v_cache + v_base + static_cast<size_t>(head - H) * page_size * vd;
-            for (int d = lane; d < vd; d += 32) vdst[d] = from_float<T>(vbias ? vsrc[d] + vbias[d] : vsrc[d]);
-        }
-        if (nw) {
-            ss = warp_sum(ss);
-            const float scale = wide ? wide_scale[is_q ? 0 : 1] : 1.0f / sqrtf(ss / static_cast<float>(hd) + eps);
+        };
 #pragma unroll
-            for (int u = 0; u < kNrsPairs; ++u) {
-                if (lane + 32 * u < n_pairs) {
-                    va[u] = nw[ia[u]] * (scale * va[u]);
-                    vb[u] = nw[ib[u]] * (scale * vb[u]);
+        for (int b = 0; b < kBatch; ++b) {
+            const int head = first + b * step;
+            const bool value = head >= n_heads;
+            const int col = head < H ? q_off + head * hd : !value ? k_off + (head - H) * hd : v_off + (head - n_heads) * vd;
+            const int n_pairs = head < n_items ? (value ? vd : hd) / 2 : 0;
+#pragma unroll
+            for (int u = 0; u < kPairs; ++u) {
+                const int pr = lane + 32 * u;
+                int ia, ib;
+                dims(pr, value, ia, ib);
+                va[b][u] = vb[b][u] = 0.f;
+                if (pr < n_pairs) {
+                    va[b][u] = row[col + ia];
+                    vb[b][u] = row[col + ib];
+                    if (bias) { va[b][u] += bias[col + ia]; vb[b][u] += bias[col + ib]; }
                 }
             }
         }
 #pragma unroll
-        for (int u = 0; u < kNrsPairs; ++u) {
-            const int pr = lane + 32 * u;
-            if (pr >= n_pairs) continue;
-            float a = va[u], b = vb[u];
-            if (pr < half) {
-                const float sn = s_sin[pr], cs = s_cos[pr];
-                const float ra = a * cs - b * sn, rb = b * cs + a * sn;
-                a = ra; b = rb;
+        for (int b = 0; b < kBatch; ++b) {
+            const int head = first + b * step;
+            if (head >= n_items) break;
+            const bool is_q = head < H, value = head >= n_heads;
+            const int n_pairs = (value ? vd : hd) / 2;
+            const float* nw = is_q ? q_norm : k_norm;
+            if (value) nw = nullptr;
+            if (nw && wide) nw += (is_q ? head : head - H) * hd;
+            T* dst = is_q ? q_out + (static_cast<size_t>(t) * H + head) * hd
+                          : !value ? k_cache + kv_base + static_cast<size_t>(head - H) * page_size * hd
+                                   : v_cache + v_base + static_cast<size_t>(head - n_heads) * page_size * vd;
+            if (!is_q && !plain_values) {
+                // the values: copied from their columns as they are (the keys themselves where the design says so)
+                const int vcol = v_off + (head - H) * vd;
+                T* vdst = v_cache + v_base + static_cast<size_t>(head - H) * page_size * vd;
+                for (int d = lane; d < vd; d += 32) vdst[d] = from_float<T>(bias ? row[vcol + d] + bias[vcol + d] : row[vcol + d]);
             }
-            dst[ia[u]] = from_float<T>(a);
-            dst[ib[u]] = from_float<T>(b);
+            float scale = 1.f;
+            if (nw) {
+                float ss = 0.f;
+#pragma unroll
+                for (int u = 0; u < kPairs; ++u) {
+                    ss = fmaf(va[b][u], va[b][u], ss);
+                    ss = fmaf(vb[b][u], vb[b][u], ss);
+                }
+                ss = warp_sum(ss);
+                scale = wide ? wide_scale[is_q ? 0 : 1] : 1.0f / sqrtf(ss / static_cast<float>(hd) + eps);
+            }
+#pragma unroll
+            for (int u = 0; u < kPairs; ++u) {
+                const int pr = lane + 32 * u;
+                if (pr >= n_pairs) continue;
+                int ia, ib;
+                dims(pr, value, ia, ib);
+                float a = va[b][u], c = vb[b][u];
+                if (nw) {
+                    a = nw[ia] * (scale * a);
+                    c = nw[ib] * (scale * c);
+                }
+                if (pr < half && !value) {
+                    const float sn = s_sin[pr], cs = s_cos[pr];
+                    const float ra = a * cs - c * sn, rc = c * cs + a * sn;
+                    a = ra; c = rc;
+                }
+                dst[ia] = from_float<T>(a);
+                dst[ib] = from_float<T>(c);
+            }
         }
     }
 }
@@ -251,9 +353,11 @@ add_normed_kernel(float* __restrict__ y, const float* __restrict__ weight, float
     }
 }
 
-// One block per token. The two latents are normed by the block (sums in the order of block_sum_256); the rotated part
-// is a pair per thread.
-template <typename T>
+// One block per token. The two latents are normed by the block; the rotated part
+// is a pair per thread. kKeep > 0: latents of at most 256 kKeep values, which the threads hold in registers: everything is asked for
+// at once and both sums go through one exchange (one after the other, and read again for the scaling, a row of
+// 768 + 512 + 32 values took 9.0 us for eight tokens and 15.7 for 1,273). 0: any size.
+template <typename T, int kKeep>
 __global__ void __launch_bounds__(256)
 latent_store_kernel(const float* __restrict__ in, int ld, int q_off, int q_rank, const float* __restrict__ q_weight,
                     T* __restrict__ q_latent, int c_off, int rank, const float* __restrict__ c_weight, int r_off, int rot,
@@ -261,24 +365,34 @@ latent_store_kernel(const float* __restrict__ in, int ld, int q_off, int q_rank,
                     const int* __restrict__ row_req, const int* __restrict__ block_tables, int table_stride,
                     T* __restrict__ cache, int page_size, int write_cache) {
     pdl_prologue();
-    __shared__ float warp_part[8];
+    __shared__ float warp_part[2][8];
     const int t = blockIdx.x;
     const float* row = in + static_cast<size_t>(t) * ld;
-    if (q_latent) {
-        float ss = 0.f;
-        for (int d = threadIdx.x; d < q_rank; d += 256) ss = fmaf(row[q_off + d], row[q_off + d], ss);
-        const float scale = 1.0f / sqrtf(block_sum_256(ss, warp_part) / static_cast<float>(q_rank) + eps);
-        for (int d = threadIdx.x; d < q_rank; d += 256)
-            q_latent[static_cast<size_t>(t) * q_rank + d] = from_float<T>(q_weight[d] * (scale * row[q_off + d]));
+    int pos = 0, page = 0;
+    if (write_cache) {
+        pos = positions[t];
+        page = block_tables[static_cast<size_t>(row_req[t]) * table_stride + pos / page_size];
     }
-    if (!write_cache) return;
-    const int pos = positions[t];
-    const int page = block_tables[static_cast<size_t>(row_req[t]) * table_stride + pos / page_size];
+    if (!q_latent) q_rank = 0;
+    if (!write_cache) rank = rot = 0;
+    constexpr int kHeld = kKeep > 0 ? kKeep : 1;
+    float qv[kHeld], cv[kHeld], qw[kHeld], cw[kHeld], sq = 0.f, sc = 0.f;
+    if constexpr (kKeep > 0) {
+#pragma unroll
+        for (int u = 0; u < kKeep; ++u) {
+            const int d = threadIdx.x + u * 256;
+            qv[u] = d < q_rank ? row[q_off + d] : 0.f;
+            cv[u] = d < rank ? row[c_off + d] : 0.f;
+            qw[u] = d < q_rank ? q_weight[d] : 0.f;
+            cw[u] = d < rank ? c_weight[d] : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < kKeep; ++u) { sq = fmaf(qv[u], qv[u], sq); sc = fmaf(cv[u], cv[u], sc); }
+    } else {
+        for (int d = threadIdx.x; d < q_rank; d += 256) sq = fmaf(row[q_off + d], row[q_off + d], sq);
+        for (int d = threadIdx.x; d < rank; d += 256) sc = fmaf(row[c_off + d], row[c_off + d], sc);
+    }
     T* dst = cache + (static_cast<size_t>(page) * page_size + (pos % page_size)) * (rank + rot);
-    float ss = 0.f;
-    for (int d = threadIdx.x; d < rank; d += 256) ss = fmaf(row[c_off + d], row[c_off + d], ss);
-    const float scale = 1.0f / sqrtf(block_sum_256(ss, warp_part) / static_cast<float>(rank) + eps);
-    for (int d = threadIdx.x; d < rank; d += 256) dst[d] = from_float<T>(c_weight[d] * (scale * row[c_off + d]));
     for (int pr = threadIdx.x; pr < rot / 2; pr += 256) {
         float sn, cs;
         sincosf(static_cast<float>(pos) * freq[pr], &sn, &cs);
@@ -287,6 +401,26 @@ latent_store_kernel(const float* __restrict__ in, int ld, int q_off, int q_rank,
         const float u = row[r_off + iu], v = row[r_off + iv];
         dst[rank + iu] = from_float<T>(u * cs - v * sn);
         dst[rank + iv] = from_float<T>(v * cs + u * sn);
+    }
+    sq = warp_sum(sq);
+    sc = warp_sum(sc);
+    if ((threadIdx.x & 31) == 0) { warp_part[0][threadIdx.x >> 5] = sq; warp_part[1][threadIdx.x >> 5] = sc; }
+    __syncthreads();
+    sq = sc = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) { sq += warp_part[0][w]; sc += warp_part[1][w]; }
+    const float q_scale = 1.0f / sqrtf(sq / static_cast<float>(q_rank) + eps), c_scale = 1.0f / sqrtf(sc / static_cast<float>(rank) + eps);
+    if constexpr (kKeep > 0) {
+#pragma unroll
+        for (int u = 0; u < kKeep; ++u) {
+            const int d = threadIdx.x + u * 256;
+            if (d < q_rank) q_latent[static_cast<size_t>(t) * q_rank + d] = from_float<T>(qw[u] * (q_scale * qv[u]));
+            if (d < rank) dst[d] = from_float<T>(cw[u] * (c_scale * cv[u]));
+        }
+    } else {
+        for (int d = threadIdx.x; d < q_rank; d += 256)
+            q_latent[static_cast<size_t>(t) * q_rank + d] = from_float<T>(q_weight[d] * (q_scale * row[q_off + d]));
+        for (int d = threadIdx.x; d < rank; d += 256) dst[d] = from_float<T>(c_weight[d] * (c_scale * row[c_off + d]));
     }
 }
 
@@ -311,6 +445,9 @@ static int gi_residual_norm_impl(const float* acc_in, const float* weight, float
     if (rows == 0) return 0;
     GI_REQUIRE(rows > 0 && D > 0, "residual_norm: sizes must be positive (rows=%d, D=%d)", rows, D);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (xn_dtype == kBF16 ? launch_normed_rows<__nv_bfloat16, false>(acc_in, weight, x_out, acc_out, static_cast<__nv_bfloat16*>(xn_out), rows, D, eps, alpha, st)
+                          : launch_normed_rows<float, false>(acc_in, weight, x_out, acc_out, static_cast<float*>(xn_out), rows, D, eps, alpha, st))
+        return check_launch("residual_norm");
     if (xn_dtype == kBF16)
         launch_kernel((residual_norm_kernel<__nv_bfloat16>), dim3(rows), dim3(256), 0, st, acc_in, weight, x_out, acc_out,
                       static_cast<__nv_bfloat16*>(xn_out), D, eps, alpha);
@@ -360,19 +497,21 @@ static int gi_norm_rope_store_impl(const float* in, int ld, int q_off, int k_off
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     GI_REQUIRE(T <= 2147483647, "norm_rope_store: too many rows");
     // few rows (decoding): the heads of a token are spread over blocks; many rows: a block per token
-    const unsigned head_blocks = T >= 256 ? 1u : static_cast<unsigned>(std::min((H + Hkv + kNrsWarps - 1) / kNrsWarps, 65535));
-    if (dtype == kF32)
-        launch_kernel((norm_rope_store_kernel<float>), dim3(T, head_blocks), dim3(kNrsWarps * 32), 0, st, in, ld, q_off, k_off, v_off, bias, q_norm,
-                      k_norm, eps, freq, rot_half, interleaved, positions, row_req, block_tables, table_stride,
-                      static_cast<float*>(q_out), static_cast<float*>(k_cache), static_cast<float*>(v_cache), H, Hkv, hd,
-                      vd, page_size, write_kv, wide);
-    else if (dtype == kBF16)
-        launch_kernel((norm_rope_store_kernel<__nv_bfloat16>), dim3(T, head_blocks), dim3(kNrsWarps * 32), 0, st, in, ld, q_off, k_off, v_off, bias,
-                      q_norm, k_norm, eps, freq, rot_half, interleaved, positions, row_req, block_tables, table_stride,
-                      static_cast<__nv_bfloat16*>(q_out), static_cast<__nv_bfloat16*>(k_cache),
-                      static_cast<__nv_bfloat16*>(v_cache), H, Hkv, hd, vd, page_size, write_kv, wide);
-    else
-        GI_REQUIRE(false, "norm_rope_store: unsupported dtype code %d", dtype);
+    const unsigned head_blocks = T >= 256 ? 1u : static_cast<unsigned>(std::min((H + 2 * Hkv + kNrsWarps - 1) / kNrsWarps, 65535));
+    auto launch = [&](auto zero, auto pairs) {
+        using T_ = decltype(zero);
+        launch_kernel((norm_rope_store_kernel<T_, decltype(pairs)::value>), dim3(T, head_blocks), dim3(kNrsWarps * 32), 0, st, in, ld, q_off, k_off, v_off,
+                      bias, q_norm, k_norm, eps, freq, rot_half, interleaved, positions, row_req, block_tables, table_stride, static_cast<T_*>(q_out),
+                      static_cast<T_*>(k_cache), static_cast<T_*>(v_cache), H, Hkv, hd, vd, page_size, write_kv, wide);
+    };
+    auto launch_as = [&](auto zero) {
+        if (hd <= 64) launch(zero, std::integral_constant<int, 1>{});
+        else if (hd <= 128) launch(zero, std::integral_constant<int, 2>{});
+        else launch(zero, std::integral_constant<int, 4>{});
+    };
+    if (dtype == kF32) launch_as(0.f);
+    else if (dtype == kBF16) launch_as(__nv_bfloat16());
+    else GI_REQUIRE(false, "norm_rope_store: unsupported dtype code %d", dtype);
     return check_launch("norm_rope_store");
 }
 
@@ -397,6 +536,10 @@ static int gi_add_normed_impl(float* y, const float* weight, float* x, void* xn_
     if (rows == 0) return 0;
     GI_REQUIRE(rows > 0 && D > 0, "add_normed: sizes must be positive (rows=%d, D=%d)", rows, D);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    float* cleared = clear_y ? y : nullptr;
+    if (xn_dtype == kBF16 ? launch_normed_rows<__nv_bfloat16, true>(y, weight, x, cleared, static_cast<__nv_bfloat16*>(xn_out), rows, D, eps, 1.f, st)
+                          : launch_normed_rows<float, true>(y, weight, x, cleared, static_cast<float*>(xn_out), rows, D, eps, 1.f, st))
+        return check_launch("add_normed");
     if (xn_dtype == kBF16)
         launch_kernel((add_normed_kernel<__nv_bfloat16>), dim3(rows), dim3(256), 0, st, y, weight, x, static_cast<__nv_bfloat16*>(xn_out), D, eps, clear_y);
     else
@@ -414,16 +557,21 @@ static int gi_latent_store_impl(const float* in, int ld, int q_off, int q_rank, 
     GI_REQUIRE(c_off >= 0 && c_off + rank <= ld && r_off >= 0 && r_off + rot <= ld, "latent_store: the key/value latent lies outside the row of %d", ld);
     GI_REQUIRE(rot == 0 || freq, "latent_store: the rotated part needs frequencies");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (dtype == kF32)
-        launch_kernel((latent_store_kernel<float>), dim3(T), dim3(256), 0, st, in, ld, q_off, q_rank, q_weight, static_cast<float*>(q_latent),
-                      c_off, rank, c_weight, r_off, rot, freq, amplitude, interleaved, eps, positions, row_req, block_tables, table_stride,
-                      static_cast<float*>(cache), page_size, write_cache);
-    else if (dtype == kBF16)
-        launch_kernel((latent_store_kernel<__nv_bfloat16>), dim3(T), dim3(256), 0, st, in, ld, q_off, q_rank, q_weight,
-                      static_cast<__nv_bfloat16*>(q_latent), c_off, rank, c_weight, r_off, rot, freq, amplitude, interleaved, eps, positions, row_req,
-                      block_tables, table_stride, static_cast<__nv_bfloat16*>(cache), page_size, write_cache);
-    else
-        GI_REQUIRE(false, "latent_store: unsupported dtype code %d", dtype);
+    auto launch = [&](auto zero, auto keep) {
+        using T_ = decltype(zero);
+        launch_kernel((latent_store_kernel<T_, decltype(keep)::value>), dim3(T), dim3(256), 0, st, in, ld, q_off, q_rank, q_weight,
+                      static_cast<T_*>(q_latent), c_off, rank, c_weight, r_off, rot, freq, amplitude, interleaved, eps, positions, row_req, block_tables,
+                      table_stride, static_cast<T_*>(cache), page_size, write_cache);
+    };
+    auto launch_as = [&](auto zero) {
+        const int most = std::max(q_latent ? q_rank : 0, rank);
+        if (most <= 1024) launch(zero, std::integral_constant<int, 4>{});
+        else if (most <= 2048) launch(zero, std::integral_constant<int, 8>{});
+        else launch(zero, std::integral_constant<int, 0>{});
+    };
+    if (dtype == kF32) launch_as(0.f);
+    else if (dtype == kBF16) launch_as(__nv_bfloat16());
+    else GI_REQUIRE(false, "latent_store: unsupported dtype code %d", dtype);
     return check_launch("latent_store");
 }
 

@@ -303,6 +303,41 @@ def test_norm_over_the_whole_projection_then_partial_rotation_in_halves(H, Hkv, 
     _close(vals, proj[:, (H + Hkv) * hd:].view(T, Hkv, vd), torch.float32, "values in their pages", f32=1e-7)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("hd, vd, wide", [(64, 64, True), (64, 65, False), (128, 130, False), (40, 48, True), (200, 256, False), (256, 30, True)])
+def test_heads_of_many_rows_and_of_few(hd, vd, wide, dtype):
+    """A block per row with several heads a warp at once (256 rows on) against a warp per head (fewer rows): the same bits, for
+    values that are items of their own and for those that are copied beside their keys."""
+    from geneinfer_b200.ops import kernels
+    g = torch.Generator().manual_seed(hd + vd)
+    T, H, G, page = 259, 5, 3, 16
+    ld = (H + G) * hd + G * vd
+    proj, bias = (torch.randn(T, ld, generator=g) * 2).to(DEV), torch.randn(ld, generator=g).to(DEV)
+    qw, kw = torch.randn(H * hd if wide else hd, generator=g).to(DEV), torch.randn(G * hd if wide else hd, generator=g).to(DEV)
+    freq, pos = torch.rand(hd // 4, generator=g).to(DEV), torch.arange(T, dtype=torch.int32, device=DEV)
+    tables = torch.randperm(17, generator=g).to(torch.int32)[None].to(DEV)
+    results = []
+    for rows in (T, 100):
+        q = torch.full((T, H * hd), float("nan"), dtype=dtype, device=DEV)
+        kc, vc = (torch.full((17, G, page, d), float("nan"), dtype=dtype, device=DEV) for d in (hd, vd))
+        for at in range(0, T, rows):
+            n = min(rows, T - at)
+            kernels.norm_rope_store(proj[at:at + n].contiguous(), 0, H * hd, (H + G) * hd, qw, kw, EPS, freq, False, pos[at:at + n].contiguous(),
+                                    torch.zeros(n, dtype=torch.int32, device=DEV), tables, q[at:at + n], kc, vc, H, G, hd, page, value_dim=vd,
+                                    wide_norm=wide, bias=bias)
+        results.append((q.cpu(), kc.cpu(), vc.cpu()))
+    for one, two in zip(*results):
+        assert torch.equal(one.nan_to_num(7.0), two.nan_to_num(7.0))
+    want = (proj + bias)[:, (H + G) * hd:].view(T, G, vd).to(dtype).cpu()
+    order = tables[0].tolist()
+    assert torch.equal(torch.stack([results[0][2][order[t // page], :, t % page] for t in range(T)]), want)
+    pq = (proj + bias)[:, :H * hd].double().cpu()
+    pq = (pf.norm_plain(pq, qw.cpu(), EPS).view(T, H, hd) if wide else pf.norm_plain(pq.view(T, H, hd), qw.cpu(), EPS))
+    # the angles are 32-bit products of positions up to 258: about 258 * 2^-24 off
+    pq = pf.rotate_half_layout(pq, freq.double().cpu(), 2 * (hd // 4))
+    _close(results[0][0].float().view(T, H, hd), pq, dtype, "queries", f32=5e-5, b16=1e-2)
+
+
 def test_wavelength_scaling_of_the_rotation_frequencies():
     from geneinfer_b200.parts import POSITION_ENCODINGS
     rot = {"base": 250.0, "dims": 32, "scaling": {"factor": 4.0, "low": 1.0, "high": 4.0, "original": 64}}

@@ -70,6 +70,54 @@ def test_add_normed(dtype):
         kernels.add_normed(y.to(DEV), w.to(DEV), xd, 1e-3)            # neither cast nor cleared
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("D", [4, 1028, 2048, 2052, 4096, 4100])
+def test_norms_on_the_output_and_after_the_sum_of_wide_rows(D, dtype):
+    """Rows held in registers up to 2,048 and up to 4,096 values, and wider ones."""
+    from geneinfer_b200.ops import kernels
+    g = torch.Generator().manual_seed(D)
+    x, y, w = torch.randn(9, D, generator=g) * 3, torch.randn(9, D, generator=g), 1 + 0.1 * torch.randn(D, generator=g)
+    xd, yd, xn = x.to(DEV), y.to(DEV), torch.empty(9, D, dtype=dtype, device=DEV)
+    kernels.add_normed(yd, w.to(DEV), xd, 1e-3, xn_out=xn, clear_y=True)
+    want = x.double() + pg.rms_norm(y.double(), w.double(), 1e-3)
+    assert float((xd.cpu() - want).abs().max()) < 2e-6 * float(want.abs().max())
+    assert torch.equal(xn.cpu().float(), xd.cpu().to(dtype).float()) and not yd.any()
+    again, kept = x.to(DEV), y.to(DEV)
+    kernels.add_normed(kept, w.to(DEV), again, 1e-3)              # neither cast nor cleared
+    assert torch.equal(again, xd) and torch.equal(kept.cpu(), y)
+    acc, out = y.to(DEV), torch.empty(9, D, device=DEV)
+    kernels.residual_norm(acc, w.to(DEV), out, 1e-3, 1.7, acc_out=acc, xn_out=xn)
+    want = pg.rms_norm(y.double(), w.double(), 1e-3)
+    assert float((out.cpu() - want).abs().max()) < 2e-6 * float(want.abs().max())
+    assert torch.equal(acc.cpu(), 1.7 * out.cpu()) and torch.equal(xn.cpu().float(), out.cpu().to(dtype).float())
+
+
+@pytest.mark.parametrize("q_rank, rank", [(768, 512), (1025, 1300), (2049, 64), (30, 2500)])
+def test_latents_of_every_size_into_their_pages(q_rank, rank):
+    from geneinfer_b200.ops import kernels
+    g = torch.Generator().manual_seed(rank)
+    T, page, rot = 9, 4, 24
+    proj = torch.randn(T, q_rank + rank + rot + 3, generator=g) * 2
+    qw, cw, freq = torch.randn(q_rank, generator=g), torch.randn(rank, generator=g), torch.rand(rot // 2, generator=g)
+    tables, pos = torch.tensor([[2, 0, 1]], dtype=torch.int32, device=DEV), torch.arange(T, dtype=torch.int32, device=DEV)
+    req = torch.zeros(T, dtype=torch.int32, device=DEV)
+    outs = []
+    for with_q, with_cache in ((True, True), (True, False), (False, True)):
+        q = torch.full((T, q_rank), float("nan"), device=DEV)
+        cache = torch.full((3, 1, page, rank + rot), float("nan"), device=DEV)
+        kernels.latent_store(proj.to(DEV), 3, qw.to(DEV) if with_q else None, q if with_q else None, 3 + q_rank, cw.to(DEV), 3 + q_rank + rank,
+                             freq.to(DEV), 1.3, 1e-3, pos, req, tables, cache, page, write_cache=with_cache)
+        outs.append((q.cpu(), torch.stack([cache[[2, 0, 1][t // page], 0, t % page].cpu() for t in range(T)])))
+    assert torch.equal(outs[1][0], outs[0][0]) and torch.equal(outs[2][1], outs[0][1])
+    assert torch.isnan(outs[2][0]).all() and torch.isnan(outs[1][1]).all()
+    _close(outs[0][0], pg.rms_norm(proj[:, 3:3 + q_rank].double(), qw.double(), 1e-3), torch.float32, "query latent", f32=3e-6)
+    _close(outs[0][1][:, :rank], pg.rms_norm(proj[:, 3 + q_rank:3 + q_rank + rank].double(), cw.double(), 1e-3), torch.float32, "latent", f32=3e-6)
+    u, v = proj[:, 3 + q_rank + rank:].double().view(T, rot // 2, 2).unbind(2)
+    angle = torch.arange(T).double()[:, None] * freq.double()
+    want = 1.3 * torch.stack((u * angle.cos() - v * angle.sin(), v * angle.cos() + u * angle.sin()), 2).view(T, rot)
+    _close(outs[0][1][:, rank:], want, torch.float32, "rotated part", f32=5e-6)
+
+
 def _paged(rows, dtype, page_size, seed):
     """Lays rows [n, Hkv, d] of one request into scattered pages; returns (pages [P, Hkv, page, d], table [1, stride])."""
     n, Hkv, d = rows.shape
