@@ -27,6 +27,8 @@
 // an output element is one chain of multiply-adds in the order of k over its own row, whichever tile the row landed in;
 // in the few-row form it is the sum of a warp's lanes' chains by a fixed tree. (Many rows through the experts' matrices
 // in bfloat16 run on the tensor cores: gi_gemm_tc_grouped.)
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace gi {
@@ -447,83 +449,164 @@ head_product64_kernel(const GroupedArgs p) {
 
 // ------------------------------------------------------------------------------------------------ routing
 constexpr int kRouteMaxExperts = 1024;
-constexpr int kRouteThreads = 256;
+constexpr int kRouteManyTokens = 4;            // tokens of a block where there are many
 
-template <typename TX>
-__global__ void __launch_bounds__(kRouteThreads)
+// Where the pairs go: tiles of tile_rows rows per expert, in the order of the experts.
+struct RouteAlign {
+    const int* ids; int n_pairs, E;
+    int* sorted_rows; int* tile_group; int* n_tiles; int max_tiles, tile_rows; int* pair_row;
+};
+// One block: counts per expert, then tiles per expert in expert order. `empty`: the places hold -1 already.
+__device__ __forceinline__ void route_align_block(const RouteAlign& p, int* s_count, int* s_start, bool empty) {
+    const int tid = threadIdx.x, threads = blockDim.x;
+    for (int e = tid; e < p.E; e += threads) s_count[e] = 0;
+    if (!empty) for (int i = tid; i < p.max_tiles * p.tile_rows; i += threads) p.sorted_rows[i] = -1;
+    __syncthreads();
+    for (int i = tid; i < p.n_pairs; i += threads) atomicAdd(&s_count[p.ids[i]], 1);
+    __syncthreads();
+    if (tid == 0) {
+        int tiles = 0;
+        for (int e = 0; e < p.E; ++e) {
+            s_start[e] = tiles * p.tile_rows;
+            const int n = (s_count[e] + p.tile_rows - 1) / p.tile_rows;
+            for (int i = 0; i < n; ++i) p.tile_group[tiles + i] = e;
+            tiles += n;
+        }
+        *p.n_tiles = tiles;
+    }
+    __syncthreads();
+    // a pair takes the next free row of its expert (which row does not matter: an output element is computed from
+    // its own row alone, in the same order of operations in every row of a tile)
+    for (int i = tid; i < p.n_pairs; i += threads) {
+        const int row = atomicAdd(&s_start[p.ids[i]], 1);
+        p.sorted_rows[row] = i;
+        if (p.pair_row) p.pair_row[i] = row;
+    }
+}
+__global__ void __launch_bounds__(1024)
+route_align_kernel(const RouteAlign p) {
+    pdl_prologue();
+    __shared__ int s_count[kRouteMaxExperts], s_start[kRouteMaxExperts];
+    route_align_block(p, s_count, s_start, false);
+}
+
+// A warp per expert (and one for the gate). A step of few tokens waits for the router's weights, 8 KB a row of 2,048: with few
+// tokens there are as many warps as rows, and a warp's first 1,024 weights are asked for before the wait for the kernel ahead
+// (they belong to no earlier kernel). With eight loads in flight and a ninth row in a second round two tokens took 17 us.
+// FUSED (up to eight tokens): the tokens' blocks are one cluster, whose first block also buckets the pairs once all are there (a
+// launch less on the way from the router to the experts' weights). TOK: tokens of a block; many tokens share what is
+// read of the weights (1,273 tokens read them from L2 for 15.5 us, a token a block).
+template <typename TX, bool FUSED, int TOK>
+__global__ void __launch_bounds__(1024)
 route_kernel(const TX* __restrict__ x, int D, const float* __restrict__ w, const float* __restrict__ correction, int E, int top,
              int softmax, int renormalise, float factor, int* __restrict__ ids, float* __restrict__ weights,
-             const float* __restrict__ gate_w, float* __restrict__ gate_out) {
-    pdl_prologue();
-    extern __shared__ float s_x[];                 // [D]
-    __shared__ float s_score[kRouteMaxExperts], s_choice[kRouteMaxExperts];
-    const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int d = threadIdx.x; d < D; d += kRouteThreads) s_x[d] = to_float(x[static_cast<size_t>(t) * D + d]);
+             const float* __restrict__ gate_w, float* __restrict__ gate_out, int T, const RouteAlign align) {
+    pdl_launch_dependents();
+    extern __shared__ float s_x[];                 // [TOK][D], then the scores and the choice scores [TOK][E]
+    float* all_scores = s_x + TOK * D;
+    float* all_choices = all_scores + TOK * E;
+    constexpr int kBatch = TOK == 1 ? 32 : 16;     // weights a lane has in flight
+    const int t0 = blockIdx.x * TOK, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x / 32;
+    const int n_rows = E + (gate_w ? 1 : 0);
+    float v[kBatch];
+    auto request = [&](int e, int d0) {
+        const float* row = (e < E ? w + static_cast<size_t>(e) * D : gate_w) + d0 + lane;
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) v[i] = d0 + lane + 32 * i < D ? row[32 * i] : 0.f;
+    };
+    if (warp < n_rows) request(warp, 0);
+    pdl_wait();
+    if (FUSED) {
+        if (t0 == 0)                                   // the places of the pairs, while the weights are on their way
+            for (int i = threadIdx.x; i < align.max_tiles * align.tile_rows; i += blockDim.x) align.sorted_rows[i] = -1;
+        if (t0 >= T) {                                 // a cluster has a power of two of blocks
+            cooperative_groups::this_cluster().sync();
+            return;
+        }
+    }
+    const int here = min(TOK, T - t0);
+    for (int d = threadIdx.x; d < here * D; d += blockDim.x) s_x[d] = to_float(x[static_cast<size_t>(t0) * D + d]);
+    if (TOK > 1) for (int d = here * D + threadIdx.x; d < TOK * D; d += blockDim.x) s_x[d] = 0.f;
     __syncthreads();
-    for (int e = warp; e < E + (gate_w ? 1 : 0); e += kRouteThreads / 32) {
-        const float* row = e < E ? w + static_cast<size_t>(e) * D : gate_w;
-        float z = 0.f;
-        int d = lane;
-        for (; d + 7 * 32 < D; d += 8 * 32) {            // eight loads in flight, one chain of multiply-adds
-            float v[8];
+    for (int e = warp; e < n_rows; e += warps) {
+        float z[TOK];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = row[d + 32 * i];
+        for (int k = 0; k < TOK; ++k) z[k] = 0.f;
+        for (int d0 = 0; d0 < D; d0 += 32 * kBatch) {
+            if (e != warp || d0 > 0) request(e, d0);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) z = fmaf(v[i], s_x[d + 32 * i], z);
+            for (int i = 0; i < kBatch; ++i) {
+                const int d = d0 + lane + 32 * i;
+                if (d < D) {
+#pragma unroll
+                    for (int k = 0; k < TOK; ++k) z[k] = fmaf(v[i], s_x[k * D + d], z[k]);
+                }
+            }
         }
-        for (; d < D; d += 32) z = fmaf(row[d], s_x[d], z);
-        z = warp_sum(z);
-        if (e == E) {
-            if (lane == 0) gate_out[t] = sigmoid_f(z);
-        } else if (lane == 0) {
-            const float s = softmax ? z : 1.0f / (1.0f + expf(-z));
-            s_score[e] = s;
-            s_choice[e] = s + (correction ? correction[e] : 0.f);
+#pragma unroll
+        for (int k = 0; k < TOK; ++k) {
+            const float sum = warp_sum(z[k]);
+            if (lane != 0 || k >= here) continue;
+            if (e == E) {
+                gate_out[t0 + k] = sigmoid_f(sum);
+            } else {
+                const float s = softmax ? sum : 1.0f / (1.0f + expf(-sum));
+                all_scores[k * E + e] = s;
+                all_choices[k * E + e] = s + (correction ? correction[e] : 0.f);
+            }
         }
     }
     __syncthreads();
-    if (warp != 0) return;
-    if (softmax) {
-        float m = -INFINITY;
-        for (int e = lane; e < E; e += 32) m = fmaxf(m, s_score[e]);
-        m = warp_max(m);
-        float sum = 0.f;
-        for (int e = lane; e < E; e += 32) sum += expf(s_score[e] - m);
-        const float inv = 1.0f / warp_sum(sum);
-        for (int e = lane; e < E; e += 32) {
-            const float s = expf(s_score[e] - m) * inv;
-            s_score[e] = s;
-            s_choice[e] = s + (correction ? correction[e] : 0.f);
+    if (warp < here) {
+        const int t = t0 + warp;
+        float* s_score = all_scores + warp * E;
+        float* s_choice = all_choices + warp * E;
+        if (softmax) {
+            float m = -INFINITY;
+            for (int e = lane; e < E; e += 32) m = fmaxf(m, s_score[e]);
+            m = warp_max(m);
+            float sum = 0.f;
+            for (int e = lane; e < E; e += 32) sum += expf(s_score[e] - m);
+            const float inv = 1.0f / warp_sum(sum);
+            for (int e = lane; e < E; e += 32) {
+                const float s = expf(s_score[e] - m) * inv;
+                s_score[e] = s;
+                s_choice[e] = s + (correction ? correction[e] : 0.f);
+            }
+            __syncwarp();
         }
-        __syncwarp();
-    }
-    float chosen = 0.f;
-    // the ``top`` largest choice scores, the lowest index among equals; a chosen expert leaves the contest
-    for (int k = 0; k < top; ++k) {
-        float best = -INFINITY;
-        int best_e = 0x7fffffff;
-        for (int e = lane; e < E; e += 32) {
-            const float c = s_choice[e];
-            if (c > best) { best = c; best_e = e; }
-        }
+        float chosen = 0.f;
+        // the ``top`` largest choice scores, the lowest index among equals; a chosen expert leaves the contest
+        for (int k = 0; k < top; ++k) {
+            float best = -INFINITY;
+            int best_e = 0x7fffffff;
+            for (int e = lane; e < E; e += 32) {
+                const float c = s_choice[e];
+                if (c > best) { best = c; best_e = e; }
+            }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oe = __shfl_xor_sync(0xffffffffu, best_e, o);
-            if (ob > best || (ob == best && oe < best_e)) { best = ob; best_e = oe; }
+            for (int o = 16; o > 0; o >>= 1) {
+                const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+                const int oe = __shfl_xor_sync(0xffffffffu, best_e, o);
+                if (ob > best || (ob == best && oe < best_e)) { best = ob; best_e = oe; }
+            }
+            if (best_e >= E) best_e = 0;                 // no comparable score (a row of NaN): any expert, but a real one
+            chosen += s_score[best_e];
+            if (lane == 0) {
+                ids[static_cast<size_t>(t) * top + k] = best_e;
+                weights[static_cast<size_t>(t) * top + k] = s_score[best_e] * factor;
+                s_choice[best_e] = -INFINITY;
+            }
+            __syncwarp();
         }
-        if (best_e >= E) best_e = 0;                 // no comparable score (a row of NaN): any expert, but a real one
-        chosen += s_score[best_e];
-        if (lane == 0) {
-            ids[static_cast<size_t>(t) * top + k] = best_e;
-            weights[static_cast<size_t>(t) * top + k] = s_score[best_e] * factor;
-            s_choice[best_e] = -INFINITY;
+        if (renormalise) {
+            const float inv = 1.0f / (chosen + 1e-20f);
+            for (int k = lane; k < top; k += 32) weights[static_cast<size_t>(t) * top + k] *= inv;
         }
-        __syncwarp();
     }
-    if (renormalise) {
-        const float inv = 1.0f / (chosen + 1e-20f);
-        for (int k = lane; k < top; k += 32) weights[static_cast<size_t>(t) * top + k] *= inv;
+    if (FUSED) {
+        cooperative_groups::this_cluster().sync();     // every token's experts are in memory
+        if (t0 == 0) route_align_block(align, reinterpret_cast<int*>(all_scores), reinterpret_cast<int*>(all_choices), true);
     }
 }
 
@@ -542,38 +625,6 @@ route_table_kernel(const int* __restrict__ tokens, const int* __restrict__ feedb
     e = e < 0 ? 0 : (e >= E ? E - 1 : e);                  // the table is checked when the model is built
     ids[i] = e;
     weights[i] = 1.0f / static_cast<float>(top);
-}
-
-// One block: counts per expert, then tiles of 16 rows per expert in expert order.
-__global__ void __launch_bounds__(1024)
-route_align_kernel(const int* __restrict__ ids, int n_pairs, int E, int* __restrict__ sorted_rows, int* __restrict__ tile_group,
-                   int* __restrict__ n_tiles, int max_tiles, int tile_rows, int* __restrict__ pair_row) {
-    pdl_prologue();
-    __shared__ int s_count[kRouteMaxExperts], s_start[kRouteMaxExperts];
-    const int tid = threadIdx.x;
-    for (int e = tid; e < E; e += 1024) s_count[e] = 0;
-    for (int i = tid; i < max_tiles * tile_rows; i += 1024) sorted_rows[i] = -1;
-    __syncthreads();
-    for (int i = tid; i < n_pairs; i += 1024) atomicAdd(&s_count[ids[i]], 1);
-    __syncthreads();
-    if (tid == 0) {
-        int tiles = 0;
-        for (int e = 0; e < E; ++e) {
-            s_start[e] = tiles * tile_rows;
-            const int n = (s_count[e] + tile_rows - 1) / tile_rows;
-            for (int i = 0; i < n; ++i) tile_group[tiles + i] = e;
-            tiles += n;
-        }
-        *n_tiles = tiles;
-    }
-    __syncthreads();
-    // a pair takes the next free row of its expert (which row does not matter: an output element is computed from
-    // its own row alone, in the same order of operations in every row of a tile)
-    for (int i = tid; i < n_pairs; i += 1024) {
-        const int row = atomicAdd(&s_start[ids[i]], 1);
-        sorted_rows[row] = i;
-        if (pair_row) pair_row[i] = row;
-    }
 }
 
 template <typename T>
@@ -750,18 +801,49 @@ static int gi_route_impl(const void* x, int x_dtype, int T, int D, const float* 
     GI_REQUIRE(tile_rows > 0, "route: tiles must have rows");
     GI_REQUIRE(max_tiles >= (pairs + tile_rows - 1) / tile_rows + std::min<long long>(E, pairs) - 1, "route: room for %d tiles is too little", max_tiles);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const size_t smem = static_cast<size_t>(D) * 4;
+    const int rows = E + (gate_w ? 1 : 0);
+    const int threads = T <= 64 ? std::min(1024, 32 * std::max(8, rows)) : 256;
+    const RouteAlign align{ids, static_cast<int>(pairs), E, sorted_rows, tile_group, n_tiles, max_tiles, tile_rows, pair_row};
+    // a cluster of up to eight blocks is portable; the places are few there (tiles of 128 rows belong to many tokens)
+    const bool fused = T <= 8 && tile_rows == kGpTM;
+    const size_t per_token = (static_cast<size_t>(D) + 2 * static_cast<size_t>(E)) * 4;
+    const bool many = T > 64 && kRouteManyTokens * per_token <= 96 * 1024;
+    auto launch = [&](auto kernel, auto* values) {
+        const size_t smem = per_token * (many ? kRouteManyTokens : 1);
+        if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        int blocks = many ? (T + kRouteManyTokens - 1) / kRouteManyTokens : T;
+        if (fused) for (blocks = 1; blocks < T; blocks *= 2) {}
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(blocks);
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = g_pdl_enabled ? 1 : 0;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = fused ? blocks : 1;
+        attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = fused ? 2 : 1;
+        cudaLaunchKernelEx(&cfg, kernel, values, D, w, correction, E, top, softmax, renormalise, factor, ids, weights, gate_w, gate_out, T, align);
+    };
     if (x_dtype == kF32) {
-        if (smem > 40 * 1024) cudaFuncSetAttribute(route_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        launch_kernel((route_kernel<float>), dim3(T), dim3(kRouteThreads), smem, st, static_cast<const float*>(x), D, w, correction, E, top, softmax, renormalise, factor, ids, weights, gate_w, gate_out);
+        const float* values = static_cast<const float*>(x);
+        if (fused) launch(route_kernel<float, true, 1>, values);
+        else if (many) launch(route_kernel<float, false, kRouteManyTokens>, values);
+        else launch(route_kernel<float, false, 1>, values);
     } else if (x_dtype == kBF16) {
-        if (smem > 40 * 1024) cudaFuncSetAttribute(route_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        launch_kernel((route_kernel<__nv_bfloat16>), dim3(T), dim3(kRouteThreads), smem, st, static_cast<const __nv_bfloat16*>(x), D, w, correction, E, top, softmax, renormalise, factor, ids, weights, gate_w, gate_out);
+        const __nv_bfloat16* values = static_cast<const __nv_bfloat16*>(x);
+        if (fused) launch(route_kernel<__nv_bfloat16, true, 1>, values);
+        else if (many) launch(route_kernel<__nv_bfloat16, false, kRouteManyTokens>, values);
+        else launch(route_kernel<__nv_bfloat16, false, 1>, values);
     } else {
         GI_REQUIRE(false, "route: unsupported dtype code %d", x_dtype);
     }
     if (check_launch("route")) return 1;
-    launch_kernel(route_align_kernel, dim3(1), dim3(1024), 0, st, static_cast<const int*>(ids), static_cast<int>(pairs), E, sorted_rows, tile_group, n_tiles, max_tiles, tile_rows, pair_row);
+    if (fused) return 0;
+    launch_kernel(route_align_kernel, dim3(1), dim3(1024), 0, st, align);
     return check_launch("route_align");
 }
 
@@ -778,7 +860,7 @@ static int gi_route_table_impl(const int* tokens, const int* feedback, const int
     launch_kernel(route_table_kernel, dim3(static_cast<unsigned>((pairs + 255) / 256)), dim3(256), 0, st, tokens, feedback, table, vocab, E, top,
                   ids, weights, static_cast<int>(pairs));
     if (check_launch("route_table")) return 1;
-    launch_kernel(route_align_kernel, dim3(1), dim3(1024), 0, st, static_cast<const int*>(ids), static_cast<int>(pairs), E, sorted_rows, tile_group, n_tiles, max_tiles, tile_rows, pair_row);
+    launch_kernel(route_align_kernel, dim3(1), dim3(1024), 0, st, RouteAlign{ids, static_cast<int>(pairs), E, sorted_rows, tile_group, n_tiles, max_tiles, tile_rows, pair_row});
     return check_launch("route_align");
 }
 

@@ -307,6 +307,38 @@ def test_routing_and_expert_products(dtype, T, E, top, D, I):
     _close(y.cpu(), want, torch.float32, "routed experts", f32=1e-5)
 
 
+@pytest.mark.parametrize("scores", ["sigmoid", "softmax"])
+@pytest.mark.parametrize("E, D, T", [(8, 2048, 131), (9, 1100, 66), (40, 96, 65)])
+def test_routing_of_many_tokens_and_of_few(E, D, T, scores):
+    """Several tokens a block, one a block, and up to eight in a cluster that also buckets them: the same experts and the same bits."""
+    from geneinfer_b200.ops import kernels
+    g = torch.Generator().manual_seed(E)
+    x, w, corr, gw = (torch.randn(*s, generator=g).to(DEV) for s in ((T, D), (E, D), (E,), (D,)))
+    w, top = w * 0.05, 3
+    results = []
+    for tm in (kernels.grouped_tile_rows(), 128):
+        for step in (T, 20, 8, 5, 1):
+            ids, wts, gate = [], [], []
+            for at in range(0, T, step):
+                n = min(step, T - at)
+                tiles = kernels.route_tiles(n, top, E, tm)
+                i, v, o = torch.empty(n, top, dtype=torch.int32, device=DEV), torch.empty(n, top, device=DEV), torch.empty(n, device=DEV)
+                srt, grp, cnt = (torch.full((k,), 77, dtype=torch.int32, device=DEV) for k in (tiles * tm, tiles, 1))
+                pair_row = torch.empty(n * top, dtype=torch.int32, device=DEV)
+                kernels.route(x[at:at + n].contiguous(), w, corr, top, i, v, srt, grp, cnt, scores=scores, renormalise=True, factor=1.5, gate_w=gw, gate_out=o,
+                              tile_rows=tm, pair_row=pair_row)
+                used = srt.cpu()[:int(cnt) * tm].view(-1, tm)
+                assert sorted(used[used >= 0].tolist()) == list(range(n * top)) and torch.equal(srt[pair_row.long()].cpu(), torch.arange(n * top).int())
+                for tile, e in zip(used, grp.cpu().tolist()):
+                    assert all(int(i.view(-1)[p]) == e for p in tile[tile >= 0].tolist())
+                ids, wts, gate = ids + [i], wts + [v], gate + [o]
+            results.append([torch.cat(z) for z in (ids, wts, gate)])
+    for r in results[1:]:
+        assert all(torch.equal(one, two) for one, two in zip(r, results[0]))
+    want = torch.sigmoid(x.double() @ gw.double())
+    assert float((results[0][2] - want).abs().max()) < 1e-5
+
+
 @pytest.mark.parametrize("gated", ["silu", None])
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("N, K", [(18, 8), (33, 264), (16, 2056)])
