@@ -370,6 +370,14 @@ grouped_rows_kernel(const GroupedArgs p, int tiles) {
     for (int unit = first; unit < q.units; unit += q.stride) {
         if (unit / q.per_tile != x) { x = unit / q.per_tile; m_count = q.tile(x, g, row); }
         const int n_first = unit % q.per_tile * kGrWarpRows;
+        if (p.tail > 0 && n_first == 0) {              // the rotated tail of the tile's rows, by the warp of its first outputs
+            const TA* tails = static_cast<const TA*>(p.a) + p.a_off + static_cast<size_t>(g) * p.a_gs + p.K;
+            const int pairs = p.tail / 2;
+            for (int base = 0; base < m_count * pairs; base += 32) {
+                const int i = base + lane, r = __shfl_sync(0xffffffffu, row, min(i / pairs, m_count - 1));
+                if (i < m_count * pairs) gp_rotate_pair(p, tails + static_cast<size_t>(r) * p.lda, r, g, i % pairs);
+            }
+        }
         for (int m0 = 0; m0 < m_count; m0 += kGrFew) {
             const int m_here = min(kGrFew, m_count - m0);
             if (m_here == 1) grouped_rows_unit<1>(q, g, row, n_first, m0, m_here, done);
@@ -449,7 +457,6 @@ head_product64_kernel(const GroupedArgs p) {
 
 // ------------------------------------------------------------------------------------------------ routing
 constexpr int kRouteMaxExperts = 1024;
-constexpr int kRouteManyTokens = 4;            // tokens of a block where there are many
 
 // Where the pairs go: tiles of tile_rows rows per expert, in the order of the experts.
 struct RouteAlign {
@@ -494,73 +501,67 @@ route_align_kernel(const RouteAlign p) {
 // tokens there are as many warps as rows, and a warp's first 1,024 weights are asked for before the wait for the kernel ahead
 // (they belong to no earlier kernel). With eight loads in flight and a ninth row in a second round two tokens took 17 us.
 // FUSED (up to eight tokens): the tokens' blocks are one cluster, whose first block also buckets the pairs once all are there (a
-// launch less on the way from the router to the experts' weights). TOK: tokens of a block; many tokens share what is
-// read of the weights (1,273 tokens read them from L2 for 15.5 us, a token a block).
-template <typename TX, bool FUSED, int TOK>
-__global__ void __launch_bounds__(1024)
+// launch less on the way from the router to the experts' weights). BATCH: weights a lane has in flight; with many
+// tokens 8, whose blocks hide one another's waits (1,273 tokens: 15.5 us; with 32 22 us; four tokens a block, sharing what is read: 24 us).
+template <typename TX, bool FUSED, int BATCH>
+__global__ void __launch_bounds__(BATCH > 8 ? 1024 : 256)
 route_kernel(const TX* __restrict__ x, int D, const float* __restrict__ w, const float* __restrict__ correction, int E, int top,
              int softmax, int renormalise, float factor, int* __restrict__ ids, float* __restrict__ weights,
              const float* __restrict__ gate_w, float* __restrict__ gate_out, int T, const RouteAlign align) {
     pdl_launch_dependents();
-    extern __shared__ float s_x[];                 // [TOK][D], then the scores and the choice scores [TOK][E]
-    float* all_scores = s_x + TOK * D;
-    float* all_choices = all_scores + TOK * E;
-    constexpr int kBatch = TOK == 1 ? 32 : 16;     // weights a lane has in flight
-    const int t0 = blockIdx.x * TOK, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x / 32;
+    extern __shared__ float s_x[];                 // [D], then the scores and the choice scores [E]
+    float* s_score = s_x + D;
+    float* s_choice = s_score + E;
+    const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x / 32;
     const int n_rows = E + (gate_w ? 1 : 0);
-    float v[kBatch];
+    float v[BATCH];
     auto request = [&](int e, int d0) {
         const float* row = (e < E ? w + static_cast<size_t>(e) * D : gate_w) + d0 + lane;
+        if (d0 + 32 * BATCH <= D) {
 #pragma unroll
-        for (int i = 0; i < kBatch; ++i) v[i] = d0 + lane + 32 * i < D ? row[32 * i] : 0.f;
+            for (int i = 0; i < BATCH; ++i) v[i] = row[32 * i];
+        } else {
+#pragma unroll
+            for (int i = 0; i < BATCH; ++i) v[i] = d0 + lane + 32 * i < D ? row[32 * i] : 0.f;
+        }
     };
     if (warp < n_rows) request(warp, 0);
     pdl_wait();
     if (FUSED) {
-        if (t0 == 0)                                   // the places of the pairs, while the weights are on their way
+        if (t == 0)                                    // the places of the pairs, while the weights are on their way
             for (int i = threadIdx.x; i < align.max_tiles * align.tile_rows; i += blockDim.x) align.sorted_rows[i] = -1;
-        if (t0 >= T) {                                 // a cluster has a power of two of blocks
+        if (t >= T) {                                  // a cluster has a power of two of blocks
             cooperative_groups::this_cluster().sync();
             return;
         }
     }
-    const int here = min(TOK, T - t0);
-    for (int d = threadIdx.x; d < here * D; d += blockDim.x) s_x[d] = to_float(x[static_cast<size_t>(t0) * D + d]);
-    if (TOK > 1) for (int d = here * D + threadIdx.x; d < TOK * D; d += blockDim.x) s_x[d] = 0.f;
+    for (int d = threadIdx.x; d < D; d += blockDim.x) s_x[d] = to_float(x[static_cast<size_t>(t) * D + d]);
     __syncthreads();
     for (int e = warp; e < n_rows; e += warps) {
-        float z[TOK];
-#pragma unroll
-        for (int k = 0; k < TOK; ++k) z[k] = 0.f;
-        for (int d0 = 0; d0 < D; d0 += 32 * kBatch) {
+        float z = 0.f;
+        for (int d0 = 0; d0 < D; d0 += 32 * BATCH) {
             if (e != warp || d0 > 0) request(e, d0);
+            if (d0 + 32 * BATCH <= D) {
 #pragma unroll
-            for (int i = 0; i < kBatch; ++i) {
-                const int d = d0 + lane + 32 * i;
-                if (d < D) {
+                for (int i = 0; i < BATCH; ++i) z = fmaf(v[i], s_x[d0 + lane + 32 * i], z);
+            } else {
 #pragma unroll
-                    for (int k = 0; k < TOK; ++k) z[k] = fmaf(v[i], s_x[k * D + d], z[k]);
-                }
+                for (int i = 0; i < BATCH; ++i)
+                    if (d0 + lane + 32 * i < D) z = fmaf(v[i], s_x[d0 + lane + 32 * i], z);
             }
         }
-#pragma unroll
-        for (int k = 0; k < TOK; ++k) {
-            const float sum = warp_sum(z[k]);
-            if (lane != 0 || k >= here) continue;
-            if (e == E) {
-                gate_out[t0 + k] = sigmoid_f(sum);
-            } else {
-                const float s = softmax ? sum : 1.0f / (1.0f + expf(-sum));
-                all_scores[k * E + e] = s;
-                all_choices[k * E + e] = s + (correction ? correction[e] : 0.f);
-            }
+        z = warp_sum(z);
+        if (lane != 0) continue;
+        if (e == E) {
+            gate_out[t] = sigmoid_f(z);
+        } else {
+            const float s = softmax ? z : 1.0f / (1.0f + expf(-z));
+            s_score[e] = s;
+            s_choice[e] = s + (correction ? correction[e] : 0.f);
         }
     }
     __syncthreads();
-    if (warp < here) {
-        const int t = t0 + warp;
-        float* s_score = all_scores + warp * E;
-        float* s_choice = all_choices + warp * E;
+    if (warp == 0) {
         if (softmax) {
             float m = -INFINITY;
             for (int e = lane; e < E; e += 32) m = fmaxf(m, s_score[e]);
@@ -606,7 +607,7 @@ route_kernel(const TX* __restrict__ x, int D, const float* __restrict__ w, const
     }
     if (FUSED) {
         cooperative_groups::this_cluster().sync();     // every token's experts are in memory
-        if (t0 == 0) route_align_block(align, reinterpret_cast<int*>(all_scores), reinterpret_cast<int*>(all_choices), true);
+        if (t == 0) route_align_block(align, reinterpret_cast<int*>(s_score), reinterpret_cast<int*>(s_choice), true);
     }
 }
 
@@ -680,6 +681,26 @@ route_combine_kernel(const float* __restrict__ part, const float* __restrict__ w
         v = fmaf(weights ? weights[t * top + k] : 1.f, part[row * D + d], v);
     }
     if (more) v = fmaf(more_gate[t], more[i], v);
+    y[i] = v;
+}
+
+// The same, four values a thread in 16-byte pieces (D a multiple of 4, pointers aligned; a value at a time: 17 us for 1,273 tokens
+// of two experts, whose bytes need 7).
+__global__ void __launch_bounds__(256)
+route_combine4_kernel(const float4* __restrict__ part, const float* __restrict__ weights, const int* __restrict__ pair_row,
+                      const float4* __restrict__ more, const float* __restrict__ more_gate, float4* __restrict__ y, int D4, int top, size_t total4) {
+    pdl_prologue();
+    const size_t i = static_cast<size_t>(blockIdx.x) * 256 + threadIdx.x;
+    if (i >= total4) return;
+    const int t = static_cast<int>(i / D4), d = static_cast<int>(i % D4);
+    float4 v = y[i];
+    auto add = [&](float f, const float4& x) { v.x = fmaf(f, x.x, v.x); v.y = fmaf(f, x.y, v.y); v.z = fmaf(f, x.z, v.z); v.w = fmaf(f, x.w, v.w); };
+#pragma unroll 2
+    for (int k = 0; k < top; ++k) {
+        const size_t pair = static_cast<size_t>(t) * top + k, row = pair_row ? static_cast<size_t>(pair_row[pair]) : pair;
+        add(weights ? weights[pair] : 1.f, part[row * D4 + d]);
+    }
+    if (more) add(more_gate[t], more[i]);
     y[i] = v;
 }
 
@@ -760,8 +781,9 @@ static int gi_head_product_impl(const void* a, int a_dtype, long long lda, int a
         else launch_kernel((head_product64_kernel<__nv_bfloat16, __nv_bfloat16>), grid64, dim3(256), 0, st64, p);
         return check_launch("head_product (tiles of 64)");
     }
-    // few tokens: the heads' matrices are what is read; the rotated tail stays with the tiled form
-    if (rows <= 2 * kGpTM && tail == 0 && rows_form_fits(p, a_dtype, w_dtype))
+    // few tokens: the heads' matrices are what is read. A rotated tail comes with short inputs and many outputs, where the few-row
+    // form spends its time on its sums: 18 us in tiles and 11 us in rows at two tokens of 16 heads (64 to 512), 19 and 25 at eight
+    if (rows <= (tail == 0 ? 2 * kGpTM : 4) && rows_form_fits(p, a_dtype, w_dtype))
         return launch_grouped_rows<false>(p, a_dtype, w_dtype, static_cast<unsigned>(tiles), static_cast<cudaStream_t>(stream));
     return launch_grouped<false>(p, a_dtype, w_dtype, grid, static_cast<cudaStream_t>(stream));
 }
@@ -807,11 +829,11 @@ static int gi_route_impl(const void* x, int x_dtype, int T, int D, const float* 
     // a cluster of up to eight blocks is portable; the places are few there (tiles of 128 rows belong to many tokens)
     const bool fused = T <= 8 && tile_rows == kGpTM;
     const size_t per_token = (static_cast<size_t>(D) + 2 * static_cast<size_t>(E)) * 4;
-    const bool many = T > 64 && kRouteManyTokens * per_token <= 96 * 1024;
+    const bool many = T > 64;
     auto launch = [&](auto kernel, auto* values) {
-        const size_t smem = per_token * (many ? kRouteManyTokens : 1);
+        const size_t smem = per_token;
         if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        int blocks = many ? (T + kRouteManyTokens - 1) / kRouteManyTokens : T;
+        int blocks = T;
         if (fused) for (blocks = 1; blocks < T; blocks *= 2) {}
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(blocks);
@@ -830,14 +852,14 @@ static int gi_route_impl(const void* x, int x_dtype, int T, int D, const float* 
     };
     if (x_dtype == kF32) {
         const float* values = static_cast<const float*>(x);
-        if (fused) launch(route_kernel<float, true, 1>, values);
-        else if (many) launch(route_kernel<float, false, kRouteManyTokens>, values);
-        else launch(route_kernel<float, false, 1>, values);
+        if (fused) launch(route_kernel<float, true, 32>, values);
+        else if (many) launch(route_kernel<float, false, 8>, values);
+        else launch(route_kernel<float, false, 32>, values);
     } else if (x_dtype == kBF16) {
         const __nv_bfloat16* values = static_cast<const __nv_bfloat16*>(x);
-        if (fused) launch(route_kernel<__nv_bfloat16, true, 1>, values);
-        else if (many) launch(route_kernel<__nv_bfloat16, false, kRouteManyTokens>, values);
-        else launch(route_kernel<__nv_bfloat16, false, 1>, values);
+        if (fused) launch(route_kernel<__nv_bfloat16, true, 32>, values);
+        else if (many) launch(route_kernel<__nv_bfloat16, false, 8>, values);
+        else launch(route_kernel<__nv_bfloat16, false, 32>, values);
     } else {
         GI_REQUIRE(false, "route: unsupported dtype code %d", x_dtype);
     }
@@ -885,6 +907,12 @@ static int gi_route_combine_impl(const float* part, const float* weights, const 
     GI_REQUIRE(T > 0 && D > 0 && top > 0, "route_combine: sizes must be positive");
     GI_REQUIRE((more == nullptr) == (more_gate == nullptr), "route_combine: a gated part needs its gate");
     const size_t total = static_cast<size_t>(T) * D;
+    auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+    if (D % 4 == 0 && aligned(part) && aligned(more) && aligned(y)) {
+        launch_kernel(route_combine4_kernel, dim3(static_cast<unsigned>((total / 4 + 255) / 256)), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                      reinterpret_cast<const float4*>(part), weights, pair_row, reinterpret_cast<const float4*>(more), more_gate, reinterpret_cast<float4*>(y), D / 4, top, total / 4);
+        return check_launch("route_combine");
+    }
     launch_kernel(route_combine_kernel, dim3(static_cast<unsigned>((total + 255) / 256)), dim3(256), 0, static_cast<cudaStream_t>(stream),
                   part, weights, pair_row, more, more_gate, y, D, top, total);
     return check_launch("route_combine");

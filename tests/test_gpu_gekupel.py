@@ -270,6 +270,51 @@ def test_head_product_with_a_rotated_tail(dtype):
         assert torch.isnan(out.cpu()[:, :2]).all()
 
 
+@pytest.mark.parametrize("interleaved", [True, False])
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("T, H, N, K, tail", [(1, 3, 70, 24, 6), (2, 16, 512, 64, 32), (3, 2, 5, 264, 72), (4, 5, 64, 32, 2), (5, 5, 64, 32, 2)])
+def test_head_product_of_very_few_rows_with_a_rotated_tail(T, H, N, K, tail, dtype, interleaved):
+    """Up to four rows in the few-row form, more in tiles; tails wider than a warp."""
+    from geneinfer_b200.ops import kernels
+    g = torch.Generator().manual_seed(T)
+    a, w = torch.randn(T, 8 + H * (K + tail + 8 - (K + tail) % 8), generator=g), _bf(torch.randn(H, N, K, generator=g))
+    step = K + tail + 8 - (K + tail) % 8
+    freq, pos = torch.rand(tail // 2, generator=g), torch.randint(0, 900, (T,), generator=g)
+    out = torch.full((T, 2 + H * (N + tail)), float("nan"), device=DEV)
+    kernels.head_product(a.to(DEV), 8, step, w.to(DEV).to(dtype), out, 2, N + tail, tail=tail, freq=freq.to(DEV), amplitude=1.3,
+                         positions=pos.int().to(DEV), interleaved=interleaved)
+    x = a[:, 8:].view(T, H, step).double()
+    got = out.cpu()[:, 2:].view(T, H, N + tail)
+    _close(got[..., :N], torch.einsum("thk,hnk->thn", x[..., :K], w.double()), torch.float32, "head product")
+    one, two = (slice(K, K + tail, 2), slice(K + 1, K + tail, 2)) if interleaved else (slice(K, K + tail // 2), slice(K + tail // 2, K + tail))
+    angle = (pos.double()[:, None] * freq.double())[:, None]
+    u, v = x[..., one], x[..., two]
+    ru, rv = 1.3 * (u * angle.cos() - v * angle.sin()), 1.3 * (v * angle.cos() + u * angle.sin())
+    want = torch.stack((ru, rv), 3).flatten(2) if interleaved else torch.cat((ru, rv), 2)
+    # the angles are 32-bit products below 900: about 900 * 2^-24 off
+    assert float((got[..., N:] - want).abs().max()) < 900 * 2.0 ** -23 * float(x.abs().max()) * 1.3 * 2
+
+
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("D", [4, 7, 2056])
+def test_combination_of_the_experts_outputs(D, gated):
+    from geneinfer_b200.ops import kernels
+    g = torch.Generator().manual_seed(D)
+    T, top = 37, 3
+    part, wts, y, more, gate = (torch.randn(*s, generator=g) for s in ((T * top + 5, D), (T, top), (T, D), (T, D), (T,)))
+    rows = torch.randperm(T * top + 5, generator=g)[:T * top].to(torch.int32)
+    for pair_row, weights in ((rows, wts), (None, wts), (rows, None)):
+        out = y.to(DEV)
+        dev = lambda t: None if t is None else t.to(DEV)  # noqa: E731
+        kernels.route_combine(part[:T * top].to(DEV) if pair_row is None else part.to(DEV), dev(weights), out, pair_row=dev(pair_row), top=top,
+                              more=dev(more) if gated else None, more_gate=dev(gate) if gated else None)
+        picked = part[:T * top] if pair_row is None else part[pair_row.long()]
+        want = y.double() + ((wts if weights is not None else torch.ones(T, top)).double()[:, :, None] * picked.view(T, top, D).double()).sum(1)
+        if gated:
+            want = want + gate.double()[:, None] * more.double()
+        assert float((out.cpu() - want).abs().max()) < 1e-5
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("T, E, top, D, I", [(1, 4, 1, 64, 24), (5, 3, 3, 40, 72), (150, 9, 2, 96, 40), (64, 40, 6, 72, 16)])
 def test_routing_and_expert_products(dtype, T, E, top, D, I):
