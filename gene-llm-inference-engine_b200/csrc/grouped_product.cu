@@ -180,9 +180,8 @@ grouped_product_kernel(const GroupedArgs p) {
 // pieces are multiplied with up to eight rows of the tile, read through the cache; more rows stream the weights again, from
 // L2. An output element is the sum of its lanes' partial sums (lane l takes the
 // pieces l, l + 32, ...), added by a fixed xor tree: it depends on its own row only.
-constexpr int kGrWarps = 4, kGrWarpRows = 4;
+constexpr int kGrWarps = 4;
 constexpr int kGrFew = 8;             // rows of a tile that are multiplied with a piece of the weights while it is in registers
-constexpr int kGrSmem = 64 * 1024;    // the block's ring: three blocks an SM
 
 template <typename T> struct Vec16;
 template <> struct Vec16<float> {
@@ -211,20 +210,24 @@ template <> __device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bf
     return make_float4(a.x, a.y, b.x, b.y);
 }
 
-// The few-row form's units of work, taken by the grid's warps in turn: (tile, four output rows), and for a tile of more than
+// The few-row form's units of work, taken by the grid's warps in turn: (tile, four or eight output rows), and for a tile of more than
 // kGrFew rows a second pass over the same weights. A warp's ring runs on from unit to unit.
-template <typename TA, typename TW, bool GATED>
+// ROWS: output rows of a unit, 4 or, not gated, 8.
+template <typename TA, typename TW, bool GATED, int ROWS>
 struct RowsStream {
     static constexpr int kPiece = Vec16<TW>::N;          // values per step of a lane: the weights' 16 bytes
-    static constexpr int kW = GATED ? 2 * kGrWarpRows : kGrWarpRows;
-    static constexpr int kStages = kGrSmem / (kGrWarps * kW * 512);
+    static constexpr int kW = GATED ? 2 * ROWS : ROWS;   // rows of weights that it streams (gated: and the up rows)
+    static constexpr int kBlocks = ROWS == 8 ? 2 : 3;    // blocks an SM: 8 rows need more than the 168 registers of three
+    static constexpr int kSmem = (ROWS == 8 ? 96 : 64) * 1024;
+    static constexpr int kStages = kSmem / (kGrWarps * kW * 512);
 
     const GroupedArgs& p;
     uint4* ring;                 // this lane's place in the warp's first stage
     int lane, units, per_tile, stride, pieces, steps;
     // the step that is requested next
     int unit, pass, passes, step, issued = 0;
-    const TW* wrow[kGrWarpRows];
+    const TW* wrow;              // the unit's first row of weights; `last`: the last that there is
+    int last;
 
     // Group and rows of tile x; lane i gets the i-th of its rows.
     __device__ __forceinline__ int tile(int x, int& g, int& row) const {
@@ -248,9 +251,9 @@ struct RowsStream {
             passes = (tile(unit / per_tile, g, row) + kGrFew - 1) / kGrFew;
             if (passes == 0) continue;
             const TW* W = static_cast<const TW*>(p.w) + static_cast<size_t>(g) * p.w_gs;
-            const int n_first = unit % per_tile * kGrWarpRows;
-#pragma unroll
-            for (int r = 0; r < kGrWarpRows; ++r) wrow[r] = W + static_cast<size_t>(min(n_first + r, p.N - 1)) * p.ldw;
+            const int n_first = unit % per_tile * ROWS;
+            wrow = W + static_cast<size_t>(n_first) * p.ldw;
+            last = p.N - 1 - n_first;
             pass = step = 0;
             return;
         }
@@ -262,7 +265,7 @@ struct RowsStream {
                 const unsigned at = static_cast<unsigned>(__cvta_generic_to_shared(ring + (issued % kStages) * (kW * 32)));
 #pragma unroll
                 for (int r = 0; r < kW; ++r) {
-                    const TW* src = wrow[r % kGrWarpRows] + (r >= kGrWarpRows ? p.up_off : 0) + c * kPiece;
+                    const TW* src = wrow + static_cast<long long>(min(r % ROWS, last)) * p.ldw + (r >= ROWS ? p.up_off : 0) + c * kPiece;
                     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(at + r * 512), "l"(src) : "memory");
                 }
             }
@@ -276,40 +279,65 @@ struct RowsStream {
     }
 };
 
-// MR rows of a tile (m_here of them are real, the last is repeated) against the four output rows from n_first on. ``row``:
-// lane i has the tile's i-th row; ``done``: steps of the warp's ring taken so far.
-template <int MR, typename TA, typename TW, bool GATED>
-__device__ __forceinline__ void grouped_rows_unit(RowsStream<TA, TW, GATED>& q, int g, int row, int n_first, int m0, int m_here, int& done) {
+// MR rows of a tile (m_here of them are real, the last is repeated) against the output rows from n_first on. ``row``:
+// lane i has the tile's i-th row; ``done``: steps of the warp's ring taken so far. With 8 output rows up to two rows' inputs are
+// asked for a step ahead.
+template <int MR, typename TA, typename TW, bool GATED, int ROWS>
+__device__ __forceinline__ void grouped_rows_unit(RowsStream<TA, TW, GATED, ROWS>& q, int g, int row, int n_first, int m0, int m_here, int& done) {
     const GroupedArgs& p = q.p;
-    constexpr int kW = RowsStream<TA, TW, GATED>::kW, kStages = RowsStream<TA, TW, GATED>::kStages, kPiece = Vec16<TW>::N;
+    using Stream = RowsStream<TA, TW, GATED, ROWS>;
+    constexpr int kW = Stream::kW, kStages = Stream::kStages, kPiece = Vec16<TW>::N;
+    constexpr bool kAhead = ROWS == 8 && MR <= 2;
     const TA* A = static_cast<const TA*>(p.a) + p.a_off + static_cast<size_t>(g) * p.a_gs;
     const TA* arow[MR];
 #pragma unroll
     for (int i = 0; i < MR; ++i) arow[i] = A + static_cast<size_t>(__shfl_sync(0xffffffffu, row, m0 + min(i, m_here - 1)) / p.a_div) * p.lda;
-    // the output gate's values of the unit's 4 x 8 outputs, a lane each, asked for before the weights arrive
-    float gate_z = 0.f;
+    // the output gate's values of the unit's outputs, (row of weights, row of the tile) by lane, asked for before the weights arrive
+    constexpr int kGates = ROWS * kGrFew / 32;
+    float gate_z[kGates];
     if (p.gate != nullptr) {
-        const int gr = q.lane / kGrFew, gi_ = q.lane % kGrFew;
-        const int gate_row = __shfl_sync(0xffffffffu, row, m0 + min(gi_, m_here - 1));
-        if (gi_ < m_here && n_first + gr < p.N) gate_z = gp_gate_value(p, gate_row, g, n_first + gr);
+#pragma unroll
+        for (int u = 0; u < kGates; ++u) {
+            const int gr = (q.lane + 32 * u) / kGrFew, gi_ = q.lane % kGrFew;
+            const int gate_row = __shfl_sync(0xffffffffu, row, m0 + min(gi_, m_here - 1));
+            gate_z[u] = (gi_ < m_here && n_first + gr < p.N) ? gp_gate_value(p, gate_row, g, n_first + gr) : 0.f;
+        }
     }
     float acc[kW][MR];
 #pragma unroll
     for (int r = 0; r < kW; ++r)
 #pragma unroll
         for (int i = 0; i < MR; ++i) acc[r][i] = 0.f;
+    constexpr int kHeld = kAhead ? kPiece : 4;
+    float av[MR][kHeld], next[kAhead ? MR : 1][kHeld];
+    auto fetch = [&](float* dst, int i, int at) {
+        const float4 v = load4<TA>(arow[i] + at);
+        dst[0] = v.x; dst[1] = v.y; dst[2] = v.z; dst[3] = v.w;
+    };
+    if constexpr (kAhead) {
+        if (q.lane < q.pieces)
+#pragma unroll
+            for (int i = 0; i < MR; ++i)
+#pragma unroll
+                for (int h = 0; h < kPiece; h += 4) fetch(&av[i][h], i, q.lane * kPiece + h);
+    }
     for (int step = 0; step < q.steps; ++step, ++done) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
         const int c = step * 32 + q.lane;
+        if constexpr (kAhead) {
+            if (c + 32 < q.pieces)
+#pragma unroll
+                for (int i = 0; i < MR; ++i)
+#pragma unroll
+                    for (int h = 0; h < kPiece; h += 4) fetch(&next[i][h], i, (c + 32) * kPiece + h);
+        }
+        asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
         if (c < q.pieces) {
             const uint4* stage = q.ring + (done % kStages) * (kW * 32);
 #pragma unroll
             for (int h = 0; h < kPiece; h += 4) {
-                float av[MR][4];
+                if constexpr (!kAhead) {
 #pragma unroll
-                for (int i = 0; i < MR; ++i) {
-                    const float4 v = load4<TA>(arow[i] + c * kPiece + h);
-                    av[i][0] = v.x; av[i][1] = v.y; av[i][2] = v.z; av[i][3] = v.w;
+                    for (int i = 0; i < MR; ++i) fetch(&av[i][0], i, c * kPiece + h);
                 }
 #pragma unroll
                 for (int r = 0; r < kW; ++r) {
@@ -318,9 +346,15 @@ __device__ __forceinline__ void grouped_rows_unit(RowsStream<TA, TW, GATED>& q, 
 #pragma unroll
                     for (int i = 0; i < MR; ++i)
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) acc[r][i] = fmaf(av[i][j], wv[h + j], acc[r][i]);
+                        for (int j = 0; j < 4; ++j) acc[r][i] = fmaf(av[i][(kAhead ? h : 0) + j], wv[h + j], acc[r][i]);
                 }
             }
+        }
+        if constexpr (kAhead) {
+#pragma unroll
+            for (int i = 0; i < MR; ++i)
+#pragma unroll
+                for (int j = 0; j < kHeld; ++j) av[i][j] = next[i][j];
         }
         q.request();                                  // into the stage read a step ago, by this lane alone
     }
@@ -331,14 +365,14 @@ __device__ __forceinline__ void grouped_rows_unit(RowsStream<TA, TW, GATED>& q, 
         const float sc = p.scales ? p.scales[out_row] : 1.f;
         float mine = 0.f;                             // lane r ends up with output row r
 #pragma unroll
-        for (int r = 0; r < kGrWarpRows; ++r) {
+        for (int r = 0; r < ROWS; ++r) {
             float v = sc * warp_sum(acc[r][i]);
-            if (GATED) v = gated_value(v, sc * warp_sum(acc[GATED ? r + kGrWarpRows : 0][i]), p.act, p.act_limit);
+            if (GATED) v = gated_value(v, sc * warp_sum(acc[GATED ? r + ROWS : 0][i]), p.act, p.act_limit);
             else v = plain_value(v, p.out_act);
-            if (p.gate != nullptr) v *= 1.0f / (1.0f + expf(-__shfl_sync(0xffffffffu, gate_z, r * kGrFew + i)));
+            if (p.gate != nullptr) v *= 1.0f / (1.0f + expf(-__shfl_sync(0xffffffffu, gate_z[r * kGrFew / 32], (r * kGrFew + i) % 32)));
             if (q.lane == r) mine = v;
         }
-        if (q.lane < kGrWarpRows && n_first + q.lane < p.N) {
+        if (q.lane < ROWS && n_first + q.lane < p.N) {
             const size_t o = static_cast<size_t>(out_row) * p.ldo + p.o_off + static_cast<size_t>(g) * p.o_gs + n_first + q.lane;
             if (p.out_is_f32) static_cast<float*>(p.out)[o] = mine;
             else static_cast<__nv_bfloat16*>(p.out)[o] = __float2bfloat16_rn(mine);
@@ -347,17 +381,17 @@ __device__ __forceinline__ void grouped_rows_unit(RowsStream<TA, TW, GATED>& q, 
 }
 
 // tiles: how many there are (experts form: at most; the number is read on the device)
-template <typename TA, typename TW, bool GATED>
-__global__ void __launch_bounds__(kGrWarps * 32, 3)
+template <typename TA, typename TW, bool GATED, int ROWS>
+__global__ void __launch_bounds__(kGrWarps * 32, (RowsStream<TA, TW, GATED, ROWS>::kBlocks))
 grouped_rows_kernel(const GroupedArgs p, int tiles) {
     extern __shared__ uint4 s_ring[];
     pdl_prologue();
-    using Stream = RowsStream<TA, TW, GATED>;
+    using Stream = RowsStream<TA, TW, GATED, ROWS>;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     Stream q{p};
     q.ring = s_ring + warp * (Stream::kStages * Stream::kW * 32) + lane;
     q.lane = lane;
-    q.per_tile = (p.N + kGrWarpRows - 1) / kGrWarpRows;
+    q.per_tile = (p.N + ROWS - 1) / ROWS;
     q.units = (p.tile_group ? *p.n_tiles : tiles) * q.per_tile;
     q.stride = gridDim.x * kGrWarps;
     q.pieces = p.K / Stream::kPiece;
@@ -369,7 +403,7 @@ grouped_rows_kernel(const GroupedArgs p, int tiles) {
     int done = 0, x = -1, g = 0, row = -1, m_count = 0;
     for (int unit = first; unit < q.units; unit += q.stride) {
         if (unit / q.per_tile != x) { x = unit / q.per_tile; m_count = q.tile(x, g, row); }
-        const int n_first = unit % q.per_tile * kGrWarpRows;
+        const int n_first = unit % q.per_tile * ROWS;
         if (p.tail > 0 && n_first == 0) {              // the rotated tail of the tile's rows, by the warp of its first outputs
             const TA* tails = static_cast<const TA*>(p.a) + p.a_off + static_cast<size_t>(g) * p.a_gs + p.K;
             const int pairs = p.tail / 2;
@@ -715,24 +749,32 @@ static bool rows_form_fits(const GroupedArgs& p, int a_dtype, int w_dtype) {
     return p.lda % a_piece == 0 && p.a_off % a_piece == 0 && p.a_gs % a_piece == 0;
 }
 
-template <typename TA, typename TW, bool GATED>
+template <typename TA, typename TW, bool GATED, int ROWS>
 static int launch_grouped_rows_as(const GroupedArgs& p, unsigned tiles, cudaStream_t st) {
-    static const cudaError_t ready = cudaFuncSetAttribute(grouped_rows_kernel<TA, TW, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGrSmem);
+    using Stream = RowsStream<TA, TW, GATED, ROWS>;
+    static const cudaError_t ready = cudaFuncSetAttribute(grouped_rows_kernel<TA, TW, GATED, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Stream::kSmem);
     if (ready != cudaSuccess) { set_error("grouped_product (rows): %s", cudaGetErrorString(ready)); return 1; }
     int sms = 0, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const long long blocks = (static_cast<long long>(tiles) * ((p.N + kGrWarpRows - 1) / kGrWarpRows) + kGrWarps - 1) / kGrWarps;
+    const long long blocks = (static_cast<long long>(tiles) * ((p.N + ROWS - 1) / ROWS) + kGrWarps - 1) / kGrWarps;
     GI_REQUIRE(blocks * kGrWarps <= 2147483647LL - 3 * 1024 * kGrWarps, "grouped_product: too many tiles");
-    launch_kernel((grouped_rows_kernel<TA, TW, GATED>), dim3(static_cast<unsigned>(blocks < 3LL * sms ? blocks : 3LL * sms)), dim3(kGrWarps * 32), kGrSmem, st, p,
-                  static_cast<int>(tiles));
+    launch_kernel((grouped_rows_kernel<TA, TW, GATED, ROWS>), dim3(static_cast<unsigned>(std::min<long long>(blocks, Stream::kBlocks * sms))), dim3(kGrWarps * 32),
+                  Stream::kSmem, st, p, static_cast<int>(tiles));
     return check_launch("grouped_product (rows)");
 }
 template <bool GATED>
 static int launch_grouped_rows(const GroupedArgs& p, int a_dtype, int w_dtype, unsigned tiles, cudaStream_t st) {
-    if (a_dtype == kF32 && w_dtype == kF32) return launch_grouped_rows_as<float, float, GATED>(p, tiles, st);
-    if (a_dtype == kF32 && w_dtype == kBF16) return launch_grouped_rows_as<float, __nv_bfloat16, GATED>(p, tiles, st);
-    return launch_grouped_rows_as<__nv_bfloat16, __nv_bfloat16, GATED>(p, tiles, st);
+    if (a_dtype == kF32 && w_dtype == kF32) return launch_grouped_rows_as<float, float, GATED, 4>(p, tiles, st);
+    if (a_dtype == kF32 && w_dtype == kBF16) {
+        // 32-bit inputs are as many bytes as four rows of bfloat16 weights for every two of them, and come from L2: eight rows a
+        // unit (2,048 outputs of 4,096 and of 3,072 inputs, sixteen and four pairs: 47.0 -> 43.4 us and 21.9 -> 15.3). Heads' matrices are too
+        // small to give every warp such a unit (19 against 26 us), two gated rows' registers leave no third block (68 against 84).
+        if constexpr (!GATED)
+            if (p.tile_group) return launch_grouped_rows_as<float, __nv_bfloat16, false, 8>(p, tiles, st);
+        return launch_grouped_rows_as<float, __nv_bfloat16, GATED, 4>(p, tiles, st);
+    }
+    return launch_grouped_rows_as<__nv_bfloat16, __nv_bfloat16, GATED, 4>(p, tiles, st);
 }
 
 template <bool GATED>

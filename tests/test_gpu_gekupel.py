@@ -385,7 +385,7 @@ def test_routing_of_many_tokens_and_of_few(E, D, T, scores):
 
 
 @pytest.mark.parametrize("gated", ["silu", None])
-@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("dtype", [*DTYPES, "32-bit inputs"])
 @pytest.mark.parametrize("N, K", [(18, 8), (33, 264), (16, 2056)])
 def test_expert_products_of_few_rows(dtype, N, K, gated):
     """Every count of rows in a tile, rows of one to nine steps with a ragged last one, blocks of outputs with a ragged last one.
@@ -401,7 +401,8 @@ def test_expert_products_of_few_rows(dtype, N, K, gated):
         srt[e, torch.randperm(tm, generator=g)[:len(r)]] = r          # empty places anywhere in a tile
     grp = torch.arange(E, dtype=torch.int32).flip(0)
     out = torch.full((T, N), float("nan"), device=DEV)
-    kernels.expert_product(a.to(DEV).to(dtype), 1, w.to(DEV).to(dtype), out, srt.flip(0).reshape(-1).to(DEV), grp.to(DEV),
+    a_dtype, w_dtype = (torch.float32, torch.bfloat16) if dtype == "32-bit inputs" else (dtype, dtype)
+    kernels.expert_product(a.to(DEV).to(a_dtype), 1, w.to(DEV).to(w_dtype), out, srt.flip(0).reshape(-1).to(DEV), grp.to(DEV),
                            torch.tensor([E], dtype=torch.int32, device=DEV), gated=gated)
     want = torch.empty(T, N, dtype=torch.float64)
     for e, r in enumerate(rows):
