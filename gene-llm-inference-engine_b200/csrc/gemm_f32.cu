@@ -11,8 +11,8 @@
 //   - a thread keeps of each output two sums, over even and over odd k: a pair of neighbouring k is then one packed
 //     multiply-add of two register pairs as they were read (no transposing, no duplicating; half the instructions);
 //   - a thread has 8 x 8 outputs for many rows (8 x 4 in twice the warps: 3 % slower; 16 x 8 single sums, which read less: 40 %
-//     slower, two warps a scheduler of 255 registers); with up to 8, 16 or 32 rows blocks of that height (few rows would
-//     multiply zeros in a tall one), for 8 and 16 rows of a single warp, so that N = 2048 still gives every SM a block or two;
+//     slower, two warps a scheduler of 255 registers); with up to 2, 4, 6, 8, 16 or 32 rows blocks of that height (few rows would
+//     multiply zeros in a tall one), up to 16 rows of a single warp, so that N = 2048 still gives every SM a block or two;
 //   - where the blocks along N alone leave SMs idle, K is cut into up to 8 chunks, one per CTA of a cluster, whose sums are
 //     added in the order of the chunks through distributed shared memory: no workspace and no second launch.
 // An output is (over chunks s) sum of (even_s + odd_s); chunks depend on N and K only. So a row's result does not depend
@@ -53,6 +53,9 @@ struct F32Tile {
     static_assert(BM * BN <= kStage * kStages, "the block's sums reuse the ring");
     static_assert(kRowsT % kLaneM == 0 && kColsT % kLaneN == 0 && BN % kCopyRows == 0 && kChunkStep % BK == 0, "");
 };
+using Tile2 = F32Tile<2, 64, 2, 2, 32, 5, 4>;
+using Tile4 = F32Tile<4, 64, 4, 2, 32, 5, 4>;
+using Tile6 = F32Tile<6, 64, 6, 2, 32, 5, 4>;
 using Tile8 = F32Tile<8, 64, 8, 2, 32, 5, 4>;
 using Tile16 = F32Tile<16, 64, 8, 4, 32, 4, 4>;
 using Tile32 = F32Tile<32, 128, 8, 4, 32, 3, 3>;
@@ -201,6 +204,9 @@ int gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int 
     int chunks = 1;
     while (chunks < kMaxChunks && (N + 127) / 128 * chunks < 148 && K / (2 * chunks) >= 256) chunks *= 2;
     const int kc = ((K + chunks - 1) / chunks + kChunkStep - 1) / kChunkStep * kChunkStep;
+    if (M <= 2) return launch<Tile2>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, st);
+    if (M <= 4) return launch<Tile4>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, st);
+    if (M <= 6) return launch<Tile6>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, st);
     if (M <= 8) return launch<Tile8>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, st);
     if (M <= 16) return launch<Tile16>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, st);
     if (M <= 32) return launch<Tile32>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, st);

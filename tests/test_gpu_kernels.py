@@ -106,7 +106,7 @@ def test_gemm_simt_tiled(M, N, K_):
     acc = base.to(DEV)
     K().gemm_simt(a, w, acc, accumulate=True)
     assert torch.equal(acc, base.to(DEV) + out)
-    for rows in (1, 8, 9, 16, 17, 32, 33, 64):      # the same rows at every block height
+    for rows in (1, 2, 3, 4, 5, 6, 7, 8, 9, 16, 17, 32, 33, 64):      # the same rows at every block height
         if rows <= M:
             part = torch.empty((rows, N), device=DEV)
             K().gemm_simt(a[M - rows:].contiguous(), w, part)
