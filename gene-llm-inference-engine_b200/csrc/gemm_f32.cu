@@ -18,9 +18,9 @@
 // An output is (over chunks s) sum of (even_s + odd_s); chunks depend on N and K only. So a row's result does not depend
 // on M, on the block's height or on where the row sits in the batch (how tokens are cut into steps), and its chains are
 // half as long or shorter than one chain over all of K.
-// Measured on prompts of 268 rows and steps of 6 (four layers of the 1B sizes, 32-bit): all products of a prompt step 10.0 ms
-// before, 3.2 ms now; the head of 128,256 rows at six tokens 1,180 us before, 224 now (4.7 TB/s); logits off from 64 bits by
-// 4.4e-6 before, 1.6e-6 now; the pass with its five sampled steps 59.5 to 8.7 ms (the sampling kernel among it).
+// Measured on prompts of 268 rows and steps of 6 (four layers of the 1B sizes, 32-bit): all products of a prompt step 9.9 ms
+// before, 4.3 ms now; of a token step 6.5 before, 0.52 now (the head of 128,256 rows 1,180 us before, 207 now); logits off from
+// 64 bits by 4.4e-6 before, 1.6e-6 now; the pass with its five sampled steps 59.5 to 8.5 ms (the sampling kernel among it).
 #include <cooperative_groups.h>
 
 #include "gemm_f32.cuh"
