@@ -1194,7 +1194,7 @@ static int launch_decode_tma(const void* q, const void* kc, const void* vc, void
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int items = n_rows * Hkv * n_chunks;
     int grid = items < sms ? items : sms;           // few items: fewer per CTA rather than fewer CTAs
-    const bool compact = n_rows >= 16 && n_rows <= Cfg::kMetaRows && items > grid;
+    const bool compact = n_rows >= 16 && n_rows <= Cfg::kMetaRows && n_chunks > 1 && items > grid;      // (one chunk: all are seen)
     auto launch = [&](auto kernel) {
         launch_kernel(kernel, dim3(grid), dim3(Cfg::kThreads), Cfg::kSmemBytes, st, mk, mv,
                   static_cast<const __nv_bfloat16*>(q), rows, n_rows, row_req, positions, tables, table_stride, H, Hkv,
