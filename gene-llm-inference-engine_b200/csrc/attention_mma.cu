@@ -372,7 +372,8 @@ struct DecodeTma {
     static constexpr int kQBytes = 16 * HD * 2;
     static constexpr int kMetaRows = 512;          // requests whose (row, position, request) are staged in shared memory
     static constexpr int kBarBytes = 256;
-    static constexpr int kSmemBytes = kWarps * kStages * kStageBytes + kWarps * kQBytes + kBarBytes + 4 * kMetaRows * 4 + 1024;
+    static constexpr int kSmemBytes = kWarps * kStages * kStageBytes + kWarps * kQBytes + kBarBytes + 3 * kMetaRows * 4 + 1024;
+    static constexpr int kCompactBytes = kSmemBytes + kMetaRows * 4;      // and the requests' ends
 };
 
 __device__ __forceinline__ void att_mbar_init(uint32_t bar) { asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar)); }
@@ -510,8 +511,9 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
             }
         } else {
             it.chunk = w % n_chunks;
-            it.g = w / n_chunks % Hkv;
-            it.idx = w / n_chunks / Hkv;
+            const int rest = w / n_chunks;
+            it.g = rest % Hkv;
+            it.idx = rest / Hkv;
         }
         if (it.idx < Cfg::kMetaRows) {
             it.t = meta[it.idx]; it.pos = meta[Cfg::kMetaRows + it.idx]; it.req = meta[2 * Cfg::kMetaRows + it.idx];
@@ -1177,8 +1179,8 @@ static int launch_decode_tma(const void* q, const void* kc, const void* vc, void
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(attention_decode_tma_kernel<HD, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_decode_tma_kernel<HD, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_decode_tma_kernel<HD, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_decode_tma_kernel<HD, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_decode_tma_kernel<HD, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kCompactBytes);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_decode_tma_kernel<HD, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kCompactBytes);
         if (e != cudaSuccess) { set_error("attention_decode: %s", cudaGetErrorString(e)); return 1; }
         configured = true;
     }
@@ -1196,7 +1198,7 @@ static int launch_decode_tma(const void* q, const void* kc, const void* vc, void
     int grid = items < sms ? items : sms;           // few items: fewer per CTA rather than fewer CTAs
     const bool compact = n_rows >= 16 && n_rows <= Cfg::kMetaRows && n_chunks > 1 && items > grid;      // (one chunk: all are seen)
     auto launch = [&](auto kernel) {
-        launch_kernel(kernel, dim3(grid), dim3(Cfg::kThreads), Cfg::kSmemBytes, st, mk, mv,
+        launch_kernel(kernel, dim3(grid), dim3(Cfg::kThreads), compact ? Cfg::kCompactBytes : Cfg::kSmemBytes, st, mk, mv,
                   static_cast<const __nv_bfloat16*>(q), rows, n_rows, row_req, positions, tables, table_stride, H, Hkv,
                   page_size, scale * kLog2e, window, part_o, part_ml, max_chunks, n_chunks, static_cast<__nv_bfloat16*>(out), status,
                   (g_stream_kv && n_rows <= 32) ? 1 : 0, ep);     // (evict-first) measured: 2 % faster at 8 requests, no gain at 64
