@@ -71,70 +71,44 @@ residual_norm_kernel(const float* __restrict__ acc_in, const float* __restrict__
     }
 }
 
-template <typename T> __device__ __forceinline__ void store_four(T* p, float a, float b, float c, float d);
-template <> __device__ __forceinline__ void store_four<float>(float* p, float a, float b, float c, float d) {
-    *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
-}
-template <> __device__ __forceinline__ void store_four<__nv_bfloat16>(__nv_bfloat16* p, float a, float b, float c, float d) {
-    const __nv_bfloat162 lo = __floats2bfloat162_rn(a, b), hi = __floats2bfloat162_rn(c, d);
-    uint2 raw;
-    raw.x = *reinterpret_cast<const uint32_t*>(&lo);
-    raw.y = *reinterpret_cast<const uint32_t*>(&hi);
-    *reinterpret_cast<uint2*>(p) = raw;
-}
-
 // residual_norm (kAdd false: x = w * unit(a), acc_out = alpha * x) and add_normed (kAdd: x += w * unit(a), acc_out = a if it
-// is to be cleared) for rows that the block holds in registers: at most 1024 PIECES values in 16-byte pieces (the host checks).
+// is to be cleared) for rows that the block holds in registers: at most 256 KEEP values, thread t those at t, t + 256, ...: the
+// order of the sums is that of the general kernels, and so is every bit.
 // Everything that is read is asked for at once (the weights even before the wait: they belong to no earlier kernel), where
-// the general kernels go to memory a second time once the sum is known, a value at a time: add_normed of 2,048 values took
+// the general kernels go to memory a second time once the sum is known: add_normed of 2,048 values took
 // 7.5 us for eight rows and 13.6 us for 1,273, of which the bytes need 7.
-template <typename TOut, int PIECES, bool kAdd>
+template <typename TOut, int KEEP, bool kAdd>
 __global__ void __launch_bounds__(256)
 normed_rows_kernel(const float* a_in, const float* __restrict__ weight, float* __restrict__ x, float* acc_out,
                    TOut* __restrict__ xn_out, int D, float eps, float alpha) {
     __shared__ float warp_part[8];
     pdl_launch_dependents();
-    const int n4 = D / 4;
     const size_t row = static_cast<size_t>(blockIdx.x) * D;
-    float4 w[PIECES], a[PIECES], old[PIECES];
+    float w[KEEP], a[KEEP], old[KEEP];
 #pragma unroll
-    for (int k = 0; k < PIECES; ++k) {
-        const int i = threadIdx.x + k * 256;
-        w[k] = i < n4 ? __ldg(reinterpret_cast<const float4*>(weight) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k = 0; k < KEEP; ++k) {
+        const int d = threadIdx.x + k * 256;
+        w[k] = d < D ? __ldg(weight + d) : 0.f;
     }
     pdl_wait();
 #pragma unroll
-    for (int k = 0; k < PIECES; ++k) {
-        const int i = threadIdx.x + k * 256;
-        a[k] = old[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (i < n4) a[k] = reinterpret_cast<const float4*>(a_in + row)[i];
-        if (kAdd && i < n4) old[k] = reinterpret_cast<const float4*>(x + row)[i];
+    for (int k = 0; k < KEEP; ++k) {
+        const int d = threadIdx.x + k * 256;
+        a[k] = d < D ? a_in[row + d] : 0.f;
+        old[k] = kAdd && d < D ? x[row + d] : 0.f;
     }
     float ss = 0.f;
 #pragma unroll
-    for (int k = 0; k < PIECES; ++k) {
-        ss = fmaf(a[k].x, a[k].x, ss); ss = fmaf(a[k].y, a[k].y, ss);
-        ss = fmaf(a[k].z, a[k].z, ss); ss = fmaf(a[k].w, a[k].w, ss);
-    }
-    ss = warp_sum(ss);
-    if ((threadIdx.x & 31) == 0) warp_part[threadIdx.x >> 5] = ss;
-    __syncthreads();
-    float total = 0.f;
+    for (int k = 0; k < KEEP; ++k) ss = fmaf(a[k], a[k], ss);
+    const float scale = 1.0f / sqrtf(block_sum_256(ss, warp_part) / static_cast<float>(D) + eps);
 #pragma unroll
-    for (int v = 0; v < 8; ++v) total += warp_part[v];
-    const float scale = 1.0f / sqrtf(total / static_cast<float>(D) + eps);
-#pragma unroll
-    for (int k = 0; k < PIECES; ++k) {
-        const int i = threadIdx.x + k * 256;
-        if (i >= n4) continue;
-        float v[4] = {w[k].x * (scale * a[k].x), w[k].y * (scale * a[k].y), w[k].z * (scale * a[k].z), w[k].w * (scale * a[k].w)};
-        if (kAdd) { v[0] += old[k].x; v[1] += old[k].y; v[2] += old[k].z; v[3] += old[k].w; }
-        store_four<float>(x + row + 4 * i, v[0], v[1], v[2], v[3]);
-        if (acc_out) {
-            if (kAdd) store_four<float>(acc_out + row + 4 * i, 0.f, 0.f, 0.f, 0.f);
-            else store_four<float>(acc_out + row + 4 * i, alpha * v[0], alpha * v[1], alpha * v[2], alpha * v[3]);
-        }
-        if (xn_out) store_four<TOut>(xn_out + row + 4 * i, v[0], v[1], v[2], v[3]);
+    for (int k = 0; k < KEEP; ++k) {
+        const int d = threadIdx.x + k * 256;
+        if (d >= D) continue;
+        const float v = kAdd ? fmaf(w[k], scale * a[k], old[k]) : w[k] * (scale * a[k]);
+        x[row + d] = v;
+        if (acc_out) acc_out[row + d] = kAdd ? 0.f : alpha * v;
+        if (xn_out) xn_out[row + d] = from_float<TOut>(v);
     }
 }
 
@@ -142,10 +116,9 @@ normed_rows_kernel(const float* a_in, const float* __restrict__ weight, float* _
 template <typename TOut, bool kAdd>
 static bool launch_normed_rows(const float* a_in, const float* weight, float* x, float* acc_out, TOut* xn_out, int rows, int D, float eps,
                                float alpha, cudaStream_t st) {
-    auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
-    if (D % 4 != 0 || D > 4096 || !aligned(a_in) || !aligned(weight) || !aligned(x) || !aligned(acc_out) || !aligned(xn_out)) return false;
-    if (D <= 2048) launch_kernel((normed_rows_kernel<TOut, 2, kAdd>), dim3(rows), dim3(256), 0, st, a_in, weight, x, acc_out, xn_out, D, eps, alpha);
-    else launch_kernel((normed_rows_kernel<TOut, 4, kAdd>), dim3(rows), dim3(256), 0, st, a_in, weight, x, acc_out, xn_out, D, eps, alpha);
+    if (D > 4096) return false;
+    if (D <= 2048) launch_kernel((normed_rows_kernel<TOut, 8, kAdd>), dim3(rows), dim3(256), 0, st, a_in, weight, x, acc_out, xn_out, D, eps, alpha);
+    else launch_kernel((normed_rows_kernel<TOut, 16, kAdd>), dim3(rows), dim3(256), 0, st, a_in, weight, x, acc_out, xn_out, D, eps, alpha);
     return true;
 }
 

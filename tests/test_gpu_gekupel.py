@@ -92,6 +92,26 @@ def test_norms_on_the_output_and_after_the_sum_of_wide_rows(D, dtype):
     assert torch.equal(acc.cpu(), 1.7 * out.cpu()) and torch.equal(xn.cpu().float(), out.cpu().to(dtype).float())
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("D, times", [(2048, 4), (3072, 4), (4096, 4), (1028, 16), (70, 64)])
+def test_norms_of_rows_in_registers_equal_the_general_ones_to_the_bit(D, times, dtype):
+    """A row of D values widened with zeros to ``times`` D is beyond what a block holds: the general kernels take it. Its mean square
+    is that of the row over a power of four, so with eps over the same its unit values are the row's times a power of two, exactly."""
+    from geneinfer_b200.ops import kernels
+    g = torch.Generator().manual_seed(D)
+    T, two = 33, int(times ** 0.5)
+    x, y, w = torch.randn(T, D, generator=g) * 3, torch.randn(T, D, generator=g), 1 + 0.1 * torch.randn(D, generator=g)
+    wide = lambda t: torch.nn.functional.pad(t, (0, (times - 1) * D)).to(DEV)  # noqa: E731
+    results = []
+    for xs, ys, ws, eps in ((x.to(DEV), y.to(DEV), w.to(DEV), 1e-3), (wide(x * two), wide(y), wide(w), 1e-3 / times)):
+        out, acc, xn, xm = torch.empty_like(ys), torch.empty_like(ys), torch.empty_like(ys, dtype=dtype), torch.empty_like(ys, dtype=dtype)
+        kernels.residual_norm(ys, ws, out, eps, 1.7, acc_out=acc, xn_out=xn)
+        kernels.add_normed(ys, ws, xs, eps, xn_out=xm)
+        results.append([t.cpu().float()[:, :D] for t in (out, acc, xn, xs, xm)])
+    for one, more in zip(*results):
+        assert torch.equal(one * two, more)
+
+
 @pytest.mark.parametrize("q_rank, rank", [(768, 512), (1025, 1300), (2049, 64), (30, 2500)])
 def test_latents_of_every_size_into_their_pages(q_rank, rank):
     from geneinfer_b200.ops import kernels
