@@ -404,14 +404,6 @@ grouped_rows_kernel(const GroupedArgs p, int tiles) {
     for (int unit = first; unit < q.units; unit += q.stride) {
         if (unit / q.per_tile != x) { x = unit / q.per_tile; m_count = q.tile(x, g, row); }
         const int n_first = unit % q.per_tile * ROWS;
-        if (p.tail > 0 && n_first == 0) {              // the rotated tail of the tile's rows, by the warp of its first outputs
-            const TA* tails = static_cast<const TA*>(p.a) + p.a_off + static_cast<size_t>(g) * p.a_gs + p.K;
-            const int pairs = p.tail / 2;
-            for (int base = 0; base < m_count * pairs; base += 32) {
-                const int i = base + lane, r = __shfl_sync(0xffffffffu, row, min(i / pairs, m_count - 1));
-                if (i < m_count * pairs) gp_rotate_pair(p, tails + static_cast<size_t>(r) * p.lda, r, g, i % pairs);
-            }
-        }
         for (int m0 = 0; m0 < m_count; m0 += kGrFew) {
             const int m_here = min(kGrFew, m_count - m0);
             if (m_here == 1) grouped_rows_unit<1>(q, g, row, n_first, m0, m_here, done);
@@ -421,6 +413,68 @@ grouped_rows_kernel(const GroupedArgs p, int tiles) {
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+// The heads form with a rotated tail for up to four rows: short inputs and many outputs, where a tile's rounds through shared
+// memory and its sixteen rows cost more than its multiply-adds, and the few-row form spends its time on its sums. A thread has one
+// output of every row, its weights in registers (asked for before the wait: they belong to no earlier kernel). The sum is one
+// chain in the order of k, as in the tiles of 16 and of 64: a token's result is the same to the bit whatever else is in the step.
+constexpr int kGcRows = 4, kGcCols = 64, kGcK = 64;
+
+template <typename TA, typename TW>
+__global__ void __launch_bounds__(kGcCols)
+head_product_few_kernel(const GroupedArgs p) {
+    pdl_launch_dependents();
+    constexpr int kPiece = Vec16<TW>::N, kPieces = kGcK / kPiece;
+    __shared__ __align__(16) float s_a[kGcK][kGcRows];
+    const int tid = threadIdx.x, g = blockIdx.x, n = blockIdx.y * kGcCols + tid;
+    const TA* A = static_cast<const TA*>(p.a) + p.a_off + static_cast<size_t>(g) * p.a_gs;
+    const TW* wrow = static_cast<const TW*>(p.w) + static_cast<size_t>(g) * p.w_gs + static_cast<size_t>(min(n, p.N - 1)) * p.ldw;
+    uint4 wv[kPieces];
+    auto request = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < kPieces; ++i) {
+            const int k = k0 + i * kPiece;                 // (K is a multiple of a piece)
+            wv[i] = k < p.K ? __ldg(reinterpret_cast<const uint4*>(wrow + k)) : make_uint4(0, 0, 0, 0);
+        }
+    };
+    request(0);
+    pdl_wait();
+    if (blockIdx.y == 0)
+        for (int i = tid; i < p.rows * (p.tail / 2); i += kGcCols) {
+            const int r = i / (p.tail / 2);
+            gp_rotate_pair(p, A + static_cast<size_t>(r) * p.lda + p.K, r, g, i % (p.tail / 2));
+        }
+    float acc[kGcRows] = {};
+    for (int k0 = 0; k0 < p.K; k0 += kGcK) {
+        __syncthreads();
+        for (int i = tid; i < kGcK * kGcRows; i += kGcCols) {
+            const int m = i / kGcK, k = i % kGcK;
+            s_a[k][m] = m < p.rows && k0 + k < p.K ? to_float(A[static_cast<size_t>(m) * p.lda + k0 + k]) : 0.f;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kPieces; ++i) {
+            float w[8];
+            Vec16<TW>::load(reinterpret_cast<const TW*>(&wv[i]), w);
+#pragma unroll
+            for (int j = 0; j < kPiece; ++j) {
+                const float4 a = *reinterpret_cast<const float4*>(s_a[i * kPiece + j]);
+                acc[0] = fmaf(a.x, w[j], acc[0]); acc[1] = fmaf(a.y, w[j], acc[1]);
+                acc[2] = fmaf(a.z, w[j], acc[2]); acc[3] = fmaf(a.w, w[j], acc[3]);
+            }
+        }
+        if (k0 + kGcK < p.K) request(k0 + kGcK);
+    }
+    if (n >= p.N) return;
+#pragma unroll
+    for (int r = 0; r < kGcRows; ++r) {
+        if (r >= p.rows) break;
+        const float v = gp_gated(p, acc[r], r, g, n);
+        const size_t o = static_cast<size_t>(r) * p.ldo + p.o_off + static_cast<size_t>(g) * p.o_gs + n;
+        if (p.out_is_f32) static_cast<float*>(p.out)[o] = v;
+        else static_cast<__nv_bfloat16*>(p.out)[o] = __float2bfloat16_rn(v);
+    }
 }
 
 // The heads form for many rows (prompt portions): tiles of 64 rows x 64 outputs, a thread 4 x 4 of them, so that two
@@ -823,10 +877,16 @@ static int gi_head_product_impl(const void* a, int a_dtype, long long lda, int a
         else launch_kernel((head_product64_kernel<__nv_bfloat16, __nv_bfloat16>), grid64, dim3(256), 0, st64, p);
         return check_launch("head_product (tiles of 64)");
     }
-    // few tokens: the heads' matrices are what is read. A rotated tail comes with short inputs and many outputs, where the few-row
-    // form spends its time on its sums: 18 us in tiles and 11 us in rows at two tokens of 16 heads (64 to 512), 19 and 25 at eight
-    if (rows <= (tail == 0 ? 2 * kGpTM : 4) && rows_form_fits(p, a_dtype, w_dtype))
-        return launch_grouped_rows<false>(p, a_dtype, w_dtype, static_cast<unsigned>(tiles), static_cast<cudaStream_t>(stream));
+    // few tokens: the heads' matrices are what is read; with a rotated tail every form's sums are chains in the order of k
+    if (rows <= (tail == 0 ? 2 * kGpTM : kGcRows) && rows_form_fits(p, a_dtype, w_dtype)) {
+        cudaStream_t st = static_cast<cudaStream_t>(stream);
+        if (tail == 0) return launch_grouped_rows<false>(p, a_dtype, w_dtype, static_cast<unsigned>(tiles), st);
+        const dim3 few(heads, (N + kGcCols - 1) / kGcCols);
+        if (a_dtype == kF32 && w_dtype == kF32) launch_kernel((head_product_few_kernel<float, float>), few, dim3(kGcCols), 0, st, p);
+        else if (a_dtype == kF32) launch_kernel((head_product_few_kernel<float, __nv_bfloat16>), few, dim3(kGcCols), 0, st, p);
+        else launch_kernel((head_product_few_kernel<__nv_bfloat16, __nv_bfloat16>), few, dim3(kGcCols), 0, st, p);
+        return check_launch("head_product (few rows)");
+    }
     return launch_grouped<false>(p, a_dtype, w_dtype, grid, static_cast<cudaStream_t>(stream));
 }
 

@@ -294,7 +294,7 @@ def test_head_product_with_a_rotated_tail(dtype):
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("T, H, N, K, tail", [(1, 3, 70, 24, 6), (2, 16, 512, 64, 32), (3, 2, 5, 264, 72), (4, 5, 64, 32, 2), (5, 5, 64, 32, 2)])
 def test_head_product_of_very_few_rows_with_a_rotated_tail(T, H, N, K, tail, dtype, interleaved):
-    """Up to four rows in the few-row form, more in tiles; tails wider than a warp."""
+    """Up to four rows by threads that have an output each, more in tiles; tails wider than a warp."""
     from geneinfer_b200.ops import kernels
     g = torch.Generator().manual_seed(T)
     a, w = torch.randn(T, 8 + H * (K + tail + 8 - (K + tail) % 8), generator=g), _bf(torch.randn(H, N, K, generator=g))
@@ -313,6 +313,28 @@ def test_head_product_of_very_few_rows_with_a_rotated_tail(T, H, N, K, tail, dty
     want = torch.stack((ru, rv), 3).flatten(2) if interleaved else torch.cat((ru, rv), 2)
     # the angles are 32-bit products below 900: about 900 * 2^-24 off
     assert float((got[..., N:] - want).abs().max()) < 900 * 2.0 ** -23 * float(x.abs().max()) * 1.3 * 2
+
+
+@pytest.mark.parametrize("a_dtype, w_dtype", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16), (torch.bfloat16, torch.bfloat16)])
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("H, N, K, tail", [(3, 70, 24, 8), (16, 512, 64, 32), (2, 65, 200, 72)])
+def test_head_product_with_a_rotated_tail_in_steps_of_any_size(H, N, K, tail, gated, a_dtype, w_dtype):
+    """A token's outputs are the same to the bit in steps of one row to four, of five, of whole tiles and of a prompt's many."""
+    from geneinfer_b200.ops import kernels
+    g = torch.Generator().manual_seed(N)
+    T, step = 131, K + tail
+    a, w = torch.randn(T, H * step, generator=g).to(DEV).to(a_dtype), torch.randn(H, N, K, generator=g).to(DEV).to(w_dtype)
+    freq, pos = torch.rand(tail // 2, generator=g).to(DEV), torch.randint(0, 900, (T,), generator=g).int().to(DEV)
+    gate = torch.randn(T, H * N, generator=g).to(DEV) if gated else None
+    results = []
+    for rows in (T, 1, 2, 3, 4, 5, 32, 33, 128):
+        out = torch.full((T, H * (N + tail)), float("nan"), device=DEV)
+        for at in range(0, T, rows):
+            cut = slice(at, min(at + rows, T))
+            kernels.head_product(a[cut].contiguous(), 0, step, w, out[cut], 0, N + tail, tail=tail, freq=freq, positions=pos[cut].contiguous(),
+                                 gate=None if gate is None else gate[cut].contiguous())
+        results.append(out.cpu())
+    assert not torch.isnan(results[0]).any() and all(torch.equal(r, results[0]) for r in results[1:])
 
 
 @pytest.mark.parametrize("gated", [False, True])
