@@ -548,7 +548,7 @@ constexpr int kRouteMaxExperts = 1024;
 
 // Where the pairs go: tiles of tile_rows rows per expert, in the order of the experts.
 struct RouteAlign {
-    const int* ids; int n_pairs, E;
+    int* ids; int n_pairs, E;                      // (the fused router writes the ids through this pointer too)
     int* sorted_rows; int* tile_group; int* n_tiles; int max_tiles, tile_rows; int* pair_row;
 };
 // One block: counts per expert, then tiles per expert in expert order. `empty`: the places hold -1 already.
@@ -594,7 +594,7 @@ route_align_kernel(const RouteAlign p) {
 template <typename TX, bool FUSED, int BATCH>
 __global__ void __launch_bounds__(BATCH > 8 ? 1024 : 256)
 route_kernel(const TX* __restrict__ x, int D, const float* __restrict__ w, const float* __restrict__ correction, int E, int top,
-             int softmax, int renormalise, float factor, int* __restrict__ ids, float* __restrict__ weights,
+             int softmax, int renormalise, float factor, float* __restrict__ weights,
              const float* __restrict__ gate_w, float* __restrict__ gate_out, int T, const RouteAlign align) {
     pdl_launch_dependents();
     extern __shared__ float s_x[];                 // [D], then the scores and the choice scores [E]
@@ -682,7 +682,7 @@ route_kernel(const TX* __restrict__ x, int D, const float* __restrict__ w, const
             if (best_e >= E) best_e = 0;                 // no comparable score (a row of NaN): any expert, but a real one
             chosen += s_score[best_e];
             if (lane == 0) {
-                ids[static_cast<size_t>(t) * top + k] = best_e;
+                align.ids[static_cast<size_t>(t) * top + k] = best_e;
                 weights[static_cast<size_t>(t) * top + k] = s_score[best_e] * factor;
                 s_choice[best_e] = -INFINITY;
             }
@@ -950,7 +950,7 @@ static int gi_route_impl(const void* x, int x_dtype, int T, int D, const float* 
         attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = fused ? 2 : 1;
-        cudaLaunchKernelEx(&cfg, kernel, values, D, w, correction, E, top, softmax, renormalise, factor, ids, weights, gate_w, gate_out, T, align);
+        cudaLaunchKernelEx(&cfg, kernel, values, D, w, correction, E, top, softmax, renormalise, factor, weights, gate_w, gate_out, T, align);
     };
     if (x_dtype == kF32) {
         const float* values = static_cast<const float*>(x);
