@@ -23,6 +23,7 @@
 // 64 bits by 4.4e-6 before, 1.6e-6 now; the pass with its five sampled steps 59.5 to 8.5 ms (the sampling kernel among it).
 #include <cooperative_groups.h>
 
+#include "device_limit.h"
 #include "gemm_f32.cuh"
 
 namespace gi {
@@ -170,8 +171,8 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
 template <typename T>
 int launch(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, int chunks, int kc,
            int accumulate, cudaStream_t st) {
-    static const cudaError_t ready = cudaFuncSetAttribute(gemm_f32_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                          static_cast<int>(T::kSmem));
+    static SharedLimit limit;
+    const cudaError_t ready = limit.allow(reinterpret_cast<const void*>(gemm_f32_kernel<T>), static_cast<int>(T::kSmem));
     if (ready != cudaSuccess) { set_error("gemm: %s", cudaGetErrorString(ready)); return 1; }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(chunks, (M + T::BM - 1) / T::BM, (N + T::BN - 1) / T::BN);

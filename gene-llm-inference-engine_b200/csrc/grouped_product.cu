@@ -30,6 +30,7 @@
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "device_limit.h"
 
 namespace gi {
 
@@ -806,7 +807,8 @@ static bool rows_form_fits(const GroupedArgs& p, int a_dtype, int w_dtype) {
 template <typename TA, typename TW, bool GATED, int ROWS>
 static int launch_grouped_rows_as(const GroupedArgs& p, unsigned tiles, cudaStream_t st) {
     using Stream = RowsStream<TA, TW, GATED, ROWS>;
-    static const cudaError_t ready = cudaFuncSetAttribute(grouped_rows_kernel<TA, TW, GATED, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Stream::kSmem);
+    static SharedLimit limit;
+    const cudaError_t ready = limit.allow(reinterpret_cast<const void*>(grouped_rows_kernel<TA, TW, GATED, ROWS>), Stream::kSmem);
     if (ready != cudaSuccess) { set_error("grouped_product (rows): %s", cudaGetErrorString(ready)); return 1; }
     int sms = 0, dev = 0;
     cudaGetDevice(&dev);

@@ -14,6 +14,7 @@
 // same arithmetic however the request was cut into steps and whatever else is in the batch; decays, step sizes,
 // gates, norms and the state are 32-bit.
 #include "common.cuh"
+#include "device_limit.h"
 
 namespace gi {
 
@@ -688,30 +689,31 @@ static int gi_causal_conv_impl(const float* in, int ld, int in_off, const float*
 }
 
 template <int kDk, int kDv>
-static void launch_apply(const ScanArgs& a, int R, cudaStream_t st) {
+static int launch_apply(const ScanArgs& a, int R, cudaStream_t st) {
     constexpr int smem = (kDk * (kApplyRows + 4) + kApplyStep * (kDv + 4)) * 4;
-    static const cudaError_t ready = cudaFuncSetAttribute(scan_apply_kernel<kDk, kDv>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    (void)ready;                                      // a failure shows at the launch
+    static SharedLimit limit;
+    const cudaError_t ready = limit.allow(reinterpret_cast<const void*>(scan_apply_kernel<kDk, kDv>), smem);
+    if (ready != cudaSuccess) { set_error("linear_scan: %s", cudaGetErrorString(ready)); return 1; }
     const int blocks = (a.part_len + kApplyRows - 1) / kApplyRows;
     launch_kernel((scan_apply_kernel<kDk, kDv>), dim3((a.dv + kDv - 1) / kDv * blocks, a.H, R * a.max_parts), dim3(128), smem, st, a, blocks);
+    return check_launch("linear_scan");
 }
 
 template <int kDk, int kRT>
-static void launch_scan(const ScanArgs& a, int R, cudaStream_t st) {
+static int launch_scan(const ScanArgs& a, int R, cudaStream_t st) {
     const unsigned tiles = (a.dv + kScanCols - 1) / kScanCols;
     constexpr int kThreads = kDk / kRT * 8;
     const bool rows = a.gate_raw != nullptr;
     if (a.part_len == 0) {
         if (rows) launch_kernel((linear_scan_kernel<kDk, kRT, false, true>), dim3(tiles, a.H, R), dim3(kThreads), 0, st, a);
         else launch_kernel((linear_scan_kernel<kDk, kRT, false, false>), dim3(tiles, a.H, R), dim3(kThreads), 0, st, a);
-        return;
+        return check_launch("linear_scan");
     }
     if (rows) launch_kernel((linear_scan_kernel<kDk, kRT, true, true>), dim3(tiles, a.H, R * a.max_parts), dim3(kThreads), 0, st, a);
     else launch_kernel((linear_scan_kernel<kDk, kRT, true, false>), dim3(tiles, a.H, R * a.max_parts), dim3(kThreads), 0, st, a);
     const size_t elements = static_cast<size_t>(a.H) * a.dk * a.dv;
     launch_kernel((scan_link_kernel), dim3(static_cast<unsigned>((elements + 255) / 256), R), dim3(256), 0, st, a);
-    if (a.dv <= 64) launch_apply<kDk, 64>(a, R, st);
-    else launch_apply<kDk, 128>(a, R, st);
+    return a.dv <= 64 ? launch_apply<kDk, 64>(a, R, st) : launch_apply<kDk, 128>(a, R, st);
 }
 
 // part_len 0: every segment is walked from the request's state by one block per head and column tile. Otherwise
@@ -740,12 +742,11 @@ static int gi_linear_scan_impl(const float* q, int ld_q, int q_off, const float*
                ws_decay};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // (padded state rows, rows per thread)
-    if (dk <= 16) launch_scan<16, 4>(a, R, st);
-    else if (dk <= 32) launch_scan<32, 4>(a, R, st);
-    else if (dk <= 64) launch_scan<64, 8>(a, R, st);
-    else if (dk <= 128) launch_scan<128, 8>(a, R, st);
-    else launch_scan<256, 16>(a, R, st);
-    return check_launch("linear_scan");
+    if (dk <= 16) return launch_scan<16, 4>(a, R, st);
+    if (dk <= 32) return launch_scan<32, 4>(a, R, st);
+    if (dk <= 64) return launch_scan<64, 8>(a, R, st);
+    if (dk <= 128) return launch_scan<128, 8>(a, R, st);
+    return launch_scan<256, 16>(a, R, st);
 }
 
 static int gi_gated_group_norm_impl(const float* y, const float* gate, int ld_gate, int gate_off, const float* weight, void* out,
