@@ -225,11 +225,12 @@ __device__ Found sample_descend(const float* __restrict__ probs, int begin, int 
     return f;
 }
 
-// The smallest c of 1 .. n with above + c * w >= target (inclusive) or > target; n where there is none.
+// The smallest c of 1 .. n with above + c * w >= target (inclusive) or > target; n where there is none, as for a target that is
+// no number (which must not become the integer that a search starts from: the conversion gives the smallest there is).
 __device__ __forceinline__ int sample_count_to(double above, double w, int n, double target, bool inclusive) {
-    if (!(w > 0.0)) return n;
+    if (!(w > 0.0) || !(target == target)) return n;
     const double guess = (target - above) / w;
-    int c = guess >= n ? n : guess <= 1.0 ? 1 : static_cast<int>(guess);
+    int c = guess >= n ? n : guess > 1.0 ? static_cast<int>(guess) : 1;
     auto reached = [&](int k) { const double cum = above + k * w; return inclusive ? cum >= target : cum > target; };
     while (c > 1 && reached(c - 1)) --c;
     while (c < n && !reached(c)) ++c;

@@ -367,6 +367,20 @@ def test_sample_rows_of_few_likely_tokens(V, top_k, top_p):
     assert got[3] == (0 if top_p < 1.0 else top_k - 1 if 0 < top_k < V else V - 1)      # no probabilities: an index, always the same
 
 
+@pytest.mark.parametrize("V", [5, 3000, 128256])
+@pytest.mark.parametrize("top_k,top_p", [(3, 1.0), (0, 0.999), (3, 0.999)])
+def test_sample_with_uniform_numbers_outside_their_range(V, top_k, top_p):
+    """Every row gets a token whatever its number is: below 0 the first of the order, from 1 on or no number the last that is kept."""
+    g = torch.Generator().manual_seed(V)
+    logits = torch.randn(6, V, generator=g)
+    logits[:, [4, 1, 2]] = torch.tensor([30.0, 29.0, 28.0])                     # hold all but 1e-8 of the mass; 0.999 keeps them
+    us = torch.tensor([float("nan"), -0.25, float("-inf"), float("inf"), 1.5, -1e-30])
+    out = torch.full((6,), -1, dtype=torch.int32, device=DEV)
+    K().sample(logits.to(DEV), torch.empty(6 * V, device=DEV), torch.ones(6, device=DEV),
+               torch.full((6,), top_k, dtype=torch.int32, device=DEV), torch.full((6,), top_p, device=DEV), us.to(DEV), out)
+    assert out.cpu().tolist() == [2, 4, 4, 2, 2, 4]
+
+
 @pytest.mark.parametrize("M,N,K_,plan", [
     (128, 256, 64, (False, 256, 1)), (128, 256, 512, (False, 256, 1)), (300, 520, 200, (False, 256, 1)),
     (129, 100, 96, (False, 128, 1)), (256, 64, 128, (False, 64, 1)),
