@@ -316,8 +316,10 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ probs_all, i
     } else if (!use_k && !use_p) {
         // index order: the CTA, the warp, then the value at which the running mass exceeds the target
         const double target = u * all_mass;
-        if (target >= all_mass) {
-            if (part == 0 && threadIdx.x == 0) out[r] = V - 1;          // rounding guard: u was (almost) 1
+        if (!(target < all_mass)) {
+            if (part == 0 && threadIdx.x == 0) out[r] = V - 1;          // rounding guard: u was (almost) 1, or no number
+        } else if (target < 0.0) {
+            if (part == 0 && threadIdx.x == 0) out[r] = 0;              // (no piece begins below 0)
         } else if (target >= before && target < before + mine) {
             double run = before, next = before;       // run: the mass ahead of the owner, a warp that has some
             int owner = -1;

@@ -368,7 +368,7 @@ def test_sample_rows_of_few_likely_tokens(V, top_k, top_p):
 
 
 @pytest.mark.parametrize("V", [5, 3000, 128256])
-@pytest.mark.parametrize("top_k,top_p", [(3, 1.0), (0, 0.999), (3, 0.999)])
+@pytest.mark.parametrize("top_k,top_p", [(0, 1.0), (3, 1.0), (0, 0.999), (3, 0.999)])
 def test_sample_with_uniform_numbers_outside_their_range(V, top_k, top_p):
     """Every row gets a token whatever its number is: below 0 the first of the order, from 1 on or no number the last that is kept."""
     g = torch.Generator().manual_seed(V)
@@ -378,7 +378,8 @@ def test_sample_with_uniform_numbers_outside_their_range(V, top_k, top_p):
     out = torch.full((6,), -1, dtype=torch.int32, device=DEV)
     K().sample(logits.to(DEV), torch.empty(6 * V, device=DEV), torch.ones(6, device=DEV),
                torch.full((6,), top_k, dtype=torch.int32, device=DEV), torch.full((6,), top_p, device=DEV), us.to(DEV), out)
-    assert out.cpu().tolist() == [2, 4, 4, 2, 2, 4]
+    first, last = (4, 2) if top_k or top_p < 1.0 else (0, V - 1)
+    assert out.cpu().tolist() == [last, first, first, last, last, first]
 
 
 @pytest.mark.parametrize("M,N,K_,plan", [
