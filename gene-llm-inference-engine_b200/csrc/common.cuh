@@ -7,6 +7,7 @@
 
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
@@ -133,6 +134,14 @@ __device__ __forceinline__ float plain_value(float z, int act) {
     return z;
 }
 
+// Kernels that this process has launched through the library (launches into a stream that is being captured among them). Every
+// launch below and in the files that launch clusters of their own passes its result through here.
+extern std::atomic<long long> g_launches;
+inline cudaError_t counted(cudaError_t launched) {
+    if (launched == cudaSuccess) g_launches.fetch_add(1, std::memory_order_relaxed);
+    return launched;
+}
+
 // ``early`` false: without that attribute. A kernel of about one long-running block per SM must not become resident while the
 // kernel ahead drains: its blocks would pile up on the SMs that happen to be free first and leave the others idle.
 template <typename... KArgs, typename... Args>
@@ -147,7 +156,7 @@ inline void launch_kernel_as(bool early, void (*kernel)(KArgs...), dim3 grid, di
     attr[0].val.programmaticStreamSerializationAllowed = g_pdl_enabled && early ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);      // errors surface in check_launch
+    counted(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...));      // errors surface in check_launch
 }
 template <typename... KArgs, typename... Args>
 inline void launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {

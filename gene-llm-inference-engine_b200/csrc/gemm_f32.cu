@@ -188,7 +188,7 @@ int launch(const float* A, const float* W, float* C, int M, int N, int K, int ld
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    cudaLaunchKernelEx(&cfg, gemm_f32_kernel<T>, A, W, C, M, N, K, lda, ldw, ldc, kc, accumulate);
+    counted(cudaLaunchKernelEx(&cfg, gemm_f32_kernel<T>, A, W, C, M, N, K, lda, ldw, ldc, kc, accumulate));
     return check_launch("gemm_f32");
 }
 

@@ -1454,7 +1454,7 @@ static int launch_persistent_pair(const CUtensorMap& mp, const CUtensorMap& mq, 
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tc_persistent_kernel<BLOCK_Q, EPI, true>, mp, mq, mc, p);
+    cudaError_t e = counted(cudaLaunchKernelEx(&cfg, gemm_tc_persistent_kernel<BLOCK_Q, EPI, true>, mp, mq, mc, p));
     if (e != cudaSuccess) { set_error("gemm_tc: launch of the paired product failed: %s", cudaGetErrorString(e)); return 1; }
     return check_launch("gemm_tc_persistent (pairs)");
 }
@@ -1521,7 +1521,7 @@ static int launch_tc_form(const CUtensorMap& mp, const CUtensorMap& mq, const Tc
     attr[1].val.clusterDim.z = p.splits;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BLOCK_Q, TILED, SPEC>, mp, mq, p);
+    cudaError_t e = counted(cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BLOCK_Q, TILED, SPEC>, mp, mq, p));
     if (e != cudaSuccess) { set_error("gemm_tc: cluster launch failed: %s", cudaGetErrorString(e)); return 1; }
     return check_launch("gemm_tc");
 }

@@ -952,7 +952,7 @@ static int gi_route_impl(const void* x, int x_dtype, int T, int D, const float* 
         attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = fused ? 2 : 1;
-        cudaLaunchKernelEx(&cfg, kernel, values, D, w, correction, E, top, softmax, renormalise, factor, weights, gate_w, gate_out, T, align);
+        counted(cudaLaunchKernelEx(&cfg, kernel, values, D, w, correction, E, top, softmax, renormalise, factor, weights, gate_w, gate_out, T, align));
     };
     if (x_dtype == kF32) {
         const float* values = static_cast<const float*>(x);

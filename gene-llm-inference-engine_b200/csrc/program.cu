@@ -10,11 +10,14 @@
 
 namespace gi {
 thread_local Program* tl_recording = nullptr;
+std::atomic<long long> g_launches{0};
 }
 
 using namespace gi;
 
 extern "C" {
+
+long long gi_launch_count() { return g_launches.load(std::memory_order_relaxed); }
 
 // Starts recording on the calling thread. Recordings do not nest.
 int gi_program_begin() {

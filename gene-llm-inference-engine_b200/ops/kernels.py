@@ -10,7 +10,7 @@ from typing import Optional
 
 import torch
 
-from .library import KernelError, check, lib
+from .library import KernelError, check, launches_made, lib
 
 F32, BF16 = 0, 1
 _CODES = {torch.float32: F32, torch.bfloat16: BF16}
@@ -23,18 +23,19 @@ def dtype_code(dtype: torch.dtype) -> int:
         raise KernelError(f"unsupported dtype {dtype} (float32 and bfloat16 only)") from None
 
 
-_launches = 0
+_from_graphs = 0
 
 
 def launch_count() -> int:
-    """Kernels of this library launched so far by this process (each wrapper call launches one)."""
-    return _launches
+    """Kernels of this library launched so far by this process: the library counts its own launches, the rest comes
+    through ``count_launches``."""
+    return launches_made() + _from_graphs
 
 
 def count_launches(n: int) -> None:
     """Adjusts the count for kernels that run from a replayed CUDA graph (or were only captured)."""
-    global _launches
-    _launches += n
+    global _from_graphs
+    _from_graphs += n
 
 
 _scoped_stream: Optional[int] = None
@@ -58,8 +59,6 @@ class on_current_stream:
 
 
 def _stream() -> int:
-    global _launches
-    _launches += 1
     return _scoped_stream if _scoped_stream is not None else torch.cuda.current_stream().cuda_stream
 
 
@@ -73,10 +72,8 @@ class Program:
         self.launches = launches
 
     def run(self) -> None:
-        global _launches
         stream = _scoped_stream if _scoped_stream is not None else torch.cuda.current_stream().cuda_stream
         check(lib().gi_program_run(self._handle, stream), "program")
-        _launches += self.launches
 
     def __len__(self) -> int:
         return int(lib().gi_program_size(self._handle))
@@ -98,13 +95,13 @@ class record:
 
     def __enter__(self):
         check(lib().gi_program_begin(), "program")
-        self._before = _launches
+        self._before = launches_made()
         return self
 
     def __exit__(self, exc_type, exc, tb):
         handle = lib().gi_program_end()
         if exc_type is None:
-            self.program = Program(handle, _launches - self._before)
+            self.program = Program(handle, launches_made() - self._before)
         elif handle:
             lib().gi_program_free(handle)
         return False
@@ -589,8 +586,6 @@ def attention_rows(q: torch.Tensor, k_cache: torch.Tensor, v_cache: Optional[tor
         float(scale), float(softcap or 0.0), int(window or 0), int(chunk or 0), _opt(slopes, "slopes", torch.float32), _opt(sinks, "sinks", torch.float32),
         _opt(gate, "gate", torch.float32), 0 if gate is None else gate.shape[1], int(gate_offset), _opt(lst, "rows or tiles", torch.int32), kind, n_list, int(splits), _opt(workspace, "workspace", torch.float32),
         0 if workspace is None else workspace.numel(), _stream()), "attention_rows")
-    if splits > 1:
-        count_launches(1)
 
 
 def attention_rows_of_step(ctx, q: torch.Tensor, k_cache: torch.Tensor, v_cache: Optional[torch.Tensor], out: torch.Tensor,
@@ -695,7 +690,8 @@ def route(x: torch.Tensor, w: torch.Tensor, correction: Optional[torch.Tensor], 
     (``renormalise``: divided by the chosen ones' sum + 1e-20), times ``factor``. The pairs (token, choice) are then
     bucketed by expert into tiles of ``tile_rows`` rows (grouped_tile_rows() by default): ``sorted_rows`` (pair index
     or -1), ``tile_group`` (a tile's expert), ``n_tiles`` [1], and optionally ``pair_row`` [T * top], the row each pair
-    landed in. ``gate_w`` [D] 32-bit with ``gate_out`` [T]: also gate_out = sigmoid(gate_w x). Two launches."""
+    landed in. ``gate_w`` [D] 32-bit with ``gate_out`` [T]: also gate_out = sigmoid(gate_w x). Two launches; one for up to eight
+    tokens in tiles of grouped_tile_rows()."""
     T, D = x.shape
     if (gate_w is None) != (gate_out is None) or (gate_w is not None and (gate_w.numel() != D or gate_out.numel() != T)):
         raise KernelError("route: a gate needs a row of D weights and a place for T values")
@@ -713,7 +709,6 @@ def route(x: torch.Tensor, w: torch.Tensor, correction: Optional[torch.Tensor], 
                          _dev(sorted_rows, "sorted_rows", torch.int32), _dev(tile_group, "tile_group", torch.int32),
                          _dev(n_tiles, "n_tiles", torch.int32), max_tiles, tm, _opt(pair_row, "pair_row", torch.int32),
                          _opt(gate_w, "gate_w", torch.float32), _opt(gate_out, "gate_out", torch.float32), _stream()), "route")
-    count_launches(1)
 
 
 def route_table(tokens: torch.Tensor, feedback: Optional[torch.Tensor], table: torch.Tensor, experts: int, ids: torch.Tensor,
@@ -734,7 +729,6 @@ def route_table(tokens: torch.Tensor, feedback: Optional[torch.Tensor], table: t
                                _dev(sorted_rows, "sorted_rows", torch.int32), _dev(tile_group, "tile_group", torch.int32),
                                _dev(n_tiles, "n_tiles", torch.int32), max_tiles, tm, _opt(pair_row, "pair_row", torch.int32), _stream()),
           "route_table")
-    count_launches(1)
 
 
 def gather_rows(x: torch.Tensor, a_div: int, sorted_rows: torch.Tensor, n_tiles: torch.Tensor, tile_rows: int, out: torch.Tensor,
@@ -822,7 +816,8 @@ def causal_conv(proj: torch.Tensor, offset: int, weight: torch.Tensor, bias: Opt
     is off; ``bias`` may be None) over the channels
     proj[:, offset:offset + C] of each request's rows; inputs before a segment's first row come from the request's
     state (``state`` [slots, floats per slot], the [taps-1, C] block at ``state_offset``), which afterwards
-    holds the last taps-1 inputs. Two launches."""
+    holds the last taps-1 inputs. Two launches; one for a single tap, and for as many rows as segments where channels and rows come in
+    whole 16-byte pieces and the taps are 2 to 4."""
     T, ld = proj.shape
     C, taps = weight.shape
     if out.shape != (T, C) or (bias is not None and bias.numel() != C):
@@ -835,8 +830,6 @@ def causal_conv(proj: torch.Tensor, offset: int, weight: torch.Tensor, bias: Opt
                                int(state_offset), _dev(row_req, "row_req", torch.int32), _dev(seg_start, "seg_start", torch.int32),
                                _dev(seg_len, "seg_len", torch.int32), _dev(state_slots, "state_slots", torch.int32),
                                _dev(out, "out", torch.float32), C, taps, T, R, int(bool(activate)), _stream()), "causal_conv")
-    if taps > 1 and T > R:                   # (a token per segment: one kernel does both)
-        count_launches(1)
 
 
 def gated_delta(proj: torch.Tensor, in_offset: int, b_offset: int, a_offset: int, conv: torch.Tensor, a_log: torch.Tensor,
@@ -872,7 +865,6 @@ def gated_delta(proj: torch.Tensor, in_offset: int, b_offset: int, a_offset: int
         _dev(seg_start, "seg_start", torch.int32), _dev(seg_len, "seg_len", torch.int32), _dev(state_slots, "state_slots", torch.int32),
         _dev(qkv, "qkv", torch.float32), _dev(gates, "gates", torch.float32), _opt(coefs, "coefs", torch.float32),
         _dev(out, "out", torch.float32), T, R, num_heads, key_heads, dk, dv, _stream()), "gated_delta")
-    count_launches(1 if coefs is None else 2)
 
 
 def gated_delta_coefs() -> int:
@@ -942,8 +934,6 @@ def linear_scan(q: torch.Tensor, q_offset: int, k: torch.Tensor, k_offset: int, 
         _dev(seg_len, "seg_len", torch.int32), _dev(state_slots, "state_slots", torch.int32), _dev(out, "out", torch.float32),
         R, int(part_len), max_parts, _opt(ws_state, "ws_state", torch.float32), _opt(ws_decay, "ws_decay", torch.float32),
         _stream()), "linear_scan")
-    if part_len:
-        count_launches(2)
 
 
 SCAN_PART = 128          # tokens per part of a long segment (see linear_scan)
@@ -1066,9 +1056,6 @@ def attention_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
         _dev(part_o, "part_o", torch.float32), _dev(part_ml, "part_ml", torch.float32), max_chunks, n_chunks,
         k_cache.shape[0], _tc_state(q.device).status.data_ptr(), *_epilogue(sink, gate, gate_offset, out_scale, num_heads, gate_dims, head_dim, q.shape[0]),
         float(softcap or 0.0), _stream()), "attention_decode")
-    tma = page_size % 8 == 0 and (32 % page_size == 0 or page_size % 32 == 0)
-    if n_chunks > 1 or not tma:
-        count_launches(1)     # the kernel that merges the chunks (not needed when every context is one chunk)
 
 
 def attention_prefill(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, out: torch.Tensor,
@@ -1350,8 +1337,6 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: boo
                                           _dev(out, "out", torch.float32), 1 if accumulate else 0, M, N, K, K, K, N,
                                           block_q, st.status.data_ptr(), splits, st.workspace.data_ptr() if splits > 1 else 0,
                                           st.workspace.numel() if splits > 1 else 0, _paired(M, block_q), 0.0, 0, _stream()), "gemm_tc")
-        if splits > 1:
-            count_launches(1)     # the kernel that adds the ranges up
         return
     check(lib().gi_gemm_tc(_dev(a, "a", torch.bfloat16), _dev(w, "w", torch.bfloat16), _dev(out, "out"),
                            dtype_code(out.dtype) | (PLAIN_ACTIVATIONS[act] << 8 if act else 0), int(accumulate), M, N, K, K, K, N, int(swap), block_q, splits,
@@ -1496,8 +1481,6 @@ def argmax(logits: torch.Tensor, out: torch.Tensor) -> None:
         _argmax_scratch[key] = buf
     check(lib().gi_argmax(_dev(logits, "logits", torch.float32), rows, V, _dev(out, "out", torch.int32),
                           buf[0].data_ptr(), buf[1].data_ptr(), _stream()), "argmax")
-    global _launches
-    _launches += 1            # two kernels
 
 
 def sample(logits: torch.Tensor, scratch: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor,

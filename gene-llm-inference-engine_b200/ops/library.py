@@ -152,6 +152,8 @@ def lib() -> ctypes.CDLL:
         loaded.gi_last_error.argtypes = []
         loaded.gi_program_end.restype = c_void_p
         loaded.gi_program_end.argtypes = []
+        loaded.gi_launch_count.restype = c_longlong
+        loaded.gi_launch_count.argtypes = []
         for name, argtypes in _SIGNATURES.items():
             fn = getattr(loaded, name, None)
             if fn is None:
@@ -160,6 +162,11 @@ def lib() -> ctypes.CDLL:
             fn.argtypes = argtypes
         _lib = loaded
     return _lib
+
+
+def launches_made() -> int:
+    """Kernels that the library has launched in this process (0 while it is not loaded)."""
+    return int(_lib.gi_launch_count()) if _lib is not None else 0
 
 
 def declare(name: str, argtypes) -> None:

@@ -426,6 +426,38 @@ def test_routing_of_many_tokens_and_of_few(E, D, T, scores):
     assert float((results[0][2] - want).abs().max()) < 1e-5
 
 
+def test_launches_are_counted_as_they_are_made():
+    """Routing in one launch or two, convolutions likewise, as the sizes and alignments decide; and the same when a recorded
+    program repeats them."""
+    from geneinfer_b200.ops import kernels
+    ints = lambda z: torch.tensor(z, dtype=torch.int32, device=DEV)  # noqa: E731
+    E, D, top = 5, 32, 2
+
+    def routed(T, tm):
+        tiles = kernels.route_tiles(T, top, E, tm)
+        x, w = torch.randn(T, D, device=DEV), torch.randn(E, D, device=DEV)
+        i, v, srt, grp, cnt = ints([[0] * top] * T), torch.empty(T, top, device=DEV), ints([0] * (tiles * tm)), ints([0] * tiles), ints([0])
+        return lambda: kernels.route(x, w, None, top, i, v, srt, grp, cnt, tile_rows=tm)
+
+    def convolved(lengths, C, taps):
+        R, T = len(lengths), sum(lengths)
+        x, w, state, out = (torch.randn(*s, device=DEV) for s in ((T, C), (C, taps), (R, (taps - 1) * C + 4), (T, C)))
+        starts = np.cumsum([0] + lengths)[:-1].tolist()
+        args = ints([r for r, n in enumerate(lengths) for _ in range(n)]), ints(starts), ints(lengths), ints(list(range(R)))
+        return lambda: kernels.causal_conv(x, 0, w, None, state, 0, *args, out)
+
+    small = kernels.grouped_tile_rows()
+    for call, launches in ((routed(8, small), 1), (routed(9, small), 2), (routed(8, 128), 2), (convolved([1, 1], 8, 3), 1), (convolved([1, 1], 6, 3), 2),
+                           (convolved([1, 1], 8, 5), 2), (convolved([3, 2], 8, 3), 2), (convolved([1], 8, 1), 1)):
+        before = kernels.launch_count()
+        with kernels.record() as made:
+            call()
+        assert kernels.launch_count() - before == launches == made.program.launches
+        made.program.run()
+        assert kernels.launch_count() - before == 2 * launches
+    torch.cuda.synchronize()
+
+
 @pytest.mark.parametrize("gated", ["silu", None])
 @pytest.mark.parametrize("dtype", [*DTYPES, "32-bit inputs"])
 @pytest.mark.parametrize("N, K", [(18, 8), (33, 264), (16, 2056)])
