@@ -459,9 +459,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
         meta[2 * Cfg::kMetaRows + i] = row_req[t];
     }
     __syncthreads();
-    // ends[i]: the items that requests 0 .. i have; every warp adds them up for itself (the same values to the same places), which
-    // costs less than another barrier
-    int* ends = meta + 3 * Cfg::kMetaRows;
+    int* ends = meta + 3 * Cfg::kMetaRows;             // ends[i]: the items that requests 0 .. i have
     int first_item = 0, total = n_rows * Hkv * n_chunks, rounds_end = 0, last_item = 0;
     const int stride = gridDim.x * Cfg::kWarps;
     if constexpr (COMPACT) {
@@ -478,10 +476,10 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
                 const int up = __shfl_up_sync(0xffffffffu, n, d);
                 if (lane >= d) n += up;
             }
-            if (base + lane < n_rows) ends[base + lane] = all + n;
-            all += __shfl_sync(0xffffffffu, n, 31);
+            if (warp == 0 && base + lane < n_rows) ends[base + lane] = all + n;
+            all += __shfl_sync(0xffffffffu, n, 31);    // (every warp has the sum)
         }
-        __syncwarp();
+        __syncthreads();
         // whole rounds of the grid's warps, then every CTA an equal share of what is left
         total = all;
         rounds_end = all / stride * stride;

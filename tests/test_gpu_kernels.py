@@ -488,11 +488,111 @@ def test_attention_decode_contexts_of_one_chunk(H, Hkv, hd, ps, decode_chunks):
 @pytest.mark.parametrize("window", [None, 300])
 @pytest.mark.parametrize("hd,requests", [(64, 33), (128, 70), (32, 513)])
 def test_attention_decode_of_many_lengths(hd, requests, window):
-    """Requests of one chunk to six beside each other, more than one round of a warp over them, and more than the
-    descriptors in shared memory hold."""
+    """Requests of one chunk to six beside each other, at most an item for each warp, and more than the descriptors in shared
+    memory hold."""
     lens = [1 + (i * 397) % 1400 if requests < 100 or i % 50 == 0 else 1 + (i * 37) % 80 for i in range(requests)]
     got, want = _attention_case("bfloat16", 4, 2, hd, 16, ctx_lens=lens, q_lens=[1] * requests, window=window, seed=31, fast=True)
     close(got, want, "bfloat16", "attention of many lengths", bf16_tol=1e-2)
+
+
+def _decode_rows(H, Hkv, hd, lens, seed, ps=16):
+    """A decoding step's tensors: one query for each of ``lens`` cached positions, pages scattered over a cache of random values."""
+    g = torch.Generator(DEV).manual_seed(seed)
+    need = [(n + ps - 1) // ps for n in lens]
+    order = torch.randperm(sum(need) + 3, generator=g, device=DEV, dtype=torch.int32)
+    tables = torch.full((len(lens), max(need)), -1, dtype=torch.int32, device=DEV)
+    for r, (at, n) in enumerate(zip([sum(need[:r]) for r in range(len(need))], need)):
+        tables[r, :n] = order[at:at + n]
+    kc, vc = (torch.randn(order.numel(), Hkv, ps, hd, generator=g, device=DEV).to(torch.bfloat16) for _ in range(2))
+    q = torch.randn(len(lens), H * hd, generator=g, device=DEV).to(torch.bfloat16)
+    return q, kc, vc, tables, torch.tensor(lens, dtype=torch.int32, device=DEV) - 1
+
+
+def _decode(q, kc, vc, tables, positions, H, window, group, n_chunks, **more):
+    """The step's rows in launches of ``group`` requests each."""
+    Hkv, ps, hd = kc.shape[1:]
+    out, n = torch.full_like(q, float("nan")), q.shape[0]
+    req = torch.arange(n, dtype=torch.int32, device=DEV)
+    po, ml = torch.empty(group * H * n_chunks * hd, device=DEV), torch.empty(group * H * n_chunks * 2, device=DEV)
+    for at in range(0, n, group):
+        K().attention_decode(q, kc, vc, out, req[at:at + group].contiguous(), req, positions, tables, H, Hkv, hd, ps, hd ** -0.5, window, po, ml,
+                             n_chunks, n_chunks, **more)
+    assert K().gemm_tc_status(torch.device(DEV)) == 0
+    return out
+
+
+def _lengths_of(chunks, requests, chunk):
+    """Context lengths of ``requests`` requests that reach into ``chunks`` chunks altogether, ragged ends among them."""
+    each = [1 + (i * 5) % 8 for i in range(requests)]
+    i = 0
+    while sum(each) != chunks:
+        each[i % requests] = max(1, each[i % requests] + (1 if sum(each) < chunks else -1))
+        i += 1
+    return [(n - 1) * chunk + 1 + (i * 97) % chunk for i, n in enumerate(each)]
+
+
+@pytest.mark.parametrize("over", [-1, 0, 1, 20, 100])
+@pytest.mark.parametrize("H,Hkv,hd", [(16, 8, 64), (8, 8, 128), (24, 8, 32)])
+def test_attention_decode_in_whole_rounds(H, Hkv, hd, over):
+    """Visible items of two whole rounds of the grid's warps and ``over`` chunks (of 8 key/value heads each) more: none left, fewer
+    than there are CTAs, no multiple of them, several for a CTA, and one round that is not whole. The same bits as in launches
+    of 15 requests, which deal out the whole rectangle, with a window too; against the plain result for one request."""
+    sms, chunk = torch.cuda.get_device_properties(0).multi_processor_count, K().attention_chunk_keys()
+    warps = 4 if hd == 128 else 8
+    lens = _lengths_of((2 * sms * warps) // Hkv + over, 90 if hd != 128 else 45, chunk)
+    q, kc, vc, tables, pos = _decode_rows(H, Hkv, hd, lens, over + hd)
+    chunks = (max(lens) + chunk - 1) // chunk
+    for window in (None, 700):
+        got = _decode(q, kc, vc, tables, pos, H, window, len(lens), chunks)
+        assert torch.equal(got, _decode(q, kc, vc, tables, pos, H, window, 15, chunks)) and not torch.isnan(got).any()
+    r = max(range(len(lens)), key=lambda i: lens[i])
+    k, v = (c[tables[r].long().clamp(min=0)].transpose(1, 2).reshape(-1, Hkv, hd)[:lens[r]].float().cpu() for c in (kc, vc))
+    full = torch.zeros(lens[r], H, hd)
+    full[-1] = q[r].view(H, hd).float().cpu()
+    want = pm.plain_attention(full, k, v, hd ** -0.5, 700)[-1:]
+    close(got[r].view(1, H, hd), want, "bfloat16", "the longest request", bf16_tol=1e-2)
+
+
+@pytest.mark.parametrize("more", ["plain", "sink", "gate", "gate by value", "cap"])
+@pytest.mark.parametrize("H,Hkv,hd,requests", [(12, 1, 64, 16), (18, 2, 128, 33), (9, 1, 16, 40), (4, 2, 16, 17), (6, 2, 64, 100)])
+def test_attention_decode_of_many_requests_in_every_form(H, Hkv, hd, requests, more):
+    """Groups of more than eight heads and of fewer, every head size, and what may follow the softmax, at 16 requests and more:
+    the same bits as in launches of 15."""
+    lens = [1 + (i * 397) % 1900 for i in range(requests)]
+    q, kc, vc, tables, pos = _decode_rows(H, Hkv, hd, lens, hd + requests)
+    z = torch.randn(requests, H * hd, generator=torch.Generator(DEV).manual_seed(1), device=DEV)
+    args = {"plain": {}, "sink": {"sink": True}, "gate": {"gate": z, "out_scale": 0.5}, "gate by value": {"gate": z, "gate_dims": hd},
+            "cap": {"softcap": 2.0}}[more]
+    chunks = (max(lens) + 255) // 256
+    for window in (None, 600):
+        got = _decode(q, kc, vc, tables, pos, H, window, requests, chunks, **args)
+        assert torch.equal(got, _decode(q, kc, vc, tables, pos, H, window, 15, chunks, **args)) and not torch.isnan(got).any()
+
+
+def test_attention_decode_of_a_repeated_graph_while_contexts_grow():
+    """The kernel reads positions ahead of its wait: a graph repeated over positions that are moved on in place, past the ends of
+    chunks, gives what a fresh launch gives."""
+    H, Hkv, hd, requests = 16, 4, 64, 40
+    lens = [700 + (i * 37) % 600 for i in range(requests)]
+    q, kc, vc, tables, pos = _decode_rows(H, Hkv, hd, lens, 3)
+    chunks, moving = (max(lens) + 255) // 256, pos - 690
+    req = torch.arange(requests, dtype=torch.int32, device=DEV)
+    po, ml = torch.empty(requests * H * chunks * hd, device=DEV), torch.empty(requests * H * chunks * 2, device=DEV)
+    out = torch.empty_like(q)
+
+    def step():
+        K().attention_decode(q, kc, vc, out, req, req, moving, tables, H, Hkv, hd, 16, hd ** -0.5, None, po, ml, chunks, chunks)
+
+    step()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph), K().on_current_stream():
+        step()
+    for at in (690, 650, 446, 435, 434, 178, 1, 0):
+        moving.copy_(pos - at)
+        out.fill_(float("nan"))
+        graph.replay()
+        assert torch.equal(out, _decode(q, kc, vc, tables, pos - at, H, None, 15, chunks)), at
 
 
 @pytest.mark.parametrize("far", [0, 15, 16, 63, 64, 255, 256, 511, 597])
