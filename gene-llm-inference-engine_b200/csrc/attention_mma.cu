@@ -351,7 +351,7 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
 // neighbouring pages at a time; a run of its own per CTA: 6 % slower at 64 requests of 8,192), and of what is left an equal share to every CTA: an SM's share
 // of the bytes decides when it is done (its warps share one path to memory), and with requests of different lengths, or
 // windows, many (request, chunk) pairs of the rectangle n_rows x n_chunks are empty: 64 requests of 380 to 1,900 positions
-// 42.9 -> 36.2 us a layer of the 1B sizes, 23 requests beside a portion at the 3B sizes 37.8 -> 29.2. Finding the items costs what
+// 42.9 -> 36.0 us a layer of the 1B sizes, 23 requests beside a portion at the 3B sizes 37.8 -> 28.2. Finding the items costs what
 // a few requests seldom give back: a step of eight requests of one length is 0.4 % faster with the rectangle dealt out as it is.
 // Each warp owns a ring of three stages (K tile + V tile) filled by TMA: one lane issues one box
 // per page and head (pages [pages, Hkv, page_size, hd] are rows of a 2D tensor map), running up to

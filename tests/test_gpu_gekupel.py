@@ -397,7 +397,7 @@ def test_routing_and_expert_products(dtype, T, E, top, D, I):
 @pytest.mark.parametrize("scores", ["sigmoid", "softmax"])
 @pytest.mark.parametrize("E, D, T", [(8, 2048, 131), (9, 1100, 66), (40, 96, 65)])
 def test_routing_of_many_tokens_and_of_few(E, D, T, scores):
-    """Several tokens a block, one a block, and up to eight in a cluster that also buckets them: the same experts and the same bits."""
+    """A token a block, with eight loads in flight and with 32, and up to eight in a cluster that also buckets them: the same experts and the same bits."""
     from geneinfer_b200.ops import kernels
     g = torch.Generator().manual_seed(E)
     x, w, corr, gw = (torch.randn(*s, generator=g).to(DEV) for s in ((T, D), (E, D), (E,), (D,)))
