@@ -98,11 +98,16 @@ constexpr int kSampleParts = 8, kBins = 1024, kDigit = 10;
 constexpr int kMassBits = 12;                  // a mantissa goes into two words of 12 bits: slices of up to 2^20 values cannot overflow them
 constexpr int kNarrowVocab = kSampleParts << 20;      // above: whole mantissas in 64-bit words (whose atomics are slower)
 
+// A warp's piece stays in registers, kHeld values a lane, where it fits (vocabularies of up to 131,072): read once instead of
+// in every pass, each a wait for L2 (six rows of 128,256, drawn with every kind of filter: 92 -> 62 us).
+constexpr int kHeld = 16;
+
 template <bool kWide> struct SampleShared {
     using Low = typename std::conditional<kWide, unsigned long long, unsigned>::type;
-    unsigned count[2][kBins];
-    Low low[2][kBins];
-    unsigned high[2][kBins];                   // histograms of this CTA's piece; the two sets take turns
+    static constexpr int kSets = kWide ? 2 : 3;      // histograms of this CTA's piece: two sets take turns, the third keeps the
+    unsigned count[kSets][kBins];                    // first pass, which is the same for every descent of a row
+    Low low[kSets][kBins];
+    unsigned high[kSets][kBins];
     double cta_max, cta_sum, cta_mass;         // each written once and read by the cluster behind its own barrier
     int cta_equal;
     double warp_mass[32];
@@ -148,36 +153,43 @@ __device__ __forceinline__ double block_sum_double(double v, double* scratch) {
 
 // Walks the row's values from the largest downwards, ten bits of them per pass (values are at most 1: 30 bits): in each pass
 // the bin is chosen in which the running total (of ones if by_count, else of probabilities) first reaches (inclusive) or
-// exceeds the target. Where rounding never lets it, the lowest bin that weighs anything is chosen. The piece
-// [begin, end) is the calling warp's. `turn` counts the passes of the row.
-template <bool kWide>
-__device__ Found sample_descend(const float* __restrict__ probs, int begin, int end, bool by_count, double target, bool inclusive,
-                                SampleShared<kWide>& s, int& turn, cg::cluster_group& cluster) {
+// exceeds the target. Where rounding never lets it, the lowest bin that weighs anything is chosen.
+// `each` calls its argument with every place and value of the calling warp's piece. `turn` counts the passes that take turns with the
+// histograms, `descents` the row's descents.
+template <bool kWide, typename Each>
+__device__ __forceinline__ Found sample_descend(const Each& each, bool by_count, double target, bool inclusive,
+                                SampleShared<kWide>& s, int& turn, int& descents, cg::cluster_group& cluster) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     Found f{0u, 0.0, 0, 0};
     unsigned mask = 0u;
     for (int shift = 20; shift >= 0; shift -= kDigit) {
-        const int set = turn++ & 1;
-        s.count[set][threadIdx.x] = 0u;
-        s.low[set][threadIdx.x] = 0u;
-        s.high[set][threadIdx.x] = 0u;
+        const bool first_pass = !kWide && shift == 20;
+        const int set = first_pass ? SampleShared<kWide>::kSets - 1 : turn++ & 1;
+        const bool fill = !(first_pass && descents > 0);
+        if (fill) {
+            s.count[set][threadIdx.x] = 0u;
+            s.low[set][threadIdx.x] = 0u;
+            s.high[set][threadIdx.x] = 0u;
+        }
         if (threadIdx.x == 0) { s.first = kBins; s.last = -1; }
         __syncthreads();
-        for (int i = begin + lane; i < end; i += 32) {
-            const unsigned bits = __float_as_uint(probs[i]);
-            if ((bits & mask) == f.bits) {
-                const unsigned digit = (bits >> shift) & (kBins - 1);
-                const unsigned m = static_cast<unsigned>(sample_mantissa(bits));
-                atomicAdd(&s.count[set][digit], 1u);
-                if constexpr (kWide) {
-                    atomicAdd(&s.low[set][digit], static_cast<unsigned long long>(m));
-                } else {
-                    atomicAdd(&s.low[set][digit], m & ((1u << kMassBits) - 1));
-                    atomicAdd(&s.high[set][digit], m >> kMassBits);
+        if (fill) {
+            each([&](int, float value) {
+                const unsigned bits = __float_as_uint(value);
+                if ((bits & mask) == f.bits) {
+                    const unsigned digit = (bits >> shift) & (kBins - 1);
+                    const unsigned m = static_cast<unsigned>(sample_mantissa(bits));
+                    atomicAdd(&s.count[set][digit], 1u);
+                    if constexpr (kWide) {
+                        atomicAdd(&s.low[set][digit], static_cast<unsigned long long>(m));
+                    } else {
+                        atomicAdd(&s.low[set][digit], m & ((1u << kMassBits) - 1));
+                        atomicAdd(&s.high[set][digit], m >> kMassBits);
+                    }
                 }
-            }
+            });
+            cluster.sync();
         }
-        cluster.sync();
         // thread t has the t-th bin from the top: its totals over the cluster, then a scan over the block
         const int bin = kBins - 1 - threadIdx.x;
         unsigned long long low = 0, high = 0;
@@ -222,6 +234,7 @@ __device__ Found sample_descend(const float* __restrict__ probs, int begin, int 
         f.bits |= static_cast<unsigned>(kBins - 1 - chosen) << shift;
         mask |= static_cast<unsigned>(kBins - 1) << shift;
     }
+    ++descents;
     return f;
 }
 
@@ -238,7 +251,8 @@ __device__ __forceinline__ int sample_count_to(double above, double w, int n, do
 }
 
 // probs: scratch [rows, V] floats.
-template <bool kWide>
+// kInRegs: every warp's piece fits kHeld values a lane, and probs is not used.
+template <bool kWide, bool kInRegs>
 __global__ void __cluster_dims__(kSampleParts, 1, 1) __launch_bounds__(kSampleThreads)
 sample_kernel(const float* __restrict__ logits, float* __restrict__ probs_all, int V,
               const float* __restrict__ temperature, const int* __restrict__ top_k,
@@ -258,9 +272,38 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ probs_all, i
     const int slice_begin = min(V, part * slice), slice_end = min(V, slice_begin + slice);
     const int begin = min(slice_end, slice_begin + warp * piece), end = min(slice_end, begin + piece);
 
+    float held[kInRegs ? kHeld : 1];
+    // every place of this lane and its value, in order
+    auto each = [&](auto f) {
+        if constexpr (kInRegs) {
+#pragma unroll
+            for (int u = 0; u < kHeld; ++u)
+                if (begin + lane + 32 * u < end) f(begin + lane + 32 * u, held[u]);
+        } else {
+            for (int i = begin + lane; i < end; i += 32) f(i, probs[i]);
+        }
+    };
+    // every value of this lane replaced: in registers, else in probs (from the logits the first time)
+    auto replace = [&](const float* from, auto f) {
+        if constexpr (kInRegs) {
+#pragma unroll
+            for (int u = 0; u < kHeld; ++u)
+                if (begin + lane + 32 * u < end) held[u] = f(held[u]);
+        } else {
+            for (int i = begin + lane; i < end; i += 32) probs[i] = f(from[i]);
+        }
+    };
+
     // max
     float mx = -INFINITY;
-    for (int i = begin + lane; i < end; i += 32) mx = fmaxf(mx, row[i]);
+    if constexpr (kInRegs) {
+#pragma unroll
+        for (int u = 0; u < kHeld; ++u) held[u] = begin + lane + 32 * u < end ? row[begin + lane + 32 * u] : -INFINITY;
+#pragma unroll
+        for (int u = 0; u < kHeld; ++u) mx = fmaxf(mx, held[u]);
+    } else {
+        for (int i = begin + lane; i < end; i += 32) mx = fmaxf(mx, row[i]);
+    }
     mx = warp_max(mx);
     if (lane == 0) s.red[warp] = static_cast<double>(mx);
     __syncthreads();
@@ -275,11 +318,11 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ probs_all, i
 
     // p_i = exp((l_i - max)/T), sum in double, then scaled by (float)(1/sum)
     double mine = 0.0;
-    for (int i = begin + lane; i < end; i += 32) {
-        const float e = expf((row[i] - mx) / temp);
-        probs[i] = e;
+    replace(row, [&](float x) {
+        const float e = expf((x - mx) / temp);
         mine += static_cast<double>(e);
-    }
+        return e;
+    });
     mine = block_sum_double(mine, s.red);
     if (threadIdx.x == 0) s.cta_sum = mine;
     cluster.sync();
@@ -287,11 +330,11 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ probs_all, i
     for (int p = 0; p < kSampleParts; ++p) sum += *cluster.map_shared_rank(&s.cta_sum, p);
     const float inv_sum = static_cast<float>(1.0 / sum);
     mine = 0.0;
-    for (int i = begin + lane; i < end; i += 32) {
-        const float p = probs[i] * inv_sum;
-        probs[i] = p;
+    replace(probs, [&](float x) {
+        const float p = x * inv_sum;
         mine += static_cast<double>(p);
-    }
+        return p;
+    });
     mine = warp_sum_double(mine);
     if (lane == 0) s.warp_mass[warp] = mine;
     __syncthreads();
@@ -329,9 +372,9 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ probs_all, i
             }
             if (owner == warp) {
                 int pick = -1, fallback = max(begin, end - 1);
-                for (int base = begin; base < end && pick < 0; base += 32) {
+                auto look = [&](int base, float value) {          // the 32 values from base on
                     const int i = base + lane;
-                    double cum = i < end ? static_cast<double>(probs[i]) : 0.0;
+                    double cum = i < end ? static_cast<double>(value) : 0.0;
                     const unsigned some = __ballot_sync(0xffffffffu, cum > 0.0);
                     if (some) fallback = base + 31 - __clz(some);
 #pragma unroll
@@ -343,6 +386,13 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ probs_all, i
                     const unsigned over = __ballot_sync(0xffffffffu, i < end && target < cum);
                     if (over) pick = base + __ffs(over) - 1;
                     run = __shfl_sync(0xffffffffu, cum, 31);
+                };
+                if constexpr (kInRegs) {
+#pragma unroll
+                    for (int u = 0; u < kHeld; ++u)
+                        if (begin + 32 * u < end && pick < 0) look(begin + 32 * u, held[u]);
+                } else {
+                    for (int base = begin; base < end && pick < 0; base += 32) look(base, base + lane < end ? probs[base + lane] : 0.f);
                 }
                 if (lane == 0) out[r] = pick >= 0 ? pick : fallback;
             }
@@ -355,10 +405,10 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ probs_all, i
         unsigned bound_bits = 0u;        // smallest kept probability's bits
         int bound_take = 0;              // how many elements equal to it are kept (index order)
         bool bounded = false;
-        int turn = 0;
+        int turn = 0, descents = 0;
 
         if (use_k) {
-            const Found f = sample_descend(probs, begin, end, true, static_cast<double>(k), true, s, turn, cluster);
+            const Found f = sample_descend<kWide>(each, true, static_cast<double>(k), true, s, turn, descents, cluster);
             bound_bits = f.bits;
             bound_take = k - f.count_above;
             bounded = true;
@@ -368,7 +418,7 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ probs_all, i
             // shortest prefix with cum >= top_p * kept_mass, inside the current kept set. The descent runs over all elements;
             // as the kept set is a prefix of the same order, the crossing lies inside it unless rounding pushes it out.
             const double threshold = static_cast<double>(tp) * kept_mass;
-            const Found f = sample_descend(probs, begin, end, false, threshold, true, s, turn, cluster);
+            const Found f = sample_descend<kWide>(each, false, threshold, true, s, turn, descents, cluster);
             const double w = static_cast<double>(__uint_as_float(f.bits));
             const int take = w > 0.0 ? sample_count_to(f.mass_above, w, f.equal, threshold, true) : 1;
             if (!bounded || f.bits > bound_bits || (f.bits == bound_bits && take <= bound_take)) {
@@ -381,7 +431,7 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ probs_all, i
 
         // ---- draw: first token in the order with u * kept_mass < cum ----
         const double target = u * kept_mass;
-        const Found f = sample_descend(probs, begin, end, false, target, false, s, turn, cluster);
+        const Found f = sample_descend<kWide>(each, false, target, false, s, turn, descents, cluster);
         unsigned pick_bits = f.bits;
         int rank = sample_count_to(f.mass_above, static_cast<double>(__uint_as_float(pick_bits)), f.equal, target, false) - 1;
         // clamp to the kept set (rounding guard: the last kept token)
@@ -391,7 +441,7 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ probs_all, i
         }
         // the rank-th (0-based) index with those bits: the CTA, the warp, then the place
         int c = 0;
-        for (int i = begin + lane; i < end; i += 32) c += __float_as_uint(probs[i]) == pick_bits;
+        each([&](int, float value) { c += __float_as_uint(value) == pick_bits; });
         c = __reduce_add_sync(0xffffffffu, c);
         __syncthreads();
         if (lane == 0) s.counts[warp] = c;
@@ -405,14 +455,22 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ probs_all, i
         cluster.sync();
         for (int p = 0; p < part; ++p) ahead += *cluster.map_shared_rank(&s.cta_equal, p);
         if (rank >= ahead && rank < ahead + c) {
-            for (int base = begin; base < end; base += 32) {
+            bool done = false;
+            auto look = [&](int base, float value) {              // the 32 values from base on
                 const int i = base + lane;
-                const unsigned same = __ballot_sync(0xffffffffu, i < end && __float_as_uint(probs[i]) == pick_bits);
+                const unsigned same = __ballot_sync(0xffffffffu, i < end && __float_as_uint(value) == pick_bits);
                 if (rank < ahead + __popc(same)) {
                     if ((same >> lane & 1u) && ahead + __popc(same & ((1u << lane) - 1)) == rank) out[r] = i;
-                    break;
+                    done = true;
                 }
                 ahead += __popc(same);
+            };
+            if constexpr (kInRegs) {
+#pragma unroll
+                for (int u = 0; u < kHeld; ++u)
+                    if (begin + 32 * u < end && !done) look(begin + 32 * u, held[u]);
+            } else {
+                for (int base = begin; base < end && !done; base += 32) look(base, base + lane < end ? probs[base + lane] : 0.f);
             }
         }
     }
@@ -423,8 +481,9 @@ int launch_sample(const float* logits, float* probs, int rows, int V, const floa
                   const float* uniform, int* out, cudaStream_t st) {
     GI_REQUIRE(rows <= INT_MAX / kSampleParts, "sample: %d rows exceed the grid limit", rows);
     const dim3 grid(rows * kSampleParts), block(kSampleThreads);
-    if (V <= kNarrowVocab) launch_kernel((sample_kernel<false>), grid, block, 0, st, logits, probs, V, temperature, top_k, top_p, uniform, out);
-    else launch_kernel((sample_kernel<true>), grid, block, 0, st, logits, probs, V, temperature, top_k, top_p, uniform, out);
+    if (V <= kSampleParts * kSampleThreads * kHeld) launch_kernel((sample_kernel<false, true>), grid, block, 0, st, logits, probs, V, temperature, top_k, top_p, uniform, out);
+    else if (V <= kNarrowVocab) launch_kernel((sample_kernel<false, false>), grid, block, 0, st, logits, probs, V, temperature, top_k, top_p, uniform, out);
+    else launch_kernel((sample_kernel<true, false>), grid, block, 0, st, logits, probs, V, temperature, top_k, top_p, uniform, out);
     return check_launch("sample");
 }
 

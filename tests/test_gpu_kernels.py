@@ -367,6 +367,20 @@ def test_sample_rows_of_few_likely_tokens(V, top_k, top_p):
     assert got[3] == (0 if top_p < 1.0 else top_k - 1 if 0 < top_k < V else V - 1)      # no probabilities: an index, always the same
 
 
+@pytest.mark.parametrize("V", [131072, 131073])
+@pytest.mark.parametrize("top_k,top_p", [(0, 1.0), (40, 1.0), (0, 0.9), (40, 0.95)])
+def test_sample_of_the_largest_rows_held_in_registers_and_the_smallest_not(V, top_k, top_p):
+    g = torch.Generator().manual_seed(V)
+    logits = torch.randn(3, V, generator=g) * 2.5
+    logits[1, [3, V // 2, V - 1]] = 20.0                                        # equals in the first, a middle and the last piece
+    us = torch.tensor([0.31, 0.7, 0.97])
+    out = torch.full((3,), -1, dtype=torch.int32, device=DEV)
+    K().sample(logits.to(DEV), torch.empty(3 * V, device=DEV), torch.ones(3, device=DEV), torch.full((3,), top_k, dtype=torch.int32, device=DEV),
+               torch.full((3,), top_p, device=DEV), us.to(DEV), out)
+    for r, got in enumerate(out.cpu().tolist()):        # (a draw within rounding of a boundary may land on either side)
+        assert got in {pm.PlainSampler(1.0, top_k, top_p).sample(logits[r].numpy(), u) for u in (float(us[r]) - 1e-6, float(us[r]), float(us[r]) + 1e-6)}, r
+
+
 @pytest.mark.parametrize("V", [5, 3000, 128256])
 @pytest.mark.parametrize("top_k,top_p", [(0, 1.0), (3, 1.0), (0, 0.999), (3, 0.999)])
 def test_sample_with_uniform_numbers_outside_their_range(V, top_k, top_p):
