@@ -69,7 +69,7 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
                 int lda, int ldw, int ldc, int kc, int accumulate) {
     constexpr int BM = T::BM, BN = T::BN, TM = T::TM, TN = T::TN, kStages = T::kStages, kPad = T::kPad;
     extern __shared__ __align__(16) float smem[];
-    pdl_prologue();
+    pdl_launch_dependents();
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     constexpr int kWarpsM = T::kRowsT / T::kLaneM;
     const int tm = (warp % kWarpsM) * T::kLaneM + lane / T::kLaneN;
@@ -80,28 +80,29 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
 
     // thread t copies piece t % kPieces of rows t / kPieces, + kCopyRows, ... of either operand
     const int cr = t / T::kPieces, ck = (t % T::kPieces) * 4;
-    auto load = [&](int tile) {
-        if (tile < tiles) {
-            float* s = smem + (tile % kStages) * T::kStage + ck;
-            const int k = k_begin + tile * T::BK + ck;
-            const bool in_k = k < k_end;
+    auto load_a = [&](int tile) {
+        float* s = smem + (tile % kStages) * T::kStage + ck;
+        const int k = k_begin + tile * T::BK + ck;
 #pragma unroll
-            for (int r = 0; r < (BM + T::kCopyRows - 1) / T::kCopyRows; ++r) {
-                const int row = cr + r * T::kCopyRows;
-                if (BM % T::kCopyRows == 0 || row < BM) {
-                    const bool ok = in_k && m0 + row < M;
-                    copy16(s + row * kPad, ok ? A + static_cast<size_t>(m0 + row) * lda + k : A, ok);
-                }
-            }
-#pragma unroll
-            for (int r = 0; r < BN / T::kCopyRows; ++r) {
-                const int row = cr + r * T::kCopyRows;
-                const bool ok = in_k && n0 + row < N;
-                copy16(s + (BM + row) * kPad, ok ? W + static_cast<size_t>(n0 + row) * ldw + k : W, ok);
+        for (int r = 0; r < (BM + T::kCopyRows - 1) / T::kCopyRows; ++r) {
+            const int row = cr + r * T::kCopyRows;
+            if (BM % T::kCopyRows == 0 || row < BM) {
+                const bool ok = k < k_end && m0 + row < M;
+                copy16(s + row * kPad, ok ? A + static_cast<size_t>(m0 + row) * lda + k : A, ok);
             }
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    auto load_w = [&](int tile) {
+        float* s = smem + (tile % kStages) * T::kStage + ck;
+        const int k = k_begin + tile * T::BK + ck;
+#pragma unroll
+        for (int r = 0; r < BN / T::kCopyRows; ++r) {
+            const int row = cr + r * T::kCopyRows;
+            const bool ok = k < k_end && n0 + row < N;
+            copy16(s + (BM + row) * kPad, ok ? W + static_cast<size_t>(n0 + row) * ldw + k : W, ok);
+        }
+    };
+    auto commit = []() { asm volatile("cp.async.commit_group;" ::: "memory"); };
 
     unsigned long long acc[TM][TN];
 #pragma unroll
@@ -109,11 +110,20 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
 #pragma unroll
         for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
 
-    for (int i = 0; i < kStages - 1; ++i) load(i);
+    // the weights of the first tiles are asked for before the wait for the kernel ahead: no earlier kernel writes them (six rows in a
+    // token's step: N = 16,384, K = 2,048 33.2 -> 28.9 us, N = 3,072 8.4 -> 7.5)
+    for (int i = 0; i < kStages - 1; ++i)
+        if (i < tiles) load_w(i);
+    pdl_wait();
+    for (int i = 0; i < kStages - 1; ++i) {
+        if (i < tiles) load_a(i);
+        commit();
+    }
     for (int tile = 0; tile < tiles; ++tile) {
         asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
         __syncthreads();                              // the tile is there for all, and all are done with the one before it
-        load(tile + kStages - 1);
+        if (tile + kStages - 1 < tiles) { load_a(tile + kStages - 1); load_w(tile + kStages - 1); }
+        commit();
         const float* sa = smem + (tile % kStages) * T::kStage + tm * kPad;
         const float* sw = smem + (tile % kStages) * T::kStage + (BM + tn) * kPad;
 #pragma unroll
