@@ -18,6 +18,27 @@
 
 namespace gi {
 
+// Two 32-bit multiply-adds (products) in one instruction, each rounded like fmaf's (a product's).
+__device__ __forceinline__ unsigned long long fma_pair(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ unsigned long long mul_pair(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned long long make_pair(float a, float b) {
+    unsigned long long d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+    return d;
+}
+__device__ __forceinline__ float2 split_pair(unsigned long long v) {
+    float2 f;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+    return f;
+}
 __device__ __forceinline__ float silu_f(float z) { return z * (1.0f / (1.0f + expf(-z))); }
 __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 
@@ -162,7 +183,9 @@ causal_conv_walk_kernel(const float* __restrict__ in, int ld, int in_off, const 
 }
 
 // ---------------------------------------------------------------------------------- the recurrence
-// A block owns 32 columns of one head's state of one request, each thread a few rows x 4 columns of it in registers.
+// A block owns 32 columns of one head's state of one request, each thread a few rows x 4 columns of it in registers, as pairs of
+// neighbouring columns: two multiply-adds an instruction, the factors of a row staged twice so that they are read as pairs (1,153
+// tokens of 16 heads of 128 x 128: 100 -> 93 us, 2,048 tokens of 32 heads of 128 x 64: 137 -> 121, a token with a decay per row 10.3 -> 6.6).
 // Tokens are staged a chunk at a time in shared memory (activated, with their a and b).
 //
 // Long segments are cut into parts of part_len tokens that run side by side (kParts): every part starts from a zero
@@ -172,7 +195,7 @@ causal_conv_walk_kernel(const float* __restrict__ in, int ld, int in_off, const 
 // o_t += A_t S_p^T q_t (apply kernel, a small matrix product per part). Steps whose segments all fit one part run
 // the scan kernel alone, straight on the state slot.
 constexpr int kScanCols = 32;
-constexpr int kScanChunk = 16;
+constexpr int kScanChunk = 8;
 
 struct ScanArgs {
     const float* q; const float* k; const float* v;      // rows of ld_q / ld_k / ld_v floats, at these column offsets
@@ -217,15 +240,15 @@ linear_scan_kernel(const ScanArgs p) {
     // chunk of tokens.
     constexpr int kGroups = kDk / kRT;                    // row groups
     constexpr int kThreads = kGroups * 8;
-    constexpr int kChunk = kDk >= 128 ? kScanChunk / 2 : kScanChunk;      // tokens staged at a time (shared memory)
+    constexpr int kChunk = kDk > 128 ? kScanChunk / 2 : kScanChunk;       // tokens staged at a time (shared memory)
     constexpr int kPerThread = kChunk * kDk / kThreads;   // q (and k) values a thread stages per chunk
     constexpr int kVPerThread = kChunk * kScanCols / kThreads;
-    __shared__ __align__(16) float s_q[kChunk][kDk];
-    __shared__ __align__(16) float s_k[kChunk][kDk];
+    __shared__ __align__(16) float2 s_q[kChunk][kDk];     // twice each: the factors of a pair of columns
+    __shared__ __align__(16) float2 s_k[kChunk][kDk];
     __shared__ __align__(16) float s_v[kChunk][kScanCols];
     __shared__ __align__(16) float s_o[kChunk][kGroups][kScanCols];
     __shared__ float s_a[kChunk], s_b[kChunk];
-    __shared__ __align__(16) float s_av[kRowDecay ? kChunk : 1][kRowDecay ? kDk : 4];      // per-row decays of the staged tokens
+    __shared__ __align__(16) float2 s_av[kRowDecay ? kChunk : 1][kRowDecay ? kDk : 2];      // per-row decays of the staged tokens
     const int tile = blockIdx.x, h = blockIdx.y;
     const int r = kParts ? blockIdx.z / p.max_parts : blockIdx.z;
     const int part_idx = kParts ? blockIdx.z % p.max_parts : 0;
@@ -243,13 +266,15 @@ linear_scan_kernel(const ScanArgs p) {
         S = p.state + static_cast<long long>(p.state_slots[r]) * p.slot_stride + p.state_off +
             static_cast<long long>(h) * p.dk * p.dv;
     }
-    float s[kRT][4];
+    unsigned long long s[kRT][2];                          // pairs of neighbouring columns
 #pragma unroll
     for (int i = 0; i < kRT; ++i) {
         const int row = rg * kRT + i;
+        float v[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c)
-            s[i][c] = (!kParts && row < p.dk && j0 + c < p.dv) ? S[static_cast<size_t>(row) * p.dv + j0 + c] : 0.f;
+            v[c] = (!kParts && row < p.dk && j0 + c < p.dv) ? S[static_cast<size_t>(row) * p.dv + j0 + c] : 0.f;
+        s[i][0] = make_pair(v[0], v[1]); s[i][1] = make_pair(v[2], v[3]);
     }
     const float skip = p.skip ? p.skip[h] : 0.f;
     const float a_const = p.decay ? p.decay[h] : 0.f;
@@ -292,9 +317,13 @@ linear_scan_kernel(const ScanArgs p) {
 #pragma unroll
         for (int u = 0; u < kPerThread; ++u) {
             const int e = threadIdx.x + u * kThreads;
-            s_q[e / kDk][e % kDk] = (p.act ? silu_f(qv[u]) : qv[u]) * p.q_scale;
-            s_k[e / kDk][e % kDk] = p.act ? silu_f(kv[u]) : kv[u];
-            if (kRowDecay) s_av[e / kDk][e % kDk] = (e / kDk < m && e % kDk < p.dk) ? row_decay(zv[u], p.inv_tau) : 1.f;
+            const float q = (p.act ? silu_f(qv[u]) : qv[u]) * p.q_scale, k = p.act ? silu_f(kv[u]) : kv[u];
+            s_q[e / kDk][e % kDk] = make_float2(q, q);
+            s_k[e / kDk][e % kDk] = make_float2(k, k);
+            if (kRowDecay) {
+                const float a = (e / kDk < m && e % kDk < p.dk) ? row_decay(zv[u], p.inv_tau) : 1.f;
+                s_av[e / kDk][e % kDk] = make_float2(a, a);
+            }
         }
 #pragma unroll
         for (int u = 0; u < kVPerThread; ++u) {
@@ -328,7 +357,7 @@ linear_scan_kernel(const ScanArgs p) {
                 const int i = threadIdx.x + u * kThreads;
                 if (i < p.dk) {
                     for (int tt = 0; tt < m; ++tt) {
-                        cumv[u] *= s_av[tt][i];
+                        cumv[u] *= s_av[tt][i].x;
                         p.ws_decay[(static_cast<size_t>(s0 + c0 + tt) * p.H + h) * p.dk + i] = cumv[u];
                     }
                 }
@@ -336,30 +365,30 @@ linear_scan_kernel(const ScanArgs p) {
         }
         for (int tt = 0; tt < m; ++tt) {
             const float a = s_a[tt], b = s_b[tt];
-            const float4 v4 = *reinterpret_cast<const float4*>(&s_v[tt][cg * 4]);
-            const float bv[4] = {b * v4.x, b * v4.y, b * v4.z, b * v4.w};
-            float o[4] = {0.f, 0.f, 0.f, 0.f};
-            const float4* k4 = reinterpret_cast<const float4*>(&s_k[tt][rg * kRT]);
-            const float4* q4 = reinterpret_cast<const float4*>(&s_q[tt][rg * kRT]);
+            const ulonglong2 v4 = *reinterpret_cast<const ulonglong2*>(&s_v[tt][cg * 4]);
+            const unsigned long long bb = make_pair(b, b), aa = make_pair(a, a);
+            const unsigned long long bv[2] = {mul_pair(bb, v4.x), mul_pair(bb, v4.y)};
+            unsigned long long o[2] = {0ull, 0ull};
+            const ulonglong2* k2 = reinterpret_cast<const ulonglong2*>(&s_k[tt][rg * kRT]);
+            const ulonglong2* q2 = reinterpret_cast<const ulonglong2*>(&s_q[tt][rg * kRT]);
+            const ulonglong2* a2 = reinterpret_cast<const ulonglong2*>(&s_av[kRowDecay ? tt : 0][kRowDecay ? rg * kRT : 0]);
 #pragma unroll
-            for (int i4 = 0; i4 < kRT / 4; ++i4) {
-                const float4 kk = k4[i4], qq = q4[i4];
-                const float kr[4] = {kk.x, kk.y, kk.z, kk.w}, qr[4] = {qq.x, qq.y, qq.z, qq.w};
-                float ar[4] = {a, a, a, a};
-                if (kRowDecay) {
-                    const float4 aa = reinterpret_cast<const float4*>(&s_av[tt][rg * kRT])[i4];
-                    ar[0] = aa.x; ar[1] = aa.y; ar[2] = aa.z; ar[3] = aa.w;
-                }
+            for (int i2 = 0; i2 < kRT / 2; ++i2) {
+                const ulonglong2 kk = k2[i2], qq = q2[i2];
+                const unsigned long long kr[2] = {kk.x, kk.y}, qr[2] = {qq.x, qq.y};
+                unsigned long long ar[2] = {aa, aa};
+                if (kRowDecay) { const ulonglong2 av = a2[i2]; ar[0] = av.x; ar[1] = av.y; }
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
+                for (int u = 0; u < 2; ++u) {
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        s[4 * i4 + u][c] = fmaf(ar[u], s[4 * i4 + u][c], kr[u] * bv[c]);
-                        o[c] = fmaf(s[4 * i4 + u][c], qr[u], o[c]);
+                    for (int c = 0; c < 2; ++c) {
+                        unsigned long long& x = s[2 * i2 + u][c];
+                        x = fma_pair(ar[u], x, mul_pair(kr[u], bv[c]));
+                        o[c] = fma_pair(x, qr[u], o[c]);
                     }
                 }
             }
-            *reinterpret_cast<float4*>(&s_o[tt][rg][cg * 4]) = make_float4(o[0], o[1], o[2], o[3]);
+            *reinterpret_cast<ulonglong2*>(&s_o[tt][rg][cg * 4]) = make_ulonglong2(o[0], o[1]);
         }
         __syncthreads();
         for (int e = threadIdx.x; e < m * kScanCols; e += kThreads) {
@@ -375,9 +404,11 @@ linear_scan_kernel(const ScanArgs p) {
 #pragma unroll
     for (int i = 0; i < kRT; ++i) {
         const int row = rg * kRT + i;
+        const float2 lo = split_pair(s[i][0]), hi = split_pair(s[i][1]);
+        const float v[4] = {lo.x, lo.y, hi.x, hi.y};
 #pragma unroll
         for (int c = 0; c < 4; ++c)
-            if (row < p.dk && j0 + c < p.dv) S[static_cast<size_t>(row) * p.dv + j0 + c] = s[i][c];
+            if (row < p.dk && j0 + c < p.dv) S[static_cast<size_t>(row) * p.dv + j0 + c] = v[c];
     }
 }
 
@@ -471,11 +502,11 @@ scan_apply_kernel(const ScanArgs p, int blocks_per_part) {            // grid (c
             s_q[e % kDk * kT + e / kDk] = (p.act ? silu_f(qv[u]) : qv[u]) * p.q_scale * cv[u];
         }
     }
-    float acc[8][kTN];
+    unsigned long long acc[8][kTN / 2];                // pairs of neighbouring columns
 #pragma unroll
     for (int m = 0; m < 8; ++m)
 #pragma unroll
-        for (int j = 0; j < kTN; ++j) acc[m][j] = 0.f;
+        for (int j = 0; j < kTN / 2; ++j) acc[m][j] = 0ull;
     for (int i0 = 0; i0 < p.dk; i0 += kApplyStep) {
         __syncthreads();
 #pragma unroll
@@ -485,15 +516,21 @@ scan_apply_kernel(const ScanArgs p, int blocks_per_part) {            // grid (c
         if (!works) continue;
 #pragma unroll
         for (int i = 0; i < kApplyStep; ++i) {
-            float l[8], x[kTN];
+            float l[8];
+            unsigned long long x[kTN / 2];
             *reinterpret_cast<float4*>(&l[0]) = *reinterpret_cast<const float4*>(s_q + (i0 + i) * kT + tm);
             *reinterpret_cast<float4*>(&l[4]) = *reinterpret_cast<const float4*>(s_q + (i0 + i) * kT + tm + 4);
 #pragma unroll
-            for (int j = 0; j < kTN; j += 4) *reinterpret_cast<float4*>(&x[j]) = *reinterpret_cast<const float4*>(s_x + i * kX + tn + j * 16);
+            for (int j = 0; j < kTN; j += 4) {
+                const ulonglong2 four = *reinterpret_cast<const ulonglong2*>(s_x + i * kX + tn + j * 16);
+                x[j / 2] = four.x; x[j / 2 + 1] = four.y;
+            }
 #pragma unroll
-            for (int m = 0; m < 8; ++m)
+            for (int m = 0; m < 8; ++m) {
+                const unsigned long long lm = make_pair(l[m], l[m]);
 #pragma unroll
-                for (int j = 0; j < kTN; ++j) acc[m][j] = fmaf(l[m], x[j], acc[m][j]);
+                for (int j = 0; j < kTN / 2; ++j) acc[m][j] = fma_pair(lm, x[j], acc[m][j]);
+            }
         }
     }
 #pragma unroll
@@ -505,7 +542,8 @@ scan_apply_kernel(const ScanArgs p, int blocks_per_part) {            // grid (c
 #pragma unroll
         for (int j = 0; j < kTN; ++j) {
             const int col = c0 + tn + (j & 3) + (j & 4) * 16;
-            if (col < p.dv) o[col] = fmaf(f, acc[m][j], o[col]);
+            const float2 two = split_pair(acc[m][j / 2]);
+            if (col < p.dv) o[col] = fmaf(f, j & 1 ? two.y : two.x, o[col]);
         }
     }
 }
