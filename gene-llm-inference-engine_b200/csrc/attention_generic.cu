@@ -13,16 +13,18 @@
 // p_j = exp(s_j) / (1 + sum exp(s_j))); ``gate`` multiplies head h's output by sigmoid(gate[t, h]);
 // ``out_scale`` multiplies the output by a constant.
 //
-// This kernel is the whole attention of the 32-bit path and the fallback of the bfloat16 path.
+// This kernel is the whole attention of the 32-bit path and the fallback of the bfloat16 path. A short context is a few
+// tiles, so what bounds it is how often its loads wait for one another: a lane asks for up to 16 pieces of its key's row at once, and for
+// its dimensions of a tile's first values before the scores of the tile, the rest in batches (a key's values at a time, behind a branch,
+// six rows of 100 positions and 32 heads took 25 us, 14 now; 268 rows 66, 60 now).
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace gi {
 
 constexpr int kAttWarps = 4;
 constexpr int kMaxHeadDim = 256;
-
-template <typename T>
-__device__ __forceinline__ float dot_row(const float* __restrict__ q, const T* __restrict__ k, int hd);
 
 // The same chain of multiply-adds, element by element: head sizes whose rows are not 16-byte pieces.
 template <typename T>
@@ -32,40 +34,57 @@ __device__ __forceinline__ float dot_row_scalar(const float* __restrict__ q, con
     return acc;
 }
 
-template <>
-__device__ __forceinline__ float dot_row<float>(const float* __restrict__ q, const float* __restrict__ k, int hd) {
+// PIECES 16-byte pieces of a key's row are in flight together.
+template <int PIECES>
+__device__ __forceinline__ float dot_row(const float* __restrict__ q, const float* __restrict__ k, int hd) {
     float acc = 0.f;
     const float4* k4 = reinterpret_cast<const float4*>(k);
-    for (int i = 0; i < hd / 4; ++i) {
-        const float4 v = k4[i];
-        acc = fmaf(q[4 * i + 0], v.x, acc);
-        acc = fmaf(q[4 * i + 1], v.y, acc);
-        acc = fmaf(q[4 * i + 2], v.z, acc);
-        acc = fmaf(q[4 * i + 3], v.w, acc);
+    for (int i0 = 0; i0 < hd / 4; i0 += PIECES) {
+        float4 v[PIECES];
+#pragma unroll
+        for (int u = 0; u < PIECES; ++u)
+            if (i0 + u < hd / 4) v[u] = k4[i0 + u];
+#pragma unroll
+        for (int u = 0; u < PIECES; ++u) {
+            if (i0 + u >= hd / 4) break;
+            const int i = 4 * (i0 + u);
+            acc = fmaf(q[i], v[u].x, acc);
+            acc = fmaf(q[i + 1], v[u].y, acc);
+            acc = fmaf(q[i + 2], v[u].z, acc);
+            acc = fmaf(q[i + 3], v[u].w, acc);
+        }
     }
     return acc;
 }
-
-template <>
-__device__ __forceinline__ float dot_row<__nv_bfloat16>(const float* __restrict__ q,
-                                                        const __nv_bfloat16* __restrict__ k, int hd) {
+template <int PIECES>
+__device__ __forceinline__ float dot_row(const float* __restrict__ q, const __nv_bfloat16* __restrict__ k, int hd) {
     float acc = 0.f;
     const uint4* k8 = reinterpret_cast<const uint4*>(k);
-    for (int i = 0; i < hd / 8; ++i) {
-        const uint4 raw = k8[i];
-        const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw);
+    for (int i0 = 0; i0 < hd / 8; i0 += PIECES) {
+        uint4 raw[PIECES];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float2 f = __bfloat1622float2(p[j]);
-            acc = fmaf(q[8 * i + 2 * j], f.x, acc);
-            acc = fmaf(q[8 * i + 2 * j + 1], f.y, acc);
+        for (int u = 0; u < PIECES; ++u)
+            if (i0 + u < hd / 8) raw[u] = k8[i0 + u];
+#pragma unroll
+        for (int u = 0; u < PIECES; ++u) {
+            if (i0 + u >= hd / 8) break;
+            const int i = 8 * (i0 + u);
+            const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw[u]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float2 f = __bfloat1622float2(p[j]);
+                acc = fmaf(q[i + 2 * j], f.x, acc);
+                acc = fmaf(q[i + 2 * j + 1], f.y, acc);
+            }
         }
     }
     return acc;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kAttWarps * 32)
+// DPL: dimensions per lane (hd <= 32 DPL). FEW: a few blocks an SM, each with as much in flight as its registers hold; else many blocks,
+// which hide one another's waits if there is room for them.
+template <typename T, int DPL, bool FEW>
+__global__ void __launch_bounds__(kAttWarps * 32, FEW ? 2 : 8)
 paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_cache,
                                const T* __restrict__ v_cache, T* __restrict__ out,
                                const int* __restrict__ row_req, const int* __restrict__ positions,
@@ -88,10 +107,11 @@ paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_
         s_q[d] = to_float(q[(static_cast<size_t>(t) * H + h) * hd + d]);
     __syncthreads();
 
-    constexpr int kDimsPerLane = kMaxHeadDim / 32;
-    float acc[kDimsPerLane];
+    constexpr int kPieces = FEW ? 16 : 4;
+    constexpr int kBatch = (FEW ? 32 : 8) / DPL;         // keys whose values are in flight together
+    float acc[DPL];
 #pragma unroll
-    for (int i = 0; i < kDimsPerLane; ++i) acc[i] = 0.f;
+    for (int i = 0; i < DPL; ++i) acc[i] = 0.f;
     float m = -INFINITY, l = 0.f;
 
     const int first_tile = lo / 32;
@@ -104,7 +124,22 @@ paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_
         if (valid) {
             const int page = table[j / page_size];
             row_off = ((static_cast<size_t>(page) * Hkv + g) * page_size + (j % page_size)) * hd;
-            score = (hd % 8 == 0 ? dot_row<T>(s_q, k_cache + row_off, hd) : dot_row_scalar<T>(s_q, k_cache + row_off, hd)) * scale;
+        }
+        T values[kBatch][DPL];
+        auto request = [&](int j0) {                      // the values of keys j0 .. of the tile (only of keys that the row sees)
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) {
+                const size_t off = __shfl_sync(0xffffffffu, static_cast<unsigned long long>(row_off), j0 + u);
+                const int key = tile * 32 + j0 + u;
+                if (key < lo || key > pos) continue;      // uniform across the warp
+#pragma unroll
+                for (int i = 0; i < DPL; ++i)
+                    if (lane + 32 * i < hd) values[u][i] = v_cache[off + lane + 32 * i];
+            }
+        };
+        request(0);
+        if (valid) {
+            score = (hd % 8 == 0 ? dot_row<kPieces>(s_q, k_cache + row_off, hd) : dot_row_scalar<T>(s_q, k_cache + row_off, hd)) * scale;
         }
         const float tile_max = warp_max(score);          // finite: a tile always holds a valid key
         const float m_new = fmaxf(m, tile_max);
@@ -112,24 +147,25 @@ paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_
         const float corr = (m == -INFINITY) ? 0.f : expf(m - m_new);
         l = l * corr + warp_sum(p);
 #pragma unroll
-        for (int i = 0; i < kDimsPerLane; ++i) acc[i] *= corr;
+        for (int i = 0; i < DPL; ++i) acc[i] *= corr;
         m = m_new;
-        for (int jj = 0; jj < 32; ++jj) {
-            const float pj = __shfl_sync(0xffffffffu, p, jj);
-            const size_t off = __shfl_sync(0xffffffffu, static_cast<unsigned long long>(row_off), jj);
-            if (pj == 0.f) continue;                      // uniform across the warp
-            const T* vrow = v_cache + off;
+#pragma unroll 1
+        for (int j0 = 0; j0 < 32; j0 += kBatch) {
+            if (j0 > 0) request(j0);
 #pragma unroll
-            for (int i = 0; i < kDimsPerLane; ++i) {
-                const int d = lane + 32 * i;
-                if (d < hd) acc[i] = fmaf(pj, to_float(vrow[d]), acc[i]);
+            for (int u = 0; u < kBatch; ++u) {
+                const float pj = __shfl_sync(0xffffffffu, p, j0 + u);
+                if (pj == 0.f) continue;                  // uniform across the warp (a key out of sight among them)
+#pragma unroll
+                for (int i = 0; i < DPL; ++i)
+                    if (lane + 32 * i < hd) acc[i] = fmaf(pj, to_float(values[u][i]), acc[i]);
             }
         }
     }
 
     if (lane == 0) { s_m[warp] = m; s_l[warp] = l; }
 #pragma unroll
-    for (int i = 0; i < kDimsPerLane; ++i) {
+    for (int i = 0; i < DPL; ++i) {
         const int d = lane + 32 * i;
         if (d < hd) s_acc[warp][d] = acc[i];
     }
@@ -179,16 +215,25 @@ static int gi_attention_generic_impl(const void* q, const void* k_cache, const v
     GI_REQUIRE(T <= 65535, "attention: %d rows in one step exceed the grid limit 65535", T);
     dim3 grid(H, T);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (dtype == kF32) {
-        launch_kernel((paged_attention_generic_kernel<float>), dim3(grid), dim3(kAttWarps * 32), 0, st, 
-            static_cast<const float*>(q), static_cast<const float*>(k_cache), static_cast<const float*>(v_cache),
-            static_cast<float*>(out), row_req, positions, block_tables, table_stride, H, Hkv, hd, page_size, scale,
+    auto launch = [&](auto kernel, auto* typed) {
+        using T = std::remove_pointer_t<decltype(typed)>;
+        launch_kernel(kernel, dim3(grid), dim3(kAttWarps * 32), 0, st,
+            static_cast<const T*>(q), static_cast<const T*>(k_cache), static_cast<const T*>(v_cache),
+            static_cast<T*>(out), row_req, positions, block_tables, table_stride, H, Hkv, hd, page_size, scale,
             window, sink, gate, gate_ld, gate_off, gate_dims, out_scale);
+    };
+    // up to two blocks an SM are few (268 rows with everything in flight, three blocks of 165 registers an SM: 105 us instead of 60)
+    const bool few = static_cast<long long>(H) * T <= 2 * 148;
+    auto typed = [&](auto* t) {
+        using V = std::remove_pointer_t<decltype(t)>;
+        if (hd <= 64) few ? launch(paged_attention_generic_kernel<V, 2, true>, t) : launch(paged_attention_generic_kernel<V, 2, false>, t);
+        else if (hd <= 128) few ? launch(paged_attention_generic_kernel<V, 4, true>, t) : launch(paged_attention_generic_kernel<V, 4, false>, t);
+        else few ? launch(paged_attention_generic_kernel<V, 8, true>, t) : launch(paged_attention_generic_kernel<V, 8, false>, t);
+    };
+    if (dtype == kF32) {
+        typed(static_cast<float*>(nullptr));
     } else if (dtype == kBF16) {
-        launch_kernel((paged_attention_generic_kernel<__nv_bfloat16>), dim3(grid), dim3(kAttWarps * 32), 0, st, 
-            static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k_cache),
-            static_cast<const __nv_bfloat16*>(v_cache), static_cast<__nv_bfloat16*>(out), row_req, positions,
-            block_tables, table_stride, H, Hkv, hd, page_size, scale, window, sink, gate, gate_ld, gate_off, gate_dims, out_scale);
+        typed(static_cast<__nv_bfloat16*>(nullptr));
     } else {
         GI_REQUIRE(false, "attention: unsupported dtype code %d", dtype);
     }
