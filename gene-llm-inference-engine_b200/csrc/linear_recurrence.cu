@@ -183,7 +183,7 @@ causal_conv_walk_kernel(const float* __restrict__ in, int ld, int in_off, const 
 }
 
 // ---------------------------------------------------------------------------------- the recurrence
-// A block owns 32 columns of one head's state of one request, each thread a few rows x 4 columns of it in registers, as pairs of
+// A block owns 32 columns (or more) of one head's state of one request, each thread a few rows x 4 columns of it in registers, as pairs of
 // neighbouring columns: two multiply-adds an instruction, the factors of a row staged twice so that they are read as pairs (1,153
 // tokens of 16 heads of 128 x 128: 100 -> 93 us, 2,048 tokens of 32 heads of 128 x 64: 137 -> 121, a token with a decay per row 10.3 -> 6.6).
 // Tokens are staged a chunk at a time in shared memory (activated, with their a and b).
@@ -194,7 +194,6 @@ causal_conv_walk_kernel(const float* __restrict__ in, int ld, int in_off, const 
 // (link kernel, a short loop per state element); and every token gets what the start state adds to it,
 // o_t += A_t S_p^T q_t (apply kernel, a small matrix product per part). Steps whose segments all fit one part run
 // the scan kernel alone, straight on the state slot.
-constexpr int kScanCols = 32;
 constexpr int kScanChunk = 8;
 
 struct ScanArgs {
@@ -230,31 +229,47 @@ __device__ __forceinline__ int parts_before(const ScanArgs& p, int r) {
 // (Left alone the compiler takes the kernel past 128 registers a thread, with a decay per row to 168, and a launch of a
 // few heads' blocks then needs a second, nearly empty round over the SMs: it is held to 512 threads an SM. Five blocks of 128
 // instead of four, which 96 registers allow without spills: 115 instead of 100 us at 640 blocks.)
-template <int kDk, int kRT, bool kParts, bool kRowDecay>
-__global__ void __launch_bounds__(kDk / kRT * 8, (kRowDecay || kDk <= 128) ? 512 / (kDk / kRT * 8) : 1)
+//
+// kCG: groups of four columns of a block. What a block does besides walking, activations and decays of each staged token, it does for all its
+// columns at once: parts of a long segment take 256 threads' worth of columns (1,153 tokens of 16 heads of 128 x 128 in 32
+// columns a block 93 us, in 64 86; a decay per row, 2,048 tokens of 16 heads of 64 x 128, 135 and in 128 columns 81), single
+// tokens the narrow blocks that give every SM one.
+template <int kDk, int kRT, int kCG, bool kRowDecay>
+struct ScanShared {
+    static constexpr int kGroups = kDk / kRT, kChunk = kDk > 128 ? kScanChunk / 2 : kScanChunk, kCols = 4 * kCG;      // kChunk: tokens staged at a time
+    float2 q[kChunk][kDk], k[kChunk][kDk];                // twice each: the factors of a pair of columns
+    float v[kChunk][kCols];
+    float o[kChunk][kGroups][kCols];
+    float2 av[kRowDecay ? kChunk : 1][kRowDecay ? kDk : 2];           // per-row decays of the staged tokens
+    float a[kChunk], b[kChunk];
+};
+template <int kDk, int kRT, int kCG, bool kParts, bool kRowDecay>
+__global__ void __launch_bounds__(kDk / kRT * kCG, (kRowDecay || kDk <= 128) ? 512 / (kDk / kRT * kCG) : 1)
 linear_scan_kernel(const ScanArgs p) {
     pdl_prologue();
     // A thread owns kRT rows x 4 columns of the state in registers (thread = row group x column group; a block covers
-    // all kDk padded rows and 32 columns): per token it reads kRT k and q values and 4 v values from shared memory
+    // all kDk padded rows and 4 kCG columns): per token it reads kRT k and q values and 4 v values from shared memory
     // for 4 kRT state elements. A token's output is the sum over the row groups, added up in their order once per
     // chunk of tokens.
     constexpr int kGroups = kDk / kRT;                    // row groups
-    constexpr int kThreads = kGroups * 8;
-    constexpr int kChunk = kDk > 128 ? kScanChunk / 2 : kScanChunk;       // tokens staged at a time (shared memory)
+    constexpr int kThreads = kGroups * kCG, kCols = 4 * kCG;
+    using Shared = ScanShared<kDk, kRT, kCG, kRowDecay>;
+    constexpr int kChunk = Shared::kChunk;
     constexpr int kPerThread = kChunk * kDk / kThreads;   // q (and k) values a thread stages per chunk
-    constexpr int kVPerThread = kChunk * kScanCols / kThreads;
-    __shared__ __align__(16) float2 s_q[kChunk][kDk];     // twice each: the factors of a pair of columns
-    __shared__ __align__(16) float2 s_k[kChunk][kDk];
-    __shared__ __align__(16) float s_v[kChunk][kScanCols];
-    __shared__ __align__(16) float s_o[kChunk][kGroups][kScanCols];
-    __shared__ float s_a[kChunk], s_b[kChunk];
-    __shared__ __align__(16) float2 s_av[kRowDecay ? kChunk : 1][kRowDecay ? kDk : 2];      // per-row decays of the staged tokens
+    constexpr int kVPerThread = kChunk * kCols / kThreads;
+    extern __shared__ __align__(16) unsigned char scan_smem[];
+    Shared& shared = *reinterpret_cast<Shared*>(scan_smem);
+    auto &s_q = shared.q, &s_k = shared.k;
+    auto &s_av = shared.av;
+    auto &s_v = shared.v;
+    auto &s_o = shared.o;
+    auto &s_a = shared.a, &s_b = shared.b;
     const int tile = blockIdx.x, h = blockIdx.y;
     const int r = kParts ? blockIdx.z / p.max_parts : blockIdx.z;
     const int part_idx = kParts ? blockIdx.z % p.max_parts : 0;
     const int g = h / p.group;
-    const int cg = threadIdx.x % 8, rg = threadIdx.x / 8;
-    const int j0 = tile * kScanCols + cg * 4;             // first of this thread's columns
+    const int cg = threadIdx.x % kCG, rg = threadIdx.x / kCG;
+    const int j0 = tile * kCols + cg * 4;             // first of this thread's columns
     int n = p.seg_len[r], s0 = p.seg_start[r];
     float* S;
     if (kParts) {
@@ -304,7 +319,7 @@ linear_scan_kernel(const ScanArgs p) {
 #pragma unroll
         for (int u = 0; u < kVPerThread; ++u) {
             const int e = threadIdx.x + u * kThreads;
-            const int tt = e / kScanCols, jj = tile * kScanCols + e % kScanCols;
+            const int tt = e / kCols, jj = tile * kCols + e % kCols;
             vv[u] = (tt < m && jj < p.dv) ? p.v[static_cast<size_t>(s0 + c0 + tt) * p.ld_v + p.v_off + h * p.dv + jj] : 0.f;
         }
         if (!kRowDecay && !p.decay && threadIdx.x < m)
@@ -328,7 +343,7 @@ linear_scan_kernel(const ScanArgs p) {
 #pragma unroll
         for (int u = 0; u < kVPerThread; ++u) {
             const int e = threadIdx.x + u * kThreads;
-            s_v[e / kScanCols][e % kScanCols] = p.act ? silu_f(vv[u]) : vv[u];
+            s_v[e / kCols][e % kCols] = p.act ? silu_f(vv[u]) : vv[u];
         }
         if (threadIdx.x < m) {
             if (kRowDecay) {
@@ -391,9 +406,9 @@ linear_scan_kernel(const ScanArgs p) {
             *reinterpret_cast<ulonglong2*>(&s_o[tt][rg][cg * 4]) = make_ulonglong2(o[0], o[1]);
         }
         __syncthreads();
-        for (int e = threadIdx.x; e < m * kScanCols; e += kThreads) {
-            const int tt = e / kScanCols, c = e % kScanCols;
-            const int jj = tile * kScanCols + c;
+        for (int e = threadIdx.x; e < m * kCols; e += kThreads) {
+            const int tt = e / kCols, c = e % kCols;
+            const int jj = tile * kCols + c;
             float o = 0.f;
 #pragma unroll
             for (int w = 0; w < kGroups; ++w) o += s_o[tt][w][c];
@@ -737,18 +752,30 @@ static int launch_apply(const ScanArgs& a, int R, cudaStream_t st) {
     return check_launch("linear_scan");
 }
 
+template <int kDk, int kRT, int kCG, bool kParts, bool kRowDecay>
+static int launch_scan_as(const ScanArgs& a, int blocks, cudaStream_t st) {
+    constexpr int kSmem = static_cast<int>(sizeof(ScanShared<kDk, kRT, kCG, kRowDecay>));
+    if constexpr (kSmem > 48 * 1024) {
+        static SharedLimit limit;
+        const cudaError_t ready = limit.allow(reinterpret_cast<const void*>(linear_scan_kernel<kDk, kRT, kCG, kParts, kRowDecay>), kSmem);
+        if (ready != cudaSuccess) { set_error("linear_scan: %s", cudaGetErrorString(ready)); return 1; }
+    }
+    launch_kernel((linear_scan_kernel<kDk, kRT, kCG, kParts, kRowDecay>), dim3((a.dv + 4 * kCG - 1) / (4 * kCG), a.H, blocks), dim3(kDk / kRT * kCG), kSmem, st, a);
+    return check_launch("linear_scan");
+}
+
 template <int kDk, int kRT>
 static int launch_scan(const ScanArgs& a, int R, cudaStream_t st) {
-    const unsigned tiles = (a.dv + kScanCols - 1) / kScanCols;
-    constexpr int kThreads = kDk / kRT * 8;
     const bool rows = a.gate_raw != nullptr;
-    if (a.part_len == 0) {
-        if (rows) launch_kernel((linear_scan_kernel<kDk, kRT, false, true>), dim3(tiles, a.H, R), dim3(kThreads), 0, st, a);
-        else launch_kernel((linear_scan_kernel<kDk, kRT, false, false>), dim3(tiles, a.H, R), dim3(kThreads), 0, st, a);
-        return check_launch("linear_scan");
-    }
-    if (rows) launch_kernel((linear_scan_kernel<kDk, kRT, true, true>), dim3(tiles, a.H, R * a.max_parts), dim3(kThreads), 0, st, a);
-    else launch_kernel((linear_scan_kernel<kDk, kRT, true, false>), dim3(tiles, a.H, R * a.max_parts), dim3(kThreads), 0, st, a);
+    if (a.part_len == 0) return rows ? launch_scan_as<kDk, kRT, 8, false, true>(a, R, st) : launch_scan_as<kDk, kRT, 8, false, false>(a, R, st);
+    // parts: blocks of 256 threads where the values are that wide (other state sizes: as narrow as single tokens)
+    constexpr int kWide = kDk == 128 ? 16 : kDk == 64 ? 32 : 8, kHalf = kWide > 16 ? 16 : kWide;
+    const int blocks = R * a.max_parts;
+    int rc;
+    if (kWide > kHalf && a.dv > 64) rc = rows ? launch_scan_as<kDk, kRT, kWide, true, true>(a, blocks, st) : launch_scan_as<kDk, kRT, kWide, true, false>(a, blocks, st);
+    else if (kHalf > 8 && a.dv > 32) rc = rows ? launch_scan_as<kDk, kRT, kHalf, true, true>(a, blocks, st) : launch_scan_as<kDk, kRT, kHalf, true, false>(a, blocks, st);
+    else rc = rows ? launch_scan_as<kDk, kRT, 8, true, true>(a, blocks, st) : launch_scan_as<kDk, kRT, 8, true, false>(a, blocks, st);
+    if (rc != 0) return rc;
     const size_t elements = static_cast<size_t>(a.H) * a.dk * a.dv;
     launch_kernel((scan_link_kernel), dim3(static_cast<unsigned>((elements + 255) / 256), R), dim3(256), 0, st, a);
     return a.dv <= 64 ? launch_apply<kDk, 64>(a, R, st) : launch_apply<kDk, 128>(a, R, st);
