@@ -1755,6 +1755,78 @@ __global__ void reduce_splits_kernel(const float* __restrict__ ws, float* __rest
     if (threadIdx.x == 0) timeline_record(kTlAddRanges, 6);
 }
 
+// The same added into C, a block per row, and the row's norm with it: out = weight * (row / sqrt(mean(row^2) + eps)) as bfloat16, what the
+// kernel of its own that follows such a product computes (elementwise.cu), in the same order: equal to the bit. Rows of at most 4,096
+// values in whole eights. A launch less behind every product of a prompt portion, and the stream is not read again
+// (512 rows of 3,072, three ranges: 6.3 + 4.8 us as two kernels, 8.0 as one).
+__global__ void __launch_bounds__(256)
+reduce_splits_norm_kernel(const float* __restrict__ ws, float* __restrict__ C, int N4, long long ldc, long long split_stride, int splits,
+                          const float* __restrict__ weight, __nv_bfloat16* __restrict__ out, float eps) {
+    if (threadIdx.x == 0) timeline_record(kTlAddRanges, 0);
+    __shared__ float warp_part[8];
+    __shared__ float s_scale;
+    const int m = blockIdx.x;
+    pdl_launch_dependents();
+    float4 w[4], kept[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int i = threadIdx.x + k * 256;
+        w[k] = i < N4 ? __ldg(reinterpret_cast<const float4*>(weight) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    pdl_wait();
+    if (threadIdx.x == 0) timeline_record(kTlAddRanges, 1);
+    float4* c = reinterpret_cast<float4*>(C + static_cast<long long>(m) * ldc);
+    const float4* row = reinterpret_cast<const float4*>(ws + static_cast<long long>(m) * N4 * 4);
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int i = threadIdx.x + k * 256;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i < N4) {
+            float4 part[8];
+#pragma unroll
+            for (int s = 0; s < 8; ++s)
+                if (s < splits) part[s] = __ldcg(row + i + static_cast<long long>(s) * split_stride / 4);
+            v = c[i];
+#pragma unroll
+            for (int s = 0; s < 8; ++s)
+                if (s < splits) { v.x += part[s].x; v.y += part[s].y; v.z += part[s].z; v.w += part[s].w; }
+            c[i] = v;
+        }
+        kept[k] = v;
+        ss = fmaf(v.x, v.x, ss); ss = fmaf(v.y, v.y, ss);
+        ss = fmaf(v.z, v.z, ss); ss = fmaf(v.w, v.w, ss);
+    }
+    ss = warp_sum(ss);
+    if ((threadIdx.x & 31) == 0) warp_part[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float total = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) total += warp_part[i];
+        s_scale = 1.0f / sqrtf(total / static_cast<float>(4 * N4) + eps);
+    }
+    __syncthreads();
+    const float scale = s_scale;
+    uint2* o = reinterpret_cast<uint2*>(out + static_cast<long long>(m) * N4 * 4);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int i = threadIdx.x + k * 256;
+        if (i >= N4) continue;
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(w[k].x * (scale * kept[k].x), w[k].y * (scale * kept[k].y));
+        const __nv_bfloat162 hi = __floats2bfloat162_rn(w[k].z * (scale * kept[k].z), w[k].w * (scale * kept[k].w));
+        o[i] = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    }
+    if (threadIdx.x == 0) timeline_record(kTlAddRanges, 6);
+}
+
+// What a product that is added into C in ranges of K leaves in the same pass: the norm of C's rows (null: nothing).
+struct RowNorm {
+    const float* weight;
+    __nv_bfloat16* out;
+    float eps;
+};
+
 // Many tokens, one persistent CTA per SM. epilogue 0: C[M,N] = A W^T (32-bit); 1: C += A W^T (32-bit);
 // 2: W is [2N, K] = [gate; up] and C[M,N] = act(A Wgate^T) * (A Wup^T) as bfloat16, act named by the bits above the
 // epilogue's low byte (0 SiLU, 1 ReLU, 2 tanh-GELU); 4: C[M,N] = act(A W^T) as bfloat16, act a PlainAct code there.
@@ -1763,10 +1835,10 @@ __global__ void reduce_splits_kernel(const float* __restrict__ ws, float* __rest
 // items of their own; their results go to `workspace` (splits x ceil(M / 128) x 128 x N floats) and a
 // second kernel adds them up in order into C. Few output tiles (a few hundred tokens) then still fill the GPU.
 // pair: the product runs on pairs of CTAs that share 256-row tiles of tokens (block_q 256 only).
-static int gi_gemm_tc_persistent_impl(const void* A, const void* W, void* C, int epilogue, int M, int N, int K,
-                                     long long lda, long long ldw, long long ldc, int block_q, void* status,
-                                     int splits, void* workspace, long long workspace_floats, int pair, float act_limit,
-                                     const float* gate_up_bias, void* stream) {
+static int gemm_tc_persistent(const void* A, const void* W, void* C, int epilogue, int M, int N, int K,
+                              long long lda, long long ldw, long long ldc, int block_q, void* status,
+                              int splits, void* workspace, long long workspace_floats, int pair, float act_limit,
+                              const float* gate_up_bias, const RowNorm& norm, void* stream) {
     if (M == 0 || N == 0) return 0;
     GI_REQUIRE(M > 0 && N > 0 && K > 0, "gemm_tc: sizes must be positive (M=%d, N=%d, K=%d)", M, N, K);
     GI_REQUIRE(K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0,
@@ -1814,6 +1886,11 @@ static int gi_gemm_tc_persistent_impl(const void* A, const void* W, void* C, int
     const int run_epilogue = split ? static_cast<int>(kEpiStoreF32) : epilogue;
     auto finish = [&](int rc) -> int {
         if (rc != 0 || !split) return rc;
+        if (norm.weight) {
+            launch_kernel((reduce_splits_norm_kernel), dim3(M), dim3(256), 0, st, static_cast<const float*>(workspace), static_cast<float*>(C),
+                          N / 4, ldc, static_cast<long long>(p.split_rows) * N, splits, norm.weight, norm.out, norm.eps);
+            return check_launch("gemm_tc reduce and norm");
+        }
         const long long n = static_cast<long long>(M) * (N / 4);
         launch_kernel((reduce_splits_kernel), dim3(static_cast<unsigned>((n + 255) / 256)), dim3(256), 0, st,
                       static_cast<const float*>(workspace), static_cast<float*>(C), M, N / 4, ldc,
@@ -1844,6 +1921,24 @@ static int gi_gemm_tc_persistent_impl(const void* A, const void* W, void* C, int
     }
     if (run_epilogue == kEpiAddF32) return launch_persistent<128, kEpiAddF32>(mp, mq, mc, p, st);
     return finish(launch_persistent<128, kEpiStoreF32>(mp, mq, mc, p, st));
+}
+
+static int gi_gemm_tc_persistent_impl(const void* A, const void* W, void* C, int epilogue, int M, int N, int K,
+                                     long long lda, long long ldw, long long ldc, int block_q, void* status,
+                                     int splits, void* workspace, long long workspace_floats, int pair, float act_limit,
+                                     const float* gate_up_bias, void* stream) {
+    return gemm_tc_persistent(A, W, C, epilogue, M, N, K, lda, ldw, ldc, block_q, status, splits, workspace, workspace_floats, pair, act_limit,
+                              gate_up_bias, RowNorm{}, stream);
+}
+// C += A W^T with K in ranges (splits > 1), and out [M, N] = the norm of C's rows.
+static int gi_gemm_tc_persistent_norm_impl(const void* A, const void* W, void* C, int M, int N, int K, long long lda, long long ldw, long long ldc,
+                                          int block_q, void* status, int splits, void* workspace, long long workspace_floats, int pair,
+                                          const float* weight, void* out, float eps, void* stream) {
+    GI_REQUIRE(weight != nullptr && out != nullptr && reinterpret_cast<uintptr_t>(weight) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0,
+               "gemm_tc norm: the norm's weights and output are required, on 16-byte boundaries");
+    GI_REQUIRE(splits > 1 && N % 8 == 0 && N <= 4096, "gemm_tc norm: for rows of at most 4,096 values in whole eights whose K is in ranges (N=%d, %d ranges)", N, splits);
+    return gemm_tc_persistent(A, W, C, kEpiAddF32, M, N, K, lda, ldw, ldc, block_q, status, splits, workspace, workspace_floats, pair, 0.f, nullptr,
+                              RowNorm{weight, static_cast<__nv_bfloat16*>(out), eps}, stream);
 }
 
 // A matrix per group of rows: A [M, K] holds tiles of 128 rows each of which belongs to one group (an expert's tokens,
@@ -1960,6 +2055,10 @@ extern "C" int gi_gemm_tc(const void* A, const void* W, void* C, int c_dtype, in
 
 extern "C" int gi_gemm_tc_rope(const void* A, const void* W, int M, int K, long long lda, long long ldw, int block_q, int splits, void* workspace, long long workspace_floats, void* counters, int n_counters, void* status, const void* w_tiles, const int* positions, const int* row_req, const int* block_tables, int table_stride, const float* cos_t, const float* sin_t, int rot_half, int interleaved, void* q_out, void* k_cache, void* v_cache, int H, int Hkv, int hd, int page_size, int write_kv, void* stream) {
     return gi::dispatch(gi_gemm_tc_rope_impl, A, W, M, K, lda, ldw, block_q, splits, workspace, workspace_floats, counters, n_counters, status, w_tiles, positions, row_req, block_tables, table_stride, cos_t, sin_t, rot_half, interleaved, q_out, k_cache, v_cache, H, Hkv, hd, page_size, write_kv, stream);
+}
+
+extern "C" int gi_gemm_tc_persistent_norm(const void* A, const void* W, void* C, int M, int N, int K, long long lda, long long ldw, long long ldc, int block_q, void* status, int splits, void* workspace, long long workspace_floats, int pair, const float* weight, void* out, float eps, void* stream) {
+    return gi::dispatch(gi_gemm_tc_persistent_norm_impl, A, W, C, M, N, K, lda, ldw, ldc, block_q, status, splits, workspace, workspace_floats, pair, weight, out, eps, stream);
 }
 
 extern "C" int gi_gemm_tc_persistent(const void* A, const void* W, void* C, int epilogue, int M, int N, int K, long long lda, long long ldw, long long ldc, int block_q, void* status, int splits, void* workspace, long long workspace_floats, int pair, float act_limit, const float* gate_up_bias, void* stream) {

@@ -52,14 +52,16 @@ class Linear:
             new.weight_tiles = kernels.tile_weight(weight)
         return new
 
-    def forward(self, a: torch.Tensor, out: torch.Tensor, accumulate: bool = False, then: "Linear" = None) -> torch.Tensor:
-        """``then``: the Linear whose product runs next but one (after a small kernel); a product of few tokens
+    def forward(self, a: torch.Tensor, out: torch.Tensor, accumulate: bool = False, then: "Linear" = None, norm=None) -> torch.Tensor:
+        """``norm`` = (weight, eps, xn): the norm of out's rows goes to xn (``kernels.gemm_tc``). ``then``: the Linear whose product runs next but one (after a small kernel); a product of few tokens
         asks the start of its weights into L2 meanwhile (``kernels.gemm_tc``: ``ahead``)."""
         if a.dtype != self.compute_dtype:
             raise kernels.KernelError(f"Linear: activations are {a.dtype}, the weight is {self.compute_dtype}")
         if self.compute_dtype is torch.bfloat16 and self.in_features % 8 == 0:
             kernels.gemm_tc(a, self.weight, out, accumulate, w_tiles=self.weight_tiles,   # tensor cores (TMA needs 16-byte rows)
-                            ahead=then.weight_tiles if then is not None else None)
+                            ahead=then.weight_tiles if then is not None else None, norm=norm)
         else:
             kernels.gemm_simt(a, self.weight, out, accumulate)
+            if norm is not None:
+                kernels.rmsnorm(out, norm[0], norm[2], norm[1])
         return out

@@ -306,11 +306,16 @@ class AttentionMixer:
             prefill(q, k_cache, v_cache, att, work, ctx.positions, tables, H, Hkv, hd, ctx.page_size, self.scale,
                     self.window, **epilogue)
 
-    def forward(self, ctx, run, xn: torch.Tensor, x: torch.Tensor, then=None) -> None:
+    @property
+    def takes_norm(self) -> bool:
+        """Whether ``forward`` takes the norm of the stream that follows (``norm``)."""
+        return not self.extended
+
+    def forward(self, ctx, run, xn: torch.Tensor, x: torch.Tensor, then=None, norm=None) -> None:
         """``xn``: normalised input [T, hidden] in the compute dtype; ``x``: the 32-bit residual
         stream, to which the mixer's output is added. ``run`` names whose cache to use. ``then``: the Linear
         of the large product that follows this mixer (the feed-forward's first), for the last product here to
-        ask the start of its weights into L2."""
+        ask the start of its weights into L2. ``norm`` = (weight, eps, out): the norm of x when the output is added."""
         T = xn.shape[0]
         H, Hkv, hd = self.num_heads, self.num_kv_heads, self.head_dim
         k_cache, v_cache = ctx.pages(run.cache_layer)
@@ -333,7 +338,7 @@ class AttentionMixer:
                                write_kv=run.writes_cache)
         att = ctx.scratch("att", (T, H * hd), self.dtype)
         self._attend(ctx, q, k_cache, v_cache, att, tables)
-        self.w_o.forward(att, x, accumulate=True, then=then)
+        self.w_o.forward(att, x, accumulate=True, then=then, norm=norm)
 
     def _forward_extended(self, ctx, run, xn, x, q, k_cache, v_cache, tables, then) -> None:
         """The mixer with options: projections to 32-bit, then per head norm, rotation and page store, attention

@@ -3,7 +3,7 @@ from __future__ import annotations
 
 import torch
 
-from .norm import LayerNorm
+from .norm import LayerNorm, RMSNorm, ScalarRMSNorm
 from .registry import FEED_FORWARDS, MIXERS, NORMS, build_part, register_block, sub_weights
 from .stream import EmbeddingAdd, EmbeddingMix
 
@@ -11,7 +11,11 @@ from .stream import EmbeddingAdd, EmbeddingMix
 @register_block("pre_norm")
 class PreNormBlock:
     """x += mixer(norm(x)); x += feed_forward(norm(x)), the residual stream x kept in 32-bit
-    (src/model/transformer.cpp:379-451)."""
+    (src/model/transformer.cpp:379-451).
+
+    Where a sublayer's last product can take the norm that follows in its own last pass (``takes_norm``), it is asked to, also for
+    the mixer of the next run (``ctx.carry`` tells its block that the normed input is there); not while a listener taps the
+    stream, which may write to it before it is normed."""
 
     def __init__(self, layer_spec, weights, build):
         self.mixer_norm = build_part(NORMS, "norm", layer_spec.mixer_norm, sub_weights(weights, "mixer_norm."), build)
@@ -21,36 +25,65 @@ class PreNormBlock:
         self.feed_forward = build_part(FEED_FORWARDS, "feed-forward", layer_spec.feed_forward,
                                        sub_weights(weights, "feed_forward."), build)
         self.dtype = build.compute_dtype
+        self._next = {}             # run -> the norm of the next run's block where that reads the stream as this one leaves it
+
+    def followed_in_run(self, run, block, stream_input) -> None:
+        after = block.mixer_norm if stream_input is None and isinstance(block, PreNormBlock) else None
+        self._next[run] = after if self._next.get(run, after) is after else None      # (a run that comes twice, before different blocks)
 
     def forward(self, ctx, run, x: torch.Tensor) -> None:
         xn = ctx.scratch("normed", tuple(x.shape), self.dtype)
         T = x.shape[0]
+        carry = getattr(ctx, "carry", None)
+        tapped = getattr(ctx, "tapping", False)
+        ready = carry is not None and carry.pop("pre_norm", None) == (x.data_ptr(), id(self.mixer_norm))
         # each half of the layer is one launch program when its parts say what their launches depend on
         # (``launch_key``); a part without that method (one that computes with other libraries) runs as it is
-        key = _launch_key(ctx, (self.mixer_norm, None), (self.mixer, run))
+        key = _launch_key(ctx, (self.mixer_norm, None), (self.mixer, run), (self.feed_forward_norm, None))
         if key is not None:
-            ctx.recorded(self, ("mixer", run, T) + key, lambda: self._mixer_half(ctx, run, xn, x))
+            ctx.recorded(self, ("mixer", run, T, ready) + key, lambda: self._mixer_half(ctx, run, xn, x, ready, tapped))
         else:
-            self._mixer_half(ctx, run, xn, x)
+            self._mixer_half(ctx, run, xn, x, ready, tapped)
         ctx.tap("attn_out", run.layer, x)
-        key = _launch_key(ctx, (self.feed_forward_norm, None), (self.feed_forward, None))
+        if tapped:
+            self.feed_forward_norm.forward(x, xn)
+        after = self._next.get(run) if carry is not None and not tapped else None
+        if after is not None and not (_norm_of(after, xn) and getattr(self.feed_forward, "takes_norm", False)):
+            after = None
+        key = _launch_key(ctx, (self.feed_forward, None))
         if key is not None:
-            ctx.recorded(self, ("feed_forward", T) + key, lambda: self._feed_forward_half(ctx, xn, x))
+            ctx.recorded(self, ("feed_forward", T, id(after)) + key, lambda: self._feed_forward_half(ctx, xn, x, after))
         else:
-            self._feed_forward_half(ctx, xn, x)
+            self._feed_forward_half(ctx, xn, x, after)
+        if after is not None:
+            carry["pre_norm"] = (x.data_ptr(), id(after))
         ctx.tap("ffn_out", run.layer, x)
 
-    def _mixer_half(self, ctx, run, xn, x) -> None:
-        self.mixer_norm.forward(x, xn)
+    def _mixer_half(self, ctx, run, xn, x, ready, tapped) -> None:
+        """Up to the feed-forward's normed input (tapped: up to what is normed)."""
+        if not ready:
+            self.mixer_norm.forward(x, xn)
+        options = {}
         then = getattr(self.feed_forward, "first_product", None)
         if then is not None and getattr(self.mixer, "takes_then", False):
-            self.mixer.forward(ctx, run, xn, x, then=then)      # the mixer's last product asks for the weights that follow
-        else:
-            self.mixer.forward(ctx, run, xn, x)
+            options["then"] = then                              # the mixer's last product asks for the weights that follow
+        norm = _norm_of(self.feed_forward_norm, xn) if getattr(self.mixer, "takes_norm", False) and not tapped else None
+        if norm is not None:
+            options["norm"] = norm
+        self.mixer.forward(ctx, run, xn, x, **options)
+        if norm is None and not tapped:
+            self.feed_forward_norm.forward(x, xn)
 
-    def _feed_forward_half(self, ctx, xn, x) -> None:
-        self.feed_forward_norm.forward(x, xn)
-        self.feed_forward.forward(ctx, xn, x)
+    def _feed_forward_half(self, ctx, xn, x, after) -> None:
+        if after is None:
+            self.feed_forward.forward(ctx, xn, x)
+        else:
+            self.feed_forward.forward(ctx, xn, x, norm=_norm_of(after, xn))
+
+
+def _norm_of(norm, xn):
+    """(weight, eps, xn) of a norm that a product can take (None for another kind)."""
+    return (norm.weight, norm.eps, xn) if type(norm) in (RMSNorm, ScalarRMSNorm) else None
 
 
 @register_block("post_norm")

@@ -62,8 +62,13 @@ class SwiGLUFeedForward:
         """Its launches depend on the token count only (which the caller's key holds)."""
         return ()
 
-    def forward(self, ctx, xn: torch.Tensor, x: torch.Tensor, accumulate: bool = True) -> None:
-        """``accumulate`` False: x is set to the output instead of being added to."""
+    @property
+    def takes_norm(self) -> bool:
+        """Whether ``forward`` takes the norm of the stream that follows (``norm``): its last product ends it."""
+        return self.b_down is None
+
+    def forward(self, ctx, xn: torch.Tensor, x: torch.Tensor, accumulate: bool = True, norm=None) -> None:
+        """``accumulate`` False: x is set to the output instead of being added to. ``norm`` = (weight, eps, out): the norm of x then."""
         T = xn.shape[0]
         h = ctx.scratch("ffn_hidden", (T, self.intermediate_size), self.dtype)
         if self.dtype is torch.bfloat16 and kernels.gemm_swiglu_supported(T, self.intermediate_size, self.hidden_size):
@@ -76,7 +81,7 @@ class SwiGLUFeedForward:
                 kernels.swiglu(gu, h)
             else:
                 kernels.gated_act(gu, h, self.activation, self.limit, self.b_gate_up)
-        self.w_down.forward(h, x, accumulate=accumulate)
+        self.w_down.forward(h, x, accumulate=accumulate, norm=norm)
         if self.b_down is not None and not self.output_bias_left:
             kernels.add_bias(x, self.b_down)
 

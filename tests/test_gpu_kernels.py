@@ -367,6 +367,20 @@ def test_sample_rows_of_few_likely_tokens(V, top_k, top_p):
     assert got[3] == (0 if top_p < 1.0 else top_k - 1 if 0 < top_k < V else V - 1)      # no probabilities: an index, always the same
 
 
+@pytest.mark.parametrize("M, N, K_", [(129, 64, 512), (300, 2048, 8192), (512, 3072, 3072), (489, 4096, 1024), (140, 4104, 4096), (512, 264, 8192), (5, 256, 512)])
+def test_gemm_takes_the_norm_of_its_sums(M, N, K_):
+    """The norm behind an adding product equals the norm's own kernel to the bit, in the pass that adds up ranges of K and elsewhere."""
+    g = torch.Generator().manual_seed(M)
+    a, w = torch.randn(M, K_, generator=g).bfloat16().to(DEV), torch.randn(N, K_, generator=g).bfloat16().to(DEV)
+    weight, start = torch.randn(N, generator=g).to(DEV), torch.randn(M, N, generator=g).to(DEV)
+    one, two = start.clone(), start.clone()
+    xn, want = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV), torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    K().gemm_tc(a, w, one, accumulate=True)
+    K().rmsnorm(one, weight, want, 1e-5)
+    K().gemm_tc(a, w, two, accumulate=True, norm=(weight, 1e-5, xn))
+    assert torch.equal(one, two) and torch.equal(xn, want)
+
+
 @pytest.mark.parametrize("V", [131072, 131073])
 @pytest.mark.parametrize("top_k,top_p", [(0, 1.0), (40, 1.0), (0, 0.9), (40, 0.95)])
 def test_sample_of_the_largest_rows_held_in_registers_and_the_smallest_not(V, top_k, top_p):
