@@ -60,6 +60,9 @@ using Tile6 = F32Tile<6, 64, 6, 2, 32, 5, 4>;
 using Tile8 = F32Tile<8, 64, 8, 2, 32, 5, 4>;
 using Tile16 = F32Tile<16, 64, 8, 4, 32, 4, 4>;
 using Tile32 = F32Tile<32, 128, 8, 4, 32, 3, 3>;
+using Tile40 = F32Tile<40, 128, 5, 8, 32, 4, 2>;
+using Tile48 = F32Tile<48, 128, 6, 8, 32, 4, 2>;
+using Tile56 = F32Tile<56, 128, 7, 8, 32, 4, 2>;
 using Tile64 = F32Tile<64, 128, 8, 8, 32, 4, 2>;
 
 // grid (chunks, blocks of rows, blocks of columns), clusters of `chunks` along x. kc: length of a chunk.
@@ -221,6 +224,23 @@ int gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int 
     if (M <= 8) return launch<Tile8>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, st);
     if (M <= 16) return launch<Tile16>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, st);
     if (M <= 32) return launch<Tile32>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, st);
+    // More rows: blocks of 8 x 5 .. 8 rows, the height whose rounds over the SMs (two blocks each) are the least work: a block that is
+    // half outside the matrix, or a last round that is nearly empty, costs as much as a full one. A block's time goes with its
+    // rows and half a row's worth of reading columns. (268 rows,
+    // blocks of 64 -> the height taken: 16,384 outputs of 2,048 inputs 495 -> 455 us in blocks of 56; 2,048 of 2,048 and 8,192 together
+    // 189 -> 171 each and 3,072 of 2,048 122 -> 112 in blocks of 48.)
+    int best = 8;
+    long long least = -1;
+    for (int tm = 8; tm >= 5; --tm) {
+        const int rows = (M + 8 * tm - 1) / (8 * tm);
+        if (rows > 65535) break;                           // the grid's limit
+        const long long blocks = static_cast<long long>(chunks) * ((N + 127) / 128) * rows;
+        const long long cost = (blocks + 2 * 148 - 1) / (2 * 148) * (2 * tm + 1);
+        if (least < 0 || cost < least) { least = cost; best = tm; }
+    }
+    if (best == 5) return launch<Tile40>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, st);
+    if (best == 6) return launch<Tile48>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, st);
+    if (best == 7) return launch<Tile56>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, st);
     return launch<Tile64>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, st);
 }
 

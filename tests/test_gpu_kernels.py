@@ -113,6 +113,18 @@ def test_gemm_simt_tiled(M, N, K_):
             assert torch.equal(part, out[M - rows:]), rows
 
 
+@pytest.mark.parametrize("M, N, K_", [(33, 300, 36), (41, 19000, 36), (48, 19000, 64), (49, 19000, 64), (56, 19000, 36), (57, 19000, 36), (268, 2056, 2052)])
+def test_gemm_simt_block_heights_agree_to_the_bit(M, N, K_):
+    """Blocks of 40, 48, 56 and 64 rows, full and with rows left over, against the same rows in blocks of 32."""
+    g = torch.Generator().manual_seed(M)
+    a, w = torch.randn(M, K_, generator=g).to(DEV), torch.randn(N, K_, generator=g).to(DEV)
+    out, part = torch.full((M, N), float("nan"), device=DEV), torch.full((M, N), float("nan"), device=DEV)
+    K().gemm_simt(a, w, out)
+    for r in range(0, M, 32):
+        K().gemm_simt(a[r:r + 32], w, part[r:r + 32])
+    assert torch.equal(out, part) and bool(out.isfinite().all())
+
+
 def _paged(dtype, n_pages, Hkv, ps, hd):
     kc = torch.full((n_pages, Hkv, ps, hd), float("nan"), dtype=dt(dtype), device=DEV)
     return kc, kc.clone()
