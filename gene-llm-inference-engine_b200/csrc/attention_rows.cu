@@ -537,7 +537,7 @@ attention_rows_mma_kernel(const RowsArgs a, const RowTiles rt) {
 // pair of value dimensions. A few KB a block, so it is as long as its loads wait for one another: a thread asks for its
 // pair of every range before the ranges' weights are worked out (a token's step, latents of 512 values: 16 heads of eight tokens and five
 // ranges 8.1 -> 4.3 us, of two tokens and fifteen ranges 14.7 -> 3.8; before, a thread had a value and four ranges in flight).
-constexpr int kRowsMaxSplits = 16;
+constexpr int kRowsMaxSplits = 32;        // a lane each
 __global__ void __launch_bounds__(kRowsMaxValueThreads)
 attention_rows_merge_kernel(const RowsArgs a, const RowTiles rt) {
     pdl_prologue();
@@ -572,7 +572,7 @@ attention_rows_merge_kernel(const RowsArgs a, const RowTiles rt) {
         float L = 0.f;
         for (int i = 0; i < rt.splits; ++i) L += __shfl_sync(0xffffffffu, ls * w, i);       // in the ranges' order
         if (a.sinks) L += expf(a.sinks[head] - M);
-        if (s < kRowsMaxSplits) s_w[s] = w;
+        s_w[s] = w;
         if (s == 0) s_inv = 1.0f / L;
     }
     __syncthreads();
@@ -718,7 +718,7 @@ static int gi_attention_rows_impl(const void* q, int q_dtype, int ldq, const voi
         GI_REQUIRE(rt.splits == 1 || (workspace != nullptr && static_cast<long long>(tiles) * Hkv * rt.head_blocks * rt.splits * rt.block_rows * (vd + 2) <= workspace_floats),
                    "attention_rows: the workspace of the key ranges is missing or too small");
         GI_REQUIRE(rt.head_blocks * rt.splits <= 65535 && a.Hkv * rt.head_blocks <= 65535 && rt.splits <= kRowsMaxSplits,
-                   "attention_rows: too many blocks of heads or ranges of keys (at most 16 ranges)");
+                   "attention_rows: too many blocks of heads or ranges of keys (at most 32 ranges)");
         const size_t smem_mma = rows_mma_smem_of(mode, hd, vd, a.alias != 0);
         if (mode == 1) return vd <= 64 ? launch_rows_mma<8, 1>(a, rt, tiles, smem_mma, st) : launch_rows_mma<16, 1>(a, rt, tiles, smem_mma, st);
         if (mode == 2) return vd <= 256 ? launch_rows_mma<16, 2>(a, rt, tiles, smem_mma, st) : launch_rows_mma<32, 2>(a, rt, tiles, smem_mma, st);

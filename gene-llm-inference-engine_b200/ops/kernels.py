@@ -531,11 +531,12 @@ _ROWS_BLOCKS = 296          # about two blocks an SM: what the ranges of keys of
 
 def attention_rows_splits(n_tiles: int, num_heads: int, num_kv_heads: int, span: int) -> int:
     """Into how many ranges the keys of every tile of a launch of ``n_tiles`` tiles are cut (1: none): few tiles
-    (decoding) with many keys to see would leave most SMs idle. ``span``: the most keys a row sees."""
+    (decoding) with many keys to see would leave most SMs idle. ``span``: the most keys a row sees. A range is a tile of 32 keys
+    where there are SMs for it: its tiles follow one another, about 2 us each, and merging a range costs a load."""
     blocks = n_tiles * num_kv_heads * ((num_heads // num_kv_heads + 15) // 16)
     if blocks <= 0 or blocks >= sm_count():
         return 1
-    return max(1, min(16, _ROWS_BLOCKS // blocks, (span + 63) // 64))
+    return max(1, min(32, _ROWS_BLOCKS // blocks, (span + 31) // 32))
 
 
 def attention_rows_workspace_rows(n_tiles: int, num_heads: int, num_kv_heads: int, splits: int) -> int:
