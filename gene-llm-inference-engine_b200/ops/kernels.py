@@ -1290,10 +1290,6 @@ _gemm_choice = {}      # (M, N, K, output dtype, tiled weights) -> (swap, block_
 AHEAD_BYTES = 24 << 20
 
 
-def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False, plan=None,
-            w_tiles: Optional[torch.Tensor] = None, ahead: Optional[torch.Tensor] = None, act: Optional[str] = None,
-            norm: Optional[Tuple[torch.Tensor, float, torch.Tensor]] = None) -> None:
-    """out[M,N] (+)= a[M,K] @ w[N,K]^T on the tensor cores: bfloat16 operands, 32-bit accumulation,
 def _norms_with_ranges(a, w, out, accumulate, plan, w_tiles, norm) -> bool:
     """Whether gemm_tc's kernel that adds up the ranges of K takes the norm of the rows too: many tokens, K in ranges, rows that a
     block holds in registers."""
@@ -1305,6 +1301,10 @@ def _norms_with_ranges(a, w, out, accumulate, plan, w_tiles, norm) -> bool:
     return not swap and block_q >= 128 and splits > 1 and splits * ((M + 255) // 256 * 256) * N <= _tc_state(a.device).workspace.numel()
 
 
+def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False, plan=None,
+            w_tiles: Optional[torch.Tensor] = None, ahead: Optional[torch.Tensor] = None, act: Optional[str] = None,
+            norm: Optional[Tuple[torch.Tensor, float, torch.Tensor]] = None) -> None:
+    """out[M,N] (+)= a[M,K] @ w[N,K]^T on the tensor cores: bfloat16 operands, 32-bit accumulation,
     output 32-bit (optionally accumulated into) or bfloat16. K must be a multiple of 8. ``w_tiles``
     (tile_weight(w)) lets products of few tokens fetch the weights with bulk copies. ``ahead``: a tensor
     that a later kernel of the step streams (the tile-by-tile weights of the next large product); a product of few
@@ -1314,13 +1314,13 @@ def _norms_with_ranges(a, w, out, accumulate, plan, w_tiles, norm) -> bool:
     in ranges that a second kernel adds up."""
     M, K = a.shape
     N = w.shape[0]
-    if act is not None and (act not in PLAIN_ACTIVATIONS or out.dtype is not torch.bfloat16 or accumulate):
-        raise KernelError(f"gemm_tc: activation '{act}' is unknown or the output is not a stored bfloat16 matrix")
-    if act is not None and plan is None and M > 128 and N % 8 == 0:      # many tokens: the activation in the persistent kernel's epilogue
     if norm is not None and not _norms_with_ranges(a, w, out, accumulate, plan, w_tiles, norm):
         gemm_tc(a, w, out, accumulate, plan, w_tiles, ahead, act)
         rmsnorm(out, norm[0], norm[2], norm[1])
         return
+    if act is not None and (act not in PLAIN_ACTIVATIONS or out.dtype is not torch.bfloat16 or accumulate):
+        raise KernelError(f"gemm_tc: activation '{act}' is unknown or the output is not a stored bfloat16 matrix")
+    if act is not None and plan is None and M > 128 and N % 8 == 0:      # many tokens: the activation in the persistent kernel's epilogue
         st = _tc_state(a.device)
         block_q = 256 if N >= 256 else 128
         check(lib().gi_gemm_tc_persistent(_dev(a, "a", torch.bfloat16), _dev(w, "w", torch.bfloat16), _dev(out, "out"),
@@ -1352,15 +1352,15 @@ def _norms_with_ranges(a, w, out, accumulate, plan, w_tiles, norm) -> bool:
         need = splits * ((M + 255) // 256 * 256) * N
         if splits > 1 and need > st.workspace.numel():
             splits = 1
-        check(lib().gi_gemm_tc_persistent(_dev(a, "a", torch.bfloat16), _dev(w, "w", torch.bfloat16),
-                                          _dev(out, "out", torch.float32), 1 if accumulate else 0, M, N, K, K, K, N,
-                                          block_q, st.status.data_ptr(), splits, st.workspace.data_ptr() if splits > 1 else 0,
         if norm is not None:
             check(lib().gi_gemm_tc_persistent_norm(_dev(a, "a", torch.bfloat16), _dev(w, "w", torch.bfloat16), _dev(out, "out", torch.float32),
                                                    M, N, K, K, K, N, block_q, st.status.data_ptr(), splits, st.workspace.data_ptr(),
                                                    st.workspace.numel(), _paired(M, block_q), _dev(norm[0], "weight", torch.float32),
                                                    _dev(norm[2], "xn", torch.bfloat16), float(norm[1]), _stream()), "gemm_tc")
             return
+        check(lib().gi_gemm_tc_persistent(_dev(a, "a", torch.bfloat16), _dev(w, "w", torch.bfloat16),
+                                          _dev(out, "out", torch.float32), 1 if accumulate else 0, M, N, K, K, K, N,
+                                          block_q, st.status.data_ptr(), splits, st.workspace.data_ptr() if splits > 1 else 0,
                                           st.workspace.numel() if splits > 1 else 0, _paired(M, block_q), 0.0, 0, _stream()), "gemm_tc")
         return
     check(lib().gi_gemm_tc(_dev(a, "a", torch.bfloat16), _dev(w, "w", torch.bfloat16), _dev(out, "out"),
