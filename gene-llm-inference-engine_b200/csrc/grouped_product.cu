@@ -21,12 +21,12 @@
 //   route_combine     y[t] += sum_k weight[t, k] * part[row of pair t * top + k] in the order of k (weights of 1 where they
 //                     scaled the experts' inputs), optionally plus gate[t] * more[t] (the gated expert of every token)
 //
-// Products run on the CUDA cores with 32-bit fused multiply-adds: the true 32-bit path, products of few rows (decoding,
-// where the weights stream once), the heads' matrices, and the bfloat16 path's fallback. Three forms: tiles of 16 x 64
-// outputs, tiles of 64 x 64 (many rows through the heads' matrices) and the few-row form further down. In the tiled forms
-// an output element is one chain of multiply-adds in the order of k over its own row, whichever tile the row landed in;
-// in the few-row form it is the sum of a warp's lanes' chains by a fixed tree. (Many rows through the experts' matrices
-// in bfloat16 run on the tensor cores: gi_gemm_tc_grouped.)
+// bfloat16 weights in aligned rows run on the tensor cores (grouped_mma_kernel for few rows, decoding, where the weights stream once;
+// head_mma_kernel for the heads' matrices), 32-bit inputs with all their bits. The true 32-bit path, a few pairs of 32-bit inputs and
+// what is not aligned run on the CUDA cores with 32-bit fused multiply-adds, in three forms: tiles of 16 x 64 outputs, tiles of 64 x 64
+// (many rows through the heads' matrices) and the few-row form further down. In the tiled forms an output element is one chain of
+// multiply-adds in the order of k over its own row, whichever tile the row landed in; in the few-row form it is the sum of
+// a warp's lanes' chains by a fixed tree. (Many rows through the experts' matrices in bfloat16: gi_gemm_tc_grouped.)
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -172,35 +172,14 @@ grouped_product_kernel(const GroupedArgs p) {
     }
 }
 
-// The same products for few rows (decoding): the weights are what takes the time. A warp streams four output rows of a
-// group's matrix (gated: and their up rows) through a ring in shared memory, 512 bytes of each a step, by asynchronous copies
+// The same products for few rows (decoding) of 32-bit inputs, with 32-bit weights or, a few pairs, bfloat16 ones: the weights are what
+// takes the time. A warp streams four or eight output rows of a group's matrix (gated: and their up rows) through a ring in shared memory, 512 bytes of each a step, by asynchronous copies
 // of 16 bytes; every lane copies exactly the pieces that it multiplies itself, so the ring needs no barrier, and 48 KB or more
-// are in flight per block whatever the warps are doing. (With the loads in registers, eight a lane and none while it
-// multiplied, eight experts of 2 x 4096 x 2048 values and sixteen pairs took 124 us, 1.9 TB/s; with the ring and a block per
-// sixteen output rows 74 us, a third of it the blocks' beginnings and ends.) Each step's
-// pieces are multiplied with up to eight rows of the tile, read through the cache; more rows stream the weights again, from
-// L2. An output element is the sum of its lanes' partial sums (lane l takes the
-// pieces l, l + 32, ...), added by a fixed xor tree: it depends on its own row only.
+// are in flight per block whatever the warps are doing. Each step's pieces are multiplied with up to eight rows of the tile, read
+// through the cache; more rows stream the weights again, from L2. An output element is the sum of its lanes' partial sums (lane l takes
+// the pieces l, l + 32, ...), added by a fixed xor tree: it depends on its own row only.
 constexpr int kGrWarps = 4;
 constexpr int kGrFew = 8;             // rows of a tile that are multiplied with a piece of the weights while it is in registers
-
-template <typename T> struct Vec16;
-template <> struct Vec16<float> {
-    static constexpr int N = 4;
-    static __device__ __forceinline__ void load(const float* p, float (&v)[8]) {
-        const float4 x = *reinterpret_cast<const float4*>(p);
-        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-    }
-};
-template <> struct Vec16<__nv_bfloat16> {
-    static constexpr int N = 8;
-    static __device__ __forceinline__ void load(const __nv_bfloat16* p, float (&v)[8]) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(p);
-        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(h[i]); v[2 * i] = f.x; v[2 * i + 1] = f.y; }
-    }
-};
 
 template <typename T> __device__ __forceinline__ float4 load4(const T* p);
 template <> __device__ __forceinline__ float4 load4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -211,12 +190,41 @@ template <> __device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bf
     return make_float4(a.x, a.y, b.x, b.y);
 }
 
+// The few-row forms: group and rows of tile x; lane i gets the i-th of its rows. Returns how many there are. HALVES: tile x is half of a
+// tile, its first eight rows or the others.
+template <bool HALVES = false>
+__device__ __forceinline__ int gm_tile(const GroupedArgs& p, int x, int lane, int& g, int& row) {
+    int r = -1, half = 0;
+    if (HALVES) { half = x & 1; x >>= 1; }
+    if (p.tile_group) {
+        g = p.tile_group[x];
+        if (lane < kGpTM) r = p.sorted_rows[x * kGpTM + lane];
+    } else {
+        g = x % p.groups;
+        if (lane < kGpTM) r = x / p.groups * kGpTM + lane;
+        if (r >= p.rows) r = -1;
+    }
+    const unsigned some = __ballot_sync(0xffffffffu, r >= 0);       // the empty places left out
+    row = r;
+    if (some & (some + 1)) row = __shfl_sync(0xffffffffu, r, __fns(some, 0, lane + 1) & 31);
+    if (HALVES) {
+        if (half) row = __shfl_sync(0xffffffffu, row, (lane + 8) & 31);
+        return max(0, min(8, __popc(some) - 8 * half));
+    }
+    return __popc(some);
+}
+
+// Four neighbouring weights of a lane's piece in shared memory, as 32-bit values.
+__device__ __forceinline__ float4 piece4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 piece4(const __nv_bfloat16* p) { return load4<__nv_bfloat16>(p); }
+
 // The few-row form's units of work, taken by the grid's warps in turn: (tile, four or eight output rows), and for a tile of more than
-// kGrFew rows a second pass over the same weights. A warp's ring runs on from unit to unit.
-// ROWS: output rows of a unit, 4 or, not gated, 8.
-template <typename TA, typename TW, bool GATED, int ROWS>
+// kGrFew rows a second pass over the same weights. A warp's ring runs on from unit to unit. 32-bit inputs.
+// ROWS: output rows of a unit: 4 of 32-bit weights; 8 of bfloat16 weights, whose few pairs' inputs are as many bytes as four rows
+// of weights for every two of them.
+template <typename TW, bool GATED, int ROWS>
 struct RowsStream {
-    static constexpr int kPiece = Vec16<TW>::N;          // values per step of a lane: the weights' 16 bytes
+    static constexpr int kPiece = 16 / sizeof(TW);       // values per step of a lane: the weights' 16 bytes
     static constexpr int kW = GATED ? 2 * ROWS : ROWS;   // rows of weights that it streams (gated: and the up rows)
     static constexpr int kBlocks = ROWS == 8 ? 2 : 3;    // blocks an SM: 8 rows need more than the 168 registers of three
     static constexpr int kSmem = (ROWS == 8 ? 96 : 64) * 1024;
@@ -230,26 +238,10 @@ struct RowsStream {
     const TW* wrow;              // the unit's first row of weights; `last`: the last that there is
     int last;
 
-    // Group and rows of tile x; lane i gets the i-th of its rows.
-    __device__ __forceinline__ int tile(int x, int& g, int& row) const {
-        int r = -1;
-        if (p.tile_group) {
-            g = p.tile_group[x];
-            if (lane < kGpTM) r = p.sorted_rows[x * kGpTM + lane];
-        } else {
-            g = x % p.groups;
-            if (lane < kGpTM) r = x / p.groups * kGpTM + lane;
-            if (r >= p.rows) r = -1;
-        }
-        const unsigned some = __ballot_sync(0xffffffffu, r >= 0);       // the empty places left out
-        row = r;
-        if (some & (some + 1)) row = __shfl_sync(0xffffffffu, r, __fns(some, 0, lane + 1) & 31);
-        return __popc(some);
-    }
     __device__ __forceinline__ void seek() {
         for (; unit < units; unit += stride) {
             int g, row;
-            passes = (tile(unit / per_tile, g, row) + kGrFew - 1) / kGrFew;
+            passes = (gm_tile(p, unit / per_tile, lane, g, row) + kGrFew - 1) / kGrFew;
             if (passes == 0) continue;
             const TW* W = static_cast<const TW*>(p.w) + static_cast<size_t>(g) * p.w_gs;
             const int n_first = unit % per_tile * ROWS;
@@ -283,14 +275,14 @@ struct RowsStream {
 // MR rows of a tile (m_here of them are real, the last is repeated) against the output rows from n_first on. ``row``:
 // lane i has the tile's i-th row; ``done``: steps of the warp's ring taken so far. With 8 output rows up to two rows' inputs are
 // asked for a step ahead.
-template <int MR, typename TA, typename TW, bool GATED, int ROWS>
-__device__ __forceinline__ void grouped_rows_unit(RowsStream<TA, TW, GATED, ROWS>& q, int g, int row, int n_first, int m0, int m_here, int& done) {
+template <int MR, typename TW, bool GATED, int ROWS>
+__device__ __forceinline__ void grouped_rows_unit(RowsStream<TW, GATED, ROWS>& q, int g, int row, int n_first, int m0, int m_here, int& done) {
     const GroupedArgs& p = q.p;
-    using Stream = RowsStream<TA, TW, GATED, ROWS>;
-    constexpr int kW = Stream::kW, kStages = Stream::kStages, kPiece = Vec16<TW>::N;
+    using Stream = RowsStream<TW, GATED, ROWS>;
+    constexpr int kW = Stream::kW, kStages = Stream::kStages, kPiece = Stream::kPiece;
     constexpr bool kAhead = ROWS == 8 && MR <= 2;
-    const TA* A = static_cast<const TA*>(p.a) + p.a_off + static_cast<size_t>(g) * p.a_gs;
-    const TA* arow[MR];
+    const float* A = static_cast<const float*>(p.a) + p.a_off + static_cast<size_t>(g) * p.a_gs;
+    const float* arow[MR];
 #pragma unroll
     for (int i = 0; i < MR; ++i) arow[i] = A + static_cast<size_t>(__shfl_sync(0xffffffffu, row, m0 + min(i, m_here - 1)) / p.a_div) * p.lda;
     // the output gate's values of the unit's outputs, (row of weights, row of the tile) by lane, asked for before the weights arrive
@@ -309,45 +301,41 @@ __device__ __forceinline__ void grouped_rows_unit(RowsStream<TA, TW, GATED, ROWS
     for (int r = 0; r < kW; ++r)
 #pragma unroll
         for (int i = 0; i < MR; ++i) acc[r][i] = 0.f;
-    constexpr int kHeld = kAhead ? kPiece : 4;
-    float av[MR][kHeld], next[kAhead ? MR : 1][kHeld];
-    auto fetch = [&](float* dst, int i, int at) {
-        const float4 v = load4<TA>(arow[i] + at);
-        dst[0] = v.x; dst[1] = v.y; dst[2] = v.z; dst[3] = v.w;
+    float4 av[MR][kAhead ? kPiece / 4 : 1], next[kAhead ? MR : 1][kPiece / 4];
+    auto fetch = [&](float4 (&dst)[kPiece / 4], const float* src, int at) {
+#pragma unroll
+        for (int h = 0; h < kPiece / 4; ++h) dst[h] = *reinterpret_cast<const float4*>(src + at * kPiece + 4 * h);
     };
     if constexpr (kAhead) {
         if (q.lane < q.pieces)
 #pragma unroll
-            for (int i = 0; i < MR; ++i)
-#pragma unroll
-                for (int h = 0; h < kPiece; h += 4) fetch(&av[i][h], i, q.lane * kPiece + h);
+            for (int i = 0; i < MR; ++i) fetch(av[i], arow[i], q.lane);
     }
     for (int step = 0; step < q.steps; ++step, ++done) {
         const int c = step * 32 + q.lane;
         if constexpr (kAhead) {
             if (c + 32 < q.pieces)
 #pragma unroll
-                for (int i = 0; i < MR; ++i)
-#pragma unroll
-                    for (int h = 0; h < kPiece; h += 4) fetch(&next[i][h], i, (c + 32) * kPiece + h);
+                for (int i = 0; i < MR; ++i) fetch(next[i], arow[i], c + 32);
         }
         asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
         if (c < q.pieces) {
             const uint4* stage = q.ring + (done % kStages) * (kW * 32);
 #pragma unroll
-            for (int h = 0; h < kPiece; h += 4) {
+            for (int h = 0; h < kPiece / 4; ++h) {
                 if constexpr (!kAhead) {
 #pragma unroll
-                    for (int i = 0; i < MR; ++i) fetch(&av[i][0], i, c * kPiece + h);
+                    for (int i = 0; i < MR; ++i) av[i][0] = *reinterpret_cast<const float4*>(arow[i] + c * kPiece + 4 * h);
                 }
 #pragma unroll
                 for (int r = 0; r < kW; ++r) {
-                    float wv[8];
-                    Vec16<TW>::load(reinterpret_cast<const TW*>(stage + r * 32), wv);
+                    const float4 w = piece4(reinterpret_cast<const TW*>(stage + r * 32) + 4 * h);
 #pragma unroll
-                    for (int i = 0; i < MR; ++i)
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) acc[r][i] = fmaf(av[i][(kAhead ? h : 0) + j], wv[h + j], acc[r][i]);
+                    for (int i = 0; i < MR; ++i) {
+                        const float4 x = av[i][kAhead ? h : 0];
+                        acc[r][i] = fmaf(x.x, w.x, acc[r][i]); acc[r][i] = fmaf(x.y, w.y, acc[r][i]);
+                        acc[r][i] = fmaf(x.z, w.z, acc[r][i]); acc[r][i] = fmaf(x.w, w.w, acc[r][i]);
+                    }
                 }
             }
         }
@@ -355,7 +343,7 @@ __device__ __forceinline__ void grouped_rows_unit(RowsStream<TA, TW, GATED, ROWS
 #pragma unroll
             for (int i = 0; i < MR; ++i)
 #pragma unroll
-                for (int j = 0; j < kHeld; ++j) av[i][j] = next[i][j];
+                for (int h = 0; h < kPiece / 4; ++h) av[i][h] = next[i][h];
         }
         q.request();                                  // into the stage read a step ago, by this lane alone
     }
@@ -382,12 +370,12 @@ __device__ __forceinline__ void grouped_rows_unit(RowsStream<TA, TW, GATED, ROWS
 }
 
 // tiles: how many there are (experts form: at most; the number is read on the device)
-template <typename TA, typename TW, bool GATED, int ROWS>
-__global__ void __launch_bounds__(kGrWarps * 32, (RowsStream<TA, TW, GATED, ROWS>::kBlocks))
+template <typename TW, bool GATED, int ROWS>
+__global__ void __launch_bounds__(kGrWarps * 32, (RowsStream<TW, GATED, ROWS>::kBlocks))
 grouped_rows_kernel(const GroupedArgs p, int tiles) {
     extern __shared__ uint4 s_ring[];
     pdl_prologue();
-    using Stream = RowsStream<TA, TW, GATED, ROWS>;
+    using Stream = RowsStream<TW, GATED, ROWS>;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     Stream q{p};
     q.ring = s_ring + warp * (Stream::kStages * Stream::kW * 32) + lane;
@@ -403,7 +391,7 @@ grouped_rows_kernel(const GroupedArgs p, int tiles) {
     for (int i = 0; i < Stream::kStages - 1; ++i) q.request();
     int done = 0, x = -1, g = 0, row = -1, m_count = 0;
     for (int unit = first; unit < q.units; unit += q.stride) {
-        if (unit / q.per_tile != x) { x = unit / q.per_tile; m_count = q.tile(x, g, row); }
+        if (unit / q.per_tile != x) { x = unit / q.per_tile; m_count = gm_tile(p, x, lane, g, row); }
         const int n_first = unit % q.per_tile * ROWS;
         for (int m0 = 0; m0 < m_count; m0 += kGrFew) {
             const int m_here = min(kGrFew, m_count - m0);
@@ -416,21 +404,408 @@ grouped_rows_kernel(const GroupedArgs p, int tiles) {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-// The heads form with a rotated tail for up to four rows: short inputs and many outputs, where a tile's rounds through shared
+// The few-row form of bfloat16 weights, on the tensor cores (mma.sync m16n8k16: tcgen05 would want the rows of 64 or 128 outputs in one
+// tile, too coarse to share a few experts' matrices evenly among 148 SMs, and multiplies a few tokens no faster than memory brings
+// the weights). A unit is MT x 16 rows of weights (gated: eight gate rows and the eight up rows of the same outputs) over all of K,
+// the work of a block; its eight warps share K in blocks of 64 values, dealt in turn, each with a ring of cp.async pieces of its own
+// that runs on from unit to unit. The ring's lane mapping is the fragments': a lane's 16 bytes are eight neighbouring k of one row, its
+// share of two products whose k are taken in an order of their own (the same for weights and inputs), so nothing is rearranged and no
+// lane reads what another one copied. Inputs are asked for a step ahead, in registers. Per unit the warps' sums meet once in shared
+// memory, where they are added in pairs.
+// bfloat16 inputs are multiplied as they are, up to sixteen rows of a tile with a piece of the weights; a 32-bit input is cut into three
+// bfloat16 values whose sum it is (24 bits of mantissa in three times eight; a part below 2^-126 may count as zero), so its products are
+// exact as well. The cutting costs more instructions than the products, so its units are of 32 rows, and of eight rows of a tile
+// (a tile with more is two, whose weights meet in L2). The tensor cores cut the sums that they carry on, so each
+// product of sixteen k starts from zero and is added by the CUDA cores, rounded (the second and third parts' sums are carried on: a
+// cut there is 2^-8 of one in the first). An output element depends on its own row only, not on the row's place in a tile.
+// Measured, sixteen pairs of eight experts, on the CUDA cores -> here: gated 2 x 4,096 outputs of 2,048 bfloat16 inputs 62.6 -> 48.6 us
+// when they spread evenly (41.6 of bytes), 90 -> 46 in a token's step; 2,048 outputs of 4,096 32-bit inputs there 54 -> 30. Errors against 64 bits:
+// 1.25e-7 of the outputs' size (1.29e-7 before) and 0.87e-7 (2.1e-7 before).
+constexpr int kGmWarps = 8, kGmSub = 2;                      // sub-blocks of 32 k per step of a warp's ring
+constexpr int kGmBlocks = 2;                                 // an SM
+template <typename TA> struct GmShape;
+template <> struct GmShape<__nv_bfloat16> { static constexpr int MT = 1, NT = 2, kStages = 6; };
+template <> struct GmShape<float> { static constexpr int MT = 2, NT = 1, kStages = 3; };
+template <typename TA> struct GmSizes {                      // bytes
+    static constexpr int kStage = kGmSub * GmShape<TA>::MT * 1024, kRing = kGmWarps * GmShape<TA>::kStages * kStage;
+    static constexpr int kSums = 2 * kGmWarps * 2 * 32 * 16;             // MT x NT fragments of a warp, twice
+};
+
+__device__ __forceinline__ void gm_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// Two products of sixteen k, added up and into a sum of the CUDA cores.
+__device__ __forceinline__ void gm_mma_add(float (&c)[4], const uint4& w0, const uint4& w1, const uint32_t (&x)[4]) {
+    float d[4] = {0.f, 0.f, 0.f, 0.f}, e[4] = {0.f, 0.f, 0.f, 0.f};
+    gm_mma(d, w0.x, w1.x, w0.y, w1.y, x[0], x[1]);
+    gm_mma(e, w0.z, w1.z, w0.w, w1.w, x[2], x[3]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c[i] += d[i] + e[i];
+}
+
+// Two 32-bit sums or differences in one instruction.
+__device__ __forceinline__ unsigned long long gm_pair(float a, float b) {
+    unsigned long long d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+    return d;
+}
+__device__ __forceinline__ float2 gm_split(unsigned long long v) {
+    float2 f;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+    return f;
+}
+__device__ __forceinline__ unsigned long long gm_plus(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned long long gm_minus(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(b), "l"(gm_pair(-1.f, -1.f)), "l"(a));
+    return d;
+}
+
+// Eight neighbouring values of an input row as they are read (GmInput) and as they are multiplied (GmParts): what they add to the
+// sums with eight values of weight rows w0 and w1.
+template <typename TA> struct GmParts;
+template <typename TA> struct GmInput;
+template <> struct GmParts<__nv_bfloat16> {
+    uint4 v;
+    __device__ __forceinline__ void multiply(float (&c)[4], float (&)[4], const uint4& w0, const uint4& w1) const {
+        const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+        gm_mma_add(c, w0, w1, x);
+    }
+};
+template <> struct GmInput<__nv_bfloat16> {
+    uint4 v;
+    __device__ __forceinline__ void zero() { v = make_uint4(0, 0, 0, 0); }
+    __device__ __forceinline__ void load(const __nv_bfloat16* p) { v = *reinterpret_cast<const uint4*>(p); }
+    __device__ __forceinline__ GmParts<__nv_bfloat16> parts() const { return {v}; }
+};
+template <> struct GmParts<float> {
+    uint32_t top[4], mid[4], low[4];
+    __device__ __forceinline__ void multiply(float (&c)[4], float (&rest)[4], const uint4& w0, const uint4& w1) const {
+        gm_mma(rest, w0.x, w1.x, w0.y, w1.y, low[0], low[1]);
+        gm_mma(rest, w0.z, w1.z, w0.w, w1.w, low[2], low[3]);
+        gm_mma(rest, w0.x, w1.x, w0.y, w1.y, mid[0], mid[1]);
+        gm_mma(rest, w0.z, w1.z, w0.w, w1.w, mid[2], mid[3]);
+        gm_mma_add(c, w0, w1, top);
+    }
+};
+template <> struct GmInput<float> {
+    float4 a, b;
+    __device__ __forceinline__ void zero() { a = b = make_float4(0.f, 0.f, 0.f, 0.f); }
+    __device__ __forceinline__ void load(const float* p) {
+        a = *reinterpret_cast<const float4*>(p);
+        b = *(reinterpret_cast<const float4*>(p) + 1);
+    }
+    __device__ __forceinline__ GmParts<float> parts() const {
+        const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        float top[8], mid[8], low[8];
+        auto cut = [](float v) { return __uint_as_float(__float_as_uint(v) & 0xffff0000u); };
+        unsigned long long sum = 0ull;
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) {               // cut, not rounded: each difference is exact
+            top[i] = cut(x[i]); top[i + 1] = cut(x[i + 1]);
+            const unsigned long long rest = gm_minus(gm_pair(x[i], x[i + 1]), gm_pair(top[i], top[i + 1]));
+            const float2 r = gm_split(rest);
+            mid[i] = cut(r.x); mid[i + 1] = cut(r.y);
+            const unsigned long long last = gm_minus(rest, gm_pair(mid[i], mid[i + 1]));
+            const float2 l = gm_split(last);
+            low[i] = l.x; low[i + 1] = l.y;
+            sum = gm_plus(sum, last);
+        }
+        const float2 sums = gm_split(sum);
+        const float any = sums.x + sums.y;
+        if (any != any) {                              // an infinity or none: it alone, its differences are none
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if ((__float_as_uint(x[i]) & 0x7f800000u) == 0x7f800000u) {
+                    top[i] = x[i] != x[i] ? __uint_as_float(0x7fc00000u) : x[i];
+                    mid[i] = low[i] = 0.f;
+                }
+        }
+        GmParts<float> p;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {                  // the upper halves of two values
+            p.top[i] = __byte_perm(__float_as_uint(top[2 * i]), __float_as_uint(top[2 * i + 1]), 0x7632);
+            p.mid[i] = __byte_perm(__float_as_uint(mid[2 * i]), __float_as_uint(mid[2 * i + 1]), 0x7632);
+            p.low[i] = __byte_perm(__float_as_uint(low[2 * i]), __float_as_uint(low[2 * i + 1]), 0x7632);
+        }
+        return p;
+    }
+};
+
+// Where a walk through a block's units stands: tile, unit within it, and the tile's group and rows.
+template <bool HALVES>
+struct GmWalk {
+    int x, n, g = 0, row = -1, count = 0;            // x: tile, n: unit of the tile (its outputs start at n * kOut)
+    int known = -1;
+    // To the first unit from (x, n) on, in strides, whose tile has rows; false: there is none.
+    __device__ __forceinline__ bool seek(const GroupedArgs& p, int tiles, int per_tile, int stride, int lane) {
+        for (;; n += stride) {
+            while (n >= per_tile) { n -= per_tile; ++x; }
+            if (x >= tiles) return false;
+            if (known != x) { known = x; count = gm_tile<HALVES>(p, x, lane, g, row); }
+            if (count > 0) return true;
+        }
+    }
+};
+
+template <typename TA, bool GATED>
+__global__ void __launch_bounds__(kGmWarps * 32, kGmBlocks)
+grouped_mma_kernel(const GroupedArgs p, int tiles_given) {
+    extern __shared__ uint4 s_ring[];
+    pdl_prologue();
+    constexpr int MT = GmShape<TA>::MT, NT = GmShape<TA>::NT, kStages = GmShape<TA>::kStages, kStage = GmSizes<TA>::kStage;
+    constexpr bool kHalves = NT == 1;
+    constexpr int kOut = GATED ? 8 * MT : 16 * MT;                  // outputs of a unit
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gr = lane >> 2, kq = (lane & 3) * 8;
+    uint4* ring = s_ring + warp * (kStages * kStage / 16) + lane;
+    float4* sums = reinterpret_cast<float4*>(s_ring + GmSizes<TA>::kRing / 16);
+    const int per_tile = (p.N + kOut - 1) / kOut, stride = gridDim.x;
+    const int tiles = (p.tile_group ? *p.n_tiles : tiles_given) * (kHalves ? 2 : 1);
+    constexpr int kStepK = kGmSub * 32;
+    const int steps = (p.K + kGmWarps * kStepK - 1) / (kGmWarps * kStepK);      // step i of warp w: k from (i * kGmWarps + w) * kStepK on
+
+    // what is requested next: weights. Row gr + 8 r of the unit (r < 2 MT); gated: the up rows are the odd r
+    GmWalk<kHalves> rq{static_cast<int>(blockIdx.x) / per_tile, static_cast<int>(blockIdx.x) % per_tile};
+    int rq_k = 0;                                                   // of the unit's K, without this warp's and lane's own offset
+    const __nv_bfloat16* rq_w[2 * MT];
+    bool rq_on = false;
+    const int k_mine = warp * kStepK + kq;
+    auto seek = [&]() {
+        rq_on = rq.seek(p, tiles, per_tile, stride, lane);
+        if (!rq_on) return;
+        const int n_first = rq.n * kOut, last = p.N - 1 - n_first;
+        const __nv_bfloat16* w = static_cast<const __nv_bfloat16*>(p.w) + static_cast<size_t>(rq.g) * p.w_gs + static_cast<size_t>(n_first) * p.ldw;
+#pragma unroll
+        for (int r = 0; r < 2 * MT; ++r)
+            rq_w[r] = w + static_cast<long long>(min(gr + 8 * (GATED ? r / 2 : r), last)) * p.ldw + (GATED && (r & 1) ? p.up_off : 0);
+        rq_k = 0;
+    };
+    const unsigned ring_at = static_cast<unsigned>(__cvta_generic_to_shared(ring));
+    unsigned rq_at = 0;
+    auto request = [&]() {
+        if (rq_on) {
+#pragma unroll
+            for (int j = 0; j < kGmSub; ++j) {
+                const int k = rq_k + k_mine + j * 32;
+                const int bytes = k < p.K ? 16 : 0, off = k < p.K ? k : 0;      // 0: zeros, nothing is read (K is a multiple of 8)
+#pragma unroll
+                for (int r = 0; r < 2 * MT; ++r)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ring_at + rq_at + (j * 2 * MT + r) * 512), "l"(rq_w[r] + off), "r"(bytes) : "memory");
+            }
+            rq_k += kGmWarps * kStepK;
+            if (rq_k >= p.K) { rq.n += stride; seek(); }
+        }
+        rq_at = rq_at + kStage == kStages * kStage ? 0 : rq_at + kStage;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // ... and inputs: rows gr (and gr + 8) of the tile of the unit that `in_at` walks to
+    GmWalk<kHalves> in_at = rq;
+    int in_k = 0;
+    bool in_on = false;
+    const TA* in_a[NT];
+    GmInput<TA> in[NT][kGmSub];
+    auto in_seek = [&]() {
+        const int before = in_at.known;
+        in_on = in_at.seek(p, tiles, per_tile, stride, lane);
+        in_k = 0;
+        if (!in_on || before == in_at.known) return;
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            const int r = __shfl_sync(0xffffffffu, in_at.row, gr + 8 * t);
+            in_a[t] = static_cast<const TA*>(p.a) + static_cast<size_t>(gr + 8 * t < in_at.count ? r / p.a_div : 0) * p.lda + p.a_off + static_cast<size_t>(in_at.g) * p.a_gs;
+        }
+    };
+    auto fetch = [&]() {
+        if (!in_on) return;
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+#pragma unroll
+            for (int j = 0; j < kGmSub; ++j) {
+                const int k = in_k + k_mine + j * 32;
+                if (gr + 8 * t < in_at.count && k < p.K) in[t][j].load(in_a[t] + k);
+                else in[t][j].zero();
+            }
+        in_k += kGmWarps * kStepK;
+        if (in_k >= p.K) { in_at.n += stride; in_seek(); }
+    };
+
+    seek();
+    for (int i = 0; i < kStages - 1; ++i) request();
+    in_seek();
+    fetch();
+    GmWalk<kHalves> at{static_cast<int>(blockIdx.x) / per_tile, static_cast<int>(blockIdx.x) % per_tile};
+    unsigned got = 0;
+    for (int turn = 0; at.seek(p, tiles, per_tile, stride, lane); at.n += stride, ++turn) {
+        float acc[kGmSub][MT][NT][4], rest[MT][NT][4];              // (a sum for each sub-block: chains half as long)
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int t = 0; t < NT; ++t)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[0][m][t][i] = acc[1][m][t][i] = rest[m][t][i] = 0.f;
+        for (int step = 0; step < steps; ++step) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+            const uint4* stage = ring + got / 16;
+            got = got + kStage == kStages * kStage ? 0 : got + kStage;
+#pragma unroll
+            for (int j = 0; j < kGmSub; ++j)
+#pragma unroll
+                for (int t = 0; t < NT; ++t) {
+                    if (t > 0 && at.count <= 8) break;
+                    const GmParts<TA> x = in[t][j].parts();
+#pragma unroll
+                    for (int m = 0; m < MT; ++m) {
+                        const uint4 w0 = stage[(j * 2 * MT + 2 * m) * 32], w1 = stage[(j * 2 * MT + 2 * m + 1) * 32];
+                        x.multiply(acc[j][m][t], rest[m][t], w0, w1);
+                    }
+                }
+            fetch();
+            request();                                              // into the stage read a step ago, by this lane alone
+        }
+        float4* mine = sums + (turn & 1) * (kGmWarps * 2 * 32) + lane;
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int t = 0; t < NT; ++t)
+                if (8 * t < at.count) {
+                    float v[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) v[i] = acc[0][m][t][i] + (acc[1][m][t][i] + rest[m][t][i]);
+                    mine[(warp * 2 + m * NT + t) * 32] = make_float4(v[0], v[1], v[2], v[3]);
+                }
+        __syncthreads();         // (this half is written again two units on, behind the next barrier, which every reader of it meets later)
+        // warps 0 .. 3, warp w: fragment w / 2 (of rows of weights, or of the tile's rows), of the tile's rows 2 (lane % 4) + w % 2 of eight
+        const int f = warp >> 1, t = NT == 2 ? f : 0, m_rows = NT == 2 ? 0 : f * (GATED ? 8 : 16), m = 8 * t + (lane & 3) * 2 + (warp & 1);
+        if (warp < 4 && 8 * t < at.count) {
+            const int out_row = __shfl_sync(0xffffffffu, at.row, m);
+            if (m < at.count) {
+                float u0[kGmWarps], u1[kGmWarps];
+#pragma unroll
+                for (int w = 0; w < kGmWarps; ++w) {
+                    const float4 part = mine[(w * 2 + f) * 32];
+                    u0[w] = warp & 1 ? part.y : part.x;
+                    u1[w] = warp & 1 ? part.w : part.z;
+                }
+                float v0 = ((u0[0] + u0[1]) + (u0[2] + u0[3])) + ((u0[4] + u0[5]) + (u0[6] + u0[7]));
+                float v1 = ((u1[0] + u1[1]) + (u1[2] + u1[3])) + ((u1[4] + u1[5]) + (u1[6] + u1[7]));
+                const int n_first = at.n * kOut + m_rows;
+                if (p.scales) { const float sc = p.scales[out_row]; v0 *= sc; v1 *= sc; }
+                auto store = [&](int n, float value) {
+                    if (n >= p.N) return;
+                    value = gp_gated(p, value, out_row, at.g, n);
+                    const size_t o = static_cast<size_t>(out_row) * p.ldo + p.o_off + static_cast<size_t>(at.g) * p.o_gs + n;
+                    if (p.out_is_f32) static_cast<float*>(p.out)[o] = value;
+                    else static_cast<__nv_bfloat16*>(p.out)[o] = __float2bfloat16_rn(value);
+                };
+                if (GATED) {
+                    store(n_first + gr, gated_value(v0, v1, p.act, p.act_limit));
+                } else {
+                    store(n_first + gr, plain_value(v0, p.out_act));
+                    store(n_first + gr + 8, plain_value(v1, p.out_act));
+                }
+            }
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+// The heads form of bfloat16 weights: every row count with a rotated tail, and without one where the rows are more than the few-row form
+// takes. A warp has MT x 16 outputs of NT x 8 rows, its operands straight from memory in the fragments' layout (as in the few-row
+// form), a step of 32 k ahead, the first weights asked for before the wait (they belong to no earlier kernel). kFew: the block's four
+// warps lie along the outputs (few rows: the weights are what is read), else along the rows. A sum goes through K in the same
+// order with the same products in either shape: a token's result is the same to the bit whatever else is in the step. Measured, 16 heads,
+// on the CUDA cores -> here: 512 to 64, 1,273 rows 91 -> 34 us; 64 to 512 with a tail, 8 rows 14.6 -> 2.7, 1,273 rows 51 -> 43; 128 to 1,024
+// 28 -> 4.7 and 173 -> 110.
+template <typename TA, int MT, int NT, bool kFew>
+__global__ void __launch_bounds__(128)
+head_mma_kernel(const GroupedArgs p) {
+    pdl_launch_dependents();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gr = lane >> 2, kq = (lane & 3) * 8, g = blockIdx.x;
+    const int n0 = (kFew ? blockIdx.y * 4 + warp : blockIdx.y) * (16 * MT);
+    const int row0 = (kFew ? blockIdx.z : blockIdx.z * 4 + warp) * (8 * NT), rows = min(8 * NT, p.rows - row0);
+    if (rows <= 0) return;
+    const TA* A = static_cast<const TA*>(p.a) + static_cast<size_t>(row0) * p.lda + p.a_off + static_cast<size_t>(g) * p.a_gs;
+    const __nv_bfloat16* W = static_cast<const __nv_bfloat16*>(p.w) + static_cast<size_t>(g) * p.w_gs;
+    uint4 w[MT][2], w_next[MT][2];
+    GmInput<TA> in[NT], in_next[NT];
+    auto weights = [&](uint4 (&dst)[MT][2], int k0) {
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+#pragma unroll
+            for (int half = 0; half < 2; ++half)
+                dst[i][half] = k0 + kq < p.K ? __ldg(reinterpret_cast<const uint4*>(W + static_cast<size_t>(min(n0 + 16 * i + 8 * half + gr, p.N - 1)) * p.ldw + k0 + kq))
+                                             : make_uint4(0, 0, 0, 0);
+    };
+    auto inputs = [&](GmInput<TA> (&dst)[NT], int k0) {
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            if (8 * t + gr < rows && k0 + kq < p.K) dst[t].load(A + static_cast<size_t>(8 * t + gr) * p.lda + k0 + kq);
+            else dst[t].zero();
+        }
+    };
+    if (n0 < p.N) weights(w, 0);
+    pdl_wait();
+    if (p.tail > 0 && blockIdx.y == 0) {                // the rotated tail, by the blocks of the first outputs
+        const int first = kFew ? threadIdx.x : lane, step = kFew ? 128 : 32, half = p.tail / 2;
+        for (int i = first; i < rows * half; i += step)
+            gp_rotate_pair(p, A + static_cast<size_t>(i / half) * p.lda + p.K, row0 + i / half, g, i % half);
+    }
+    if (n0 >= p.N) return;
+    float acc[MT][NT][4], rest[MT][NT][4];
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[i][t][e] = rest[i][t][e] = 0.f;
+    inputs(in, 0);
+    for (int k0 = 0; k0 < p.K; k0 += 32) {
+        if (k0 + 32 < p.K) { weights(w_next, k0 + 32); inputs(in_next, k0 + 32); }
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            const GmParts<TA> x = in[t].parts();
+#pragma unroll
+            for (int i = 0; i < MT; ++i) x.multiply(acc[i][t], rest[i][t], w[i][0], w[i][1]);
+        }
+#pragma unroll
+        for (int i = 0; i < MT; ++i) { w[i][0] = w_next[i][0]; w[i][1] = w_next[i][1]; }
+#pragma unroll
+        for (int t = 0; t < NT; ++t) in[t] = in_next[t];
+    }
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int m = 8 * t + (lane & 3) * 2 + (e & 1), n = n0 + 16 * i + 8 * (e >> 1) + gr;
+                if (m >= rows || n >= p.N) continue;
+                const float v = gp_gated(p, acc[i][t][e] + rest[i][t][e], row0 + m, g, n);
+                const size_t o = static_cast<size_t>(row0 + m) * p.ldo + p.o_off + static_cast<size_t>(g) * p.o_gs + n;
+                if (p.out_is_f32) static_cast<float*>(p.out)[o] = v;
+                else static_cast<__nv_bfloat16*>(p.out)[o] = __float2bfloat16_rn(v);
+            }
+}
+
+// The heads form of 32-bit weights with a rotated tail for up to four rows: short inputs and many outputs, where a tile's rounds through shared
 // memory and its sixteen rows cost more than its multiply-adds, and the few-row form spends its time on its sums. A thread has one
 // output of every row, its weights in registers (asked for before the wait: they belong to no earlier kernel). The sum is one
 // chain in the order of k, as in the tiles of 16 and of 64: a token's result is the same to the bit whatever else is in the step.
 constexpr int kGcRows = 4, kGcCols = 64, kGcK = 64;
 
-template <typename TA, typename TW>
 __global__ void __launch_bounds__(kGcCols)
 head_product_few_kernel(const GroupedArgs p) {
     pdl_launch_dependents();
-    constexpr int kPiece = Vec16<TW>::N, kPieces = kGcK / kPiece;
+    constexpr int kPiece = 4, kPieces = kGcK / kPiece;
     __shared__ __align__(16) float s_a[kGcK][kGcRows];
     const int tid = threadIdx.x, g = blockIdx.x, n = blockIdx.y * kGcCols + tid;
-    const TA* A = static_cast<const TA*>(p.a) + p.a_off + static_cast<size_t>(g) * p.a_gs;
-    const TW* wrow = static_cast<const TW*>(p.w) + static_cast<size_t>(g) * p.w_gs + static_cast<size_t>(min(n, p.N - 1)) * p.ldw;
+    const float* A = static_cast<const float*>(p.a) + p.a_off + static_cast<size_t>(g) * p.a_gs;
+    const float* wrow = static_cast<const float*>(p.w) + static_cast<size_t>(g) * p.w_gs + static_cast<size_t>(min(n, p.N - 1)) * p.ldw;
     uint4 wv[kPieces];
     auto request = [&](int k0) {
 #pragma unroll
@@ -456,8 +831,7 @@ head_product_few_kernel(const GroupedArgs p) {
         __syncthreads();
 #pragma unroll
         for (int i = 0; i < kPieces; ++i) {
-            float w[8];
-            Vec16<TW>::load(reinterpret_cast<const TW*>(&wv[i]), w);
+            const float w[kPiece] = {__uint_as_float(wv[i].x), __uint_as_float(wv[i].y), __uint_as_float(wv[i].z), __uint_as_float(wv[i].w)};
 #pragma unroll
             for (int j = 0; j < kPiece; ++j) {
                 const float4 a = *reinterpret_cast<const float4*>(s_a[i * kPiece + j]);
@@ -804,33 +1178,45 @@ static bool rows_form_fits(const GroupedArgs& p, int a_dtype, int w_dtype) {
     return p.lda % a_piece == 0 && p.a_off % a_piece == 0 && p.a_gs % a_piece == 0;
 }
 
-template <typename TA, typename TW, bool GATED, int ROWS>
+template <typename TW, bool GATED, int ROWS>
 static int launch_grouped_rows_as(const GroupedArgs& p, unsigned tiles, cudaStream_t st) {
-    using Stream = RowsStream<TA, TW, GATED, ROWS>;
+    using Stream = RowsStream<TW, GATED, ROWS>;
     static SharedLimit limit;
-    const cudaError_t ready = limit.allow(reinterpret_cast<const void*>(grouped_rows_kernel<TA, TW, GATED, ROWS>), Stream::kSmem);
+    const cudaError_t ready = limit.allow(reinterpret_cast<const void*>(grouped_rows_kernel<TW, GATED, ROWS>), Stream::kSmem);
     if (ready != cudaSuccess) { set_error("grouped_product (rows): %s", cudaGetErrorString(ready)); return 1; }
     int sms = 0, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const long long blocks = (static_cast<long long>(tiles) * ((p.N + ROWS - 1) / ROWS) + kGrWarps - 1) / kGrWarps;
     GI_REQUIRE(blocks * kGrWarps <= 2147483647LL - 3 * 1024 * kGrWarps, "grouped_product: too many tiles");
-    launch_kernel((grouped_rows_kernel<TA, TW, GATED, ROWS>), dim3(static_cast<unsigned>(std::min<long long>(blocks, Stream::kBlocks * sms))), dim3(kGrWarps * 32),
+    launch_kernel((grouped_rows_kernel<TW, GATED, ROWS>), dim3(static_cast<unsigned>(std::min<long long>(blocks, Stream::kBlocks * sms))), dim3(kGrWarps * 32),
                   Stream::kSmem, st, p, static_cast<int>(tiles));
     return check_launch("grouped_product (rows)");
 }
+template <typename TA, bool GATED>
+static int launch_grouped_mma(const GroupedArgs& p, unsigned tiles, cudaStream_t st) {
+    constexpr int kSmem = GmSizes<TA>::kRing + GmSizes<TA>::kSums, kOut = (GATED ? 8 : 16) * GmShape<TA>::MT;
+    static SharedLimit limit;
+    const cudaError_t ready = limit.allow(reinterpret_cast<const void*>(grouped_mma_kernel<TA, GATED>), kSmem);
+    if (ready != cudaSuccess) { set_error("grouped_product (few rows): %s", cudaGetErrorString(ready)); return 1; }
+    int sms = 0, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const long long units = static_cast<long long>(tiles) * (2 / GmShape<TA>::NT) * ((p.N + kOut - 1) / kOut);
+    GI_REQUIRE(units <= 2147483647LL - 4 * 1024, "grouped_product: too many tiles");
+    launch_kernel((grouped_mma_kernel<TA, GATED>), dim3(static_cast<unsigned>(std::min<long long>(units, kGmBlocks * sms))), dim3(kGmWarps * 32), kSmem, st, p, static_cast<int>(tiles));
+    return check_launch("grouped_product (few rows)");
+}
 template <bool GATED>
 static int launch_grouped_rows(const GroupedArgs& p, int a_dtype, int w_dtype, unsigned tiles, cudaStream_t st) {
-    if (a_dtype == kF32 && w_dtype == kF32) return launch_grouped_rows_as<float, float, GATED, 4>(p, tiles, st);
-    if (a_dtype == kF32 && w_dtype == kBF16) {
-        // 32-bit inputs are as many bytes as four rows of bfloat16 weights for every two of them, and come from L2: eight rows a
-        // unit (2,048 outputs of 4,096 and of 3,072 inputs, sixteen and four pairs: 47.0 -> 43.4 us and 21.9 -> 15.3). Heads' matrices are too
-        // small to give every warp such a unit (19 against 26 us), two gated rows' registers leave no third block (68 against 84).
-        if constexpr (!GATED)
-            if (p.tile_group) return launch_grouped_rows_as<float, __nv_bfloat16, false, 8>(p, tiles, st);
-        return launch_grouped_rows_as<float, __nv_bfloat16, GATED, 4>(p, tiles, st);
-    }
-    return launch_grouped_rows_as<__nv_bfloat16, __nv_bfloat16, GATED, 4>(p, tiles, st);
+    if (w_dtype == kF32) return launch_grouped_rows_as<float, GATED, 4>(p, tiles, st);
+    // 32-bit inputs with room for at most five tiles (up to four pairs, or few experts): mostly a pair or two a tile, so that the
+    // multiply-adds are few, and cutting eight rows' inputs into parts costs more than they do (2,048 outputs of 4,096 inputs, 2 / 4
+    // pairs: 14.1 / 17.1 us on the CUDA cores, 14.7 / 26.1 on the tensor cores; 8 pairs 30.2 against 29.4, sixteen 36.7 against 40.8 when
+    // they spread evenly and 54 against 31 when they crowd a few experts).
+    if constexpr (!GATED)
+        if (a_dtype == kF32 && p.tile_group && tiles <= 5) return launch_grouped_rows_as<__nv_bfloat16, false, 8>(p, tiles, st);
+    return a_dtype == kF32 ? launch_grouped_mma<float, GATED>(p, tiles, st) : launch_grouped_mma<__nv_bfloat16, GATED>(p, tiles, st);
 }
 
 template <bool GATED>
@@ -840,6 +1226,17 @@ static int launch_grouped(const GroupedArgs& p, int a_dtype, int w_dtype, dim3 g
     else if (a_dtype == kBF16 && w_dtype == kBF16) launch_kernel((grouped_product_kernel<__nv_bfloat16, __nv_bfloat16, GATED>), grid, dim3(128), 0, st, p);
     else { set_error("grouped_product: inputs of dtype code %d with weights of %d are not built", a_dtype, w_dtype); return 2; }
     return check_launch("grouped_product");
+}
+
+// bfloat16 weights in pieces that rows_form_fits has looked at. Up to 8 rows a block has 64 outputs, with more 64 rows and 64 outputs.
+template <typename TA>
+static int launch_head_mma(const GroupedArgs& p, cudaStream_t st) {
+    const unsigned heads = static_cast<unsigned>(p.groups), blocks_n = static_cast<unsigned>((p.N + 63) / 64);
+    GI_REQUIRE(blocks_n <= 65535 && (p.rows + 63) / 64 <= 65535, "head_product: too many tiles");
+    if (p.rows <= 8) launch_kernel((head_mma_kernel<TA, 1, 1, true>), dim3(heads, blocks_n), dim3(128), 0, st, p);
+    else if (p.rows <= 32) launch_kernel((head_mma_kernel<TA, 1, 2, true>), dim3(heads, blocks_n, (p.rows + 15) / 16), dim3(128), 0, st, p);
+    else launch_kernel((head_mma_kernel<TA, 4, 2, false>), dim3(heads, blocks_n, (p.rows + 63) / 64), dim3(128), 0, st, p);
+    return check_launch("head_product (tensor cores)");
 }
 
 }  // namespace gi
@@ -867,6 +1264,17 @@ static int gi_head_product_impl(const void* a, int a_dtype, long long lda, int a
     const long long tiles = static_cast<long long>((rows + kGpTM - 1) / kGpTM) * heads;
     GI_REQUIRE(tiles <= 2147483647LL, "head_product: too many tiles");
     dim3 grid(static_cast<unsigned>(tiles), (N + kGpTN - 1) / kGpTN);
+    // few tokens without a tail: the heads' matrices are what is read, their K shared by a block's warps; else bfloat16 weights on the
+    // tensor cores at every row count. (With a tail every row count has the same sums to the bit, whatever form it runs.)
+    if (rows_form_fits(p, a_dtype, w_dtype)) {
+        cudaStream_t st = static_cast<cudaStream_t>(stream);
+        if (tail == 0 && rows <= 2 * kGpTM) return launch_grouped_rows<false>(p, a_dtype, w_dtype, static_cast<unsigned>(tiles), st);
+        if (w_dtype == kBF16) return a_dtype == kF32 ? launch_head_mma<float>(p, st) : launch_head_mma<__nv_bfloat16>(p, st);
+        if (tail > 0 && rows <= kGcRows) {
+            launch_kernel(head_product_few_kernel, dim3(heads, (N + kGcCols - 1) / kGcCols), dim3(kGcCols), 0, st, p);
+            return check_launch("head_product (few rows)");
+        }
+    }
     // many tokens: tiles of 64 x 64 where every group of four values is aligned (K in whole fours: no ragged piece)
     if (rows >= 2 * kG64 && K % 4 == 0 && lda % 4 == 0 && a_off % 4 == 0 && a_gs % 4 == 0 && w_gs % 4 == 0 &&
         reinterpret_cast<uintptr_t>(a) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0 && !(a_dtype == kBF16 && w_dtype == kF32)) {
@@ -878,17 +1286,6 @@ static int gi_head_product_impl(const void* a, int a_dtype, long long lda, int a
         else if (a_dtype == kF32) launch_kernel((head_product64_kernel<float, __nv_bfloat16>), grid64, dim3(256), 0, st64, p);
         else launch_kernel((head_product64_kernel<__nv_bfloat16, __nv_bfloat16>), grid64, dim3(256), 0, st64, p);
         return check_launch("head_product (tiles of 64)");
-    }
-    // few tokens: the heads' matrices are what is read; with a rotated tail every form's sums are chains in the order of k. 16 heads of 64
-    // to 512, bfloat16 weights, launches of one graph: 2.8 to 3.3 us for one to four rows, 13.2 to 13.4 in tiles (as long for eight)
-    if (rows <= (tail == 0 ? 2 * kGpTM : kGcRows) && rows_form_fits(p, a_dtype, w_dtype)) {
-        cudaStream_t st = static_cast<cudaStream_t>(stream);
-        if (tail == 0) return launch_grouped_rows<false>(p, a_dtype, w_dtype, static_cast<unsigned>(tiles), st);
-        const dim3 few(heads, (N + kGcCols - 1) / kGcCols);
-        if (a_dtype == kF32 && w_dtype == kF32) launch_kernel((head_product_few_kernel<float, float>), few, dim3(kGcCols), 0, st, p);
-        else if (a_dtype == kF32) launch_kernel((head_product_few_kernel<float, __nv_bfloat16>), few, dim3(kGcCols), 0, st, p);
-        else launch_kernel((head_product_few_kernel<__nv_bfloat16, __nv_bfloat16>), few, dim3(kGcCols), 0, st, p);
-        return check_launch("head_product (few rows)");
     }
     return launch_grouped<false>(p, a_dtype, w_dtype, grid, static_cast<cudaStream_t>(stream));
 }

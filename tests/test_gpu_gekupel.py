@@ -485,6 +485,47 @@ def test_expert_products_of_few_rows(dtype, N, K, gated):
     _close(out.cpu(), want, torch.float32, "few rows", f32=1e-5)
 
 
+@pytest.mark.parametrize("form", ["experts", "experts, room for five tiles", "gated experts", "heads, 9 rows", "heads, 33 rows", "heads, 70 rows", "heads with a tail, 12 rows"])
+@pytest.mark.parametrize("N, K", [(16, 264), (70, 40)])
+def test_products_of_32_bit_inputs_with_bfloat16_weights(form, N, K):
+    """Inputs all of whose bits count, of any size, infinite or none. The parts that an input is cut into add up to it, so what is left are
+    roundings of 32-bit sums: K / 16 + 16 additions, each off by at most 2^-23 of the products' total size; a part below the smallest
+    normal number, 2^-126, may count as zero: two such parts a product."""
+    from geneinfer_b200.ops import kernels
+    g = torch.Generator().manual_seed(K)
+    heads = form.startswith("heads")
+    T = int(form.split(", ")[1].split()[0]) if heads else 9
+    G, tail = (3, 8 if "tail" in form else 0) if heads else (1, 0)
+    gated = form == "gated experts"
+    x, w = torch.randn(T, G, K, generator=g), _bf(torch.randn(G, (2 if gated else 1) * N, K, generator=g))
+    x[2] *= 2.0 ** 118
+    x[3] *= 1e-35
+    x[0, :, 5], x[1, :, 7], x[4, :, 9] = float("inf"), float("nan"), float("-inf")
+    out = torch.full((T, G * (N + tail)), float("nan"), device=DEV)
+    if heads:
+        a = torch.cat([x, torch.zeros(T, G, tail)], 2).reshape(T, -1).to(DEV)
+        kernels.head_product(a, 0, K + tail, w.to(DEV).bfloat16(), out, 0, N + tail, tail=tail,
+                             freq=torch.ones(tail // 2, device=DEV) if tail else None, positions=torch.zeros(T, dtype=torch.int32, device=DEV) if tail else None)
+    else:
+        room = 5 if "room" in form else 6
+        rows = torch.full((room * kernels.grouped_tile_rows(),), -1, dtype=torch.int32)
+        rows[:T] = torch.arange(T, dtype=torch.int32)
+        kernels.expert_product(x[:, 0].contiguous().to(DEV), 1, w.to(DEV).bfloat16(), out, rows.to(DEV), torch.zeros(room, dtype=torch.int32, device=DEV),
+                               torch.ones(1, dtype=torch.int32, device=DEV), gated="relu" if gated else None)
+    got = out.cpu().view(T, G, N + tail)[..., :N].double()
+    want = torch.einsum("tgk,gnk->tgn", x.double(), w.double())
+    size = torch.einsum("tgk,gnk->tgn", x.double().abs(), w.double().abs())
+    bound = (K / 16 + 16) * 2.0 ** -23 * size + 2 * 2.0 ** -126 * w.double().abs().sum(2)
+    if gated:                   # relu(gate) * up: each factor off by its bound (of rows whose products stay finite in 32 bits)
+        gate, up, eg, eu = want[..., :N].relu(), want[..., N:], bound[..., :N], bound[..., N:]
+        want, bound = gate * up, eg * (up.abs() + eu) + eu * (gate + eg) + 2.0 ** -23 * (gate * up).abs()
+        keep = [i for i in range(T) if i not in (0, 1, 2, 3, 4)]
+    else:
+        assert torch.equal(got[0], want[0]) and torch.isnan(got[1]).all() and torch.equal(got[4], want[4])
+        keep = [i for i in range(T) if i not in (0, 1, 4)]
+    assert bool(((got - want).abs() <= bound)[keep].all()), float(((got - want).abs() / bound)[keep].max())
+
+
 # ------------------------------------------------------------------------------------------ mixers alone
 ATT = {"heads": 6, "kv_heads": 2, "dim": 16, "vdim": 24, "mask": {"size": 11}, "scale": 0.45}
 LAT = {"heads": 3, "dim": 24, "rot_dim": 8, "vdim": 40, "q_rank": 32, "kv_rank": 48, "mask": {"size": 13}, "scale": 0.3,
