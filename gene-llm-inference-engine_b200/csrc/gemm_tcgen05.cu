@@ -1726,7 +1726,7 @@ static int gi_gemm_tc_rope_impl(const void* A, const void* W, int M, int K, long
 
 // Reads the status word (synchronises the stream): 0 = no bounded wait ever gave up.
 extern "C" int gi_gemm_tc_status(const void* status, void* stream, int* out) {
-    cudaError_t e = cudaMemcpyAsync(out, status, sizeof(int), cudaMemcpyDeviceToHost, static_cast<cudaStream_t>(stream));
+    cudaError_t e = cudaMemcpyAsync(out, status, sizeof(int), cudaMemcpyDefault, static_cast<cudaStream_t>(stream));      // (the word may be the host's)
     if (e == cudaSuccess) e = cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) { set_error("gemm_tc_status: %s", cudaGetErrorString(e)); return 1; }
     return 0;

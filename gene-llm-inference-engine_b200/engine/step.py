@@ -260,9 +260,9 @@ class StepEngine:
         self.max_graphs = 512
         # a listener for intermediate activations: tap(tag, layer, tensor, ctx); steps run outside graphs while it is set
         self.tap = None
-        # the kernels' status word (a bounded wait that gave up) follows every step to pinned memory
-        self._status_host = [torch.zeros(1, dtype=torch.int32).pin_memory() for _ in range(4)]
+        # an event behind every step: once it is over, the kernels' status word (a bounded wait that gave up) includes the step
         self._status_events: List[Optional[torch.cuda.Event]] = [None] * 4
+        self._status_failures = [0] * 4
         self._status_next = 0
         self.scratch_generation = 0     # counts replaced scratch buffers: what was recorded before is stale
 
@@ -551,32 +551,33 @@ class StepEngine:
 
     # ------------------------------------------------------------------ the kernels' status word
     def _post_status(self) -> None:
-        """Sends the status word after the step's kernels to pinned memory (no wait)."""
+        """Marks where the step's kernels end (no wait)."""
         slot = self._status_next
-        self._status_next = (slot + 1) % len(self._status_host)
+        self._status_next = (slot + 1) % len(self._status_events)
         if self._status_events[slot] is not None:
             self._status_events[slot].synchronize()
-            self._raise_on(self._status_host[slot])
-        self._status_host[slot].copy_(kernels.status_word(self.device), non_blocking=True)
+            self._raise_on_failure(self._status_failures[slot])
         ev = torch.cuda.Event()
         ev.record()
         self._status_events[slot] = ev
+        self._status_failures[slot] = kernels.status_failures(self.device)
 
     def _poll_status(self, wait: bool) -> None:
-        """Looks at the status words of steps that have finished (of all steps with ``wait``) and
+        """Looks at the status word behind steps that have finished (behind all steps with ``wait``) and
         raises ``KernelError`` if a kernel recorded that one of its bounded waits gave up: what
         that step computed is not to be trusted."""
         for slot, ev in enumerate(self._status_events):
             if ev is not None and (wait or ev.query()):
                 ev.synchronize()
                 self._status_events[slot] = None
-                self._raise_on(self._status_host[slot])
+                self._raise_on_failure(self._status_failures[slot])
 
-    def _raise_on(self, word: torch.Tensor) -> None:
-        code = int(word[0])
-        if code:
-            word[0] = 0
-            kernels.status_word(self.device).zero_()
+    def _raise_on_failure(self, failures: int) -> None:
+        """``failures``: how many the device had when the step was launched (more now: another reader has cleared the word)."""
+        code = int(kernels.status_word(self.device)[0])
+        if code or kernels.status_failures(self.device) != failures:
+            if code:
+                kernels.clear_status(self.device)
             for i in range(len(self._status_events)):
                 self._status_events[i] = None
             raise kernels.KernelError(f"a kernel gave up a bounded wait (status {code:#x}): the results of the "

@@ -1120,7 +1120,8 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: b
 
 class _TensorCoreState:
     """Per-device buffers of the tensor-core matrix product: the workspace and tile counters of the
-    split over K, and the status word in which a kernel records a wait that gave up."""
+    split over K, and the status word in which a kernel records a wait that gave up. The word lies in pinned host
+    memory that the device writes to (only when a wait gives up), so looking at it behind a step costs no copy."""
 
     WORKSPACE_FLOATS = 8 * 1024 * 1024
     COUNTERS = 4096
@@ -1129,7 +1130,8 @@ class _TensorCoreState:
         self.device = device
         self._workspace = None
         self.counters = torch.zeros(self.COUNTERS, dtype=torch.int32, device=device)
-        self.status = torch.zeros(1, dtype=torch.int32, device=device)
+        self.status = torch.zeros(1, dtype=torch.int32).pin_memory()
+        self.failures = 0           # how often the word was found set and cleared
 
     @property
     def workspace(self) -> torch.Tensor:
@@ -1478,8 +1480,22 @@ def specialised_products(on: Optional[bool] = None) -> bool:
 
 
 def status_word(device: torch.device) -> torch.Tensor:
-    """The device word [1] (int32) in which a kernel records a bounded wait that gave up (0 = none)."""
+    """The word [1] (int32, pinned host memory) in which the device's kernels record a bounded wait that gave up (0 = none): what it
+    holds once an event behind a kernel is over includes that kernel."""
     return _tc_state(device).status
+
+
+def status_failures(device: torch.device) -> int:
+    """How often the status word has been cleared after a failure: who noted the number before a launch knows by it that someone
+    else has seen (and cleared) a failure since."""
+    return _tc_state(device).failures
+
+
+def clear_status(device: torch.device) -> None:
+    """Clears the status word after a failure."""
+    st = _tc_state(device)
+    st.failures += 1
+    st.status.zero_()
 
 
 def gemm_tc_status(device: torch.device) -> int:

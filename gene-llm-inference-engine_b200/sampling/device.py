@@ -19,19 +19,21 @@ _RING = 4          # samples that may be in flight before the oldest must have b
 class PendingSample:
     """The token ids of one sampling call, on their way to the host."""
 
-    def __init__(self, host: torch.Tensor, rows: int, event, status: Optional[torch.Tensor] = None, on_failure=None):
-        """``status``: the host copy [1] of the kernels' status word, taken behind the ids; a value
+    def __init__(self, host: torch.Tensor, rows: int, event, status: Optional[torch.Tensor] = None, on_failure=None, failed=None):
+        """``status``: the kernels' status word [1] as the host sees it behind the ids; a value
         other than 0 says that a kernel of the steps before gave up a bounded wait, so the ids are
-        not to be trusted. ``on_failure`` is called (to clear the device's word) before the error."""
-        self._host, self._rows, self._event, self._status, self._on_failure = host, rows, event, status, on_failure
+        not to be trusted. ``on_failure`` is called (to clear the word) before the error. ``failed()``: whether someone else has
+        found the word set, and cleared it, since the ids were drawn."""
+        self._host, self._rows, self._event, self._status, self._on_failure, self._failed = host, rows, event, status, on_failure, failed
 
     def result(self) -> List[int]:
         self._event.synchronize()
-        if self._status is not None and int(self._status[0]) != 0:
-            code = int(self._status[0])
-            self._status[0] = 0
-            if self._on_failure is not None:
-                self._on_failure()
+        code = int(self._status[0]) if self._status is not None else 0
+        if code != 0 or (self._failed is not None and self._failed()):
+            if code != 0:
+                self._status[0] = 0
+                if self._on_failure is not None:
+                    self._on_failure()
             raise kernels.KernelError(f"a kernel gave up a bounded wait (status {code:#x}): the sampled tokens are not valid")
         return self._host[:self._rows].tolist()
 
@@ -52,7 +54,6 @@ class DeviceSampler:
         if rows > self._rows:
             self._rows = max(rows, 2 * self._rows, 8, self._ids.numel())
             self._host_ids = [torch.empty(self._rows, dtype=torch.int32).pin_memory() for _ in range(_RING)]
-            self._host_status = [torch.zeros(1, dtype=torch.int32).pin_memory() for _ in range(_RING)]
             self._host = [torch.empty((4, self._rows), dtype=torch.float32).pin_memory() for _ in range(_RING)]
             self._dev = torch.empty((4, self._rows), dtype=torch.float32, device=self.device)
             self._top_k = torch.empty(self._rows, dtype=torch.int32, device=self.device)
@@ -88,12 +89,11 @@ class DeviceSampler:
         host_ids = self._host_ids[slot]
         host_ids[:rows].copy_(ids, non_blocking=True)
         word = kernels.status_word(self.device)
-        status = self._host_status[slot]
-        status.copy_(word, non_blocking=True)
         event = torch.cuda.Event()
         event.record()
         self._events[slot] = event
-        return PendingSample(host_ids, rows, event, status, word.zero_)
+        before, device = kernels.status_failures(self.device), self.device
+        return PendingSample(host_ids, rows, event, word, lambda: kernels.clear_status(device), lambda: kernels.status_failures(device) != before)
 
     def sample(self, logits: torch.Tensor, params: Sequence[SamplingParams], uniforms: Sequence[float]) -> List[int]:
         if logits.shape[0] == 0:

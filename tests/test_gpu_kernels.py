@@ -393,6 +393,23 @@ def test_gemm_takes_the_norm_of_its_sums(M, N, K_):
     assert torch.equal(one, two) and torch.equal(xn, want)
 
 
+def test_a_failed_wait_ends_every_call_that_was_under_way():
+    """The status word is one for all: who finds it set clears it, and the others still learn of it."""
+    from geneinfer_b200 import SamplingParams
+    from geneinfer_b200.sampling.device import DeviceSampler
+    device = torch.device(DEV)
+    sampler = DeviceSampler(64, device)
+    logits = torch.zeros(1, 64, device=DEV)
+    logits[0, 7] = 1.0
+    calls = [sampler.sample_async(logits, [SamplingParams(0.0)], [0.0]) for _ in range(2)]
+    torch.cuda.synchronize()
+    K().status_word(device)[0] = 0x21                       # what a kernel would leave there
+    for call in calls:
+        with pytest.raises(K().KernelError):
+            call.result()
+    assert K().gemm_tc_status(device) == 0 and sampler.sample(logits, [SamplingParams(0.0)], [0.0]) == [7]
+
+
 @pytest.mark.parametrize("V", [131072, 131073])
 @pytest.mark.parametrize("top_k,top_p", [(0, 1.0), (40, 1.0), (0, 0.9), (40, 0.95)])
 def test_sample_of_the_largest_rows_held_in_registers_and_the_smallest_not(V, top_k, top_p):
