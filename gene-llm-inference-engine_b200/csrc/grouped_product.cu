@@ -467,7 +467,9 @@ __device__ __forceinline__ unsigned long long gm_minus(unsigned long long a, uns
 }
 
 // Eight neighbouring values of an input row as they are read (GmInput) and as they are multiplied (GmParts): what they add to the
-// sums with eight values of weight rows w0 and w1.
+// sums with eight values of weight rows w0 and w1. An input's second and third parts may be zero, and zero times an infinite weight is
+// none, where the input times the weight is infinite: then the first parts' sums alone, which are infinite or none too, are the answer (the parts
+// have the input's sign, so what the others add could not change it).
 template <typename TA> struct GmParts;
 template <typename TA> struct GmInput;
 template <> struct GmParts<__nv_bfloat16> {
@@ -675,7 +677,10 @@ grouped_mma_kernel(const GroupedArgs p, int tiles_given) {
                 if (8 * t < at.count) {
                     float v[4];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) v[i] = acc[0][m][t][i] + (acc[1][m][t][i] + rest[m][t][i]);
+                    for (int i = 0; i < 4; ++i) {
+                        v[i] = acc[0][m][t][i] + (acc[1][m][t][i] + rest[m][t][i]);
+                        if (sizeof(TA) == 4 && v[i] != v[i]) v[i] = acc[0][m][t][i] + acc[1][m][t][i];      // (GmParts: a part that is zero and an infinite weight)
+                    }
                     mine[(warp * 2 + m * NT + t) * 32] = make_float4(v[0], v[1], v[2], v[3]);
                 }
         __syncthreads();         // (this half is written again two units on, behind the next barrier, which every reader of it meets later)
@@ -785,7 +790,9 @@ head_mma_kernel(const GroupedArgs p) {
             for (int e = 0; e < 4; ++e) {
                 const int m = 8 * t + (lane & 3) * 2 + (e & 1), n = n0 + 16 * i + 8 * (e >> 1) + gr;
                 if (m >= rows || n >= p.N) continue;
-                const float v = gp_gated(p, acc[i][t][e] + rest[i][t][e], row0 + m, g, n);
+                float v = acc[i][t][e] + rest[i][t][e];
+                if (sizeof(TA) == 4 && v != v) v = acc[i][t][e];                 // (GmParts: a part that is zero and an infinite weight)
+                v = gp_gated(p, v, row0 + m, g, n);
                 const size_t o = static_cast<size_t>(row0 + m) * p.ldo + p.o_off + static_cast<size_t>(g) * p.o_gs + n;
                 if (p.out_is_f32) static_cast<float*>(p.out)[o] = v;
                 else static_cast<__nv_bfloat16*>(p.out)[o] = __float2bfloat16_rn(v);

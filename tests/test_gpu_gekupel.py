@@ -526,6 +526,43 @@ def test_products_of_32_bit_inputs_with_bfloat16_weights(form, N, K):
     assert bool(((got - want).abs() <= bound)[keep].all()), float(((got - want).abs() / bound)[keep].max())
 
 
+@pytest.mark.parametrize("form", ["experts", "four experts' pairs", "gated experts", "heads, 9 rows", "heads, 33 rows", "heads, 70 rows", "heads with a tail, 12 rows"])
+@pytest.mark.parametrize("N, K", [(16, 264), (70, 40)])
+def test_infinite_weights_with_32_bit_inputs(form, N, K):
+    """An infinite weight gives an infinity of the input's sign, none where the input is zero or another one is infinite the other
+    way, and nothing to the outputs beside it: whatever parts an input is cut into."""
+    from geneinfer_b200.ops import kernels
+    g = torch.Generator().manual_seed(K)
+    heads = form.startswith("heads")
+    T = int(form.split(", ")[1].split()[0]) if heads else 4 if "four" in form else 9
+    G, tail = (3, 8 if "tail" in form else 0) if heads else (1, 0)
+    gated = form == "gated experts"
+    x, w = torch.randn(T, G, K, generator=g), _bf(torch.randn(G, (2 if gated else 1) * N, K, generator=g))
+    x[1] = _bf(x[1])                                        # nothing is left of these behind the first part
+    x[2, :, K - 3] = 0.0
+    w[:, 3, K - 3], w[:, N - 2, 0] = float("inf"), float("-inf")
+    if not gated:
+        w[:, 5, 1], w[:, 5, K - 1], w[:, 7, 2] = float("inf"), float("-inf"), float("nan")
+    out = torch.full((T, G * (N + tail)), 7.0, device=DEV)
+    if heads:
+        a = torch.cat([x, torch.zeros(T, G, tail)], 2).reshape(T, -1).to(DEV)
+        kernels.head_product(a, 0, K + tail, w.to(DEV).bfloat16(), out, 0, N + tail, tail=tail,
+                             freq=torch.ones(tail // 2, device=DEV) if tail else None, positions=torch.zeros(T, dtype=torch.int32, device=DEV) if tail else None)
+    else:
+        rows = torch.full((6 * kernels.grouped_tile_rows(),), -1, dtype=torch.int32)
+        rows[:T] = torch.arange(T, dtype=torch.int32)
+        kernels.expert_product(x[:, 0].contiguous().to(DEV), 1, w.to(DEV).bfloat16(), out, rows.to(DEV), torch.zeros(6, dtype=torch.int32, device=DEV),
+                               torch.ones(1, dtype=torch.int32, device=DEV), gated="silu" if gated else None)
+    got = out.cpu().view(T, G, N + tail)[..., :N].double()
+    want = torch.einsum("tgk,gnk->tgn", x.double(), w.double())
+    if gated:                   # (silu of minus infinity is none: minus infinity times zero)
+        want = want[..., :N] * torch.sigmoid(want[..., :N]) * want[..., N:]
+    special = ~want.isfinite()
+    assert bool(special[1].any()) and torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got[special & ~want.isnan()], want[special & ~want.isnan()])
+    _close(got[~special], want[~special], torch.float32, form, f32=1e-5)
+
+
 # ------------------------------------------------------------------------------------------ mixers alone
 ATT = {"heads": 6, "kv_heads": 2, "dim": 16, "vdim": 24, "mask": {"size": 11}, "scale": 0.45}
 LAT = {"heads": 3, "dim": 24, "rot_dim": 8, "vdim": 40, "q_rank": 32, "kv_rank": 48, "mask": {"size": 13}, "scale": 0.3,
