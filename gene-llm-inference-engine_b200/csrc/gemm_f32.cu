@@ -69,7 +69,7 @@ using Tile64 = F32Tile<64, 128, 8, 8, 32, 4, 2>;
 template <typename T>
 __global__ void __launch_bounds__(T::kThreads, T::kBlocks)
 gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N, int K,
-                int lda, int ldw, int ldc, int kc, int accumulate) {
+                int lda, int ldw, int ldc, int kc, int accumulate, int w_constant) {
     constexpr int BM = T::BM, BN = T::BN, TM = T::TM, TN = T::TN, kStages = T::kStages, kPad = T::kPad;
     extern __shared__ __align__(16) float smem[];
     pdl_launch_dependents();
@@ -113,13 +113,14 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
 #pragma unroll
         for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
 
-    // the weights of the first tiles are asked for before the wait for the kernel ahead: no earlier kernel writes them (six rows in a
-    // token's step: N = 16,384, K = 2,048 33.2 -> 28.9 us, N = 3,072 8.4 -> 7.5)
-    for (int i = 0; i < kStages - 1; ++i)
-        if (i < tiles) load_w(i);
+    // w_constant: the weights of the first tiles are asked for before the wait for the kernel ahead, as no kernel that may still be running
+    // writes them (six rows in a token's step: N = 16,384, K = 2,048 33.2 -> 28.9 us, N = 3,072 8.4 -> 7.5)
+    if (w_constant)
+        for (int i = 0; i < kStages - 1; ++i)
+            if (i < tiles) load_w(i);
     pdl_wait();
     for (int i = 0; i < kStages - 1; ++i) {
-        if (i < tiles) load_a(i);
+        if (i < tiles) { load_a(i); if (!w_constant) load_w(i); }
         commit();
     }
     for (int tile = 0; tile < tiles; ++tile) {
@@ -183,7 +184,7 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
 
 template <typename T>
 int launch(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, int chunks, int kc,
-           int accumulate, cudaStream_t st) {
+           int accumulate, int w_constant, cudaStream_t st) {
     static SharedLimit limit;
     const cudaError_t ready = limit.allow(reinterpret_cast<const void*>(gemm_f32_kernel<T>), static_cast<int>(T::kSmem));
     if (ready != cudaSuccess) { set_error("gemm: %s", cudaGetErrorString(ready)); return 1; }
@@ -201,7 +202,7 @@ int launch(const float* A, const float* W, float* C, int M, int N, int K, int ld
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    counted(cudaLaunchKernelEx(&cfg, gemm_f32_kernel<T>, A, W, C, M, N, K, lda, ldw, ldc, kc, accumulate));
+    counted(cudaLaunchKernelEx(&cfg, gemm_f32_kernel<T>, A, W, C, M, N, K, lda, ldw, ldc, kc, accumulate, w_constant));
     return check_launch("gemm_f32");
 }
 
@@ -213,17 +214,17 @@ bool gemm_f32_takes(const float* A, const float* W, int M, int N, int K, int lda
     return K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && aligned(A) && aligned(W) && (M + 63) / 64 <= 65535 && (N + 63) / 64 <= 65535;
 }
 
-int gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, int accumulate, cudaStream_t st) {
+int gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, int accumulate, int w_constant, cudaStream_t st) {
     // Chunks of K until the blocks along N fill the 148 SMs, none shorter than 256: by N and K alone (see above).
     int chunks = 1;
     while (chunks < kMaxChunks && (N + 127) / 128 * chunks < 148 && K / (2 * chunks) >= 256) chunks *= 2;
     const int kc = ((K + chunks - 1) / chunks + kChunkStep - 1) / kChunkStep * kChunkStep;
-    if (M <= 2) return launch<Tile2>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, st);
-    if (M <= 4) return launch<Tile4>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, st);
-    if (M <= 6) return launch<Tile6>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, st);
-    if (M <= 8) return launch<Tile8>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, st);
-    if (M <= 16) return launch<Tile16>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, st);
-    if (M <= 32) return launch<Tile32>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, st);
+    if (M <= 2) return launch<Tile2>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, w_constant, st);
+    if (M <= 4) return launch<Tile4>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, w_constant, st);
+    if (M <= 6) return launch<Tile6>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, w_constant, st);
+    if (M <= 8) return launch<Tile8>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, w_constant, st);
+    if (M <= 16) return launch<Tile16>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, w_constant, st);
+    if (M <= 32) return launch<Tile32>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, w_constant, st);
     // More rows: blocks of 8 x 5 .. 8 rows, the height whose rounds over the SMs (two blocks each) are the least work: a block that is
     // half outside the matrix, or a last round that is nearly empty, costs as much as a full one. A block's time goes with its
     // rows and half a row's worth of reading columns. (268 rows,
@@ -238,10 +239,10 @@ int gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int 
         const long long cost = (blocks + 2 * 148 - 1) / (2 * 148) * (2 * tm + 1);
         if (least < 0 || cost < least) { least = cost; best = tm; }
     }
-    if (best == 5) return launch<Tile40>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, st);
-    if (best == 6) return launch<Tile48>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, st);
-    if (best == 7) return launch<Tile56>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, st);
-    return launch<Tile64>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, st);
+    if (best == 5) return launch<Tile40>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, w_constant, st);
+    if (best == 6) return launch<Tile48>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, w_constant, st);
+    if (best == 7) return launch<Tile56>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, w_constant, st);
+    return launch<Tile64>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, w_constant, st);
 }
 
 }  // namespace gi

@@ -92,9 +92,10 @@ int launch_simt(const void* A, const void* W, void* C, int c_dtype, int accumula
 
 using namespace gi;
 
-// C[M,N] (+)= A[M,K] * W[N,K]^T; row strides lda, ldw, ldc in elements.
+// C[M,N] (+)= A[M,K] * W[N,K]^T; row strides lda, ldw, ldc in elements. w_constant: no launch before this one that may still be running writes
+// W, so that its first values may be asked for before the wait for them.
 static int gi_gemm_simt_impl(const void* A, int a_dtype, const void* W, int w_dtype, void* C, int c_dtype,
-                            int accumulate, int M, int N, int K, int lda, int ldw, int ldc, void* stream) {
+                            int accumulate, int M, int N, int K, int lda, int ldw, int ldc, int w_constant, void* stream) {
     if (M == 0 || N == 0) return 0;
     GI_REQUIRE(M > 0 && N > 0 && K > 0, "gemm: sizes must be positive (M=%d, N=%d, K=%d)", M, N, K);
     GI_REQUIRE((M + kBM - 1) / kBM <= 65535, "gemm: M=%d exceeds the grid limit", M);
@@ -102,7 +103,7 @@ static int gi_gemm_simt_impl(const void* A, int a_dtype, const void* W, int w_dt
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (a_dtype == kF32 && w_dtype == kF32 && c_dtype == kF32 &&
         gemm_f32_takes(static_cast<const float*>(A), static_cast<const float*>(W), M, N, K, lda, ldw))
-        return gemm_f32(static_cast<const float*>(A), static_cast<const float*>(W), static_cast<float*>(C), M, N, K, lda, ldw, ldc, accumulate, st);
+        return gemm_f32(static_cast<const float*>(A), static_cast<const float*>(W), static_cast<float*>(C), M, N, K, lda, ldw, ldc, accumulate, w_constant, st);
     if (a_dtype == kF32 && w_dtype == kF32) return launch_simt<float, float>(A, W, C, c_dtype, accumulate, M, N, K, lda, ldw, ldc, st);
     if (a_dtype == kF32 && w_dtype == kBF16) return launch_simt<float, __nv_bfloat16>(A, W, C, c_dtype, accumulate, M, N, K, lda, ldw, ldc, st);
     if (a_dtype == kBF16 && w_dtype == kBF16) return launch_simt<__nv_bfloat16, __nv_bfloat16>(A, W, C, c_dtype, accumulate, M, N, K, lda, ldw, ldc, st);
@@ -111,6 +112,6 @@ static int gi_gemm_simt_impl(const void* A, int a_dtype, const void* W, int w_dt
 
 // The exported names: each runs its implementation above and, while a launch program is recorded, leaves a copy of
 // its arguments in the program (common.cuh).
-extern "C" int gi_gemm_simt(const void* A, int a_dtype, const void* W, int w_dtype, void* C, int c_dtype, int accumulate, int M, int N, int K, int lda, int ldw, int ldc, void* stream) {
-    return gi::dispatch(gi_gemm_simt_impl, A, a_dtype, W, w_dtype, C, c_dtype, accumulate, M, N, K, lda, ldw, ldc, stream);
+extern "C" int gi_gemm_simt(const void* A, int a_dtype, const void* W, int w_dtype, void* C, int c_dtype, int accumulate, int M, int N, int K, int lda, int ldw, int ldc, int w_constant, void* stream) {
+    return gi::dispatch(gi_gemm_simt_impl, A, a_dtype, W, w_dtype, C, c_dtype, accumulate, M, N, K, lda, ldw, ldc, w_constant, stream);
 }

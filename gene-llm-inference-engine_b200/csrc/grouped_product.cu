@@ -42,6 +42,7 @@ struct GroupedArgs {
     void* out; int out_is_f32; long long ldo; int o_off; int o_gs;
     int N, K, rows, groups;
     const int* tile_group; const int* sorted_rows; const int* n_tiles;   // experts form (else null)
+    int w_constant;                                               // no kernel that may still be running writes w: it may be read before the wait
     int act; float act_limit;                                     // gated: a GateAct code and its limit
     int out_act;                                                  // not gated: a PlainAct code
     // rotated tail (heads form)
@@ -721,7 +722,7 @@ grouped_mma_kernel(const GroupedArgs p, int tiles_given) {
 
 // The heads form of bfloat16 weights: every row count with a rotated tail, and without one where the rows are more than the few-row form
 // takes. A warp has MT x 16 outputs of NT x 8 rows, its operands straight from memory in the fragments' layout (as in the few-row
-// form), a step of 32 k ahead, the first weights asked for before the wait (they belong to no earlier kernel). kFew: the block's four
+// form), a step of 32 k ahead, the first weights asked for before the wait where they are constant. kFew: the block's four
 // warps lie along the outputs (few rows: the weights are what is read), else along the rows. A sum goes through K in the same
 // order with the same products in either shape: a token's result is the same to the bit whatever else is in the step. Measured, 16 heads,
 // on the CUDA cores -> here: 512 to 64, 1,273 rows 91 -> 34 us; 64 to 512 with a tail, 8 rows 14.6 -> 2.7, 1,273 rows 51 -> 43; 128 to 1,024
@@ -743,7 +744,7 @@ head_mma_kernel(const GroupedArgs p) {
         for (int i = 0; i < MT; ++i)
 #pragma unroll
             for (int half = 0; half < 2; ++half)
-                dst[i][half] = k0 + kq < p.K ? __ldg(reinterpret_cast<const uint4*>(W + static_cast<size_t>(min(n0 + 16 * i + 8 * half + gr, p.N - 1)) * p.ldw + k0 + kq))
+                dst[i][half] = k0 + kq < p.K ? *reinterpret_cast<const uint4*>(W + static_cast<size_t>(min(n0 + 16 * i + 8 * half + gr, p.N - 1)) * p.ldw + k0 + kq)
                                              : make_uint4(0, 0, 0, 0);
     };
     auto inputs = [&](GmInput<TA> (&dst)[NT], int k0) {
@@ -753,8 +754,9 @@ head_mma_kernel(const GroupedArgs p) {
             else dst[t].zero();
         }
     };
-    if (n0 < p.N) weights(w, 0);
+    if (p.w_constant && n0 < p.N) weights(w, 0);
     pdl_wait();
+    if (!p.w_constant && n0 < p.N) weights(w, 0);
     if (p.tail > 0 && blockIdx.y == 0) {                // the rotated tail, by the blocks of the first outputs
         const int first = kFew ? threadIdx.x : lane, step = kFew ? 128 : 32, half = p.tail / 2;
         for (int i = first; i < rows * half; i += step)
@@ -801,7 +803,7 @@ head_mma_kernel(const GroupedArgs p) {
 
 // The heads form of 32-bit weights with a rotated tail for up to four rows: short inputs and many outputs, where a tile's rounds through shared
 // memory and its sixteen rows cost more than its multiply-adds, and the few-row form spends its time on its sums. A thread has one
-// output of every row, its weights in registers (asked for before the wait: they belong to no earlier kernel). The sum is one
+// output of every row, its weights in registers (asked for before the wait where they are constant). The sum is one
 // chain in the order of k, as in the tiles of 16 and of 64: a token's result is the same to the bit whatever else is in the step.
 constexpr int kGcRows = 4, kGcCols = 64, kGcK = 64;
 
@@ -818,11 +820,12 @@ head_product_few_kernel(const GroupedArgs p) {
 #pragma unroll
         for (int i = 0; i < kPieces; ++i) {
             const int k = k0 + i * kPiece;                 // (K is a multiple of a piece)
-            wv[i] = k < p.K ? __ldg(reinterpret_cast<const uint4*>(wrow + k)) : make_uint4(0, 0, 0, 0);
+            wv[i] = k < p.K ? *reinterpret_cast<const uint4*>(wrow + k) : make_uint4(0, 0, 0, 0);
         }
     };
-    request(0);
+    if (p.w_constant) request(0);
     pdl_wait();
+    if (!p.w_constant) request(0);
     if (blockIdx.y == 0)
         for (int i = tid; i < p.rows * (p.tail / 2); i += kGcCols) {
             const int r = i / (p.tail / 2);
@@ -1255,7 +1258,7 @@ extern "C" int gi_grouped_tile_rows() { return kGpTM; }
 static int gi_head_product_impl(const void* a, int a_dtype, long long lda, int a_off, int a_gs, const void* w, int w_dtype,
                                 long long w_gs, void* out, int out_dtype, long long ldo, int o_off, int o_gs, int rows, int heads,
                                 int N, int K, int tail, const float* freq, float amplitude, int tail_interleaved, const int* positions, const float* gate,
-                                long long ldg, int gate_off, int gate_per_head, void* stream) {
+                                long long ldg, int gate_off, int gate_per_head, int w_constant, void* stream) {
     if (rows == 0) return 0;
     GI_REQUIRE(rows > 0 && heads > 0 && N > 0 && K > 0, "head_product: sizes must be positive");
     GI_REQUIRE(gate == nullptr || (gate_off >= 0 && gate_off + static_cast<long long>(heads) * (gate_per_head ? 1 : N) <= ldg), "head_product: the gate's columns lie outside its rows");
@@ -1263,7 +1266,7 @@ static int gi_head_product_impl(const void* a, int a_dtype, long long lda, int a
     GI_REQUIRE(out_dtype == kF32 || out_dtype == kBF16, "head_product: unsupported output dtype");
     GroupedArgs p = {};
     p.a = a; p.lda = lda; p.a_off = a_off; p.a_gs = a_gs; p.a_div = 1;
-    p.w = w; p.w_gs = w_gs; p.ldw = K; p.up_off = 0;
+    p.w = w; p.w_gs = w_gs; p.ldw = K; p.up_off = 0; p.w_constant = w_constant;
     p.out = out; p.out_is_f32 = out_dtype == kF32; p.ldo = ldo; p.o_off = o_off; p.o_gs = o_gs;
     p.N = N; p.K = K; p.rows = rows; p.groups = heads;
     p.tail = tail; p.freq = freq; p.amplitude = amplitude; p.tail_interleaved = tail_interleaved; p.positions = positions;
@@ -1430,9 +1433,9 @@ static int gi_route_combine_impl(const float* part, const float* weights, const 
 extern "C" int gi_head_product(const void* a, int a_dtype, long long lda, int a_off, int a_gs, const void* w, int w_dtype,
                                long long w_gs, void* out, int out_dtype, long long ldo, int o_off, int o_gs, int rows, int heads,
                                int N, int K, int tail, const float* freq, float amplitude, int tail_interleaved, const int* positions, const float* gate,
-                               long long ldg, int gate_off, int gate_per_head, void* stream) {
+                               long long ldg, int gate_off, int gate_per_head, int w_constant, void* stream) {
     return gi::dispatch(gi_head_product_impl, a, a_dtype, lda, a_off, a_gs, w, w_dtype, w_gs, out, out_dtype, ldo, o_off, o_gs, rows,
-                        heads, N, K, tail, freq, amplitude, tail_interleaved, positions, gate, ldg, gate_off, gate_per_head, stream);
+                        heads, N, K, tail, freq, amplitude, tail_interleaved, positions, gate, ldg, gate_off, gate_per_head, w_constant, stream);
 }
 
 extern "C" int gi_expert_product(const void* a, int a_dtype, long long lda, int a_div, const void* w, int w_dtype, long long w_gs,

@@ -648,13 +648,14 @@ def attention_rows_launch_key(ctx, num_heads: int, num_kv_heads: int, head_dim: 
 def head_product(a: torch.Tensor, a_offset: int, a_head_stride: int, w: torch.Tensor, out: torch.Tensor, out_offset: int,
                  out_head_stride: int, tail: int = 0, freq: Optional[torch.Tensor] = None, amplitude: float = 1.0,
                  positions: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None, gate_offset: int = 0,
-                 interleaved: bool = True, gate_per_head: bool = False) -> None:
+                 interleaved: bool = True, gate_per_head: bool = False, w_constant: bool = False) -> None:
     """out[t, out_offset + h * out_head_stride + n] = sum_k w[h, n, k] * a[t, a_offset + h * a_head_stride + k] for
     every head h of ``w`` [H, N, K]: a matrix per head, applied to that head's slice of a row. ``tail`` > 0: the tail
     columns behind a head's K inputs are rotated pair by pair ((2i, 2i+1), or (i, i + tail / 2) when not ``interleaved``)
     by positions[t] * freq[i] (cos and sin times ``amplitude``) and written behind the head's N outputs. ``gate`` [T, ld] 32-bit: output n of head h is multiplied by
     sigmoid(gate[t, gate_offset + h * N + n]) (an element-wise output gate laid out head by head), with ``gate_per_head``
-    by sigmoid(gate[t, gate_offset + h])."""
+    by sigmoid(gate[t, gate_offset + h]). ``w_constant``: no launch of this library that may still be running writes ``w`` (a model's
+    weights), so that the kernel may read it before the launch ahead has ended."""
     T = a.shape[0]
     H, N, K = w.shape
     if gate is not None and (gate.dim() != 2 or gate.shape[0] != T or gate_offset < 0 or
@@ -670,7 +671,7 @@ def head_product(a: torch.Tensor, a_offset: int, a_head_stride: int, w: torch.Te
         _dev(a, "a"), dtype_code(a.dtype), a.shape[1], int(a_offset), int(a_head_stride), _dev(w, "w"), dtype_code(w.dtype), N * K,
         _dev(out, "out"), dtype_code(out.dtype), out.shape[1], int(out_offset), int(out_head_stride), T, H, N, K, int(tail),
         _opt(freq, "freq", torch.float32), float(amplitude), int(interleaved), 0 if positions is None else _dev(positions, "positions", torch.int32),
-        _opt(gate, "gate", torch.float32), 0 if gate is None else gate.shape[1], int(gate_offset), int(gate_per_head), _stream()), "head_product")
+        _opt(gate, "gate", torch.float32), 0 if gate is None else gate.shape[1], int(gate_offset), int(gate_per_head), int(w_constant), _stream()), "head_product")
 
 
 def grouped_tile_rows() -> int:
@@ -1114,14 +1115,15 @@ def attention_prefill_tc(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.
         float(softcap or 0.0), _stream()), "attention_prefill_tc")
 
 
-def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False) -> None:
-    """out[M,N] (+)= a[M,K] @ w[N,K]^T with 32-bit fused multiply-adds on the CUDA cores."""
+def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False, w_constant: bool = False) -> None:
+    """out[M,N] (+)= a[M,K] @ w[N,K]^T with 32-bit fused multiply-adds on the CUDA cores. ``w_constant``: no launch of this library that
+    may still be running writes ``w`` (a model's weights), so that the kernel may read it before the launch ahead has ended."""
     M, K = a.shape
     N = w.shape[0]
     if w.shape[1] != K or out.shape != (M, N):
         raise KernelError(f"gemm: shapes do not agree (a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)})")
     check(lib().gi_gemm_simt(_dev(a, "a"), dtype_code(a.dtype), _dev(w, "w"), dtype_code(w.dtype), _dev(out, "out"),
-                             dtype_code(out.dtype), int(accumulate), M, N, K, K, K, N, _stream()), "gemm")
+                             dtype_code(out.dtype), int(accumulate), M, N, K, K, K, N, int(w_constant), _stream()), "gemm")
 
 
 class _TensorCoreState:

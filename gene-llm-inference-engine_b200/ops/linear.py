@@ -61,7 +61,7 @@ class Linear:
             kernels.gemm_tc(a, self.weight, out, accumulate, w_tiles=self.weight_tiles,   # tensor cores (TMA needs 16-byte rows)
                             ahead=then.weight_tiles if then is not None else None, norm=norm)
         else:
-            kernels.gemm_simt(a, self.weight, out, accumulate)
+            kernels.gemm_simt(a, self.weight, out, accumulate, w_constant=True)
             if norm is not None:
                 kernels.rmsnorm(out, norm[0], norm[2], norm[1])
         return out

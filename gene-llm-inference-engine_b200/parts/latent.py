@@ -121,12 +121,12 @@ class LatentAttentionMixer:
         # the queries as the latent rows see them: [W_uk,h^T q_h^p, rotated q_h^r] per head
         qa = ctx.scratch("latent_queries_absorbed", (T, H * (kr + r)), torch.float32)
         kernels.head_product(q, 0, d + r, self.w_uk_t, qa, 0, kr + r, tail=r, freq=self.freq, amplitude=self.amplitude,
-                             positions=ctx.positions, interleaved=self.interleaved)
+                             positions=ctx.positions, interleaved=self.interleaved, w_constant=True)
         ol = ctx.scratch("latent_out", (T, H * kr), torch.float32)
         kernels.attention_rows_of_step(ctx, qa, cache, None, ol, tables, H, 1, kr + r, kr, self.scale, self.window, None, None,
                                        self.sink)
         att = ctx.scratch("att", (T, H * dv), self.dtype)
         # the heads' value matrices; the output gate (its values lie in the first product's columns) in the same kernel
         kernels.head_product(ol, 0, kr, self.w_uv, att, 0, dv, gate=down if self.output_gate or self.head_gate else None,
-                             gate_offset=self.gate_offset, gate_per_head=self.head_gate)
+                             gate_offset=self.gate_offset, gate_per_head=self.head_gate, w_constant=True)
         self.w_o.forward(att, x, accumulate=True, then=then)

@@ -125,6 +125,36 @@ def test_gemm_simt_block_heights_agree_to_the_bit(M, N, K_):
     assert torch.equal(out, part) and bool(out.isfinite().all())
 
 
+@pytest.mark.parametrize("product", ["5 rows", "40 rows", "heads, 5 rows", "heads, 40 rows", "heads with a tail, 5 rows", "heads with a tail and 32 bits, 3 rows"])
+def test_products_with_weights_of_the_launch_before(product):
+    """Weights that the launch ahead writes (a product over many inputs, whose sums are stored at its end) are read when they are there."""
+    heads, T = product.startswith("heads"), int(product.split()[-2])
+    N, K_, long, tail = 256 if heads else 2048, 64, 8192, 8 if "tail" in product else 0
+    g = torch.Generator().manual_seed(N + T)
+    left, right = torch.randn(N, long, generator=g).to(DEV), torch.randn(K_, long, generator=g).to(DEV)
+    a = torch.randn(T, K_ + tail, generator=g).to(DEV)
+    w = torch.empty(N, K_, device=DEV, dtype=torch.bfloat16 if heads and "32 bits" not in product else torch.float32)
+    freq, positions = torch.ones(4, device=DEV), torch.zeros(T, dtype=torch.int32, device=DEV)
+
+    def run(wait):
+        w.zero_()
+        out = torch.empty(T, N + tail, device=DEV)
+        torch.cuda.synchronize()
+        K().gemm_simt(left, right, w)
+        if wait:
+            torch.cuda.synchronize()
+        if heads:
+            K().head_product(a, 0, K_ + tail, w.view(1, N, K_), out, 0, N + tail, tail=tail, freq=freq if tail else None, positions=positions if tail else None)
+        else:
+            K().gemm_simt(a, w, out)
+        return out
+
+    want = run(True)
+    assert bool((want[:, :N] != 0).any())
+    for _ in range(3):
+        assert torch.equal(run(False), want)
+
+
 def _paged(dtype, n_pages, Hkv, ps, hd):
     kc = torch.full((n_pages, Hkv, ps, hd), float("nan"), dtype=dt(dtype), device=DEV)
     return kc, kc.clone()
