@@ -574,10 +574,8 @@ class StepEngine:
 
     def _raise_on_failure(self, failures: int) -> None:
         """``failures``: how many the device had when the step was launched (more now: another reader has cleared the word)."""
-        code = int(kernels.status_word(self.device)[0])
-        if code or kernels.status_failures(self.device) != failures:
-            if code:
-                kernels.clear_status(self.device)
+        code = kernels.take_failure(self.device, failures)
+        if code:
             for i in range(len(self._status_events)):
                 self._status_events[i] = None
             raise kernels.KernelError(f"a kernel gave up a bounded wait (status {code:#x}): the results of the "

@@ -1499,11 +1499,15 @@ def status_failures(device: torch.device) -> int:
     return _tc_state(device).failures
 
 
-def clear_status(device: torch.device) -> None:
-    """Clears the status word after a failure."""
+def take_failure(device: torch.device, failures: int) -> int:
+    """For who noted ``failures`` (``status_failures``): other than 0 if the status word holds a failure, which is then counted and the
+    word cleared, or if someone else has done so since."""
     st = _tc_state(device)
-    st.failures += 1
-    st.status.zero_()
+    code = int(st.status[0])            # (looked at before the count, and cleared behind it: a failure is always in one of the two)
+    if code:
+        st.failures += 1
+        st.status.zero_()
+    return code or st.failures - failures
 
 
 def gemm_tc_status(device: torch.device) -> int:

@@ -20,20 +20,21 @@ class PendingSample:
     """The token ids of one sampling call, on their way to the host."""
 
     def __init__(self, host: torch.Tensor, rows: int, event, status: Optional[torch.Tensor] = None, on_failure=None, failed=None):
-        """``status``: the kernels' status word [1] as the host sees it behind the ids; a value
-        other than 0 says that a kernel of the steps before gave up a bounded wait, so the ids are
-        not to be trusted. ``on_failure`` is called (to clear the word) before the error. ``failed()``: whether someone else has
-        found the word set, and cleared it, since the ids were drawn."""
+        """``failed()``: looked at behind the ids; a value other than 0 says that a kernel gave up a bounded wait, so the ids are
+        not to be trusted. ``status``: or a word [1] of this call's own that says so, cleared with the error; ``on_failure`` is called
+        before it."""
         self._host, self._rows, self._event, self._status, self._on_failure, self._failed = host, rows, event, status, on_failure, failed
 
     def result(self) -> List[int]:
         self._event.synchronize()
         code = int(self._status[0]) if self._status is not None else 0
-        if code != 0 or (self._failed is not None and self._failed()):
-            if code != 0:
-                self._status[0] = 0
-                if self._on_failure is not None:
-                    self._on_failure()
+        if code:
+            if self._on_failure is not None:
+                self._on_failure()
+            self._status[0] = 0
+        elif self._failed is not None:
+            code = self._failed()
+        if code:
             raise kernels.KernelError(f"a kernel gave up a bounded wait (status {code:#x}): the sampled tokens are not valid")
         return self._host[:self._rows].tolist()
 
@@ -88,12 +89,11 @@ class DeviceSampler:
             kernels.sample(logits, self._probs, self._dev[0, :rows], top_k, self._dev[2, :rows], self._dev[3, :rows], ids)
         host_ids = self._host_ids[slot]
         host_ids[:rows].copy_(ids, non_blocking=True)
-        word = kernels.status_word(self.device)
         event = torch.cuda.Event()
         event.record()
         self._events[slot] = event
         before, device = kernels.status_failures(self.device), self.device
-        return PendingSample(host_ids, rows, event, word, lambda: kernels.clear_status(device), lambda: kernels.status_failures(device) != before)
+        return PendingSample(host_ids, rows, event, failed=lambda: kernels.take_failure(device, before))
 
     def sample(self, logits: torch.Tensor, params: Sequence[SamplingParams], uniforms: Sequence[float]) -> List[int]:
         if logits.shape[0] == 0:

@@ -1,0 +1,81 @@
+"""The kernels' status word and those who look at it, on the host alone: a sampler whose kernels are stood in for, and a word that
+tells when it is cleared."""
+import pytest
+import torch
+
+from geneinfer_b200 import SamplingParams
+from geneinfer_b200.ops import kernels
+from geneinfer_b200.sampling.device import DeviceSampler
+
+
+class Word:
+    """The word [1], calling ``cleared`` at the moment when it no longer holds a failure."""
+
+    def __init__(self):
+        self.value, self.cleared = 0, lambda: None
+
+    def __getitem__(self, i):
+        return self.value
+
+    def __setitem__(self, i, value):
+        was, self.value = self.value, int(value)
+        if was and not self.value:
+            self.cleared()
+
+    def zero_(self):
+        self[0] = 0
+
+
+class Event:
+    def record(self):
+        pass
+
+    def synchronize(self):
+        pass
+
+
+class Host:
+    """A sampler of two tokens on the host; ``sample()`` is a call under way, ``launched`` runs where its kernels are launched."""
+
+    def __init__(self):
+        self.device = torch.device("cpu", 0)
+        self.state = kernels._tc_states[0]
+        self.sampler = DeviceSampler(2, self.device)
+        self.launched = lambda: None
+
+    def argmax(self, logits, ids):
+        self.launched()
+        ids.copy_(logits.argmax(1))
+
+    def sample(self):
+        return self.sampler.sample_async(torch.tensor([[0.0, 1.0]]), [SamplingParams(0.0)], [0.0])
+
+
+@pytest.fixture
+def host(monkeypatch):
+    monkeypatch.setattr(torch.Tensor, "pin_memory", lambda self, *a: self)
+    monkeypatch.setattr(torch.cuda, "Event", Event)
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda *a: None)
+    state = kernels._TensorCoreState(torch.device("cpu", 0))
+    state.status = Word()
+    monkeypatch.setitem(kernels._tc_states, 0, state)
+    h = Host()
+    monkeypatch.setattr(kernels, "argmax", h.argmax)
+    return h
+
+
+def test_a_failure_is_counted_before_the_word_is_cleared(host):
+    """Another thread that looks at the very moment when the word is cleared still learns of the failure."""
+    one, other = host.sample(), host.sample()
+    seen = []
+
+    def look():
+        with pytest.raises(kernels.KernelError):
+            other.result()
+        seen.append(True)
+
+    host.state.status[0] = 0x21
+    host.state.status.cleared = look
+    with pytest.raises(kernels.KernelError, match="0x21"):
+        one.result()
+    assert seen == [True] and host.sample().result() == [1]
