@@ -415,6 +415,7 @@ class StepEngine:
             raise ValueError(f"{n_want} wanted rows exceed the limit {self.max_logit_rows}")
 
         self._poll_status(wait=False)      # before anything is reserved: an earlier step's failure ends this call
+        failures = kernels.status_failures(self.device)
 
         # ---- reserve pages for every entry, all or nothing
         reserved: List[RequestCache] = []
@@ -485,7 +486,7 @@ class StepEngine:
         ctx = StepContext(self, total, R, k, segments, views)
         with ctx.range(f"step {total} tokens {R} requests"):
             logits = self._run(ctx)
-        self._post_status()
+        self._post_status(failures)
         for e in entries:
             self.cache.advance(self.cache.requests[e.key], len(e.tokens))
         return logits
@@ -550,8 +551,8 @@ class StepEngine:
             raise AssertionError("step descriptor: two requests of one step write into the same page")
 
     # ------------------------------------------------------------------ the kernels' status word
-    def _post_status(self) -> None:
-        """Marks where the step's kernels end (no wait)."""
+    def _post_status(self, failures: int) -> None:
+        """Marks where the step's kernels end (no wait). ``failures``: how many the device had before they were launched."""
         slot = self._status_next
         self._status_next = (slot + 1) % len(self._status_events)
         if self._status_events[slot] is not None:
@@ -560,7 +561,7 @@ class StepEngine:
         ev = torch.cuda.Event()
         ev.record()
         self._status_events[slot] = ev
-        self._status_failures[slot] = kernels.status_failures(self.device)
+        self._status_failures[slot] = failures
 
     def _poll_status(self, wait: bool) -> None:
         """Looks at the status word behind steps that have finished (behind all steps with ``wait``) and
@@ -573,7 +574,7 @@ class StepEngine:
                 self._raise_on_failure(self._status_failures[slot])
 
     def _raise_on_failure(self, failures: int) -> None:
-        """``failures``: how many the device had when the step was launched (more now: another reader has cleared the word)."""
+        """``failures``: how many the device had before the step was launched (more now: another reader has cleared the word)."""
         code = kernels.take_failure(self.device, failures)
         if code:
             for i in range(len(self._status_events)):

@@ -71,6 +71,7 @@ class DeviceSampler:
         if self._events[slot] is not None:
             self._events[slot].synchronize()       # the slot's host buffers are free again
         ids = self._ids[:rows]
+        device, before = self.device, kernels.status_failures(self.device)
         greedy = [p.greedy for p in params]
         if any(greedy) or rows == 0:
             kernels.argmax(logits, ids)
@@ -92,7 +93,6 @@ class DeviceSampler:
         event = torch.cuda.Event()
         event.record()
         self._events[slot] = event
-        before, device = kernels.status_failures(self.device), self.device
         return PendingSample(host_ids, rows, event, failed=lambda: kernels.take_failure(device, before))
 
     def sample(self, logits: torch.Tensor, params: Sequence[SamplingParams], uniforms: Sequence[float]) -> List[int]:

@@ -225,3 +225,25 @@ def test_trace_run_taps(tmp_path):
             assert tt.rel_err(got, full[rows].numpy()) < gf.TOL_F32, f"step {step}, tap {tag}"
         for l in range(cfg["layers"]):
             assert (out / f"{step}.layer{l:02d}_attn_out.f32").stat().st_size == len(rows) * D * 4
+
+
+def test_a_failure_cleared_while_a_step_is_launched_ends_it():
+    """Another thread finds a failure, and clears it, between the launches of a step and the end of the call that makes them."""
+    from geneinfer_b200 import StepEntry
+    from geneinfer_b200.ops import kernels
+    engine = gf.make_engine("b", "bfloat16", n_pages=4)
+    run = engine._run
+
+    def failing(ctx):
+        kernels.status_word(engine.device)[0] = 0x22
+        assert kernels.take_failure(engine.device, kernels.status_failures(engine.device))
+        return run(ctx)
+
+    engine.open(0)
+    engine._run = failing
+    engine.step([StepEntry(0, [3, 4, 5])])
+    engine._run = run
+    with pytest.raises(kernels.KernelError):
+        engine.check_status()
+    engine.step([StepEntry(0, [6])])
+    engine.check_status()

@@ -79,3 +79,17 @@ def test_a_failure_is_counted_before_the_word_is_cleared(host):
     with pytest.raises(kernels.KernelError, match="0x21"):
         one.result()
     assert seen == [True] and host.sample().result() == [1]
+
+
+def test_a_failure_while_a_sample_is_launched_is_its_own(host):
+    """Another thread finds and clears a failure between the launch of a sample's kernels and the end of the call that launches them."""
+    def fail():
+        host.state.status[0] = 0x22
+        assert kernels.take_failure(host.device, kernels.status_failures(host.device))
+
+    host.launched = fail
+    call = host.sample()
+    host.launched = lambda: None
+    with pytest.raises(kernels.KernelError):
+        call.result()
+    assert host.sample().result() == [1]
