@@ -6,6 +6,7 @@ refuses a size. Nothing here computes on the host.
 """
 from __future__ import annotations
 
+import threading
 from typing import Optional, Tuple
 
 import torch
@@ -1140,6 +1141,7 @@ class _TensorCoreState:
         self.counters = torch.zeros(self.COUNTERS, dtype=torch.int32, device=device)
         self.status = torch.zeros(1, dtype=torch.int32).pin_memory()
         self.failures = 0           # how often the word was found set and cleared
+        self.lock = threading.Lock()
 
     @property
     def workspace(self) -> torch.Tensor:
@@ -1501,12 +1503,16 @@ def status_failures(device: torch.device) -> int:
 
 def take_failure(device: torch.device, failures: int) -> int:
     """For who noted ``failures`` (``status_failures``): other than 0 if the status word holds a failure, which is then counted and the
-    word cleared, or if someone else has done so since."""
+    word cleared once nothing runs on the device, or if someone else has done so since. The failure may be that of a kernel behind what
+    the caller has waited for."""
     st = _tc_state(device)
     code = int(st.status[0])            # (looked at before the count, and cleared behind it: a failure is always in one of the two)
     if code:
-        st.failures += 1
-        st.status.zero_()
+        torch.cuda.synchronize(device)  # what still runs may set the word again, for the same failure
+        with st.lock:
+            if int(st.status[0]):       # (else someone else has taken it meanwhile)
+                st.failures += 1
+                st.status.zero_()
     return code or st.failures - failures
 
 

@@ -20,8 +20,8 @@ class PendingSample:
     """The token ids of one sampling call, on their way to the host."""
 
     def __init__(self, host: torch.Tensor, rows: int, event, status: Optional[torch.Tensor] = None, on_failure=None, failed=None):
-        """``failed()``: looked at behind the ids; a value other than 0 says that a kernel gave up a bounded wait, so the ids are
-        not to be trusted. ``status``: or a word [1] of this call's own that says so, cleared with the error; ``on_failure`` is called
+        """``failed()``: looked at behind the ids; a value other than 0 says that a kernel gave up a bounded wait, of the steps
+        before or of one launched since: the ids are not to be trusted. ``status``: or a word [1] of this call's own that says so, cleared with the error; ``on_failure`` is called
         before it."""
         self._host, self._rows, self._event, self._status, self._on_failure, self._failed = host, rows, event, status, on_failure, failed
 

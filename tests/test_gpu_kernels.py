@@ -440,6 +440,43 @@ def test_a_failed_wait_ends_every_call_that_was_under_way():
     assert K().gemm_tc_status(device) == 0 and sampler.sample(logits, [SamplingParams(0.0)], [0.0]) == [7]
 
 
+def _writes_word_later(code, device):
+    """Launches, behind some 25 ms, a kernel that stores ``code`` in the status word: the place of a row's largest value, written where
+    its id would go."""
+    from geneinfer_b200.ops.library import lib
+    logits = torch.zeros(1, 64, device=device)
+    logits[0, code] = 1.0
+    values, places = torch.empty(32, device=device), torch.empty(32, dtype=torch.int32, device=device)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(50_000_000)
+    assert lib().gi_argmax(logits.data_ptr(), 1, 64, K().status_word(device).data_ptr(), values.data_ptr(), places.data_ptr(),
+                           torch.cuda.current_stream().cuda_stream) == 0
+
+
+def test_the_status_word_as_kernels_write_it():
+    """What a kernel stores in the word is seen behind the event of the call that launched it, and what it stores after a failure has
+    been found, while it runs on, ends with that failure."""
+    from geneinfer_b200 import SamplingParams
+    from geneinfer_b200.sampling.device import DeviceSampler
+    device = torch.device(DEV)
+    sampler = DeviceSampler(64, device)
+    logits = torch.zeros(1, 64, device=DEV)
+    logits[0, 7] = 1.0
+    call = lambda: sampler.sample_async(logits, [SamplingParams(0.0)], [0.0])  # noqa: E731
+    assert call().result() == [7]
+    _writes_word_later(0x21, device)
+    with pytest.raises(K().KernelError, match="0x21"):
+        call().result()
+    assert call().result() == [7]
+    one = call()
+    _writes_word_later(0x22, device)
+    K().status_word(device)[0] = 0x21                       # its first
+    with pytest.raises(K().KernelError, match="0x21"):
+        one.result()
+    torch.cuda.synchronize()
+    assert call().result() == [7] and K().gemm_tc_status(device) == 0
+
+
 @pytest.mark.parametrize("V", [131072, 131073])
 @pytest.mark.parametrize("top_k,top_p", [(0, 1.0), (40, 1.0), (0, 0.9), (40, 0.95)])
 def test_sample_of_the_largest_rows_held_in_registers_and_the_smallest_not(V, top_k, top_p):

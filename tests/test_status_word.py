@@ -93,3 +93,22 @@ def test_a_failure_while_a_sample_is_launched_is_its_own(host):
     with pytest.raises(kernels.KernelError):
         call.result()
     assert host.sample().result() == [1]
+
+
+def test_a_failure_ends_when_its_kernels_have(host, monkeypatch):
+    """A kernel that has given up one wait gives up others while it runs on: they belong to the same failure, and a call that is made
+    after it has been raised is not ended by them."""
+    running = [True]
+
+    def ends():
+        if running.pop() and not host.state.status[0]:
+            host.state.status[0] = 0x23
+        running.append(False)
+
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda *a: ends())
+    call = host.sample()
+    host.state.status[0] = 0x21
+    with pytest.raises(kernels.KernelError):
+        call.result()
+    ends()
+    assert host.sample().result() == [1]
