@@ -1141,6 +1141,7 @@ class _TensorCoreState:
         self.counters = torch.zeros(self.COUNTERS, dtype=torch.int32, device=device)
         self.status = torch.zeros(1, dtype=torch.int32).pin_memory()
         self.failures = 0           # how often the word was found set and cleared
+        self.failure = 0            # what it held the last time
         self.lock = threading.Lock()
 
     @property
@@ -1502,8 +1503,8 @@ def status_failures(device: torch.device) -> int:
 
 
 def take_failure(device: torch.device, failures: int) -> int:
-    """For who noted ``failures`` (``status_failures``): other than 0 if the status word holds a failure, which is then counted and the
-    word cleared once nothing runs on the device, or if someone else has done so since. The failure may be that of a kernel behind what
+    """For who noted ``failures`` (``status_failures``): the failure that the status word holds, which is then counted and the word
+    cleared once nothing runs on the device, or that someone else has found since (0: none). The failure may be that of a kernel behind what
     the caller has waited for."""
     st = _tc_state(device)
     code = int(st.status[0])            # (looked at before the count, and cleared behind it: a failure is always in one of the two)
@@ -1511,9 +1512,10 @@ def take_failure(device: torch.device, failures: int) -> int:
         torch.cuda.synchronize(device)  # what still runs may set the word again, for the same failure
         with st.lock:
             if int(st.status[0]):       # (else someone else has taken it meanwhile)
+                st.failure = code
                 st.failures += 1
                 st.status.zero_()
-    return code or st.failures - failures
+    return code or (st.failure if st.failures != failures else 0)
 
 
 def gemm_tc_status(device: torch.device) -> int:

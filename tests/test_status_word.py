@@ -112,3 +112,12 @@ def test_a_failure_ends_when_its_kernels_have(host, monkeypatch):
         call.result()
     ends()
     assert host.sample().result() == [1]
+
+
+def test_every_call_under_way_names_the_failure(host):
+    """Who learns of a failure by the count gives its code too."""
+    calls = [host.sample(), host.sample()]
+    host.state.status[0] = 0x21
+    for call in calls:
+        with pytest.raises(kernels.KernelError, match="status 0x21"):
+            call.result()
