@@ -175,10 +175,11 @@ def _plain_row_decay_scan(q, k, v, z, tau, S0=None):
     return o, S
 
 
-@pytest.mark.parametrize("H, dk, dv", [(3, 16, 24), (2, 48, 40), (1, 100, 33), (2, 200, 8), (5, 8, 64)])
-def test_recurrence_with_a_decay_per_row(H, dk, dv):
-    """One walk from a state that an earlier step left; a step of more than 128 tokens cut into parts that run side by
-    side; single tokens; the bias on z and the constant on the queries."""
+@pytest.mark.parametrize("H, dk, dv, part", [(3, 16, 24, 128), (2, 48, 40, 128), (1, 100, 33, 128), (2, 200, 8, 128), (5, 8, 64, 128),
+                                             (2, 64, 128, 128), (1, 40, 130, 128), (2, 64, 128, 70), (1, 33, 200, 70), (2, 50, 65, 131), (1, 128, 100, 70)])
+def test_recurrence_with_a_decay_per_row(H, dk, dv, part):
+    """One walk from a state that an earlier step left; a step of more than ``part`` tokens cut into parts that run side by
+    side, in blocks of 32, 64 and 128 columns, the last one partly empty; single tokens; the bias on z and the constant on the queries."""
     from geneinfer_b200.ops import kernels
     g = torch.Generator().manual_seed(H * 100 + dk)
     tau, qs = 4.0, 0.37
@@ -204,8 +205,8 @@ def test_recurrence_with_a_decay_per_row(H, dk, dv):
             starts = np.cumsum([0] + [lengths[r] for r in live])
             out = torch.full((T, H * dv), float("nan"), device=DEV)
             extra = {}
-            if T > kernels.SCAN_PART:
-                extra = {"part_len": kernels.SCAN_PART, "ws_state": torch.full((kernels.scan_parts(T, len(live)), H * dk * dv), float("nan"), device=DEV),
+            if T > part:
+                extra = {"part_len": part, "ws_state": torch.full((kernels.scan_parts(T, len(live), part), H * dk * dv), float("nan"), device=DEV),
                          "ws_decay": torch.full((T, H * dk), float("nan"), device=DEV)}
             kernels.linear_scan(x, 3, x, 3 + H * dk, x, 3 + 2 * H * dk, H, 1, dk, dv, False, state, 5,
                                 torch.tensor(starts[:-1], dtype=torch.int32, device=DEV),
@@ -222,7 +223,7 @@ def test_recurrence_with_a_decay_per_row(H, dk, dv):
 
 
 @pytest.mark.parametrize("stepped", [False, True])
-@pytest.mark.parametrize("H, group, dk, dv", [(4, 2, 16, 24), (2, 1, 48, 64), (3, 3, 128, 65), (2, 1, 100, 130)])
+@pytest.mark.parametrize("H, group, dk, dv", [(4, 2, 16, 24), (2, 1, 48, 64), (3, 3, 128, 65), (2, 1, 100, 130), (2, 2, 64, 128), (2, 1, 40, 130), (1, 1, 33, 65)])
 def test_recurrence_cut_into_parts(H, group, dk, dv, stepped):
     """Constant decays (one of them 0) and decays from step sizes: parts whose last one has a token, tokens around the 64 of an
     output block, a segment of one token, against the walk in 64 bits and against the walk without parts."""

@@ -252,7 +252,7 @@ def test_attention_rows_in_tiles_and_ranges_of_keys(H, Hkv, hd, vd, window, chun
     args = (q.reshape(n, H * hd).to(DEV), k_pages, v_pages)
     rest = (torch.zeros(n, dtype=torch.int32, device=DEV), pos.int().to(DEV), table, H, Hkv, hd, vd, page, 0.21)
     kw = dict(window=window, chunk=chunk, slopes=None if slopes is None else slopes.to(DEV), sinks=None if sinks is None else sinks.to(DEV))
-    for splits in (1, 3, 16):
+    for splits in (1, 3, 16, 17, 30, 32):
         ws = None
         if splits > 1:
             ws = torch.full((kernels.attention_rows_workspace_rows(len(tiles), H, Hkv, splits), vd + 2), float("nan"), device=DEV)

@@ -300,7 +300,7 @@ def _attention_case(dtype, H, Hkv, hd, ps, ctx_lens, q_lens, window, seed, spike
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("H,Hkv,hd,ps", [(4, 2, 16, 16), (3, 1, 32, 8), (6, 3, 48, 16), (8, 2, 128, 32), (2, 1, 256, 16),
-                                          (5, 5, 80, 4)])
+                                          (5, 5, 80, 4), (8, 2, 256, 16), (4, 1, 128, 16), (12, 4, 64, 16)])
 def test_attention_mixed_rows(dtype, H, Hkv, hd, ps):
     # a whole prompt, a single decoded token deep in a context, a portion over page edges, position 0 alone
     got, want = _attention_case(dtype, H, Hkv, hd, ps, ctx_lens=[37, 130, 3 * ps + 1, 1], q_lens=[37, 1, ps + 2, 1],
@@ -475,6 +475,69 @@ def test_the_status_word_as_kernels_write_it():
         one.result()
     torch.cuda.synchronize()
     assert call().result() == [7] and K().gemm_tc_status(device) == 0
+
+
+_GIVES_UP = """
+__global__ void gives_up(int* status, const volatile int* flag, int code, long long cycles) {
+    const long long t0 = clock64();
+    while (!*flag)
+        if (clock64() - t0 > cycles) { atomicCAS(status, 0, code); break; }
+}
+extern "C" int launch(int* status, const int* flag, int code, long long cycles, void* stream) {
+    gives_up<<<1, 1, 0, static_cast<cudaStream_t>(stream)>>>(status, flag, code, cycles);
+    return cudaGetLastError();
+}
+"""
+
+
+def test_a_bounded_wait_that_gives_up_ends_steps_and_samples(tmp_path):
+    """A kernel (of the test's own) that waits some milliseconds for a flag that nothing sets and then leaves its code in the word as the
+    library's do, ahead of a sample and of a step."""
+    import ctypes
+    import subprocess
+    import gpu_fixtures as gf
+    from geneinfer_b200 import SamplingParams, StepEntry
+    from geneinfer_b200.ops.build import _nvcc
+    from geneinfer_b200.sampling.device import DeviceSampler
+    (tmp_path / "gives_up.cu").write_text(_GIVES_UP)
+    subprocess.run([_nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-Xcompiler", "-fPIC", "-o", str(tmp_path / "gives_up.so"),
+                    str(tmp_path / "gives_up.cu")], check=True)
+    launch = ctypes.CDLL(str(tmp_path / "gives_up.so")).launch
+    launch.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_void_p]
+    device = torch.device(DEV)
+    flag = torch.zeros(1, dtype=torch.int32, device=device)
+
+    def gives_up(code):
+        assert launch(K().status_word(device).data_ptr(), flag.data_ptr(), code, 20_000_000, torch.cuda.current_stream().cuda_stream) == 0
+
+    sampler = DeviceSampler(64, device)
+    engine = gf.make_engine("b", "bfloat16", n_pages=4)
+    engine.open(0)
+    logits = torch.zeros(1, 64, device=device)
+    gives_up(5)
+    gives_up(6)                                             # (the first code stays)
+    with pytest.raises(K().KernelError, match="0x5"):
+        sampler.sample(logits, [SamplingParams(0.0)], [0.0])
+    engine.step([StepEntry(0, [3])])
+    engine.check_status()
+    gives_up(7)
+    engine.step([StepEntry(0, [4])])
+    with pytest.raises(K().KernelError, match="0x7"):
+        engine.check_status()
+    engine.step([StepEntry(0, [5])])
+    engine.check_status()
+    assert sampler.sample(logits, [SamplingParams(0.0)], [0.0]) == [0] and K().gemm_tc_status(device) == 0
+
+
+def test_the_status_word_is_read_behind_the_kernels():
+    """What a kernel still in the stream stores in the word is in the answer."""
+    device = torch.device(DEV)
+    assert K().gemm_tc_status(device) == 0
+    _writes_word_later(0x23, device)
+    got = K().gemm_tc_status(device)
+    torch.cuda.synchronize()
+    K().status_word(device).zero_()
+    assert got == 0x23 and K().gemm_tc_status(device) == 0
 
 
 @pytest.mark.parametrize("V", [131072, 131073])

@@ -344,3 +344,60 @@ def test_engine_with_sixteen_running_requests_across_context_buckets(dtype, tmp_
         w, rnd = pm.round_weights_bf16(w), pm.bf16_rounding
     for i in (0, 2, 5, 8, 15, 19):                           # the shortest, the longest, the ones at the buckets' edges
         _check_greedy_continuation(w, cfg, rnd, prompts[i], got[i], dtype, f"request {i}")
+
+
+# ------------------------------------------------------------------ the norm that a layer hands on to the next
+def _model_of_runs(case, dtype, looped):
+    import torch
+    from geneinfer_b200.config.base import ScheduleEntry
+    from geneinfer_b200.engine.loading import parse_dtype
+    from geneinfer_b200.parts import DecoderModel
+    from geneinfer_b200.weights import load_model_folder
+    _, cfg, params = load_model_folder(gf.model_dir(case))
+    spec = cfg.model_spec()
+    if looped:               # layer 0 with two caches, layer 1 once as a writer and once as a reader, ahead of 0 and at the end
+        spec.schedule = [ScheduleEntry(0), ScheduleEntry(1), ScheduleEntry(0, cache_of=2), ScheduleEntry(1, writes_cache=False)]
+    return DecoderModel(spec, params, parse_dtype(dtype), torch.device("cuda:0"))
+
+
+@pytest.mark.parametrize("dtype, case, looped", [("float32", "d", False), ("float32", "d", True), ("bfloat16", "c", False), ("bfloat16", "d", False),
+                                                 ("bfloat16", "d", True), ("bfloat16", "w", False)])
+def test_norms_handed_on_with_a_listener_that_comes_and_goes(dtype, case, looped, monkeypatch):
+    """A layer's last product also takes the norm that follows, for the next layer too. The logits are those of norms that are taken
+    where they are needed, to the bit, also when a listener changes the stream between two of them, steps before and behind it run from
+    recorded programs and graphs, and layers run twice. ("w": the prompt's norms are taken by the kernel that adds up ranges of K.)"""
+    from geneinfer_b200 import StepEngine, StepEntry
+    from geneinfer_b200.ops import kernels
+    from geneinfer_b200.parts.attention import AttentionMixer
+    from geneinfer_b200.parts.feed_forward import SwiGLUFeedForward
+    model = _model_of_runs(case, dtype, looped)
+    vocab = gf.CASES[case][0]["vocab_size"]
+    text = tc.random_tokens(364, vocab, 77)
+    listening = []
+
+    def listener(tag, layer, x, ctx):
+        listening.append((tag, layer))
+        if tag in ("attn_out", "ffn_out"):
+            x[:, :3] += 0.5
+
+    def run():
+        engine = StepEngine(model, page_size=16, n_pages=64, max_requests=2, max_step_tokens=256)
+        engine.open(0)
+        out, at = [], 0
+        for n, listens in ((129, False), (100, True), (129, False), (1, False), (1, True), (1, False), (1, False), (1, True), (1, False)):
+            engine.tap = listener if listens else None
+            out.append(engine.step([StepEntry(0, text[at:at + n], [0, n - 1] if n > 1 else [0])]).clone())
+            at += n
+        engine.check_status()
+        return out
+
+    got = run()
+    heard = len(listening)
+    if case == "w":
+        assert kernels.gemm_tc_plan(129, model.hidden_size, 8192, True)[2] > 1
+    monkeypatch.setattr(AttentionMixer, "takes_norm", False)
+    monkeypatch.setattr(SwiGLUFeedForward, "takes_norm", False)
+    want = run()
+    assert heard > 0 and len(listening) == 2 * heard
+    for i, (a, b) in enumerate(zip(got, want)):
+        assert bool((a == b).all()), i
