@@ -1242,7 +1242,7 @@ static int launch_grouped(const GroupedArgs& p, int a_dtype, int w_dtype, dim3 g
 template <typename TA>
 static int launch_head_mma(const GroupedArgs& p, cudaStream_t st) {
     const unsigned heads = static_cast<unsigned>(p.groups), blocks_n = static_cast<unsigned>((p.N + 63) / 64);
-    GI_REQUIRE(blocks_n <= 65535 && (p.rows + 63) / 64 <= 65535, "head_product: too many tiles");
+    GI_REQUIRE(blocks_n <= 65535, "head_product: too many tiles");
     if (p.rows <= 8) launch_kernel((head_mma_kernel<TA, 1, 1, true>), dim3(heads, blocks_n), dim3(128), 0, st, p);
     else if (p.rows <= 32) launch_kernel((head_mma_kernel<TA, 1, 2, true>), dim3(heads, blocks_n, (p.rows + 15) / 16), dim3(128), 0, st, p);
     else launch_kernel((head_mma_kernel<TA, 4, 2, false>), dim3(heads, blocks_n, (p.rows + 63) / 64), dim3(128), 0, st, p);
@@ -1279,7 +1279,8 @@ static int gi_head_product_impl(const void* a, int a_dtype, long long lda, int a
     if (rows_form_fits(p, a_dtype, w_dtype)) {
         cudaStream_t st = static_cast<cudaStream_t>(stream);
         if (tail == 0 && rows <= 2 * kGpTM) return launch_grouped_rows<false>(p, a_dtype, w_dtype, static_cast<unsigned>(tiles), st);
-        if (w_dtype == kBF16) return a_dtype == kF32 ? launch_head_mma<float>(p, st) : launch_head_mma<__nv_bfloat16>(p, st);
+        if (w_dtype == kBF16 && rows <= 65535 * 64)                   // (blocks of rows along the grid's third axis; more: below)
+            return a_dtype == kF32 ? launch_head_mma<float>(p, st) : launch_head_mma<__nv_bfloat16>(p, st);
         if (tail > 0 && rows <= kGcRows) {
             launch_kernel(head_product_few_kernel, dim3(heads, (N + kGcCols - 1) / kGcCols), dim3(kGcCols), 0, st, p);
             return check_launch("head_product (few rows)");

@@ -290,6 +290,19 @@ def test_head_product_with_a_rotated_tail(dtype):
         assert torch.isnan(out.cpu()[:, :2]).all()
 
 
+@pytest.mark.parametrize("T", [65535 * 64, 65535 * 64 + 1])
+def test_head_product_of_the_most_rows(T):
+    """A row more than a grid has places for in tiles of 64."""
+    from geneinfer_b200.ops import kernels
+    a = torch.randn(T, 8, generator=torch.Generator(DEV).manual_seed(1), device=DEV)
+    w = _bf(torch.randn(1, 8, 8, generator=torch.Generator().manual_seed(2)))
+    out = torch.full((T, 8), float("nan"), device=DEV)
+    kernels.head_product(a, 0, 8, w.to(DEV).bfloat16(), out, 0, 8)
+    for rows in (slice(0, 1000), slice(T - 1000, T)):
+        _close(out[rows].cpu(), a[rows].cpu().double() @ w[0].double().T, torch.float32, "first and last rows")
+    assert bool(out.isfinite().all())
+
+
 @pytest.mark.parametrize("interleaved", [True, False])
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("T, H, N, K, tail", [(1, 3, 70, 24, 6), (2, 16, 512, 64, 32), (3, 2, 5, 264, 72), (4, 5, 64, 32, 2), (5, 5, 64, 32, 2)])
