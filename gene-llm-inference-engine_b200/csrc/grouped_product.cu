@@ -40,7 +40,7 @@ struct GroupedArgs {
     const void* a; long long lda; int a_off; int a_gs; int a_div;
     const void* w; long long w_gs; int ldw; long long up_off;     // W[g] = w + g * w_gs, rows of ldw; the up rows start at up_off
     void* out; int out_is_f32; long long ldo; int o_off; int o_gs;
-    int N, K, rows, groups;
+    int N, K, rows, groups;                                       // rows: the pairs in the experts form
     const int* tile_group; const int* sorted_rows; const int* n_tiles;   // experts form (else null)
     int w_constant;                                               // no kernel that may still be running writes w: it may be read before the wait
     int act; float act_limit;                                     // gated: a GateAct code and its limit
@@ -1220,12 +1220,14 @@ static int launch_grouped_mma(const GroupedArgs& p, unsigned tiles, cudaStream_t
 template <bool GATED>
 static int launch_grouped_rows(const GroupedArgs& p, int a_dtype, int w_dtype, unsigned tiles, cudaStream_t st) {
     if (w_dtype == kF32) return launch_grouped_rows_as<float, GATED, 4>(p, tiles, st);
-    // 32-bit inputs with room for at most five tiles (up to four pairs, or few experts): mostly a pair or two a tile, so that the
-    // multiply-adds are few, and cutting eight rows' inputs into parts costs more than they do (2,048 outputs of 4,096 inputs, 2 / 4
-    // pairs: 14.1 / 17.1 us on the CUDA cores, 14.7 / 26.1 on the tensor cores; 8 pairs 30.2 against 29.4, sixteen 36.7 against 40.8 when
-    // they spread evenly and 54 against 31 when they crowd a few experts).
+    // 32-bit inputs of a few pairs, about two for each expert that there is (room for tiles: one and an expert's each): the multiply-adds
+    // are few, and cutting eight rows' inputs into parts costs more than they do. The time on the CUDA cores goes with the rows of the
+    // fullest tile, on the tensor cores with the tiles, and jumps at the third. Measured, 2,048 outputs of 4,096 inputs, us on the CUDA cores /
+    // on the tensor cores, pairs of each expert: 1,1 13.5 / 15.0; 2,2 14.8 / 15.2; 2,2,2 16.9 / 25.9; 2,2,2,2 18.5 / 26.6; 1,1,1,1 of eight experts
+    // 17.7 / 24.8; but 4 18.5 / 13.8; 3,3 18.7 / 15.3; 5,1,1,1 28.4 / 26.7; 6,5,5 28.1 / 26.8; 10,4,1,1 45.2 / 27.5; five experts of one pair
+    // 29.0 / 28.9.
     if constexpr (!GATED)
-        if (a_dtype == kF32 && p.tile_group && tiles <= 5) return launch_grouped_rows_as<__nv_bfloat16, false, 8>(p, tiles, st);
+        if (a_dtype == kF32 && p.tile_group && tiles <= 5 && p.rows <= 2 * (static_cast<int>(tiles) - 1)) return launch_grouped_rows_as<__nv_bfloat16, false, 8>(p, tiles, st);
     return a_dtype == kF32 ? launch_grouped_mma<float, GATED>(p, tiles, st) : launch_grouped_mma<__nv_bfloat16, GATED>(p, tiles, st);
 }
 
@@ -1304,7 +1306,7 @@ static int gi_head_product_impl(const void* a, int a_dtype, long long lda, int a
 static int gi_expert_product_impl(const void* a, int a_dtype, long long lda, int a_div, const void* w, int w_dtype, long long w_gs,
                                   int ldw, long long up_off, int gated, int act, float act_limit, const float* scales, void* out, int out_dtype, long long ldo,
                                   int N, int K, const int* tile_group, const int* sorted_rows, const int* n_tiles, int max_tiles,
-                                  void* stream) {
+                                  int pairs, void* stream) {
     if (max_tiles == 0) return 0;
     GI_REQUIRE(max_tiles > 0 && N > 0 && K > 0 && a_div > 0, "expert_product: sizes must be positive");
     GI_REQUIRE(tile_group && sorted_rows && n_tiles, "expert_product: the sorted rows are missing");
@@ -1313,7 +1315,7 @@ static int gi_expert_product_impl(const void* a, int a_dtype, long long lda, int
     p.a = a; p.lda = lda; p.a_div = a_div;
     p.w = w; p.w_gs = w_gs; p.ldw = ldw; p.up_off = up_off;
     p.out = out; p.out_is_f32 = out_dtype == kF32; p.ldo = ldo;
-    p.N = N; p.K = K; p.groups = 1;
+    p.N = N; p.K = K; p.groups = 1; p.rows = pairs;
     p.tile_group = tile_group; p.sorted_rows = sorted_rows; p.n_tiles = n_tiles; p.act = gated ? act : 0; p.act_limit = act_limit;
     p.out_act = gated ? kPlainNone : act;
     p.scales = scales;
@@ -1441,9 +1443,9 @@ extern "C" int gi_head_product(const void* a, int a_dtype, long long lda, int a_
 
 extern "C" int gi_expert_product(const void* a, int a_dtype, long long lda, int a_div, const void* w, int w_dtype, long long w_gs,
                                  int ldw, long long up_off, int gated, int act, float act_limit, const float* scales, void* out, int out_dtype, long long ldo, int N, int K,
-                                 const int* tile_group, const int* sorted_rows, const int* n_tiles, int max_tiles, void* stream) {
+                                 const int* tile_group, const int* sorted_rows, const int* n_tiles, int max_tiles, int pairs, void* stream) {
     return gi::dispatch(gi_expert_product_impl, a, a_dtype, lda, a_div, w, w_dtype, w_gs, ldw, up_off, gated, act, act_limit, scales, out, out_dtype, ldo,
-                        N, K, tile_group, sorted_rows, n_tiles, max_tiles, stream);
+                        N, K, tile_group, sorted_rows, n_tiles, max_tiles, pairs, stream);
 }
 
 extern "C" int gi_route(const void* x, int x_dtype, int T, int D, const float* w, const float* correction, int E, int top,

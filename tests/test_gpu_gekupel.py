@@ -498,7 +498,7 @@ def test_expert_products_of_few_rows(dtype, N, K, gated):
     _close(out.cpu(), want, torch.float32, "few rows", f32=1e-5)
 
 
-@pytest.mark.parametrize("form", ["experts", "experts, room for five tiles", "gated experts", "heads, 9 rows", "heads, 33 rows", "heads, 70 rows", "heads with a tail, 12 rows"])
+@pytest.mark.parametrize("form", ["experts", "experts, room for five tiles", "experts, eight pairs, room for five tiles", "gated experts", "heads, 9 rows", "heads, 33 rows", "heads, 70 rows", "heads with a tail, 12 rows"])
 @pytest.mark.parametrize("N, K", [(16, 264), (70, 40)])
 def test_products_of_32_bit_inputs_with_bfloat16_weights(form, N, K):
     """Inputs all of whose bits count, of any size, infinite or none. The parts that an input is cut into add up to it, so what is left are
@@ -507,7 +507,7 @@ def test_products_of_32_bit_inputs_with_bfloat16_weights(form, N, K):
     from geneinfer_b200.ops import kernels
     g = torch.Generator().manual_seed(K)
     heads = form.startswith("heads")
-    T = int(form.split(", ")[1].split()[0]) if heads else 9
+    T = int(form.split(", ")[1].split()[0]) if heads else 8 if "eight" in form else 9
     G, tail = (3, 8 if "tail" in form else 0) if heads else (1, 0)
     gated = form == "gated experts"
     x, w = torch.randn(T, G, K, generator=g), _bf(torch.randn(G, (2 if gated else 1) * N, K, generator=g))
@@ -539,7 +539,7 @@ def test_products_of_32_bit_inputs_with_bfloat16_weights(form, N, K):
     assert bool(((got - want).abs() <= bound)[keep].all()), float(((got - want).abs() / bound)[keep].max())
 
 
-@pytest.mark.parametrize("form", ["experts", "four experts' pairs", "gated experts", "heads, 9 rows", "heads, 33 rows", "heads, 70 rows", "heads with a tail, 12 rows"])
+@pytest.mark.parametrize("form", ["experts", "experts, four pairs, room for five tiles", "gated experts", "heads, 9 rows", "heads, 33 rows", "heads, 70 rows", "heads with a tail, 12 rows"])
 @pytest.mark.parametrize("N, K", [(16, 264), (70, 40)])
 def test_infinite_weights_with_32_bit_inputs(form, N, K):
     """An infinite weight gives an infinity of the input's sign, none where the input is zero or another one is infinite the other
@@ -562,9 +562,10 @@ def test_infinite_weights_with_32_bit_inputs(form, N, K):
         kernels.head_product(a, 0, K + tail, w.to(DEV).bfloat16(), out, 0, N + tail, tail=tail,
                              freq=torch.ones(tail // 2, device=DEV) if tail else None, positions=torch.zeros(T, dtype=torch.int32, device=DEV) if tail else None)
     else:
-        rows = torch.full((6 * kernels.grouped_tile_rows(),), -1, dtype=torch.int32)
+        room = 5 if "room" in form else 6
+        rows = torch.full((room * kernels.grouped_tile_rows(),), -1, dtype=torch.int32)
         rows[:T] = torch.arange(T, dtype=torch.int32)
-        kernels.expert_product(x[:, 0].contiguous().to(DEV), 1, w.to(DEV).bfloat16(), out, rows.to(DEV), torch.zeros(6, dtype=torch.int32, device=DEV),
+        kernels.expert_product(x[:, 0].contiguous().to(DEV), 1, w.to(DEV).bfloat16(), out, rows.to(DEV), torch.zeros(room, dtype=torch.int32, device=DEV),
                                torch.ones(1, dtype=torch.int32, device=DEV), gated="silu" if gated else None)
     got = out.cpu().view(T, G, N + tail)[..., :N].double()
     want = torch.einsum("tgk,gnk->tgn", x.double(), w.double())
