@@ -20,6 +20,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "device_limit.h"
 
 namespace gi {
 
@@ -223,7 +224,7 @@ static int gi_attention_generic_impl(const void* q, const void* k_cache, const v
             window, sink, gate, gate_ld, gate_off, gate_dims, out_scale);
     };
     // up to two blocks an SM are few (268 rows with everything in flight, three blocks of 165 registers an SM: 105 us instead of 60)
-    const bool few = static_cast<long long>(H) * T <= 2 * 148;
+    const bool few = static_cast<long long>(H) * T <= 2 * sm_count();
     auto typed = [&](auto* t) {
         using V = std::remove_pointer_t<decltype(t)>;
         if (hd <= 64) few ? launch(paged_attention_generic_kernel<V, 2, true>, t) : launch(paged_attention_generic_kernel<V, 2, false>, t);

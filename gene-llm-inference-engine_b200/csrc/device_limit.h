@@ -1,4 +1,4 @@
-// The dynamic shared memory above 48 KB that a kernel may be launched with is set per device. A launcher keeps one of these per
+// What launchers ask of the device. The dynamic shared memory above 48 KB that a kernel may be launched with is set per device. A launcher keeps one of these per
 // kernel: the limit is set at the kernel's first launch on each device of the process and remembered by device.
 #pragma once
 
@@ -26,5 +26,13 @@ class SharedLimit {
   private:
     std::atomic<unsigned long long> set_{0};
 };
+
+// Multiprocessors of the current device.
+inline int sm_count() {
+    int sms = 0, device = 0;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    return sms > 0 ? sms : 1;
+}
 
 }  // namespace gi

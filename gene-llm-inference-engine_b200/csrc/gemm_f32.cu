@@ -232,11 +232,12 @@ int gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int 
     // 189 -> 171 each and 3,072 of 2,048 122 -> 112 in blocks of 48.)
     int best = 8;
     long long least = -1;
+    const int at_once = 2 * sm_count();
     for (int tm = 8; tm >= 5; --tm) {
         const int rows = (M + 8 * tm - 1) / (8 * tm);
         if (rows > 65535) break;                           // the grid's limit
         const long long blocks = static_cast<long long>(chunks) * ((N + 127) / 128) * rows;
-        const long long cost = (blocks + 2 * 148 - 1) / (2 * 148) * (2 * tm + 1);
+        const long long cost = (blocks + at_once - 1) / at_once * (2 * tm + 1);
         if (least < 0 || cost < least) { least = cost; best = tm; }
     }
     if (best == 5) return launch<Tile40>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, w_constant, st);

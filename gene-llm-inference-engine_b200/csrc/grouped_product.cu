@@ -1194,9 +1194,7 @@ static int launch_grouped_rows_as(const GroupedArgs& p, unsigned tiles, cudaStre
     static SharedLimit limit;
     const cudaError_t ready = limit.allow(reinterpret_cast<const void*>(grouped_rows_kernel<TW, GATED, ROWS>), Stream::kSmem);
     if (ready != cudaSuccess) { set_error("grouped_product (rows): %s", cudaGetErrorString(ready)); return 1; }
-    int sms = 0, dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = sm_count();
     const long long blocks = (static_cast<long long>(tiles) * ((p.N + ROWS - 1) / ROWS) + kGrWarps - 1) / kGrWarps;
     GI_REQUIRE(blocks * kGrWarps <= 2147483647LL - 3 * 1024 * kGrWarps, "grouped_product: too many tiles");
     launch_kernel((grouped_rows_kernel<TW, GATED, ROWS>), dim3(static_cast<unsigned>(std::min<long long>(blocks, Stream::kBlocks * sms))), dim3(kGrWarps * 32),
@@ -1209,9 +1207,7 @@ static int launch_grouped_mma(const GroupedArgs& p, unsigned tiles, cudaStream_t
     static SharedLimit limit;
     const cudaError_t ready = limit.allow(reinterpret_cast<const void*>(grouped_mma_kernel<TA, GATED>), kSmem);
     if (ready != cudaSuccess) { set_error("grouped_product (few rows): %s", cudaGetErrorString(ready)); return 1; }
-    int sms = 0, dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = sm_count();
     const long long units = static_cast<long long>(tiles) * (2 / GmShape<TA>::NT) * ((p.N + kOut - 1) / kOut);
     GI_REQUIRE(units <= 2147483647LL - 4 * 1024, "grouped_product: too many tiles");
     launch_kernel((grouped_mma_kernel<TA, GATED>), dim3(static_cast<unsigned>(std::min<long long>(units, kGmBlocks * sms))), dim3(kGmWarps * 32), kSmem, st, p, static_cast<int>(tiles));
