@@ -115,12 +115,12 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
 
     // w_constant: the weights of the first tiles are asked for before the wait for the kernel ahead, as no kernel that may still be running
     // writes them (six rows in a token's step: N = 16,384, K = 2,048 33.2 -> 28.9 us, N = 3,072 8.4 -> 7.5)
-    if (w_constant)
-        for (int i = 0; i < kStages - 1; ++i)
-            if (i < tiles) load_w(i);
+    if (!w_constant) pdl_wait();
+    for (int i = 0; i < kStages - 1; ++i)
+        if (i < tiles) load_w(i);
     pdl_wait();
     for (int i = 0; i < kStages - 1; ++i) {
-        if (i < tiles) { load_a(i); if (!w_constant) load_w(i); }
+        if (i < tiles) load_a(i);
         commit();
     }
     for (int tile = 0; tile < tiles; ++tile) {

@@ -754,9 +754,9 @@ head_mma_kernel(const GroupedArgs p) {
             else dst[t].zero();
         }
     };
-    if (p.w_constant && n0 < p.N) weights(w, 0);
+    if (!p.w_constant) pdl_wait();
+    if (n0 < p.N) weights(w, 0);
     pdl_wait();
-    if (!p.w_constant && n0 < p.N) weights(w, 0);
     if (p.tail > 0 && blockIdx.y == 0) {                // the rotated tail, by the blocks of the first outputs
         const int first = kFew ? threadIdx.x : lane, step = kFew ? 128 : 32, half = p.tail / 2;
         for (int i = first; i < rows * half; i += step)
@@ -823,9 +823,9 @@ head_product_few_kernel(const GroupedArgs p) {
             wv[i] = k < p.K ? *reinterpret_cast<const uint4*>(wrow + k) : make_uint4(0, 0, 0, 0);
         }
     };
-    if (p.w_constant) request(0);
+    if (!p.w_constant) pdl_wait();
+    request(0);
     pdl_wait();
-    if (!p.w_constant) request(0);
     if (blockIdx.y == 0)
         for (int i = tid; i < p.rows * (p.tail / 2); i += kGcCols) {
             const int r = i / (p.tail / 2);
