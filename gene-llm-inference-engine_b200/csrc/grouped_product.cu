@@ -470,7 +470,7 @@ __device__ __forceinline__ unsigned long long gm_minus(unsigned long long a, uns
 // Eight neighbouring values of an input row as they are read (GmInput) and as they are multiplied (GmParts): what they add to the
 // sums with eight values of weight rows w0 and w1. An input's second and third parts may be zero, and zero times an infinite weight is
 // none, where the input times the weight is infinite: then the first parts' sums alone, which are infinite or none too, are the answer (the parts
-// have the input's sign, so what the others add could not change it).
+// have the input's sign, so what the others add could not change it; of an input below 2^-126 there may be no first part either).
 template <typename TA> struct GmParts;
 template <typename TA> struct GmInput;
 template <> struct GmParts<__nv_bfloat16> {

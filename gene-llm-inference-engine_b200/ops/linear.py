@@ -53,8 +53,9 @@ class Linear:
         return new
 
     def forward(self, a: torch.Tensor, out: torch.Tensor, accumulate: bool = False, then: "Linear" = None, norm=None) -> torch.Tensor:
-        """``norm`` = (weight, eps, xn): the norm of out's rows goes to xn (``kernels.gemm_tc``). ``then``: the Linear whose product runs next but one (after a small kernel); a product of few tokens
-        asks the start of its weights into L2 meanwhile (``kernels.gemm_tc``: ``ahead``)."""
+        """``norm`` = (weight, eps, xn): the norm of out's rows goes to xn (``kernels.gemm_tc``). ``then``: the Linear whose
+        product runs next but one (after a small kernel); a product of few tokens asks the start of its weights into L2
+        meanwhile (``kernels.gemm_tc``: ``ahead``)."""
         if a.dtype != self.compute_dtype:
             raise kernels.KernelError(f"Linear: activations are {a.dtype}, the weight is {self.compute_dtype}")
         if self.compute_dtype is torch.bfloat16 and self.in_features % 8 == 0:

@@ -150,8 +150,8 @@ class RoutedExpertsFeedForward:
     the shared expert's under ``shared.``. The ``correction`` may be absent (no correction).
 
     The step's (token, choice) pairs are bucketed by expert on the device into tiles of rows; each tile runs its
-    expert's matrices. Few pairs (decoding) and the 32-bit path: tiles of a few rows on the CUDA cores, the expert
-    weights streamed once. Many pairs in bfloat16: the rows are gathered into tiles of 128 in the experts' order and
+    expert's matrices. Few pairs (decoding) and the 32-bit path: tiles of a few rows, the expert weights streamed once
+    (bfloat16 weights on mma.sync, a very few pairs and the 32-bit path on the CUDA cores). Many pairs in bfloat16: the rows are gathered into tiles of 128 in the experts' order and
     the two products run on the tensor cores (the many-token product with a matrix per token tile, the activation in
     the first one's epilogue). The launches depend on the token count only (tiles beyond the step's number are not
     run), so the part is recorded into launch programs and CUDA graphs like the dense one."""
