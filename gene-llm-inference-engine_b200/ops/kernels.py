@@ -1303,7 +1303,8 @@ _gemm_choice = {}      # (M, N, K, output dtype, tiled weights) -> (swap, block_
 AHEAD_BYTES = 24 << 20
 
 
-def _norms_with_ranges(a, w, out, accumulate, plan, w_tiles, norm) -> bool:
+def gemm_tc_takes_norm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool,
+                       norm: Tuple[torch.Tensor, float, torch.Tensor], plan=None) -> bool:
     """Whether gemm_tc's kernel that adds up the ranges of K takes the norm of the rows too: many tokens, K in ranges, rows that a
     block holds in registers."""
     (M, K), N = a.shape, w.shape[0]
@@ -1327,7 +1328,7 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: boo
     in ranges that a second kernel adds up."""
     M, K = a.shape
     N = w.shape[0]
-    if norm is not None and not _norms_with_ranges(a, w, out, accumulate, plan, w_tiles, norm):
+    if norm is not None and not gemm_tc_takes_norm(a, w, out, accumulate, norm, plan):
         gemm_tc(a, w, out, accumulate, plan, w_tiles, ahead, act)
         rmsnorm(out, norm[0], norm[2], norm[1])
         return

@@ -59,10 +59,12 @@ class Linear:
         if a.dtype != self.compute_dtype:
             raise kernels.KernelError(f"Linear: activations are {a.dtype}, the weight is {self.compute_dtype}")
         if self.compute_dtype is torch.bfloat16 and self.in_features % 8 == 0:
+            fused = norm is not None and kernels.gemm_tc_takes_norm(a, self.weight, out, accumulate, norm)
             kernels.gemm_tc(a, self.weight, out, accumulate, w_tiles=self.weight_tiles,   # tensor cores (TMA needs 16-byte rows)
-                            ahead=then.weight_tiles if then is not None else None, norm=norm)
+                            ahead=then.weight_tiles if then is not None else None, norm=norm if fused else None)
         else:
+            fused = False
             kernels.gemm_simt(a, self.weight, out, accumulate, w_constant=True)
-            if norm is not None:
-                kernels.rmsnorm(out, norm[0], norm[2], norm[1])
+        if norm is not None and not fused:        # (an operation of its own, also for who times them one by one)
+            kernels.rmsnorm(out, norm[0], norm[2], norm[1])
         return out

@@ -247,3 +247,16 @@ def test_a_failure_cleared_while_a_step_is_launched_ends_it():
         engine.check_status()
     engine.step([StepEntry(0, [6])])
     engine.check_status()
+
+
+@pytest.mark.parametrize("dtype, products", [("bfloat16", "matrix products (tensor cores)"), ("float32", "matrix products (32-bit)")])
+def test_the_profile_counts_every_operation_once(dtype, products):
+    """Two layers of [q; k; v], O, [gate; up] and down products with a norm ahead of the first and the third, and the head's."""
+    from geneinfer_b200 import Engine
+    from geneinfer_b200.engine.profile import profile_report
+    engine = Engine(gf.model_dir("c"), dtype=dtype, max_running=1, kv_pages=24)
+    calls = {}
+    for line in profile_report(engine, [3, 1, 4, 1, 5]).splitlines()[2:]:
+        calls[line[2:38].strip()] = int(line[38:44])
+    fused = calls.get("q/k/v projections + rope + store", 0)
+    assert calls["rmsnorm"] == 5 and calls[products] + fused == 9, calls
