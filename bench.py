@@ -660,7 +660,7 @@ def gekupel_kernel_table(width, heads, kv_heads, head_dim, span, ff, T, pk):
         wuk = (torch.randn(lh, kr, head_dim, device=dev) * 0.05).to(bf)
         qa = torch.empty(N, lh * (kr + rot), device=dev)
         add(f"head_product, queries ({what})", "product", lambda: K.head_product(q, 0, head_dim + rot, wuk, qa, 0, kr + rot, tail=rot,
-                                                                                 freq=freq, amplitude=1.1, positions=pos),
+                                                                                 freq=freq, amplitude=1.1, positions=pos, w_constant=True),
             lh * kr * head_dim * 2 + N * lh * (head_dim + kr + 2 * rot) * 4, flops=2.0 * N * lh * kr * head_dim,
             simt=N * lh * kr * head_dim)
         ol = torch.empty(N, lh * kr, device=dev)
@@ -675,7 +675,7 @@ def gekupel_kernel_table(width, heads, kv_heads, head_dim, span, ff, T, pk):
             else:
                 kw = {"tiles": torch.tensor([(t, min(pt, n - t), 0) for t in range(0, n, pt)][::-1], **i32)}
                 count = kw["tiles"].shape[0]
-            sp = K.attention_rows_splits(count, Hq, Hk, span)
+            sp = K.attention_rows_splits(count, Hq, Hk, span, vd_)
             if sp > 1:
                 kw.update(splits=sp, workspace=torch.empty(K.attention_rows_workspace_rows(count, Hq, Hk, sp), vd_ + 2, device=dev))
             return kw
@@ -686,7 +686,7 @@ def gekupel_kernel_table(width, heads, kv_heads, head_dim, span, ff, T, pk):
             lat_bytes, flops=2.0 * R * seen * lh * (2 * kr + rot))
         wuv = (torch.randn(lh, head_dim, kr, device=dev) * 0.05).to(bf)
         att = torch.empty(N, lh * head_dim, dtype=bf, device=dev)
-        add(f"head_product, values ({what})", "product", lambda: K.head_product(ol, 0, kr, wuv, att, 0, head_dim),
+        add(f"head_product, values ({what})", "product", lambda: K.head_product(ol, 0, kr, wuv, att, 0, head_dim, w_constant=True),
             lh * kr * head_dim * 2 + N * lh * (kr * 4 + head_dim * 2), flops=2.0 * N * lh * kr * head_dim, simt=N * lh * kr * head_dim)
         # attention in blocks with a distance bias and sinks, beside Llama's attention over the same context
         kc = torch.randn(n_pages, kv_heads, page, head_dim, device=dev).to(bf)
@@ -888,7 +888,7 @@ def pinorax_kernel_table(width, heads, head_dim, ff, vocab, layers, T, pk):
         wuk = (torch.randn(lh, kr, head_dim, device=dev) * 0.05).to(bf)
         qa = torch.empty(N, lh * kr, device=dev)
         add(f"head_product, queries from the first product ({what})", "head_product",
-            lambda: K.head_product(down, 0, head_dim, wuk, qa, 0, kr), lh * kr * head_dim * 2 + N * lh * (head_dim + kr) * 4,
+            lambda: K.head_product(down, 0, head_dim, wuk, qa, 0, kr, w_constant=True), lh * kr * head_dim * 2 + N * lh * (head_dim + kr) * 4,
             flops=2.0 * N * lh * kr * head_dim, simt=N * lh * kr * head_dim)
         ol = torch.empty(N, lh * kr, device=dev)
         sinks = torch.randn(lh, device=dev)
@@ -901,7 +901,7 @@ def pinorax_kernel_table(width, heads, head_dim, ff, vocab, layers, T, pk):
             else:
                 kw = {"tiles": torch.tensor([(t, min(pt, n - t), 0) for t in range(0, n, pt)][::-1], **i32)}
                 count = kw["tiles"].shape[0]
-            sp = K.attention_rows_splits(count, lh, 1, span)
+            sp = K.attention_rows_splits(count, lh, 1, span, kr)
             if sp > 1:
                 kw.update(splits=sp, workspace=torch.empty(K.attention_rows_workspace_rows(count, lh, 1, sp), kr + 2, device=dev))
             return kw
@@ -917,7 +917,7 @@ def pinorax_kernel_table(width, heads, head_dim, ff, vocab, layers, T, pk):
         att = torch.empty(N, lh * head_dim, dtype=bf, device=dev)
         for name, like, gate in ((f"head_product, values with the output gate ({what})", "head_product", down),
                                  (f"head_product, values, Gekupel ({what})", "", None)):
-            add(name, like, lambda: K.head_product(ol, 0, kr, wuv, att, 0, head_dim, gate=gate, gate_offset=lh * head_dim + kr),
+            add(name, like, lambda: K.head_product(ol, 0, kr, wuv, att, 0, head_dim, gate=gate, gate_offset=lh * head_dim + kr, w_constant=True),
                 lh * kr * head_dim * 2 + N * lh * (kr * 4 + head_dim * (6 if gate is not None else 2)), flops=2.0 * N * lh * kr * head_dim,
                 simt=N * lh * kr * head_dim)
         # experts chosen by a table beside experts chosen by scores; the capped activation beside SiLU
@@ -1606,7 +1606,7 @@ def kidarax_kernel_table(width, ff, heads, head_dim, kv_heads, T, pk):
         qa = torch.empty(N, lh * (kr + rot), device=dev)
         for name, like, il in ((f"head_product, queries with a rotated tail of halves ({what})", "head_product", False),
                                (f"head_product, queries with a rotated tail of neighbours, Gekupel ({what})", "", True)):
-            add(name, like, lambda: K.head_product(down, 0, head_dim + rot, wuk, qa, 0, kr + rot, tail=rot, freq=fr, amplitude=1.2, positions=pos, interleaved=il),
+            add(name, like, lambda: K.head_product(down, 0, head_dim + rot, wuk, qa, 0, kr + rot, tail=rot, freq=fr, amplitude=1.2, positions=pos, interleaved=il, w_constant=True),
                 lh * kr * head_dim * 2 + N * lh * (head_dim + kr + 2 * rot) * 4, simt=float(N * lh * kr * head_dim))
         ol, lsink = torch.empty(N, lh * kr, device=dev), torch.zeros(lh, device=dev)
         add(f"attention_rows over the latent and the rotated part, sink (unchanged) ({what})", "", lambda: K.attention_rows_of_step(
@@ -1616,9 +1616,9 @@ def kidarax_kernel_table(width, ff, heads, head_dim, kv_heads, T, pk):
         lat = torch.empty(N, lh * head_dim, dtype=bf, device=dev)
         gz = torch.randn(N, lh * head_dim, device=dev)
         add(f"head_product, values with a gate per head ({what})", "head_product", lambda: K.head_product(
-            ol, 0, kr, wuv, lat, 0, head_dim, gate=down, gate_offset=c0 + kr + rot, gate_per_head=True), lh * kr * head_dim * 2 + N * lh * (kr * 4 + head_dim * 2),
+            ol, 0, kr, wuv, lat, 0, head_dim, gate=down, gate_offset=c0 + kr + rot, gate_per_head=True, w_constant=True), lh * kr * head_dim * 2 + N * lh * (kr * 4 + head_dim * 2),
             simt=float(N * lh * kr * head_dim))
-        add(f"head_product, values with a gate per value, Pinorax ({what})", "", lambda: K.head_product(ol, 0, kr, wuv, lat, 0, head_dim, gate=gz),
+        add(f"head_product, values with a gate per value, Pinorax ({what})", "", lambda: K.head_product(ol, 0, kr, wuv, lat, 0, head_dim, gate=gz, w_constant=True),
             lh * kr * head_dim * 2 + N * lh * (kr * 4 + head_dim * 6), simt=float(N * lh * kr * head_dim))
         # experts whose weights scale what they read, and the gated shared expert
         E, top, I, Is = 8, 2, 3 * ff // 8, ff // 4
