@@ -537,7 +537,9 @@ attention_rows_mma_kernel(const RowsArgs a, const RowTiles rt) {
 // pair of value dimensions. A few KB a block, so it is as long as its loads wait for one another: a thread asks for its
 // pair of every range before the ranges' weights are worked out (a token's step, latents of 512 values: 16 heads of eight tokens and five
 // ranges 8.1 -> 4.3 us, of two tokens and fifteen ranges 14.7 -> 3.8; before, a thread had a value and four ranges in flight).
+// PAIRS: the workspace starts on 8 bytes, so that a pair is one load.
 constexpr int kRowsMaxSplits = 32;        // a lane each
+template <bool PAIRS>
 __global__ void __launch_bounds__(kRowsMaxValueThreads)
 attention_rows_merge_kernel(const RowsArgs a, const RowTiles rt) {
     pdl_prologue();
@@ -555,11 +557,15 @@ attention_rows_merge_kernel(const RowsArgs a, const RowTiles rt) {
     const float* row = rt.workspace + (((static_cast<size_t>(blockIdx.x) * a.Hkv + g) * rt.head_blocks + zb) * rt.splits) * stride +
                        static_cast<size_t>(r) * (a.vd + 2);
     const int head = g * group + first_head + tr.head(r);
-    const int d = 2 * threadIdx.x;                    // (vd is a multiple of 64, so rows of vd + 2 values start on 8 bytes)
+    const int d = 2 * threadIdx.x;                    // (vd is a multiple of 64: rows of vd + 2 values start on 8 bytes if the workspace does)
     float2 part[kRowsMaxSplits];
 #pragma unroll
     for (int s = 0; s < kRowsMaxSplits; ++s)
-        if (s < rt.splits) part[s] = *reinterpret_cast<const float2*>(row + s * stride + d);
+        if (s < rt.splits) {
+            const float* pair = row + s * stride + d;
+            if (PAIRS) part[s] = *reinterpret_cast<const float2*>(pair);
+            else part[s] = make_float2(pair[0], pair[1]);
+        }
     const float* gz = gate_row(a, tr.row0 + tr.token(r), head);
     const float2 z = gz ? make_float2(gz[d], gz[d + 1]) : make_float2(0.f, 0.f);
     if (threadIdx.x < 32) {
@@ -599,7 +605,9 @@ static int launch_rows_mma(const RowsArgs& a, const RowTiles& rt, int n_tiles, s
     if (rt.splits > 1) {
         // single tokens: the rows behind a token's heads are not there
         const int rows = rt.kind == 2 ? rt.block_rows : std::min(a.H / a.Hkv, kMmaHeads);
-        launch_kernel(attention_rows_merge_kernel, dim3(n_tiles, a.Hkv * rt.head_blocks, rows), dim3(a.vd / 2), 0, st, a, rt);
+        const bool pairs = reinterpret_cast<uintptr_t>(rt.workspace) % 8 == 0;
+        launch_kernel(pairs ? attention_rows_merge_kernel<true> : attention_rows_merge_kernel<false>, dim3(n_tiles, a.Hkv * rt.head_blocks, rows),
+                      dim3(a.vd / 2), 0, st, a, rt);
         return check_launch("attention_rows (merge)");
     }
     return 0;
