@@ -1306,10 +1306,11 @@ AHEAD_BYTES = 24 << 20
 def gemm_tc_takes_norm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool,
                        norm: Tuple[torch.Tensor, float, torch.Tensor], plan=None) -> bool:
     """Whether gemm_tc's kernel that adds up the ranges of K takes the norm of the rows too: many tokens, K in ranges, rows that a
-    block holds in registers."""
+    block holds in registers, in pieces of 16 bytes."""
     (M, K), N = a.shape, w.shape[0]
     if not accumulate or plan is not None or N % 8 or N > 4096 or out.shape != (M, N) or out.dtype is not torch.float32 or \
-            norm[2].shape != (M, N) or norm[2].dtype is not torch.bfloat16 or norm[0].numel() != N:
+            norm[2].shape != (M, N) or norm[2].dtype is not torch.bfloat16 or norm[0].numel() != N or \
+            norm[0].data_ptr() % 16 or norm[2].data_ptr() % 16:
         return False
     swap, block_q, splits = gemm_tc_plan(M, N, K, True)
     return not swap and block_q >= 128 and splits > 1 and splits * ((M + 255) // 256 * 256) * N <= _tc_state(a.device).workspace.numel()

@@ -440,6 +440,24 @@ def test_a_failed_wait_ends_every_call_that_was_under_way():
     assert K().gemm_tc_status(device) == 0 and sampler.sample(logits, [SamplingParams(0.0)], [0.0]) == [7]
 
 
+@pytest.mark.parametrize("weight_at, xn_at", [(1, 0), (2, 0), (0, 1), (0, 2)])
+def test_gemm_takes_norms_of_pieces_of_buffers(weight_at, xn_at):
+    """Weights and outputs of the norm that do not start on 16 bytes: the norm's own kernel."""
+    M, N, K_ = 140, 256, 4096
+    g = torch.Generator().manual_seed(M)
+    a, w = torch.randn(M, K_, generator=g).bfloat16().to(DEV), torch.randn(N, K_, generator=g).bfloat16().to(DEV)
+    weight = torch.randn(N + 4, generator=g).to(DEV)[weight_at:weight_at + N]
+    one = torch.zeros(M, N, device=DEV)
+    two = one.clone()
+    want = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    xn = torch.full((M * N + 4,), float("nan"), dtype=torch.bfloat16, device=DEV)[xn_at:xn_at + M * N].view(M, N)
+    K().gemm_tc(a, w, one, accumulate=True)
+    K().rmsnorm(one, weight, want, 1e-5)
+    K().gemm_tc(a, w, two, accumulate=True, norm=(weight, 1e-5, xn))
+    assert torch.equal(one, two)
+    close(xn, want.float().cpu(), "bfloat16", "norm", bf16_tol=1e-2)
+
+
 def _writes_word_later(code, device):
     """Launches, behind some 25 ms, a kernel that stores ``code`` in the status word: the place of a row's largest value, written where
     its id would go."""
