@@ -227,18 +227,21 @@ int gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int 
     if (M <= 32) return launch<Tile32>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, w_constant, st);
     // More rows: blocks of 8 x 5 .. 8 rows, the height whose rounds over the SMs (two blocks each) are the least work: a block that is
     // half outside the matrix, or a last round that is nearly empty, costs as much as a full one. A block's time goes with its
-    // rows and half a row's worth of reading columns. (268 rows,
-    // blocks of 64 -> the height taken: 16,384 outputs of 2,048 inputs 495 -> 455 us in blocks of 56; 2,048 of 2,048 and 8,192 together
-    // 189 -> 171 each and 3,072 of 2,048 122 -> 112 in blocks of 48.)
+    // rows and a row's worth of the rest; a last round of a block an SM takes 0.7 of one of two; clusters of four and eight leave
+    // places that no further one fits; and another height has to promise 4 %, as the promise is that rough. Of 551 products of 33 to 2,048
+    // rows (100 to 128,256 outputs of 36 to 14,336 inputs) the height taken is 1.2 % slower than the best (blocks of 64: 20 %), and two
+    // are more than 3 % slower than blocks of 64 (by 5 at most). (268 rows, blocks of 64 -> the height taken: 16,384 outputs of
+    // 2,048 inputs 495 -> 455 us in blocks of 56; 2,048 of 2,048 and 8,192 together 189 -> 171 each and 3,072 of 2,048 122 -> 112 in blocks of 48.)
     int best = 8;
     long long least = -1;
-    const int at_once = 2 * sm_count();
+    const int at_once = 2 * sm_count() - (chunks > 2 ? 12 : 0);
     for (int tm = 8; tm >= 5; --tm) {
         const int rows = (M + 8 * tm - 1) / (8 * tm);
         if (rows > 65535) break;                           // the grid's limit
         const long long blocks = static_cast<long long>(chunks) * ((N + 127) / 128) * rows;
-        const long long cost = (blocks + at_once - 1) / at_once * (2 * tm + 1);
-        if (least < 0 || cost < least) { least = cost; best = tm; }
+        const long long left = blocks % at_once;
+        const long long cost = (blocks / at_once * 10 + (left == 0 ? 0 : 2 * left <= at_once ? 7 : 10)) * (tm + 1);
+        if (least < 0 || (best == 8 ? cost * 100 < least * 96 : cost < least)) { least = cost; best = tm; }
     }
     if (best == 5) return launch<Tile40>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, w_constant, st);
     if (best == 6) return launch<Tile48>(A, W, C, M, N, K, lda, ldw, ldc, chunks, kc, accumulate, w_constant, st);
