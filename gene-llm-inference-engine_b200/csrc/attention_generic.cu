@@ -82,10 +82,10 @@ __device__ __forceinline__ float dot_row(const float* __restrict__ q, const __nv
     return acc;
 }
 
-// DPL: dimensions per lane (hd <= 32 DPL). FEW: a few blocks an SM, each with as much in flight as its registers hold; else many blocks,
+// DPL: dimensions per lane (hd <= 32 DPL). BLOCKS: that an SM holds. 2: each with as much in flight as its registers hold; 8 or 10: many blocks,
 // which hide one another's waits if there is room for them.
-template <typename T, int DPL, bool FEW>
-__global__ void __launch_bounds__(kAttWarps * 32, FEW ? 2 : 8)
+template <typename T, int DPL, int BLOCKS>
+__global__ void __launch_bounds__(kAttWarps * 32, BLOCKS)
 paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_cache,
                                const T* __restrict__ v_cache, T* __restrict__ out,
                                const int* __restrict__ row_req, const int* __restrict__ positions,
@@ -108,6 +108,7 @@ paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_
         s_q[d] = to_float(q[(static_cast<size_t>(t) * H + h) * hd + d]);
     __syncthreads();
 
+    constexpr bool FEW = BLOCKS == 2;
     constexpr int kPieces = FEW ? 16 : 4;
     constexpr int kBatch = (FEW ? 32 : 8) / DPL;         // keys whose values are in flight together
     float acc[DPL];
@@ -223,13 +224,22 @@ static int gi_attention_generic_impl(const void* q, const void* k_cache, const v
             static_cast<T*>(out), row_req, positions, block_tables, table_stride, H, Hkv, hd, page_size, scale,
             window, sink, gate, gate_ld, gate_off, gate_dims, out_scale);
     };
-    // up to two blocks an SM are few (268 rows with everything in flight, three blocks of 165 registers an SM: 105 us instead of 60)
-    const bool few = static_cast<long long>(H) * T <= 2 * sm_count();
+    // up to two blocks an SM are few (268 rows with everything in flight, three blocks of 165 registers an SM: 105 us instead of 60); ten
+    // instead of eight where that saves enough rounds over the SMs (40 rows of 32 heads of 64, 1,000 positions, 32-bit: 272 us in two rounds
+    // of eight, 175 in one of ten; 37 rows, one round either way, are faster with eight)
+    const long long blocks = static_cast<long long>(H) * T, sms = sm_count();
+    const bool few = blocks <= 2 * sms, ten = (blocks + 8 * sms - 1) / (8 * sms) * 3 > (blocks + 10 * sms - 1) / (10 * sms) * 4;
     auto typed = [&](auto* t) {
         using V = std::remove_pointer_t<decltype(t)>;
-        if (hd <= 64) few ? launch(paged_attention_generic_kernel<V, 2, true>, t) : launch(paged_attention_generic_kernel<V, 2, false>, t);
-        else if (hd <= 128) few ? launch(paged_attention_generic_kernel<V, 4, true>, t) : launch(paged_attention_generic_kernel<V, 4, false>, t);
-        else few ? launch(paged_attention_generic_kernel<V, 8, true>, t) : launch(paged_attention_generic_kernel<V, 8, false>, t);
+        auto of = [&](auto lanes) {
+            constexpr int DPL = decltype(lanes)::value;
+            if (few) launch(paged_attention_generic_kernel<V, DPL, 2>, t);
+            else if (ten) launch(paged_attention_generic_kernel<V, DPL, 10>, t);
+            else launch(paged_attention_generic_kernel<V, DPL, 8>, t);
+        };
+        if (hd <= 64) of(std::integral_constant<int, 2>{});
+        else if (hd <= 128) of(std::integral_constant<int, 4>{});
+        else of(std::integral_constant<int, 8>{});
     };
     if (dtype == kF32) {
         typed(static_cast<float*>(nullptr));
