@@ -98,9 +98,9 @@ constexpr int kSampleParts = 8, kBins = 1024, kDigit = 10;
 constexpr int kMassBits = 12;                  // a mantissa goes into two words of 12 bits: slices of up to 2^20 values cannot overflow them
 constexpr int kNarrowVocab = kSampleParts << 20;      // above: whole mantissas in 64-bit words (whose atomics are slower)
 
-// A warp's piece stays in registers, kHeld values a lane, where it fits (vocabularies of up to 131,072): read once instead of
+// A warp's piece stays in registers, up to 16 values a lane, where it fits (vocabularies of up to 131,072): read once instead of
 // in every pass, each a wait for L2 (six rows of 128,256, drawn with every kind of filter: 92 -> 62 us).
-constexpr int kHeld = 16;
+constexpr int kHeldMost = 16, kHeldFew = 4;       // (vocabularies of up to 32,768: places without a value cost time, too: forty rows of 1,000 31.2 -> 24.7 us)
 
 template <bool kWide> struct SampleShared {
     using Low = typename std::conditional<kWide, unsigned long long, unsigned>::type;
@@ -251,8 +251,8 @@ __device__ __forceinline__ int sample_count_to(double above, double w, int n, do
 }
 
 // probs: scratch [rows, V] floats.
-// kInRegs: every warp's piece fits kHeld values a lane, and probs is not used.
-template <bool kWide, bool kInRegs>
+// kHeld > 0: every warp's piece fits kHeld values a lane, and probs is not used.
+template <bool kWide, int kHeld>
 __global__ void __cluster_dims__(kSampleParts, 1, 1) __launch_bounds__(kSampleThreads)
 sample_kernel(const float* __restrict__ logits, float* __restrict__ probs_all, int V,
               const float* __restrict__ temperature, const int* __restrict__ top_k,
@@ -272,6 +272,7 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ probs_all, i
     const int slice_begin = min(V, part * slice), slice_end = min(V, slice_begin + slice);
     const int begin = min(slice_end, slice_begin + warp * piece), end = min(slice_end, begin + piece);
 
+    constexpr bool kInRegs = kHeld > 0;
     float held[kInRegs ? kHeld : 1];
     // every place of this lane and its value, in order
     auto each = [&](auto f) {
@@ -481,9 +482,10 @@ int launch_sample(const float* logits, float* probs, int rows, int V, const floa
                   const float* uniform, int* out, cudaStream_t st) {
     GI_REQUIRE(rows <= INT_MAX / kSampleParts, "sample: %d rows exceed the grid limit", rows);
     const dim3 grid(rows * kSampleParts), block(kSampleThreads);
-    if (V <= kSampleParts * kSampleThreads * kHeld) launch_kernel((sample_kernel<false, true>), grid, block, 0, st, logits, probs, V, temperature, top_k, top_p, uniform, out);
-    else if (V <= kNarrowVocab) launch_kernel((sample_kernel<false, false>), grid, block, 0, st, logits, probs, V, temperature, top_k, top_p, uniform, out);
-    else launch_kernel((sample_kernel<true, false>), grid, block, 0, st, logits, probs, V, temperature, top_k, top_p, uniform, out);
+    if (V <= kSampleParts * kSampleThreads * kHeldFew) launch_kernel((sample_kernel<false, kHeldFew>), grid, block, 0, st, logits, probs, V, temperature, top_k, top_p, uniform, out);
+    else if (V <= kSampleParts * kSampleThreads * kHeldMost) launch_kernel((sample_kernel<false, kHeldMost>), grid, block, 0, st, logits, probs, V, temperature, top_k, top_p, uniform, out);
+    else if (V <= kNarrowVocab) launch_kernel((sample_kernel<false, 0>), grid, block, 0, st, logits, probs, V, temperature, top_k, top_p, uniform, out);
+    else launch_kernel((sample_kernel<true, 0>), grid, block, 0, st, logits, probs, V, temperature, top_k, top_p, uniform, out);
     return check_launch("sample");
 }
 
