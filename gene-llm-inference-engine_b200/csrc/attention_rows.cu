@@ -537,9 +537,9 @@ attention_rows_mma_kernel(const RowsArgs a, const RowTiles rt) {
 // pair of value dimensions. A few KB a block, so it is as long as its loads wait for one another: a thread asks for its
 // pair of every range before the ranges' weights are worked out (a token's step, latents of 512 values: 16 heads of eight tokens and five
 // ranges 8.1 -> 4.3 us, of two tokens and fifteen ranges 14.7 -> 3.8; before, a thread had a value and four ranges in flight).
-// PAIRS: the workspace starts on 8 bytes, so that a pair is one load.
+// PAIRS: the workspace starts on 8 bytes, so that a pair is one load. MOST: ranges that there are at most.
 constexpr int kRowsMaxSplits = 32;        // a lane each
-template <bool PAIRS>
+template <bool PAIRS, int MOST>
 __global__ void __launch_bounds__(kRowsMaxValueThreads)
 attention_rows_merge_kernel(const RowsArgs a, const RowTiles rt) {
     pdl_prologue();
@@ -558,9 +558,9 @@ attention_rows_merge_kernel(const RowsArgs a, const RowTiles rt) {
                        static_cast<size_t>(r) * (a.vd + 2);
     const int head = g * group + first_head + tr.head(r);
     const int d = 2 * threadIdx.x;                    // (vd is a multiple of 64: rows of vd + 2 values start on 8 bytes if the workspace does)
-    float2 part[kRowsMaxSplits];
+    float2 part[MOST];
 #pragma unroll
-    for (int s = 0; s < kRowsMaxSplits; ++s)
+    for (int s = 0; s < MOST; ++s)
         if (s < rt.splits) {
             const float* pair = row + s * stride + d;
             if (PAIRS) part[s] = *reinterpret_cast<const float2*>(pair);
@@ -584,7 +584,7 @@ attention_rows_merge_kernel(const RowsArgs a, const RowTiles rt) {
     __syncthreads();
     float2 v = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int s = 0; s < kRowsMaxSplits; ++s)
+    for (int s = 0; s < MOST; ++s)
         if (s < rt.splits) { v.x = fmaf(part[s].x, s_w[s], v.x); v.y = fmaf(part[s].y, s_w[s], v.y); }
     v.x *= s_inv; v.y *= s_inv;
     if (gz) { v.x *= sigmoid_f(z.x); v.y *= sigmoid_f(z.y); }
@@ -606,7 +606,9 @@ static int launch_rows_mma(const RowsArgs& a, const RowTiles& rt, int n_tiles, s
         // single tokens: the rows behind a token's heads are not there
         const int rows = rt.kind == 2 ? rt.block_rows : std::min(a.H / a.Hkv, kMmaHeads);
         const bool pairs = reinterpret_cast<uintptr_t>(rt.workspace) % 8 == 0;
-        launch_kernel(pairs ? attention_rows_merge_kernel<true> : attention_rows_merge_kernel<false>, dim3(n_tiles, a.Hkv * rt.head_blocks, rows),
+        auto merge = !pairs ? attention_rows_merge_kernel<false, kRowsMaxSplits> : rt.splits <= 4 ? attention_rows_merge_kernel<true, 4>
+                                                                                                : attention_rows_merge_kernel<true, kRowsMaxSplits>;
+        launch_kernel(merge, dim3(n_tiles, a.Hkv * rt.head_blocks, rows),
                       dim3(a.vd / 2), 0, st, a, rt);
         return check_launch("attention_rows (merge)");
     }

@@ -532,8 +532,9 @@ _ROWS_BLOCKS = 296          # about two blocks an SM: what the ranges of keys of
 
 def _rows_blocks(value_dim: Optional[int]) -> int:
     """Four blocks an SM where values are narrow: the blocks wait for their chains of loads and products, not for one another (eight tokens
-    of eight key/value heads of 64, 310 positions: 20.2 -> 13.0 us, the merge 3.0 -> 4.6). Wide ones keep their workspace below 42 MB."""
-    return 2 * _ROWS_BLOCKS if value_dim is not None and value_dim <= 128 else _ROWS_BLOCKS
+    of eight key/value heads of 64, 310 positions: 20.2 -> 13.0 us, the merge 3.0 -> 4.6). Of wider ones an SM holds fewer at a time (values of 128, eight tokens of four
+    key/value heads, 1,024 positions, with the merge: 38.2 us, 29.3 with half as many), and their workspace stays below 42 MB."""
+    return 2 * _ROWS_BLOCKS if value_dim is not None and value_dim <= 64 else _ROWS_BLOCKS
 
 
 def attention_rows_splits(n_tiles: int, num_heads: int, num_kv_heads: int, span: int, value_dim: Optional[int] = None) -> int:
