@@ -40,7 +40,7 @@ struct GroupedArgs {
     const void* a; long long lda; int a_off; int a_gs; int a_div;
     const void* w; long long w_gs; int ldw; long long up_off;     // W[g] = w + g * w_gs, rows of ldw; the up rows start at up_off
     void* out; int out_is_f32; long long ldo; int o_off; int o_gs;
-    int N, K, rows, groups;                                       // rows: the pairs in the experts form
+    int N, K, rows, groups;                                       // experts form: the pairs and the experts
     const int* tile_group; const int* sorted_rows; const int* n_tiles;   // experts form (else null)
     int w_constant;                                               // no kernel that may still be running writes w: it may be read before the wait
     int act; float act_limit;                                     // gated: a GateAct code and its limit
@@ -173,8 +173,8 @@ grouped_product_kernel(const GroupedArgs p) {
     }
 }
 
-// The same products for few rows (decoding) of 32-bit inputs, with 32-bit weights or, a few pairs, bfloat16 ones: the weights are what
-// takes the time. A warp streams four or eight output rows of a group's matrix (gated: and their up rows) through a ring in shared memory, 512 bytes of each a step, by asynchronous copies
+// The same products for few rows (decoding), with 32-bit weights or, very few rows (few_on_cuda_cores), bfloat16 ones: the weights are
+// what takes the time. A warp streams four or eight output rows of a group's matrix (gated: and their up rows) through a ring in shared memory, 512 bytes of each a step, by asynchronous copies
 // of 16 bytes; every lane copies exactly the pieces that it multiplies itself, so the ring needs no barrier, and 48 KB or more
 // are in flight per block whatever the warps are doing. Each step's pieces are multiplied with up to eight rows of the tile, read
 // through the cache; more rows stream the weights again, from L2. An output element is the sum of its lanes' partial sums (lane l takes
@@ -220,10 +220,9 @@ __device__ __forceinline__ float4 piece4(const float* p) { return *reinterpret_c
 __device__ __forceinline__ float4 piece4(const __nv_bfloat16* p) { return load4<__nv_bfloat16>(p); }
 
 // The few-row form's units of work, taken by the grid's warps in turn: (tile, four or eight output rows), and for a tile of more than
-// kGrFew rows a second pass over the same weights. A warp's ring runs on from unit to unit. 32-bit inputs.
-// ROWS: output rows of a unit: 4 of 32-bit weights; 8 of bfloat16 weights, whose few pairs' inputs are as many bytes as four rows
-// of weights for every two of them.
-template <typename TW, bool GATED, int ROWS>
+// kGrFew rows a second pass over the same weights. A warp's ring runs on from unit to unit.
+// ROWS: output rows of a unit, 4 or, not gated, 8.
+template <typename TA, typename TW, bool GATED, int ROWS>
 struct RowsStream {
     static constexpr int kPiece = 16 / sizeof(TW);       // values per step of a lane: the weights' 16 bytes
     static constexpr int kW = GATED ? 2 * ROWS : ROWS;   // rows of weights that it streams (gated: and the up rows)
@@ -276,14 +275,14 @@ struct RowsStream {
 // MR rows of a tile (m_here of them are real, the last is repeated) against the output rows from n_first on. ``row``:
 // lane i has the tile's i-th row; ``done``: steps of the warp's ring taken so far. With 8 output rows up to two rows' inputs are
 // asked for a step ahead.
-template <int MR, typename TW, bool GATED, int ROWS>
-__device__ __forceinline__ void grouped_rows_unit(RowsStream<TW, GATED, ROWS>& q, int g, int row, int n_first, int m0, int m_here, int& done) {
+template <int MR, typename TA, typename TW, bool GATED, int ROWS>
+__device__ __forceinline__ void grouped_rows_unit(RowsStream<TA, TW, GATED, ROWS>& q, int g, int row, int n_first, int m0, int m_here, int& done) {
     const GroupedArgs& p = q.p;
-    using Stream = RowsStream<TW, GATED, ROWS>;
+    using Stream = RowsStream<TA, TW, GATED, ROWS>;
     constexpr int kW = Stream::kW, kStages = Stream::kStages, kPiece = Stream::kPiece;
     constexpr bool kAhead = ROWS == 8 && MR <= 2;
-    const float* A = static_cast<const float*>(p.a) + p.a_off + static_cast<size_t>(g) * p.a_gs;
-    const float* arow[MR];
+    const TA* A = static_cast<const TA*>(p.a) + p.a_off + static_cast<size_t>(g) * p.a_gs;
+    const TA* arow[MR];
 #pragma unroll
     for (int i = 0; i < MR; ++i) arow[i] = A + static_cast<size_t>(__shfl_sync(0xffffffffu, row, m0 + min(i, m_here - 1)) / p.a_div) * p.lda;
     // the output gate's values of the unit's outputs, (row of weights, row of the tile) by lane, asked for before the weights arrive
@@ -303,9 +302,9 @@ __device__ __forceinline__ void grouped_rows_unit(RowsStream<TW, GATED, ROWS>& q
 #pragma unroll
         for (int i = 0; i < MR; ++i) acc[r][i] = 0.f;
     float4 av[MR][kAhead ? kPiece / 4 : 1], next[kAhead ? MR : 1][kPiece / 4];
-    auto fetch = [&](float4 (&dst)[kPiece / 4], const float* src, int at) {
+    auto fetch = [&](float4 (&dst)[kPiece / 4], const TA* src, int at) {
 #pragma unroll
-        for (int h = 0; h < kPiece / 4; ++h) dst[h] = *reinterpret_cast<const float4*>(src + at * kPiece + 4 * h);
+        for (int h = 0; h < kPiece / 4; ++h) dst[h] = load4<TA>(src + at * kPiece + 4 * h);
     };
     if constexpr (kAhead) {
         if (q.lane < q.pieces)
@@ -326,7 +325,7 @@ __device__ __forceinline__ void grouped_rows_unit(RowsStream<TW, GATED, ROWS>& q
             for (int h = 0; h < kPiece / 4; ++h) {
                 if constexpr (!kAhead) {
 #pragma unroll
-                    for (int i = 0; i < MR; ++i) av[i][0] = *reinterpret_cast<const float4*>(arow[i] + c * kPiece + 4 * h);
+                    for (int i = 0; i < MR; ++i) av[i][0] = load4<TA>(arow[i] + c * kPiece + 4 * h);
                 }
 #pragma unroll
                 for (int r = 0; r < kW; ++r) {
@@ -371,12 +370,12 @@ __device__ __forceinline__ void grouped_rows_unit(RowsStream<TW, GATED, ROWS>& q
 }
 
 // tiles: how many there are (experts form: at most; the number is read on the device)
-template <typename TW, bool GATED, int ROWS>
-__global__ void __launch_bounds__(kGrWarps * 32, (RowsStream<TW, GATED, ROWS>::kBlocks))
+template <typename TA, typename TW, bool GATED, int ROWS>
+__global__ void __launch_bounds__(kGrWarps * 32, (RowsStream<TA, TW, GATED, ROWS>::kBlocks))
 grouped_rows_kernel(const GroupedArgs p, int tiles) {
     extern __shared__ uint4 s_ring[];
     pdl_prologue();
-    using Stream = RowsStream<TW, GATED, ROWS>;
+    using Stream = RowsStream<TA, TW, GATED, ROWS>;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     Stream q{p};
     q.ring = s_ring + warp * (Stream::kStages * Stream::kW * 32) + lane;
@@ -1188,16 +1187,16 @@ static bool rows_form_fits(const GroupedArgs& p, int a_dtype, int w_dtype) {
     return p.lda % a_piece == 0 && p.a_off % a_piece == 0 && p.a_gs % a_piece == 0;
 }
 
-template <typename TW, bool GATED, int ROWS>
+template <typename TA, typename TW, bool GATED, int ROWS>
 static int launch_grouped_rows_as(const GroupedArgs& p, unsigned tiles, cudaStream_t st) {
-    using Stream = RowsStream<TW, GATED, ROWS>;
+    using Stream = RowsStream<TA, TW, GATED, ROWS>;
     static SharedLimit limit;
-    const cudaError_t ready = limit.allow(reinterpret_cast<const void*>(grouped_rows_kernel<TW, GATED, ROWS>), Stream::kSmem);
+    const cudaError_t ready = limit.allow(reinterpret_cast<const void*>(grouped_rows_kernel<TA, TW, GATED, ROWS>), Stream::kSmem);
     if (ready != cudaSuccess) { set_error("grouped_product (rows): %s", cudaGetErrorString(ready)); return 1; }
     const int sms = sm_count();
     const long long blocks = (static_cast<long long>(tiles) * ((p.N + ROWS - 1) / ROWS) + kGrWarps - 1) / kGrWarps;
     GI_REQUIRE(blocks * kGrWarps <= 2147483647LL - 3 * 1024 * kGrWarps, "grouped_product: too many tiles");
-    launch_kernel((grouped_rows_kernel<TW, GATED, ROWS>), dim3(static_cast<unsigned>(std::min<long long>(blocks, Stream::kBlocks * sms))), dim3(kGrWarps * 32),
+    launch_kernel((grouped_rows_kernel<TA, TW, GATED, ROWS>), dim3(static_cast<unsigned>(std::min<long long>(blocks, Stream::kBlocks * sms))), dim3(kGrWarps * 32),
                   Stream::kSmem, st, p, static_cast<int>(tiles));
     return check_launch("grouped_product (rows)");
 }
@@ -1213,18 +1212,34 @@ static int launch_grouped_mma(const GroupedArgs& p, unsigned tiles, cudaStream_t
     launch_kernel((grouped_mma_kernel<TA, GATED>), dim3(static_cast<unsigned>(std::min<long long>(units, kGmBlocks * sms))), dim3(kGmWarps * 32), kSmem, st, p, static_cast<int>(tiles));
     return check_launch("grouped_product (few rows)");
 }
+// Where few rows of bfloat16 weights are multiplied on the CUDA cores: the time there goes with the rows of the fullest tile, on the tensor
+// cores with the tiles and the outputs (a tile's first row costs as much as eight), more with 32-bit inputs, which are cut into parts.
+static bool few_on_cuda_cores(const GroupedArgs& p, bool a_is_f32) {
+    // Heads: us on the CUDA cores / on the tensor cores, 32-bit inputs, 16 of 64 x 512: one row 3.7 / 5.5, four 4.8 / 5.6, six 5.9 / 5.5; 128
+    // of 128 x 512: one 9.7 / 28.2, eight 20.5 / 28.7, twelve 29.9 / 28.8. bfloat16 inputs: one 3.6 / 4.1 and 9.5 / 17.8, three 4.3 / 4.1 and 12.4 / 17.9.
+    if (!p.tile_group) return p.rows <= (p.groups >= 64 ? (a_is_f32 ? 10 : 5) : (a_is_f32 ? 5 : 2));
+    // Experts: p.rows pairs of p.groups experts. Most have a tile of their own while they are fewer than the experts, or two an expert of
+    // up to four or of very many. Weights from memory, 32-bit inputs: six pairs of eight experts, 2,048 outputs of 4,096 inputs 32.3 / 32.3,
+    // 4,608 of 2,048 29.2 / 40.6; eight 33.8 / 41.5 on eight of them and 19.6 / 16.0 on two (in a token's step 32.5 / 31.4); 16 of 32, 768 of 2,048
+    // 18.2 / 23.4, 32 22.8 / 28.1, 64 39.9 / 30.7; 128 of 64, 512 of 1,024 26.9 / 27.1; 2, 2, 2, 2 of four 18.5 / 26.6, 3, 3 of two 18.7 / 15.3, four of one 18.5 / 13.8.
+    // bfloat16 inputs, which need no cutting, only where K is short, so that a unit's work is little beside its beginning and end: 16 of
+    // 64, gated, 2 x 1,024 of 512 15.6 / 20.1, 32 of 128, 256 of 512 6.8 / 8.1; of 2,048 inputs 12 of 32 21.8 / 19.9.
+    const int experts = p.groups;
+    if (a_is_f32) return experts <= 4 || experts >= 64 ? p.rows <= 2 * experts : experts >= 16 ? p.rows <= experts : 4 * p.rows <= 3 * experts;
+    return p.rows >= 6 && p.rows <= experts && p.K <= 1024;
+}
 template <bool GATED>
 static int launch_grouped_rows(const GroupedArgs& p, int a_dtype, int w_dtype, unsigned tiles, cudaStream_t st) {
-    if (w_dtype == kF32) return launch_grouped_rows_as<float, GATED, 4>(p, tiles, st);
-    // 32-bit inputs of a few pairs, about two for each expert that there is (room for tiles: one and an expert's each): the multiply-adds
-    // are few, and cutting eight rows' inputs into parts costs more than they do. The time on the CUDA cores goes with the rows of the
-    // fullest tile, on the tensor cores with the tiles, and jumps at the third. Measured, 2,048 outputs of 4,096 inputs, us on the CUDA cores /
-    // on the tensor cores, pairs of each expert: 1,1 13.5 / 15.0; 2,2 14.8 / 15.2; 2,2,2 16.9 / 25.9; 2,2,2,2 18.5 / 26.6; 1,1,1,1 of eight experts
-    // 17.7 / 24.8; but 4 18.5 / 13.8; 3,3 18.7 / 15.3; 5,1,1,1 28.4 / 26.7; 6,5,5 28.1 / 26.8; 10,4,1,1 45.2 / 27.5; five experts of one pair
-    // 29.0 / 28.9.
-    if constexpr (!GATED)
-        if (a_dtype == kF32 && p.tile_group && tiles <= 5 && p.rows <= 2 * (static_cast<int>(tiles) - 1)) return launch_grouped_rows_as<__nv_bfloat16, false, 8>(p, tiles, st);
-    return a_dtype == kF32 ? launch_grouped_mma<float, GATED>(p, tiles, st) : launch_grouped_mma<__nv_bfloat16, GATED>(p, tiles, st);
+    if (w_dtype == kF32) return launch_grouped_rows_as<float, float, GATED, 4>(p, tiles, st);
+    const bool f32 = a_dtype == kF32;
+    if (few_on_cuda_cores(p, f32)) {
+        // eight rows a unit for 32-bit inputs, as many bytes as four rows of weights for every two; heads' matrices and gated
+        // ones are too small, or need too many registers, for that
+        if constexpr (!GATED)
+            if (f32 && p.tile_group) return launch_grouped_rows_as<float, __nv_bfloat16, false, 8>(p, tiles, st);
+        return f32 ? launch_grouped_rows_as<float, __nv_bfloat16, GATED, 4>(p, tiles, st) : launch_grouped_rows_as<__nv_bfloat16, __nv_bfloat16, GATED, 4>(p, tiles, st);
+    }
+    return f32 ? launch_grouped_mma<float, GATED>(p, tiles, st) : launch_grouped_mma<__nv_bfloat16, GATED>(p, tiles, st);
 }
 
 template <bool GATED>
@@ -1302,7 +1317,7 @@ static int gi_head_product_impl(const void* a, int a_dtype, long long lda, int a
 static int gi_expert_product_impl(const void* a, int a_dtype, long long lda, int a_div, const void* w, int w_dtype, long long w_gs,
                                   int ldw, long long up_off, int gated, int act, float act_limit, const float* scales, void* out, int out_dtype, long long ldo,
                                   int N, int K, const int* tile_group, const int* sorted_rows, const int* n_tiles, int max_tiles,
-                                  int pairs, void* stream) {
+                                  int pairs, int experts, void* stream) {
     if (max_tiles == 0) return 0;
     GI_REQUIRE(max_tiles > 0 && N > 0 && K > 0 && a_div > 0, "expert_product: sizes must be positive");
     GI_REQUIRE(tile_group && sorted_rows && n_tiles, "expert_product: the sorted rows are missing");
@@ -1311,7 +1326,7 @@ static int gi_expert_product_impl(const void* a, int a_dtype, long long lda, int
     p.a = a; p.lda = lda; p.a_div = a_div;
     p.w = w; p.w_gs = w_gs; p.ldw = ldw; p.up_off = up_off;
     p.out = out; p.out_is_f32 = out_dtype == kF32; p.ldo = ldo;
-    p.N = N; p.K = K; p.groups = 1; p.rows = pairs;
+    p.N = N; p.K = K; p.groups = experts; p.rows = pairs;
     p.tile_group = tile_group; p.sorted_rows = sorted_rows; p.n_tiles = n_tiles; p.act = gated ? act : 0; p.act_limit = act_limit;
     p.out_act = gated ? kPlainNone : act;
     p.scales = scales;
@@ -1439,9 +1454,9 @@ extern "C" int gi_head_product(const void* a, int a_dtype, long long lda, int a_
 
 extern "C" int gi_expert_product(const void* a, int a_dtype, long long lda, int a_div, const void* w, int w_dtype, long long w_gs,
                                  int ldw, long long up_off, int gated, int act, float act_limit, const float* scales, void* out, int out_dtype, long long ldo, int N, int K,
-                                 const int* tile_group, const int* sorted_rows, const int* n_tiles, int max_tiles, int pairs, void* stream) {
+                                 const int* tile_group, const int* sorted_rows, const int* n_tiles, int max_tiles, int pairs, int experts, void* stream) {
     return gi::dispatch(gi_expert_product_impl, a, a_dtype, lda, a_div, w, w_dtype, w_gs, ldw, up_off, gated, act, act_limit, scales, out, out_dtype, ldo,
-                        N, K, tile_group, sorted_rows, n_tiles, max_tiles, pairs, stream);
+                        N, K, tile_group, sorted_rows, n_tiles, max_tiles, pairs, experts, stream);
 }
 
 extern "C" int gi_route(const void* x, int x_dtype, int T, int D, const float* w, const float* correction, int E, int top,

@@ -799,7 +799,7 @@ def expert_product(a: torch.Tensor, a_div: int, w: torch.Tensor, out: torch.Tens
                                   ACTIVATIONS[gated] if gated else PLAIN_ACTIVATIONS[act or "none"], float(limit),
                                   _opt(scales, "scales", torch.float32), _dev(out, "out"), dtype_code(out.dtype), N, N, K, _dev(tile_group, "tile_group", torch.int32),
                                   _dev(sorted_rows, "sorted_rows", torch.int32), _dev(n_tiles, "n_tiles", torch.int32),
-                                  tile_group.numel(), out.shape[0], _stream()), "expert_product")
+                                  tile_group.numel(), out.shape[0], E, _stream()), "expert_product")
 
 
 def route_combine(part: torch.Tensor, weights: Optional[torch.Tensor], y: torch.Tensor, pair_row: Optional[torch.Tensor] = None,

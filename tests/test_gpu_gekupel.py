@@ -500,7 +500,7 @@ def test_expert_products_of_few_rows(dtype, N, K, gated):
     _close(out.cpu(), want, torch.float32, "few rows", f32=1e-5)
 
 
-@pytest.mark.parametrize("form", ["experts", "experts, room for five tiles", "experts, eight pairs, room for five tiles", "gated experts", "heads, 9 rows", "heads, 33 rows", "heads, 70 rows", "heads with a tail, 12 rows"])
+@pytest.mark.parametrize("form", ["experts", "experts, room for five tiles", "few pairs of sixteen experts", "gated experts", "heads, 9 rows", "heads, 33 rows", "heads, 70 rows", "heads with a tail, 12 rows"])
 @pytest.mark.parametrize("N, K", [(16, 264), (70, 40)])
 def test_products_of_32_bit_inputs_with_bfloat16_weights(form, N, K):
     """Inputs all of whose bits count, of any size, infinite or none. The parts that an input is cut into add up to it, so what is left are
@@ -509,7 +509,7 @@ def test_products_of_32_bit_inputs_with_bfloat16_weights(form, N, K):
     from geneinfer_b200.ops import kernels
     g = torch.Generator().manual_seed(K)
     heads = form.startswith("heads")
-    T = int(form.split(", ")[1].split()[0]) if heads else 8 if "eight" in form else 9
+    T = int(form.split(", ")[1].split()[0]) if heads else 9
     G, tail = (3, 8 if "tail" in form else 0) if heads else (1, 0)
     gated = form == "gated experts"
     x, w = torch.randn(T, G, K, generator=g), _bf(torch.randn(G, (2 if gated else 1) * N, K, generator=g))
@@ -525,7 +525,8 @@ def test_products_of_32_bit_inputs_with_bfloat16_weights(form, N, K):
         room = 5 if "room" in form else 6
         rows = torch.full((room * kernels.grouped_tile_rows(),), -1, dtype=torch.int32)
         rows[:T] = torch.arange(T, dtype=torch.int32)
-        kernels.expert_product(x[:, 0].contiguous().to(DEV), 1, w.to(DEV).bfloat16(), out, rows.to(DEV), torch.zeros(room, dtype=torch.int32, device=DEV),
+        experts = w.to(DEV).bfloat16().repeat(16 if "sixteen" in form else 1, 1, 1)
+        kernels.expert_product(x[:, 0].contiguous().to(DEV), 1, experts, out, rows.to(DEV), torch.zeros(room, dtype=torch.int32, device=DEV),
                                torch.ones(1, dtype=torch.int32, device=DEV), gated="relu" if gated else None)
     got = out.cpu().view(T, G, N + tail)[..., :N].double()
     want = torch.einsum("tgk,gnk->tgn", x.double(), w.double())
@@ -541,7 +542,43 @@ def test_products_of_32_bit_inputs_with_bfloat16_weights(form, N, K):
     assert bool(((got - want).abs() <= bound)[keep].all()), float(((got - want).abs() / bound)[keep].max())
 
 
-@pytest.mark.parametrize("form", ["experts", "experts, four pairs, room for five tiles", "gated experts", "heads, 9 rows", "heads, 33 rows", "heads, 70 rows", "heads with a tail, 12 rows"])
+@pytest.mark.parametrize("inputs", DTYPES)
+@pytest.mark.parametrize("N, K, gated", [(18, 8, None), (33, 264, None), (16, 1000, "silu"), (33, 264, "relu"), (70, 1024, None)])
+def test_products_of_fewer_rows_than_experts(inputs, N, K, gated):
+    """bfloat16 weights, pairs of six experts of sixteen in tiles of one to four rows, and heads of one to five rows and, many of them, to
+    ten: both sides of where the form changes. Bound: K products of values of about 1 and 0.1 in 32 bits."""
+    from geneinfer_b200.ops import kernels
+    g = torch.Generator().manual_seed(K + N)
+    E, tm = 16, kernels.grouped_tile_rows()
+    for counts in ([1], [2, 1], [1, 1, 1, 2, 1], [4, 3, 2, 1, 1, 1], [4, 4, 2, 1, 1, 1], [4, 4, 4, 2, 1, 1], [4, 4, 4, 3, 1, 1]):
+        T, n = sum(counts), len(counts)
+        a, w = _bf(torch.randn(T, K, generator=g)), _bf(torch.randn(E, (2 if gated else 1) * N, K, generator=g) * 0.1)
+        who = torch.randperm(E, generator=g)[:n].sort().values
+        rows = torch.full((T + 2, tm), -1, dtype=torch.int32)
+        for i, r in enumerate(torch.randperm(T, generator=g).to(torch.int32).split(counts)):
+            rows[i, torch.randperm(tm, generator=g)[:len(r)]] = r
+        groups = torch.zeros(T + 2, dtype=torch.int32)
+        groups[:n] = who.int()
+        out = torch.full((T, N), float("nan"), device=DEV)
+        kernels.expert_product(a.to(DEV).to(inputs), 1, w.to(DEV).bfloat16(), out, rows.view(-1).to(DEV), groups.to(DEV),
+                               torch.tensor([n], dtype=torch.int32, device=DEV), gated=gated)
+        want = torch.empty(T, N, dtype=torch.float64)
+        for i in range(n):
+            r = rows[i][rows[i] >= 0].long()
+            z = a[r].double() @ w[who[i]].double().T
+            act = torch.relu if gated == "relu" else torch.nn.functional.silu
+            want[r] = act(z[:, :N]) * z[:, N:] if gated else z
+        _close(out.cpu(), want, torch.float32, f"{counts}", f32=1e-5)
+    if not gated:
+        for H, T in ((3, 1), (3, 2), (3, 3), (3, 5), (3, 6), (64, 5), (64, 6), (64, 10), (64, 11)):
+            a, w = _bf(torch.randn(T, H * K, generator=g)), _bf(torch.randn(H, N, K, generator=g) * 0.1)
+            out = torch.full((T, H * N), float("nan"), device=DEV)
+            kernels.head_product(a.to(DEV).to(inputs), 0, K, w.to(DEV).bfloat16(), out, 0, N)
+            want = torch.einsum("thk,hnk->thn", a.view(T, H, K).double(), w.double()).reshape(T, -1)
+            _close(out.cpu(), want, torch.float32, f"{T} rows of {H} heads", f32=1e-5)
+
+
+@pytest.mark.parametrize("form", ["experts", "four pairs of sixteen experts", "gated experts", "heads, 9 rows", "heads, 33 rows", "heads, 70 rows", "heads with a tail, 12 rows"])
 @pytest.mark.parametrize("N, K", [(16, 264), (70, 40)])
 def test_infinite_weights_with_32_bit_inputs(form, N, K):
     """An infinite weight gives an infinity of the input's sign, none where the input is zero or another one is infinite the other
@@ -567,7 +604,8 @@ def test_infinite_weights_with_32_bit_inputs(form, N, K):
         room = 5 if "room" in form else 6
         rows = torch.full((room * kernels.grouped_tile_rows(),), -1, dtype=torch.int32)
         rows[:T] = torch.arange(T, dtype=torch.int32)
-        kernels.expert_product(x[:, 0].contiguous().to(DEV), 1, w.to(DEV).bfloat16(), out, rows.to(DEV), torch.zeros(room, dtype=torch.int32, device=DEV),
+        experts = w.to(DEV).bfloat16().repeat(16 if "sixteen" in form else 1, 1, 1)
+        kernels.expert_product(x[:, 0].contiguous().to(DEV), 1, experts, out, rows.to(DEV), torch.zeros(room, dtype=torch.int32, device=DEV),
                                torch.ones(1, dtype=torch.int32, device=DEV), gated="silu" if gated else None)
     got = out.cpu().view(T, G, N + tail)[..., :N].double()
     want = torch.einsum("tgk,gnk->tgn", x.double(), w.double())

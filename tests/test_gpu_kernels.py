@@ -300,7 +300,7 @@ def _attention_case(dtype, H, Hkv, hd, ps, ctx_lens, q_lens, window, seed, spike
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("H,Hkv,hd,ps", [(4, 2, 16, 16), (3, 1, 32, 8), (6, 3, 48, 16), (8, 2, 128, 32), (2, 1, 256, 16),
-                                          (5, 5, 80, 4), (8, 2, 256, 16), (4, 1, 128, 16), (12, 4, 64, 16)])
+                                          (5, 5, 80, 4), (8, 2, 256, 16), (4, 1, 128, 16), (12, 4, 64, 16), (24, 4, 64, 16), (24, 2, 128, 16), (24, 2, 256, 16)])
 def test_attention_mixed_rows(dtype, H, Hkv, hd, ps):
     # a whole prompt, a single decoded token deep in a context, a portion over page edges, position 0 alone
     got, want = _attention_case(dtype, H, Hkv, hd, ps, ctx_lens=[37, 130, 3 * ps + 1, 1], q_lens=[37, 1, ps + 2, 1],
@@ -558,7 +558,7 @@ def test_the_status_word_is_read_behind_the_kernels():
     assert got == 0x23 and K().gemm_tc_status(device) == 0
 
 
-@pytest.mark.parametrize("V", [131072, 131073])
+@pytest.mark.parametrize("V", [32768, 32769, 131072, 131073])
 @pytest.mark.parametrize("top_k,top_p", [(0, 1.0), (40, 1.0), (0, 0.9), (40, 0.95)])
 def test_sample_of_the_largest_rows_held_in_registers_and_the_smallest_not(V, top_k, top_p):
     g = torch.Generator().manual_seed(V)
