@@ -234,9 +234,10 @@ __device__ __forceinline__ int parts_before(const ScanArgs& p, int r) {
 // columns at once: parts of a long segment take 256 threads' worth of columns (1,153 tokens of 16 heads of 128 x 128 in 32
 // columns a block 93 us, in 64 86; a decay per row, 2,048 tokens of 16 heads of 64 x 128, 135 and in 128 columns 81), single
 // tokens the narrow blocks that give every SM one.
-template <int kDk, int kRT, int kCG, bool kRowDecay>
+template <int kDk, int kRT, int kCG, bool kParts, bool kRowDecay>
 struct ScanShared {
-    static constexpr int kGroups = kDk / kRT, kChunk = kRowDecay && kDk > 128 ? kScanChunk / 2 : kScanChunk, kCols = 4 * kCG;      // kChunk: tokens staged at a time
+    static constexpr int kGroups = kDk / kRT, kCols = 4 * kCG;
+    static constexpr int kChunk = kDk > 128 && (kRowDecay || !kParts) ? kScanChunk / 2 : kScanChunk;      // tokens staged at a time
     float2 q[kChunk][kDk], k[kChunk][kDk];                // twice each: the factors of a pair of columns
     float v[kChunk][kCols];
     float o[kChunk][kGroups][kCols];
@@ -253,7 +254,7 @@ linear_scan_kernel(const ScanArgs p) {
     // chunk of tokens.
     constexpr int kGroups = kDk / kRT;                    // row groups
     constexpr int kThreads = kGroups * kCG, kCols = 4 * kCG;
-    using Shared = ScanShared<kDk, kRT, kCG, kRowDecay>;
+    using Shared = ScanShared<kDk, kRT, kCG, kParts, kRowDecay>;
     constexpr int kChunk = Shared::kChunk;
     constexpr int kPerThread = kChunk * kDk / kThreads;   // q (and k) values a thread stages per chunk
     constexpr int kVPerThread = kChunk * kCols / kThreads;
@@ -332,12 +333,12 @@ linear_scan_kernel(const ScanArgs p) {
 #pragma unroll
         for (int u = 0; u < kPerThread; ++u) {
             const int e = threadIdx.x + u * kThreads;
-            if (e / kDk >= m) break;                      // (64 single tokens, 16 heads of 128 x 128: 31.1 -> 27.4 us)
+            if (!kParts && e / kDk >= m) break;           // (64 single tokens, 16 heads of 128 x 128: 31.1 -> 27.4 us)
             const float q = (p.act ? silu_f(qv[u]) : qv[u]) * p.q_scale, k = p.act ? silu_f(kv[u]) : kv[u];
             s_q[e / kDk][e % kDk] = make_float2(q, q);
             s_k[e / kDk][e % kDk] = make_float2(k, k);
             if (kRowDecay) {
-                const float a = e % kDk < p.dk ? row_decay(zv[u], p.inv_tau) : 1.f;
+                const float a = (e / kDk < m && e % kDk < p.dk) ? row_decay(zv[u], p.inv_tau) : 1.f;
                 s_av[e / kDk][e % kDk] = make_float2(a, a);
             }
         }
@@ -755,7 +756,7 @@ static int launch_apply(const ScanArgs& a, int R, cudaStream_t st) {
 
 template <int kDk, int kRT, int kCG, bool kParts, bool kRowDecay>
 static int launch_scan_as(const ScanArgs& a, int blocks, cudaStream_t st) {
-    constexpr int kSmem = static_cast<int>(sizeof(ScanShared<kDk, kRT, kCG, kRowDecay>));
+    constexpr int kSmem = static_cast<int>(sizeof(ScanShared<kDk, kRT, kCG, kParts, kRowDecay>));
     if constexpr (kSmem > 48 * 1024) {
         static SharedLimit limit;
         const cudaError_t ready = limit.allow(reinterpret_cast<const void*>(linear_scan_kernel<kDk, kRT, kCG, kParts, kRowDecay>), kSmem);
