@@ -1215,9 +1215,10 @@ static int launch_grouped_mma(const GroupedArgs& p, unsigned tiles, cudaStream_t
 // Where few rows of bfloat16 weights are multiplied on the CUDA cores: the time there goes with the rows of the fullest tile, on the tensor
 // cores with the tiles and the outputs (a tile's first row costs as much as eight), more with 32-bit inputs, which are cut into parts.
 static bool few_on_cuda_cores(const GroupedArgs& p, bool a_is_f32) {
-    // Heads: us on the CUDA cores / on the tensor cores, 32-bit inputs, 16 of 64 x 512: one row 3.7 / 5.5, four 4.8 / 5.6, six 5.9 / 5.5; 128
-    // of 128 x 512: one 9.7 / 28.2, eight 20.5 / 28.7, twelve 29.9 / 28.8. bfloat16 inputs: one 3.6 / 4.1 and 9.5 / 17.8, three 4.3 / 4.1 and 12.4 / 17.9.
-    if (!p.tile_group) return p.rows <= (p.groups >= 64 ? (a_is_f32 ? 10 : 5) : (a_is_f32 ? 5 : 2));
+    // Heads: us on the CUDA cores / on the tensor cores, 32-bit inputs, 128 of 128 x 512: one row 9.7 / 28.2, eight 20.5 / 28.7, twelve
+    // 29.9 / 28.8; bfloat16 inputs one 9.5 / 17.8, four 13.1 / 17.8. Of few heads a row or two are faster alone (16 of 64 x 512: 3.8 / 5.6), but
+    // not in a token's step (11.2 / 7.6, code and inputs cold).
+    if (!p.tile_group) return p.groups >= 64 && p.rows <= (a_is_f32 ? 10 : 5);
     // Experts: p.rows pairs of p.groups experts. Most have a tile of their own while they are fewer than the experts, or two an expert of
     // up to four or of very many. Weights from memory, 32-bit inputs: six pairs of eight experts, 2,048 outputs of 4,096 inputs 32.3 / 32.3,
     // 4,608 of 2,048 29.2 / 40.6; eight 33.8 / 41.5 on eight of them and 19.6 / 16.0 on two (in a token's step 32.5 / 31.4); 16 of 32, 768 of 2,048
